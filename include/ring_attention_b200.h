@@ -133,6 +133,8 @@ RA_API int ra_attention_step_segmented(const float* q, const float* k, const flo
 #define RA_STEP_CTA_PAIR 32u /* tcgen05 kernel, head_dim 128 / 256 with P in tensor memory: cluster
                               * pairs with M = 256 MMAs (cta_group::2), each block holding half of
                               * every K / V tile; the third, cross-checking form of the kernel */
+#define RA_STEP_KEY_SPLIT_SHIFT 8 /* bits 8..11: 0 = chosen by shape; n = 1..8: n blocks of a cluster
+                                   * share the key tiles of each query block (cross-checks) */
 
 /* The general step every other step entry point funnels into: any dtype, segmented
  * positions with a stride, optional document mask (visible only if

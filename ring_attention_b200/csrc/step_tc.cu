@@ -85,7 +85,7 @@ __device__ inline unsigned pack16(float lo, float hi) {
   }
 }
 
-template <int D, bool kPInTmem, bool kPair = false>
+template <int D, bool kPInTmem, bool kPair = false, bool kSplit = false>
 struct TcCfg {
   // head_dim 256: O alone takes 256 tensor-memory columns, so a block owns ONE 128-row query
   // tile (one MMA warp, one softmax group), and a 128-key K or V tile (64 KiB) travels through
@@ -121,7 +121,11 @@ struct TcCfg {
   static constexpr int kOffP = kOffKV + kStages * kItemBytes;
   static constexpr int kOffBar = kOffP + kTiles * kPBytes;
   static constexpr int kNumBars = 2 + 2 * kStages + 8;
-  static constexpr int kSmemBytes = kOffBar + kNumBars * 8 + 16 + 1024;  // + alignment slack
+  static constexpr int kOffMl = kOffBar + kNumBars * 8 + 16;  // (m, l) of every row: key-split form
+  static constexpr int kMlBytes = kSplit ? kTiles * kBM * 8 : 0;
+  static constexpr int kSmemBytes = kOffMl + kMlBytes + 1024;  // + alignment slack
+  static_assert(!kSplit || (kPInTmem && !kPair && kTiles * kBM * ((D + 4) * 4 + 8) <= kOffBar),
+                "the key-split merge stages O and the row factors over Q and the ring");
   // Three schedules of the two MMAs of a key tile.
   //  * early S (P in shared memory; head_dim 64 with P in tensor memory: S 256 + O 128 + P 128
   //    columns = 512): P does not overlap S, so the next S tile is issued as soon as the softmax
@@ -165,12 +169,14 @@ __device__ inline RingPos ring_pos(int which, int t, int sub) {
 
 
 // DR is the head_dim of the tensors in memory: D, or 32 on the 64-wide kernel (see launch_cfg).
-template <int D, bool kBf16, bool kPInTmem, int DR, bool kPair = false>
-__global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair>::kThreads), 1)
+// kSplit: the blocks of a cluster share the key tiles of ONE query block and merge their partial
+// states through distributed shared memory (see pick_key_split).
+template <int D, bool kBf16, bool kPInTmem, int DR, bool kPair = false, bool kSplit = false>
+__global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit>::kThreads), 1)
     step_tc_kernel(const __grid_constant__ CUtensorMap tmap_q,
                    const __grid_constant__ CUtensorMap tmap_k,
                    const __grid_constant__ CUtensorMap tmap_v, const TcArgs a) {
-  using C = TcCfg<D, kPInTmem, kPair>;
+  using C = TcCfg<D, kPInTmem, kPair, kSplit>;
   extern __shared__ unsigned char smem_raw[];
   // 128B-swizzled tiles need 1024-byte alignment
   unsigned char* smem = reinterpret_cast<unsigned char*>(
@@ -197,13 +203,14 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair>::kThreads), 1)
 
   // Rank inside the CTA pair; rank 0 (the leader) issues the pair's MMAs.
   unsigned cta_rank = 0;
-  if constexpr (kPair) cta_rank = cluster_ctarank();
+  if constexpr (kPair || kSplit) cta_rank = cluster_ctarank();
   const bool leader = cta_rank == 0;
+  constexpr bool kCluster = kPair || kSplit;
 
   // An earlier block gave up: leave at once (the vote makes the decision block-uniform). The
-  // two blocks of a pair could decide differently, so a pair starts in the aborted state instead
+  // blocks of a cluster could decide differently, so a cluster starts in the aborted state instead
   // (every wait then returns at once) and still meets at the cluster barriers below.
-  if constexpr (!kPair) {
+  if constexpr (!kCluster) {
     if (__syncthreads_or(*reinterpret_cast<volatile int*>(a.status) != 0)) return;
   }
 
@@ -228,7 +235,9 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair>::kThreads), 1)
     const int kv_lin = static_cast<int>(blockIdx.y) * a.kv_per_wave + j / group;  // batch * kvH + kv head
     bh = (kv_lin / a.kvH) * a.H + (j % group) * a.kvH + kv_lin % a.kvH;
   } else {
-    bh = kPair ? static_cast<int>(blockIdx.x >> 1) : static_cast<int>(blockIdx.x);
+    bh = kPair    ? static_cast<int>(blockIdx.x >> 1)
+         : kSplit ? static_cast<int>(blockIdx.x) / a.key_split
+                  : static_cast<int>(blockIdx.x);
     qb_lin = kPair ? 2 * static_cast<int>(gridDim.y) - 1 -
                          (2 * static_cast<int>(blockIdx.y) + static_cast<int>(blockIdx.x & 1))
                    : static_cast<int>(gridDim.y) - 1 - static_cast<int>(blockIdx.y);
@@ -249,11 +258,23 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair>::kThreads), 1)
   const int qmin = a.qmap.base[sq] + span_row0 * a.stride;
   const int qmax = a.qmap.base[sq] + (span_row0 + rows_in_span - 1) * a.stride;
 
+  // Query tiles of the block that take part. In the key-split form, whose calls have few query rows,
+  // a segment's last block of at most 128 rows leaves its second tile out (384 rows against 40384
+  // keys, H32/kvH8 D128: 735 -> 542 us before any split). The other forms run it on zeros: they
+  // have many blocks, and the check in their softmax loop costs the D64 pass 2 %.
+  const int live = (kSplit && C::kTiles == 2 && q_seg_len - row0 <= kBM) ? 1 : C::kTiles;
+
   // Tile list: segments in order, tiles [lo, hi) of each; identical in every role.
   int n_tiles = 0;
   for (int sk = 0; sk < a.kmap.n_seg; ++sk) {
     const TileRange r = tile_range<kBN>(a.kmap, sk, a.stride, causal, a.doc_len, qmin, qmax);
     n_tiles += r.hi - r.lo;
+  }
+  [[maybe_unused]] int share_beg = 0, share_end = 0;
+  if constexpr (kSplit) {  // this block's contiguous share, sizes at most one tile apart
+    share_beg = static_cast<int>(static_cast<long long>(n_tiles) * cta_rank / a.key_split);
+    share_end = static_cast<int>(static_cast<long long>(n_tiles) * (cta_rank + 1) / a.key_split);
+    n_tiles = share_end - share_beg;
   }
 
   if (tid == 0) {
@@ -264,7 +285,7 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair>::kThreads), 1)
     mbar_init(bar_q_full + 8, peers);
     for (int s = 0; s < C::kStages; ++s) {
       mbar_init(bar_kv_full + 8 * s, peers);
-      mbar_init(bar_kv_empty + 8 * s, C::kTiles);  // one commit from each issuing warp
+      mbar_init(bar_kv_empty + 8 * s, live);  // one commit from each issuing warp
     }
     for (int w = 0; w < 2; ++w) {
       mbar_init(bar_s_full + 8 * w, 1);
@@ -273,7 +294,7 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair>::kThreads), 1)
       mbar_init(bar_s_free + 8 * w, kPair ? 4 * peers : kBM);
     }
 
-    *abort_flag = (kPair && *reinterpret_cast<volatile int*>(a.status) != 0) ? 1 : 0;
+    *abort_flag = (kCluster && *reinterpret_cast<volatile int*>(a.status) != 0) ? 1 : 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -305,7 +326,7 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair>::kThreads), 1)
     // ------------------------------------------------------------ TMA producer ----
     if (lane == 0 && n_tiles > 0) {
       const int q_row = sq * q_seg_len + row0;
-      for (int w = 0; w < C::kTiles; ++w) {
+      for (int w = 0; w < live; ++w) {
         mbar_expect_tx(bar_q_full + 8 * w, C::kTileBytes);
         for (int bx = 0; bx < C::kBoxes; ++bx)
           tma_load_3d(s_q + w * C::kTileBytes + bx * (kBM * 128), &tmap_q, bar_q_full + 8 * w,
@@ -354,8 +375,10 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair>::kThreads), 1)
       // tile t - 1.
       int v_row = 0, v_head = 0;
       bool v_pending = false;
+      [[maybe_unused]] TileShare share{share_beg, share_end, 0};
       for (int sk = 0; sk < a.kmap.n_seg && ok; ++sk) {
-        const TileRange r = tile_range<kBN>(a.kmap, sk, a.stride, causal, a.doc_len, qmin, qmax);
+        TileRange r = tile_range<kBN>(a.kmap, sk, a.stride, causal, a.doc_len, qmin, qmax);
+        if constexpr (kSplit) r = share.clip(r);
         for (int t = r.lo; t < r.hi && ok; ++t, ++jt) {
           const int k_row = a.kseg_row[sk] + t * kBN;
           const int k_head = a.kseg_head[sk] + kv_bh;
@@ -405,7 +428,7 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair>::kThreads), 1)
         }
       }
     }
-  } else if (warp == 1 || (warp == 2 && C::kTiles == 2)) {
+  } else if (warp == 1 || (warp == 2 && live == 2)) {
     // ------------------------------------------------------------- MMA issuers ----
     // One issuing warp per query tile (warp 1: tile 0, warp 2: tile 1). The two tiles are
     // independent instruction streams, so a tile that is still in its exponentials never holds
@@ -560,6 +583,9 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair>::kThreads), 1)
       }
     }
   }
+  if constexpr (kSplit) {  // the three meetings of the merge below
+    for (int i = 0; i < 3; ++i) cluster_sync_threads();
+  }
   } else {
     if constexpr (C::kTiles == 2) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(RAB_REGS_HI));
     // ----------------------------------------------------------------- softmax ----
@@ -581,8 +607,11 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair>::kThreads), 1)
     bool ok = true;
 
     int j = 0;
-    for (int sk = 0; sk < a.kmap.n_seg && ok; ++sk) {
-      const TileRange tr = tile_range<kBN>(a.kmap, sk, a.stride, causal, a.doc_len, qmin, qmax);
+    const int n_seg = (!kSplit || w < live) ? a.kmap.n_seg : 0;
+    [[maybe_unused]] TileShare share{share_beg, share_end, 0};
+    for (int sk = 0; sk < n_seg && ok; ++sk) {
+      TileRange tr = tile_range<kBN>(a.kmap, sk, a.stride, causal, a.doc_len, qmin, qmax);
+      if constexpr (kSplit) tr = share.clip(tr);
       // Keys of this segment the row can see are the local indices [rel_lo, rel_hi): causal
       // and document limits are affine in the key index, so they are worked out once per
       // segment (64-bit divisions) and the per-tile work is two 32-bit clamps.
@@ -785,11 +814,17 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair>::kThreads), 1)
     }
 
     // ---------------------------------------------------------------- epilogue ----
-    if (ok && n_tiles > 0)
+    if (ok && n_tiles > 0 && (!kSplit || w < live))
       ok = mbar_wait(bar_o_done + 8 * w, (C::kEarlyS || C::kDoubleS) ? ((n_tiles - 1) & 1) : 0,
                      abort_flag, a.status, 8, n_tiles, a.wait_ns);
     ok = __all_sync(0xffffffffu, ok);
-    if (ok) {
+    if constexpr (kSplit) {
+      tc_fence_after();
+      merge_key_split<C, DR>(a, smem, s_base, t_o, w, row, row_valid,
+                             static_cast<size_t>(bh) * a.Sq + static_cast<size_t>(sq) * q_seg_len + row0,
+                             ok && w < live && n_tiles > 0, m_ref, l_run, 1.f, cta_rank, fresh,
+                             finalize);
+    } else if (ok) {
       tc_fence_after();
       const size_t grow = (static_cast<size_t>(bh) * a.Sq + static_cast<size_t>(sq) * q_seg_len +
                            (row_valid ? r_in_seg : 0));
@@ -868,9 +903,9 @@ std::atomic<unsigned long long> g_wait_ns{kWaitLimitNs};
 std::atomic<int> g_stall_after{-1};
 std::atomic<int> g_block_order{-1};  // -1: by shape, 0: heads fastest, k > 0: waves of k KV heads
 
-template <int D, bool kBf16, bool kPInTmem, int DR, bool kPair = false>
-int launch_cfg(const StepArgs& a, cudaStream_t stream) {
-  using C = TcCfg<D, kPInTmem, kPair>;
+template <int D, bool kBf16, bool kPInTmem, int DR, bool kPair = false, bool kSplit = false>
+int launch_cfg(const StepArgs& a, cudaStream_t stream, int key_split = 1) {
+  using C = TcCfg<D, kPInTmem, kPair, kSplit>;
   CUtensorMap mq, mk, mv;
   const int dtype = kBf16 ? RA_BF16 : RA_F16;
   int rc = make_map(&mq, dtype, a.q, a.D, a.Sq, static_cast<long long>(a.B) * a.H,
@@ -939,12 +974,14 @@ int launch_cfg(const StepArgs& a, cudaStream_t stream) {
   }
   const int order = g_block_order.load(std::memory_order_relaxed);  // test hook
   if (order == 0 || (order > 0 && kv_heads_total % order == 0)) kv_per_wave = order;
+  if (kSplit) kv_per_wave = 0;
   t.kv_per_wave = kv_per_wave;
+  t.key_split = key_split;
   const long long bh_total = static_cast<long long>(a.B) * a.H;
   const long long per_x = kv_per_wave > 0 ? static_cast<long long>(a.H / a.kvH) * kv_per_wave : 0;
   RAB_REQUIRE(kv_per_wave > 0 ? n_qblocks * per_x < (1ll << 31) : n_qblocks <= 65535, RA_ERR_INVALID,
               "attention step: grid too large (%lld query blocks, %lld heads)", n_qblocks, bh_total);
-  auto kern = step_tc_kernel<D, kBf16, kPInTmem, DR, kPair>;
+  auto kern = step_tc_kernel<D, kBf16, kPInTmem, DR, kPair, kSplit>;
   // once per device and instantiation: the attribute call costs microseconds that a pass of a
   // few short launches would otherwise pay every time
   static std::atomic<unsigned long long> smem_set{0};
@@ -957,16 +994,17 @@ int launch_cfg(const StepArgs& a, cudaStream_t stream) {
   dim3 grid(static_cast<unsigned>(a.B) * a.H, static_cast<unsigned>(n_qblocks));
   if (kv_per_wave > 0)
     grid = dim3(static_cast<unsigned>(n_qblocks * per_x), static_cast<unsigned>(kv_heads_total / kv_per_wave));
-  if constexpr (kPair) {
-    // the two blocks of a pair are neighbours in x; they take the query blocks 2i and 2i + 1
+  if constexpr (kPair || kSplit) {
+    // the blocks of a cluster are neighbours in x; those of a pair take the query blocks 2i and
+    // 2i + 1, those of a key split all take the same one
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = kv_per_wave > 0 ? grid : dim3(2 * grid.x, grid.y / 2);
+    cfg.gridDim = kSplit ? dim3(grid.x * key_split, grid.y) : kv_per_wave > 0 ? grid : dim3(2 * grid.x, grid.y / 2);
     cfg.blockDim = dim3(C::kThreads);
     cfg.dynamicSmemBytes = C::kSmemBytes;
     cfg.stream = stream;
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = 2;
+    attr.val.clusterDim.x = kSplit ? key_split : 2;
     attr.val.clusterDim.y = 1;
     attr.val.clusterDim.z = 1;
     cfg.attrs = &attr;
@@ -979,14 +1017,29 @@ int launch_cfg(const StepArgs& a, cudaStream_t stream) {
   return RA_OK;
 }
 
+template <int D, int DR>
+int launch_split(int dtype, const StepArgs& a, cudaStream_t stream, int n) {
+  return dtype == RA_BF16 ? launch_cfg<D, true, true, DR, false, true>(a, stream, n)
+                          : launch_cfg<D, false, true, DR, false, true>(a, stream, n);
+}
+
 template <int D>
 int launch_d(int dtype, const StepArgs& a, cudaStream_t stream) {
   // P stays in tensor memory unless the caller asks for the shared-memory path (kept as a
   // cross-check of the first one; both are tested)
   const bool p_in_tmem = (a.flags & RA_STEP_P_IN_SMEM) == 0;
+  // A key split (not under a forced block order, which is about whole blocks). Head_dim 128 and 256
+  // stay whole up to 16 key tiles, where they equal their cluster-pair form bit for bit; a
+  // merge stages 4 bytes per row and column, so it costs more tiles the wider the head.
+  const int split = p_in_tmem && (a.flags & RA_STEP_CTA_PAIR) == 0 &&
+                            g_block_order.load(std::memory_order_relaxed) < 0
+                        ? pick_key_split<kBN>(a, TcCfg<D, true>::kTiles * kBM, D == 64 ? 1.5 : 2.5,
+                                              D == 64 ? 0 : 16)
+                        : 1;
   // the 64-wide kernel also takes head_dim 32 (DR = 32)
   if constexpr (D == 64) {
     if (a.D == 32) {
+      if (split > 1) return launch_split<64, 32>(dtype, a, stream, split);
       if (dtype == RA_BF16)
         return p_in_tmem ? launch_cfg<64, true, true, 32>(a, stream)
                          : launch_cfg<64, true, false, 32>(a, stream);
@@ -994,6 +1047,7 @@ int launch_d(int dtype, const StepArgs& a, cudaStream_t stream) {
                        : launch_cfg<64, false, false, 32>(a, stream);
     }
   }
+  if (split > 1) return launch_split<D, D>(dtype, a, stream, split);
   if constexpr (D == 128 || D == 256) {
     // Cluster pairs with M = 256 MMAs (cta_group::2), on request, wherever a segment has at least
     // two query blocks to pair up. Measured on B200 the pairs are 5-15 % slower than independent

@@ -167,6 +167,28 @@ __device__ inline void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::
                    : "memory");
 }
+// The same for threads of warps that may be diverged: every thread of the cluster arrives.
+__device__ inline void cluster_sync_threads() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+// Shared memory of CTA `rank` of the cluster at this CTA's address `saddr`.
+__device__ inline unsigned cluster_addr(unsigned saddr, unsigned rank) {
+  unsigned r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
+  return r;
+}
+__device__ inline float2 ld_cluster_f2(unsigned addr) {
+  float2 v;
+  asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr));
+  return v;
+}
+__device__ inline float4 ld_cluster_f4(unsigned addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "r"(addr));
+  return v;
+}
 // Arrive on the barrier at the same shared-memory offset in CTA `rank` of the cluster.
 __device__ inline void mbar_arrive_cluster(unsigned bar, unsigned rank) {
   asm volatile(
@@ -323,7 +345,6 @@ __device__ inline float ex2(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-
 // Shared-memory matrix descriptors for 128B-swizzled tiles (8-row groups 1024 B apart).
 // K-major operand (rows = M or N index, 64 contiguous 16-bit elements of the contraction
 // dimension per 128-byte row); the leading byte offset is unused for swizzled K-major.
@@ -367,7 +388,7 @@ struct TileRange {
 // Visible key-tile range of key segment `sk` for a query block whose rows span positions
 // [qmin, qmax] (both ends are positions of real rows).
 template <int kTileKeys>
-__device__ inline TileRange tile_range(const PosMap& kmap, int sk, int stride, bool causal,
+__host__ __device__ inline TileRange tile_range(const PosMap& kmap, int sk, int stride, bool causal,
                                        long long doc_len, int qmin, int qmax) {
   const int L = kmap.seg_len;
   const long long kb = kmap.base[sk];
@@ -388,6 +409,18 @@ __device__ inline TileRange tile_range(const PosMap& kmap, int sk, int stride, b
   return {static_cast<int>(j_lo / kTileKeys), static_cast<int>(j_hi / kTileKeys) + 1};
 }
 
+// A block's share of its query block's tile list when the list is cut across the blocks of a
+// cluster: list entries [beg, end). clip() is called once per key segment, in order.
+struct TileShare {
+  int beg, end, seen;
+  __device__ TileRange clip(TileRange r) {
+    const int n = r.hi - r.lo;
+    const int lo = max(0, beg - seen), hi = min(n, end - seen);
+    seen += n;
+    return {r.lo + lo, r.lo + max(lo, hi)};
+  }
+};
+
 struct TcArgs {
   float* out;
   float* m;
@@ -404,7 +437,99 @@ struct TcArgs {
   unsigned long long wait_ns;  // limit of every device-side wait
   int stall_after;             // test hook: the producer stops after this many ring items (< 0: off)
   int kv_per_wave;             // block order: waves of this many KV heads (0: heads fastest)
+  int key_split;               // blocks of a cluster that share one query block's key tiles
 };
+
+// End of a block of the key-split form, run by the softmax threads (one per row; the other threads
+// of the cluster only join the three barriers): the partial (O, m, l) of the cluster's blocks are
+// merged and folded into the state as one step. Every block scales its O to the common reference
+// point (o_unit: what one unit
+// of the accumulator is worth) and stages it in its own shared memory, then each block sums its slice of the elements
+// over all blocks and writes it. 128 KB of staged O per block at head_dim 128 cross the cluster
+// once (about 2 us); no workspace and no second launch.
+template <class C, int DR>
+__device__ inline void merge_key_split(const TcArgs& a, unsigned char* smem, unsigned s_base,
+                                       unsigned t_o, int w, int row, bool row_valid, size_t grow0, bool worked,
+                                       float m_ref, float l_run, float o_unit, unsigned rank, bool fresh,
+                                       bool finalize) {
+  constexpr int kRows = C::kTiles * kBM;
+  constexpr int kStride = DR + 4;  // floats: rows 16 bytes apart modulo 128, so float4 stores do not collide
+  constexpr int kOffFac = kRows * kStride * 4;
+  float* const o_stage = reinterpret_cast<float*>(smem);
+  float2* const fac = reinterpret_cast<float2*>(smem + kOffFac);
+  float2* const ml = reinterpret_cast<float2*>(smem + C::kOffMl);
+  const int rb = w * kBM + row;
+  const int n = a.key_split;
+  const bool have = worked && row_valid && m_ref > -INFINITY;
+  ml[rb] = have ? make_float2(m_ref, l_run) : make_float2(-INFINITY, 0.f);
+  cluster_sync_threads();  // all (m, l) are there, no block reads its Q or ring any more
+  const unsigned ml_addr = s_base + C::kOffMl + rb * 8;
+  float m_all = -INFINITY, l_all = 0.f;
+  for (int r = 0; r < n; ++r) m_all = fmaxf(m_all, ld_cluster_f2(cluster_addr(ml_addr, r)).x);
+  for (int r = 0; r < n; ++r) {
+    const float2 p = ld_cluster_f2(cluster_addr(ml_addr, r));
+    if (p.x > -INFINITY) l_all += p.y * ex2(p.x - m_all);
+  }
+  const size_t grow = grow0 + (row_valid ? rb : 0);
+  const bool any = row_valid && m_all > -INFINITY;
+  float m_old = -INFINITY, l_old = 0.f;
+  if (!fresh && row_valid) {
+    m_old = a.m[grow];
+    l_old = a.l[grow];
+  }
+  const float m_new = any ? m_all * kLn2 : -INFINITY;
+  const float m_fin = fmaxf(m_old, m_new);
+  const float ca = (m_old == -INFINITY) ? 0.f : expf(m_old - m_fin);
+  const float cb = any ? expf(m_new - m_fin) : 0.f;
+  const float l_fin = ca * l_old + cb * l_all;
+  const float inv = finalize ? (l_fin > 0.f ? 1.f / l_fin : 0.f) : 1.f;
+  const bool touch = row_valid && (any || fresh || finalize);
+  fac[rb] = touch ? make_float2(ca * inv, cb * inv) : make_float2(-1.f, 0.f);  // factors are never negative
+  const float scale = have ? ex2(m_ref - m_all) * o_unit : 0.f;
+#pragma unroll 1
+  for (int c = 0; c < DR / 32; ++c) {
+    float o[32];
+    if (worked) {  // warp-uniform: the tensor-memory load is warp-collective
+      tmem_ld32(t_o + c * 32, o);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) o[i] = 0.f;
+    }
+    float4* dst = reinterpret_cast<float4*>(o_stage + rb * kStride + c * 32);
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      dst[i] = have ? make_float4(o[4 * i] * scale, o[4 * i + 1] * scale, o[4 * i + 2] * scale,
+                                  o[4 * i + 3] * scale)
+                    : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  cluster_sync_threads();  // every block's O is staged, every old (m, l) has been read
+  constexpr int kVec = DR / 4;
+  for (int idx = static_cast<int>(rank) * kRows + rb; idx < kRows * kVec; idx += n * kRows) {
+    const int r_out = idx / kVec, col = (idx % kVec) * 4;
+    const float2 f = fac[r_out];
+    if (f.x == -1.f) continue;
+    const unsigned addr = s_base + (r_out * kStride + col) * 4;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+    for (int r = 0; r < n; ++r) {
+      const float4 o = ld_cluster_f4(cluster_addr(addr, r));
+      acc.x += o.x;
+      acc.y += o.y;
+      acc.z += o.z;
+      acc.w += o.w;
+    }
+    float4* dst = reinterpret_cast<float4*>(a.out + (grow0 + r_out) * DR + col);
+    float4 old = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (!fresh) old = *dst;
+    *dst = make_float4(f.x * old.x + f.y * acc.x, f.x * old.y + f.y * acc.y, f.x * old.z + f.y * acc.z,
+                       f.x * old.w + f.y * acc.w);
+  }
+  if (rank == 0 && touch) {
+    a.m[grow] = m_fin;
+    a.l[grow] = l_fin;
+  }
+  cluster_sync_threads();  // nobody leaves while its shared memory is still read
+}
 
 // ---- host side ----------------------------------------------------------------------
 
@@ -453,6 +578,70 @@ inline int make_map(CUtensorMap* map, int dtype, const void* base, int D, long l
   RAB_REQUIRE(r == CUDA_SUCCESS, RA_ERR_CUDA, "cuTensorMapEncodeTiled failed with code %d",
               static_cast<int>(r));
   return RA_OK;
+}
+
+// Key split: how many blocks of a cluster share the key tiles of one query block (1: no split).
+// A block walks its key tiles one after the other, so a call with fewer query blocks than SMs
+// leaves SMs idle however many keys there are. Cutting the tile list in n shortens the walk to
+// 1/n and costs every block its own prologue and the merge (kFixed and merge_tiles, in tiles of
+// work; a query block without a visible key costs kEmpty). The estimate is the walk of the longest
+// block while the blocks with work fit the SMs that clusters of that size can occupy (a cluster
+// lives inside one GPC: cudaOccupancyMaxActiveClusters gives 148, 148, 135, 132, 130, 132, 120 for
+// n = 1, 2, 3, 4, 5, 6, 8), else the total work over them plus half a block for the last wave.
+// `longest_unsplit`: calls whose longest walk is at most this stay whole.
+// Measured, us per call at n = 1 / 2 / 4 / 8 (fp16, causal): 384 rows on 40384 keys H32/kvH8 D128
+// 542 / 296 / 303 / 410 (735 before the second tile of the last block was left out); 64 rows on
+// 65536 keys H8 D128 1077 / 540 / 277 / 146; 1024 x 1024 H8 D64 23 / 19 / 17 / 38; 2048 x 2048 H16
+// D64 (128 blocks) 36 / 38 / 59 / 122.
+template <int kTileKeys>
+inline int pick_key_split(const StepArgs& a, int q_block_rows, double merge_tiles, int longest_unsplit) {
+  const int forced = static_cast<int>((a.flags >> RA_STEP_KEY_SPLIT_SHIFT) & 15u);
+  if (forced) return forced > 8 ? 8 : forced;
+  constexpr int kSms = 148;
+  constexpr double kFixed = 3, kEmpty = 0.7;
+  const int per_seg = (a.qmap.seg_len + q_block_rows - 1) / q_block_rows;
+  const long long heads = static_cast<long long>(a.B) * a.H;
+  if (heads * per_seg * a.qmap.n_seg >= kSms) return 1;
+  const bool causal = (a.flags & RA_STEP_CAUSAL) != 0;
+  long long total = 0;
+  int longest = 0, busy = 0, idle = 0;  // per head
+  for (int sq = 0; sq < a.qmap.n_seg; ++sq)
+    for (int tq = 0; tq < per_seg; ++tq) {
+      const int row0 = tq * q_block_rows;
+      const int rows = a.qmap.seg_len - row0 < q_block_rows ? a.qmap.seg_len - row0 : q_block_rows;
+      const int qmin = a.qmap.base[sq] + row0 * a.stride;
+      int tiles = 0;
+      for (int sk = 0; sk < a.kmap.n_seg; ++sk) {
+        const TileRange r = tile_range<kTileKeys>(a.kmap, sk, a.stride, causal, a.doc_len, qmin,
+                                                  qmin + (rows - 1) * a.stride);
+        tiles += r.hi - r.lo;
+      }
+      total += tiles;
+      longest = tiles > longest ? tiles : longest;
+      tiles > 0 ? ++busy : ++idle;
+    }
+  if (busy == 0 || longest <= longest_unsplit) return 1;
+  const double mean = static_cast<double>(total) / busy;
+  constexpr int kSizes[7] = {1, 2, 3, 4, 5, 6, 8}, kSlots[7] = {kSms, kSms, 135, 132, 130, 132, 120};
+  int best = 1;
+  double best_t = 0;
+  for (int i = 0; i < 7; ++i) {
+    const int n = kSizes[i];
+    if (n > 1 && longest < 2 * n) break;  // at least two tiles to walk
+    const double fixed = kFixed + (n > 1 ? merge_tiles : 0);
+    const double empties = static_cast<double>(heads * idle) * n * kEmpty / kSlots[i];
+    double t = longest / static_cast<double>(n) + fixed + empties;
+    const double n_blocks = static_cast<double>(heads * busy) * n;
+    if (n_blocks > kSlots[i]) {
+      const double spread = (n_blocks / kSlots[i] + 0.5) * (mean / n + fixed) + empties;
+      t = t > spread ? t : spread;
+    }
+    if (i == 0 || t < best_t) {
+      best = n;
+      best_t = t;
+    }
+  }
+  return best;
 }
 
 // Limits set through the test hooks (step_tc.cu owns them).

@@ -1,0 +1,73 @@
+"""GPU parity of the forms that a call's shape selects: the key-split form of the step kernels (the
+blocks of a cluster share a query block's keys).
+
+Tolerances are those of the other step and decode tests: 1e-5 for fp32 and 1e-3 / 8e-3 for fp16 /
+bf16 P, absolute and relative, against the oracle on the same rounded inputs."""
+import ctypes as C
+
+import numpy as np
+import pytest
+import torch
+
+import oracle
+from ring_attention_b200 import api
+from ring_attention_b200._lib import RA_BF16, RA_F16, RA_F32, SegMap, lib
+from util import assert_close, normal_inputs, round_to
+
+pytestmark = pytest.mark.gpu
+
+TOL = {torch.float32: 1e-5, torch.float16: 1e-3, torch.bfloat16: 8e-3}
+CODE = {torch.float32: RA_F32, torch.float16: RA_F16, torch.bfloat16: RA_BF16}
+CAUSAL, FRESH, FINALIZE = 1, 2, 4
+
+
+def dev(x, dtype=torch.float32):
+    return torch.from_numpy(np.ascontiguousarray(x)).to("cuda").to(dtype).contiguous()
+
+
+def step(q, k, v, state, shape, qmap, kmap, flags, split=0, doc_len=0):
+    out, m, l = state
+    api.check(lib().ra_attention_step_ex(
+        CODE[q.dtype], api._ptr(q), api._ptr(k), api._ptr(v), api._ptr(out), api._ptr(m), api._ptr(l),
+        C.byref(shape.c()), C.byref(qmap), C.byref(kmap), 1, flags | split << 8, doc_len, 0, api._stream()))
+
+
+def poisoned(B, H, Sq, D):
+    return [torch.full(s, float("nan"), device="cuda") for s in ((B, H, Sq, D), (B, H, Sq), (B, H, Sq))]
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("D", [32, 64, 128, 256])
+@pytest.mark.parametrize("split", [2, 3, 8])
+def test_key_split_in_two_steps_matches_the_oracle(dtype, D, split):
+    # 300 query rows (a whole block and one of a single short tile), two key chunks of which the
+    # second has fewer tiles than blocks; document and causal limits leave some shares empty
+    if dtype == torch.float32 and D == 256:
+        pytest.skip("head_dim 256 in fp32 runs the SIMT kernel")
+    B, H, kvH, Sq, Sk, doc = 1, 4, 2, 300, 1333, 900
+    q, k, v = (round_to(x, dtype) for x in normal_inputs(5, B, H, kvH, Sq, Sk, D))
+    cut = 1100
+    qmap = SegMap.make([Sk - Sq], Sq)
+    state = poisoned(B, H, Sq, D)
+    dq = dev(q, dtype)
+    for lo, hi, flags in ((0, cut, FRESH), (cut, Sk, FINALIZE)):
+        step(dq, dev(k[:, :, lo:hi], dtype), dev(v[:, :, lo:hi], dtype), state,
+             api.AttentionShape(B, H, Sq, hi - lo, D, kvH), qmap, SegMap.make([lo], hi - lo), flags | CAUSAL, split, doc)
+    lse = api.attention_lse(state[1], state[2]).cpu().numpy()
+    assert api.device_status()[0] == 0
+    w_out, w_m, w_l = oracle.attention_init((B, H, Sq, D), (B, H, Sq))
+    oracle.attention_step(q, k, v, w_out, w_m, w_l, [Sk - Sq], [0], causal=True, kv_heads=kvH, doc_len=doc)
+    oracle.attention_finalize(w_out, w_l)
+    assert_close(state[0].cpu().numpy(), w_out, TOL[dtype], TOL[dtype], "out")
+    assert_close(lse, w_m + np.log(w_l), TOL[dtype], TOL[dtype], "lse")
+
+
+def test_key_split_leaves_rows_without_a_visible_key_alone():
+    B, H, Sq, Sk, D = 1, 2, 200, 512, 64
+    q, k, v = normal_inputs(6, B, H, H, Sq, Sk, D)
+    state = [torch.full((B, H, Sq, D), 3.0, device="cuda"), torch.full((B, H, Sq), 0.5, device="cuda"),
+             torch.full((B, H, Sq), 2.0, device="cuda")]
+    for dtype in (torch.float16, torch.float32):
+        step(dev(q, dtype), dev(k, dtype), dev(v, dtype), state, api.AttentionShape(B, H, Sq, Sk, D),
+             SegMap.make([0], Sq), SegMap.make([1000], Sk), CAUSAL, 4)
+    assert (state[0] == 3.0).all() and (state[1] == 0.5).all() and (state[2] == 2.0).all()
