@@ -75,8 +75,8 @@ int step_ex(int dtype, const void* q, const void* k, const void* v, float* out, 
   }
   if (!(flags & RA_STEP_FORCE_SIMT) && step_tc_supported(dtype, a))
     return launch_step_tc(dtype, a, stream);
-  if (!(flags & RA_STEP_FORCE_SIMT) && step_tf32_supported(dtype, a))
-    return launch_step_tf32(a, stream);
+  if (!(flags & RA_STEP_FORCE_SIMT) && step_f32_supported(dtype, a))
+    return launch_step_f32(a, stream);
   return launch_step_simt(dtype, a, stream);
 }
 

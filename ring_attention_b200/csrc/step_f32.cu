@@ -1,0 +1,821 @@
+// Blackwell (sm_100a) ring step for fp32 Q/K/V on the tensor cores: the same FlashAttention-style
+// forward as step_tc.cu (TMA, tcgen05.mma, tensor memory) with every operand split into two fp16
+// terms of a scaled value, x * 2^e ~ hi + lo (hi = fp16(x * 2^e), lo = fp16(x * 2^e - hi)), and
+// every product taken as hi*hi + lo*hi + hi*lo with fp32 accumulation. Replaces the reference's
+// fp32 step (src/attention_step.cu:114-282) for head_dim 32, 64 and 128.
+//
+// Precision. hi + lo carry 22 bits like a pair of TF32 terms, and kind::f16 runs at twice the rate
+// of kind::tf32 with half the operand bytes and half the accumulations per product. What fp16
+// lacks is range, so values are scaled by powers of two first (exact): Q by row, K by key, V by
+// key tile, each so that the largest magnitude sits in [2^14, 2^15). An element keeps all 22 bits
+// down to 2^-17 of that largest one and an absolute 2^-40 of it below. P is fp32 until it is split
+// the same way (unit 2^kPBits), the row sums stay fp32. The dropped lo*lo and the rounding of lo
+// are about 2^-22 of a product; what shows in the output is the tensor core's fp32 accumulation
+// over the key tiles, as in any such kernel. RA_STEP_FORCE_SIMT selects the plain-fp32 kernel;
+// head_dim 256 keeps it (its split Q tiles and key ring exceed shared memory).
+//
+// Work decomposition: grid = (batch * heads, 256-row query blocks), heavy blocks first; a block
+// owns two 128-row query tiles and walks the visible 64-key tiles of every key segment. Calls with
+// few query blocks cut the tile list over the blocks of a cluster (pick_key_split).
+//
+// Roles inside a block (640 threads)
+//   warp 0        TMA producer: K_0, V_0, K_1, ... as 128B-swizzled fp32 tiles into a shared-memory
+//                 ring (no multicast).
+//   warps 1, 2    MMA issuers, one per query tile (converged warp, one elected lane).
+//   warps 4-11    softmax, one thread per row, a warpgroup per query tile. At the start each thread
+//                 reads, scales and splits its row of Q into tensor memory, where the A operand
+//                 costs the scores no shared-memory reads, which bound them otherwise (head_dim
+//                 128: the hi term; lo goes as swizzled tiles into shared memory).
+//   warps 12-19   splitters: a landed raw tile is read into registers, scaled, split and written
+//                 back over itself, the hi tiles over the even 32-column boxes and the lo tiles over
+//                 the odd ones, in the layout TMA would give 16-bit data.
+//   Head_dim 32 / 64: S and P have buffers of their own, so the scores of tile t+1 are computed
+//   while the softmax of tile t runs. Head_dim 128: P is written over S and the two query tiles take
+//   turns on the tensor core.
+//
+// Tensor memory, 256 columns per query tile: S [0,64) P hi [64,96) P lo [96,128) O [128,192) Q hi
+// [192,224) Q lo [224,256); head_dim 128: S and P [0,64) O [64,192) Q hi [192,256).
+// Every wait on an mbarrier is bounded (see tc_common.cuh); a wait that runs out reports into
+// the device status word and the block unwinds.
+#include <atomic>
+
+#include "tc_common.cuh"
+
+namespace rab {
+
+using namespace tcgen;
+
+namespace {
+
+constexpr int kBNf = 64;          // keys per tile
+constexpr int kThreadsF = 640;
+constexpr int kSplitThreads = 256;
+constexpr int kTopExp = 14;       // scaled values have their largest magnitude in [2^14, 2^15)
+constexpr int kPBits = 8;         // P at the row's reference point is 2^8
+constexpr int kVSlack = 2;        // a V tile may exceed the accumulator's unit by 2^2
+constexpr float kPSumLimit = 65000.f;  // of eight P: none of them then leaves fp16's range
+
+template <int DR, bool kSplit>
+struct F32Cfg {
+  static constexpr int kTiles = 2;
+  static constexpr int D = DR < 64 ? 64 : DR;           // columns of a split tile row
+  // Where Q's terms go. Head_dim 32 / 64: both into tensor memory, beside S, P and O. Head_dim 128:
+  // hi into tensor memory, lo as swizzled tiles into shared memory; P is then written over S, and
+  // the 64 KB that Q's hi tiles do not take make the ring 5 slots instead of 3. (With Q all in
+  // shared memory and P beside S, B1 H4 S16384 causal took 1032 us: every K tile waited for the
+  // slot that P.V of the tile before last frees.)
+  static constexpr bool kQLoInTmem = D == 64;
+  static constexpr bool kAlias = D == 128;
+  static constexpr int kBoxes = DR / 32;                // raw boxes: 32 fp32 = 128 bytes of a row
+  static constexpr int kGroups = D / 64;                // 64-column groups of a split tile
+  static constexpr int kBoxBytes = kBNf * 128;
+  static constexpr int kSlotBytes = 2 * kGroups * kBoxBytes;  // raw tile = hi + lo tiles
+  static constexpr int kRawBytes = kBoxes * kBoxBytes;
+  static constexpr int kStages = D == 128 ? (kSplit ? 4 : 5) : 10;
+  // per-key factors of K are read by the softmax of their tile while later tiles are split; the
+  // ring holds the producer back far enough for this many copies
+  static constexpr int kGDepth = D == 128 ? 4 : 8;
+  static_assert(kGDepth > kStages / 2, "a key factor could be overwritten before it is read");
+  static constexpr int kQBytes = kQLoInTmem ? 0 : kBM * D * 2;  // lo of one query tile
+  static constexpr int kOffQ = 0;
+  static constexpr int kOffKV = kTiles * kQBytes;
+  static constexpr int kOffBar = kOffKV + kStages * kSlotBytes;
+  static constexpr int kNumBars = 2 + 3 * kStages + 8 + 1;
+  static constexpr int kOffSlot = kOffBar + kNumBars * 8;      // tensor-memory address, abort flag
+  static constexpr int kOffRed = kOffSlot + 8;                 // [2][8] tile maxima of V by warp
+  static constexpr int kOffVExp = kOffRed + 64;                // [16] exponents of V tiles
+  static constexpr int kOffG = (kOffVExp + 64 + 15) & ~15;     // [kGDepth][kBNf] factors of K
+  static constexpr int kOffMl = kOffG + kGDepth * kBNf * 4;
+  static constexpr int kMlBytes = kSplit ? kTiles * kBM * 8 : 0;
+  static constexpr int kSmemBytes = kOffMl + kMlBytes;
+  static constexpr int kColS = 0, kColP = kAlias ? 0 : 64, kColO = kAlias ? 64 : 128, kColQ = 192;
+  static_assert(kSmemBytes <= 232448, "shared memory budget");
+  static_assert(kTiles * kBM * ((DR + 4) * 4 + 8) <= kOffBar, "staging of the key-split merge");
+};
+
+// The power-of-two exponent that brings a largest magnitude (as its bits) to [2^14, 2^15); an
+// infinity or a NaN counts as nothing (it stays what it is under any scale), zero gives zero.
+// Clamped so that the product of two inverse scales is still a normal number.
+__device__ inline int scale_exp(unsigned max_bits) {
+  const int e = static_cast<int>(max_bits >> 23);
+  return e == 0 ? 0 : min(kTopExp + 127 - e, 62);
+}
+__device__ inline unsigned finite_abs_bits(float x) {
+  const unsigned u = __float_as_uint(x) & 0x7fffffffu;
+  return u < 0x7f800000u ? u : 0u;
+}
+__device__ inline float pow2i(int e) { return __int_as_float((e + 127) << 23); }  // -126 <= e <= 127
+// Two scaled values as packed hi and lo fp16 pairs.
+__device__ inline void split_pair(float x0, float x1, unsigned& hi, unsigned& lo) {
+  const __half2 h = __floats2half2_rn(x0, x1);
+  const float2 f = __half22float2(h);
+  const __half2 r = __floats2half2_rn(x0 - f.x, x1 - f.y);
+  hi = *reinterpret_cast<const unsigned*>(&h);
+  lo = *reinterpret_cast<const unsigned*>(&r);
+}
+__device__ inline float2 fmul2(float2 a, float2 b) {
+  float2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;"
+      : "=l"(*reinterpret_cast<unsigned long long*>(&d))
+      : "l"(*reinterpret_cast<unsigned long long*>(&a)),
+        "l"(*reinterpret_cast<unsigned long long*>(&b)));
+  return d;
+}
+__device__ inline float4 ld_shared_f4(unsigned addr) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "r"(addr));
+  return v;
+}
+__device__ inline void st_shared_u4(unsigned addr, unsigned a, unsigned b, unsigned c, unsigned d) {
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d)
+               : "memory");
+}
+
+template <int DR, bool kSplit>
+__global__ void __launch_bounds__(kThreadsF, 1)
+    step_f32_kernel(const __grid_constant__ CUtensorMap tmap_k,
+                    const __grid_constant__ CUtensorMap tmap_v, const float* __restrict__ q_g,
+                    const TcArgs a) {
+  using C = F32Cfg<DR, kSplit>;
+  extern __shared__ __align__(1024) unsigned char smem[];  // 128B-swizzled tiles
+  const unsigned s_base = smem_u32(smem);
+  const unsigned s_q = s_base + C::kOffQ;
+  const unsigned s_kv = s_base + C::kOffKV;
+  const unsigned s_bar = s_base + C::kOffBar;
+  const unsigned bar_q_full = s_bar;                             // [2] Q split
+  const unsigned bar_kv_raw = s_bar + 16;                        // [kStages] TMA bytes
+  const unsigned bar_kv_full = bar_kv_raw + 8 * C::kStages;      // [kStages] split
+  const unsigned bar_kv_empty = bar_kv_full + 8 * C::kStages;    // [kStages] MMAs done
+  const unsigned bar_s_full = bar_kv_empty + 8 * C::kStages;     // [2]
+  const unsigned bar_s_free = bar_s_full + 16;                   // [2] S held in registers
+  const unsigned bar_p_full = bar_s_free + 16;                   // [2]
+  const unsigned bar_o_done = bar_p_full + 16;                   // [2] P.V done
+  const unsigned bar_v_max = bar_o_done + 16;                    // a V tile's maxima by warp written
+  unsigned* tmem_slot = reinterpret_cast<unsigned*>(smem + C::kOffSlot);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  volatile unsigned* red = reinterpret_cast<volatile unsigned*>(smem + C::kOffRed);
+  volatile int* v_exp = reinterpret_cast<volatile int*>(smem + C::kOffVExp);
+
+  const int tid = threadIdx.x;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+  const int lane = tid & 31;
+  unsigned cta_rank = 0;
+  if constexpr (kSplit) cta_rank = cluster_ctarank();
+
+  // an earlier block gave up: leave at once; a cluster starts in the aborted state instead and
+  // still meets at its barriers (see step_tc.cu)
+  if constexpr (!kSplit) {
+    if (__syncthreads_or(*reinterpret_cast<volatile int*>(a.status) != 0)) return;
+  }
+
+  const bool causal = (a.flags & RA_STEP_CAUSAL) != 0;
+  const bool fresh = (a.flags & RA_STEP_FRESH) != 0;
+  const bool finalize = (a.flags & RA_STEP_FINALIZE) != 0;
+
+  const int bh = kSplit ? static_cast<int>(blockIdx.x) / a.key_split : static_cast<int>(blockIdx.x);
+  const int qb_lin = static_cast<int>(gridDim.y) - 1 - static_cast<int>(blockIdx.y);
+  const int sq = qb_lin / a.n_qblocks_per_seg;
+  const int tq = qb_lin - sq * a.n_qblocks_per_seg;
+  const int h = bh % a.H;
+  const int b = bh / a.H;
+  const int kv_bh = b * a.kvH + (h % a.kvH);
+  const int q_seg_len = a.qmap.seg_len;
+  constexpr int kQBlock = C::kTiles * kBM;
+  const int row0 = tq * kQBlock;
+  const int rows_in_block = min(kQBlock, q_seg_len - row0);
+  const int qmin = a.qmap.base[sq] + row0 * a.stride;
+  const int qmax = a.qmap.base[sq] + (row0 + rows_in_block - 1) * a.stride;
+  const int live = rows_in_block > kBM ? 2 : 1;  // query tiles that hold a row
+
+  int n_tiles = 0;
+  for (int sk = 0; sk < a.kmap.n_seg; ++sk) {
+    const TileRange r = tile_range<kBNf>(a.kmap, sk, a.stride, causal, a.doc_len, qmin, qmax);
+    n_tiles += r.hi - r.lo;
+  }
+  int share_beg = 0, share_end = n_tiles;
+  if constexpr (kSplit) {
+    share_beg = static_cast<int>(static_cast<long long>(n_tiles) * cta_rank / a.key_split);
+    share_end = static_cast<int>(static_cast<long long>(n_tiles) * (cta_rank + 1) / a.key_split);
+    n_tiles = share_end - share_beg;
+  }
+
+  if (tid == 0) {
+    for (int w = 0; w < 2; ++w) {
+      mbar_init(bar_q_full + 8 * w, kBM);
+      mbar_init(bar_s_full + 8 * w, 1);
+      mbar_init(bar_s_free + 8 * w, kBM);
+      mbar_init(bar_p_full + 8 * w, kBM);
+      mbar_init(bar_o_done + 8 * w, 1);
+    }
+    mbar_init(bar_v_max, kSplitThreads / 32);
+    for (int s = 0; s < C::kStages; ++s) {
+      mbar_init(bar_kv_raw + 8 * s, 1);
+      mbar_init(bar_kv_full + 8 * s, kSplitThreads);
+      mbar_init(bar_kv_empty + 8 * s, live);
+    }
+    *abort_flag = (kSplit && *reinterpret_cast<volatile int*>(a.status) != 0) ? 1 : 0;
+    if (s_base & 1023u) {  // the swizzle of TMA and the descriptors below count on it
+      *abort_flag = 1;
+      atomicCAS(&a.status[0], 0, RA_ERR_DEVICE_WAIT);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(
+                     smem_u32(tmem_slot))
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const unsigned tmem_base = *tmem_slot;
+
+  // Registers: 640 threads start with 96 each (61440 in all); 128 * 40 + 256 * 144 + 256 * 72 = 60416.
+  if (warp < 4) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+    if (warp == 0) {
+      // ---------------------------------------------------------- TMA producer ----
+      if (lane == 0 && n_tiles > 0) {
+        int it = 0;
+        bool ok = *abort_flag == 0;
+        TileShare share{share_beg, share_end, 0};
+        for (int sk = 0; sk < a.kmap.n_seg && ok; ++sk) {
+          const TileRange r =
+              share.clip(tile_range<kBNf>(a.kmap, sk, a.stride, causal, a.doc_len, qmin, qmax));
+          for (int t = r.lo; t < r.hi && ok; ++t) {
+            const int k_row = a.kseg_row[sk] + t * kBNf;
+            const int k_head = a.kseg_head[sk] + kv_bh;
+            for (int which = 0; which < 2 && ok; ++which, ++it) {
+              const int slot = it % C::kStages;
+              if (it >= C::kStages)
+                ok = mbar_wait(bar_kv_empty + 8 * slot, ((it / C::kStages) + 1) & 1, abort_flag,
+                               a.status, 1, it, a.wait_ns);
+              if (!ok) break;
+              if (a.stall_after >= 0 && it >= a.stall_after) {  // test hook, see step_tc.cu
+                ok = false;
+                break;
+              }
+              mbar_expect_tx(bar_kv_raw + 8 * slot, C::kRawBytes);
+              const CUtensorMap* map = which == 0 ? &tmap_k : &tmap_v;
+              for (int bx = 0; bx < C::kBoxes; ++bx)
+                tma_load_3d(s_kv + slot * C::kSlotBytes + bx * C::kBoxBytes, map, bar_kv_raw + 8 * slot,
+                            bx * 32, k_row, k_head);
+            }
+          }
+        }
+      }
+    } else if (warp == 1 || (warp == 2 && live == 2)) {
+      // ----------------------------------------------------------- MMA issuers ----
+      if (n_tiles > 0) {
+        const int w = warp - 1;
+        constexpr unsigned idesc_s = make_idesc(0u, 0, kBNf, kBM);
+        constexpr unsigned idesc_pv = make_idesc(0u, 1, DR, kBM);
+        constexpr unsigned kQBox = (kBM * 128) >> 4;        // one 64-column box, 16-byte units
+        constexpr unsigned kGroup = (2 * C::kBoxBytes) >> 4;  // hi and lo box of a 64-column group
+        constexpr unsigned kLo = C::kBoxBytes >> 4;
+        const unsigned t_w = tmem_base + 256 * w;
+        const unsigned t_s = t_w + C::kColS, t_p = t_w + C::kColP, t_o = t_w + C::kColO;
+        const unsigned t_q = t_w + C::kColQ;
+        [[maybe_unused]] const unsigned long long qd = desc_kmajor(s_q + w * C::kQBytes);
+        const unsigned b_s_full = bar_s_full + 8 * w, b_s_free = bar_s_free + 8 * w;
+        const unsigned b_p_full = bar_p_full + 8 * w, b_o_done = bar_o_done + 8 * w;
+        auto wait = [&](unsigned bar, unsigned parity, int which, int tile) {
+          return __all_sync(0xffffffffu,
+                            mbar_wait(bar, parity, abort_flag, a.status, which, tile, a.wait_ns)) != 0;
+        };
+        // ring item of K_t: 2t, of V_t: 2t + 1
+        auto wait_kv = [&](int it, int which, int t) {
+          return wait(bar_kv_full + 8 * (it % C::kStages), (it / C::kStages) & 1, which, t);
+        };
+        auto issue_s = [&](int t) {
+          const int slot = (2 * t) % C::kStages;
+          const unsigned long long kd = desc_kmajor(s_kv + slot * C::kSlotBytes);
+          if (elect_one()) {
+            // small terms first: lo*hi, hi*lo, hi*hi
+#pragma unroll
+            for (int term = 0; term < 3; ++term) {
+#pragma unroll
+              for (int ks = 0; ks < DR / 16; ++ks) {  // 16 columns = 32 bytes, 4 steps per group
+                const unsigned off_k = (ks / 4) * kGroup + (ks % 4) * 2 + (term == 1 ? kLo : 0);
+                const unsigned acc = (term > 0 || ks > 0) ? 1u : 0u;
+                if (C::kQLoInTmem || term > 0) {
+                  mma_ts(t_s, t_q + ks * 8 + (term == 0 ? 32 : 0), kd + off_k, idesc_s, acc);
+                } else {
+                  mma_ss(t_s, qd + (ks / 4) * kQBox + (ks % 4) * 2, kd + off_k, idesc_s, acc);
+                }
+              }
+            }
+            tc_commit(b_s_full);
+            tc_commit(bar_kv_empty + 8 * slot);
+          }
+        };
+        auto issue_pv = [&](int t) {
+          const int slot = (2 * t + 1) % C::kStages;
+          // MN-major V: 64 columns per 128-byte row, groups 2 boxes apart, 16 keys per k-step
+          const unsigned long long vd =
+              desc_mnmajor(s_kv + slot * C::kSlotBytes, 2 * C::kBoxBytes, 1024);
+          if (elect_one()) {
+#pragma unroll
+            for (int term = 0; term < 3; ++term) {
+#pragma unroll
+              for (int ks = 0; ks < kBNf / 16; ++ks)
+                mma_ts(t_o, t_p + ks * 8 + (term == 0 ? 32 : 0),
+                       vd + ks * (2048 >> 4) + (term == 1 ? kLo : 0), idesc_pv,
+                       (t > 0 || term > 0 || ks > 0) ? 1u : 0u);
+            }
+            tc_commit(b_o_done);
+            tc_commit(bar_kv_empty + 8 * slot);
+          }
+        };
+        bool ok = wait(bar_q_full + 8 * w, 0, 3, w) && wait_kv(0, 5, 0);
+        if (ok) {
+          tc_fence_after();
+          issue_s(0);
+        }
+        for (int t = 0; t < n_tiles && ok; ++t) {
+          const bool more = t + 1 < n_tiles;
+          if constexpr (C::kAlias) {
+            // P.V of tile t and the scores of tile t + 1, which overwrite P, go out together: the
+            // tensor core runs them in order
+            ok = wait_kv(2 * t + 1, 4, t) && (!more || wait_kv(2 * t + 2, 5, t)) &&
+                 wait(b_p_full, t & 1, 6, t);
+            if (!ok) break;
+            tc_fence_after();
+            issue_pv(t);
+            if (more) issue_s(t + 1);
+          } else {
+            if (more) {
+              ok = wait(b_s_free, t & 1, 9, t) && wait_kv(2 * t + 2, 5, t);
+              if (!ok) break;
+              tc_fence_after();
+              issue_s(t + 1);
+            }
+            ok = wait_kv(2 * t + 1, 4, t) && wait(b_p_full, t & 1, 6, t);
+            if (!ok) break;
+            tc_fence_after();
+            issue_pv(t);
+          }
+        }
+      }
+    }
+    if constexpr (kSplit) {  // the three meetings of merge_key_split
+      for (int i = 0; i < 3; ++i) cluster_sync_threads();
+    }
+  } else if (warp >= 12) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
+    // --------------------------------------------------------------- splitters ----
+    // A warp owns eight rows of every tile; its lanes own 16-byte pieces of the split rows (8
+    // values, 32 raw bytes): lane = (piece, row), so the eight lanes of a phase touch eight rows
+    // at one swizzled column and no bank twice.
+    if (n_tiles > 0) {
+      constexpr int kUnits = DR / 32;  // pieces per lane
+      const int sw = warp - 12, r8 = lane & 7, p4 = lane >> 3;
+      const unsigned row_off = (sw * 8 + r8) * 128;
+      bool ok = true;
+      for (int it = 0; it < 2 * n_tiles && ok; ++it) {
+        const int slot = it % C::kStages;
+        ok = __all_sync(0xffffffffu, mbar_wait(bar_kv_raw + 8 * slot, (it / C::kStages) & 1, abort_flag,
+                                               a.status, 13, it, a.wait_ns)) != 0;
+        if (!ok) break;
+        const unsigned base = s_kv + slot * C::kSlotBytes + row_off;
+        float x[kUnits][8];
+        float fm = 0.f;
+#pragma unroll
+        for (int u = 0; u < kUnits; ++u) {
+          const int piece = p4 + 4 * u;  // of the whole row; raw box = piece / 4, 2 chunks each
+          const unsigned box = base + (piece >> 2) * C::kBoxBytes;
+          const int c = (piece & 3) * 2;
+          const float4 v0 = ld_shared_f4(box + ((c ^ r8) << 4));
+          const float4 v1 = ld_shared_f4(box + (((c + 1) ^ r8) << 4));
+          x[u][0] = v0.x, x[u][1] = v0.y, x[u][2] = v0.z, x[u][3] = v0.w;
+          x[u][4] = v1.x, x[u][5] = v1.y, x[u][6] = v1.z, x[u][7] = v1.w;
+#pragma unroll
+          for (int i = 0; i < 8; i += 2) fm = max3(fm, fabsf(x[u][i]), fabsf(x[u][i + 1]));
+        }
+        unsigned mx = __float_as_uint(fm);  // (a maximum passes NaN by)
+        if (mx >= 0x7f800000u) {            // an infinity among them: the finite ones count
+          mx = 0;
+#pragma unroll
+          for (int u = 0; u < kUnits; ++u)
+#pragma unroll
+            for (int i = 0; i < 8; ++i) mx = max(mx, finite_abs_bits(x[u][i]));
+        }
+        int e;
+        if ((it & 1) == 0) {
+          // K: by key. The row's pieces sit in the four lanes r8, r8 + 8, ...
+          mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
+          mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+          e = scale_exp(mx);
+          if (p4 == 0) {
+            const unsigned g = s_base + C::kOffG + (((it >> 1) % C::kGDepth) * kBNf + sw * 8 + r8) * 4;
+            asm volatile("st.shared.f32 [%0], %1;" ::"r"(g), "f"(pow2i(-e)) : "memory");
+          }
+          __syncwarp();  // the rows of this warp have been read
+        } else {
+          // V: by tile
+          mx = __reduce_max_sync(0xffffffffu, mx);
+          const int par = (it >> 1) & 1;
+          if (lane == 0) {
+            red[par * 8 + sw] = mx;
+            mbar_arrive(bar_v_max);
+          }
+          // (an mbarrier and not bar.sync: a warp that gives up must not leave the others waiting)
+          ok = __all_sync(0xffffffffu,
+                          mbar_wait(bar_v_max, par, abort_flag, a.status, 15, it, a.wait_ns)) != 0;
+          if (!ok) break;
+          mx = 0;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) mx = max(mx, red[par * 8 + i]);
+          e = scale_exp(mx);
+          // (an all-zero tile sets no unit: marked with an exponent no other tile has)
+          if (sw == 0 && lane == 0) v_exp[(it >> 1) & 15] = mx == 0 ? 127 : e;
+        }
+        const float sc = pow2i(e);
+#pragma unroll
+        for (int u = 0; u < kUnits; ++u) {
+          const int piece = p4 + 4 * u;  // split box pair = piece / 8
+          const unsigned hi_at = base + (piece >> 3) * 2 * C::kBoxBytes + (((piece & 7) ^ r8) << 4);
+          unsigned hi[4], lo[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) split_pair(x[u][2 * i] * sc, x[u][2 * i + 1] * sc, hi[i], lo[i]);
+          st_shared_u4(hi_at, hi[0], hi[1], hi[2], hi[3]);
+          st_shared_u4(hi_at + C::kBoxBytes, lo[0], lo[1], lo[2], lo[3]);
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        mbar_arrive(bar_kv_full + 8 * slot);
+      }
+    }
+    if constexpr (kSplit) {
+      for (int i = 0; i < 3; ++i) cluster_sync_threads();
+    }
+  } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 144;");
+    // ----------------------------------------------------------------- softmax ----
+    const int w = (warp - 4) >> 2;
+    const int row = ((warp & 3) << 5) + lane;  // row of the tile = tensor-memory lane
+    const unsigned t_w = tmem_base + (static_cast<unsigned>((warp & 3) << 5) << 16) + 256 * w;
+    const unsigned t_s = t_w + C::kColS, t_p = t_w + C::kColP, t_o = t_w + C::kColO;
+    const int r_in_seg = row0 + w * kBM + row;
+    const bool row_valid = r_in_seg < q_seg_len;
+    const int qpos = a.qmap.base[sq] + r_in_seg * a.stride;
+    const long long qdoc = a.doc_len > 0 ? qpos / a.doc_len : 0;
+    const size_t grow0 = static_cast<size_t>(bh) * a.Sq + static_cast<size_t>(sq) * q_seg_len + row0;
+    const size_t grow = grow0 + (row_valid ? w * kBM + row : 0);
+    const bool mine = w < live && n_tiles > 0;
+
+    // ---- this row of Q: scale, split, hand to the MMA warp
+    float row_f = 0.f;  // turns a scaled score (K factor applied) into log2 units
+    if (mine) {
+      const float4* q4 = reinterpret_cast<const float4*>(q_g + grow * DR);
+      unsigned mx = 0;
+#pragma unroll 4
+      for (int i = 0; i < DR / 4; ++i) {
+        const float4 v = row_valid ? q4[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+        mx = max(max(max(mx, finite_abs_bits(v.x)), max(finite_abs_bits(v.y), finite_abs_bits(v.z))),
+                 finite_abs_bits(v.w));
+      }
+      const int e = scale_exp(mx);
+      const float sc = pow2i(e);
+      row_f = rsqrtf(static_cast<float>(DR)) * kLog2e * pow2i(-e);
+#pragma unroll
+      for (int g = 0; g < DR / 32; ++g) {  // 32 columns at a time (second read: L1 / L2)
+        unsigned hi[16], lo[16];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float4 v = row_valid ? q4[g * 8 + i] : make_float4(0.f, 0.f, 0.f, 0.f);
+          split_pair(v.x * sc, v.y * sc, hi[2 * i], lo[2 * i]);
+          split_pair(v.z * sc, v.w * sc, hi[2 * i + 1], lo[2 * i + 1]);
+        }
+        tmem_st16(t_w + C::kColQ + 16 * g, hi);
+        if constexpr (C::kQLoInTmem) {
+          tmem_st16(t_w + C::kColQ + 32 + 16 * g, lo);
+        } else {
+          const unsigned at = s_q + w * C::kQBytes + (g >> 1) * (kBM * 128) + row * 128;
+#pragma unroll
+          for (int p = 0; p < 4; ++p) {
+            const unsigned off = ((((g & 1) * 4 + p) ^ (row & 7)) << 4);
+            st_shared_u4(at + off, lo[4 * p], lo[4 * p + 1], lo[4 * p + 2], lo[4 * p + 3]);
+          }
+        }
+      }
+      tmem_wait_st();
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      tc_fence_before();
+      mbar_arrive(bar_q_full + 8 * w);
+    }
+
+    float m_ref = -INFINITY;  // reference point of P, O and l, log2 units
+    float l_run = 0.f;
+    int v_ref = 127;          // O is in units of 2^-(kPBits + v_ref); 127: no V seen yet
+    bool ok = true;
+    int j = 0;
+    const int n_seg = mine ? a.kmap.n_seg : 0;
+    TileShare share{share_beg, share_end, 0};
+    for (int sk = 0; sk < n_seg && ok; ++sk) {
+      const TileRange tr =
+          share.clip(tile_range<kBNf>(a.kmap, sk, a.stride, causal, a.doc_len, qmin, qmax));
+      // visible local key indices [rel_lo, rel_hi) of this segment for this row
+      int rel_lo = 0, rel_hi = row_valid ? a.kmap.seg_len : 0;
+      {
+        const long long kb = a.kmap.base[sk];
+        if (causal) {
+          const long long d = static_cast<long long>(qpos) - kb;
+          rel_hi = d < 0 ? 0 : static_cast<int>(min(static_cast<long long>(rel_hi), d / a.stride + 1));
+        }
+        if (a.doc_len > 0) {
+          const long long p_lo = qdoc * a.doc_len, p_hi = p_lo + a.doc_len - 1;
+          if (p_hi < kb) {
+            rel_hi = 0;
+          } else {
+            rel_hi = static_cast<int>(min(static_cast<long long>(rel_hi), (p_hi - kb) / a.stride + 1));
+            if (p_lo > kb)
+              rel_lo = static_cast<int>(min(static_cast<long long>(a.kmap.seg_len),
+                                            (p_lo - kb + a.stride - 1) / a.stride));
+          }
+        }
+      }
+      for (int t = tr.lo; t < tr.hi && ok; ++t, ++j) {
+        int c_lo = min(max(rel_lo - t * kBNf, 0), kBNf);
+        int c_hi = min(max(rel_hi - t * kBNf, 0), kBNf);
+        if (c_hi < c_lo) c_hi = c_lo;
+        const bool full = __all_sync(0xffffffffu, c_lo == 0 && c_hi == kBNf);
+
+        // the V tile's barrier stands for both: K_j is split before V_j, and V_j's slot is not
+        // reused before this softmax is done
+        const int vit = 2 * j + 1;
+        ok = mbar_wait(bar_kv_full + 8 * (vit % C::kStages), (vit / C::kStages) & 1, abort_flag, a.status,
+                       11, j, a.wait_ns) &&
+             mbar_wait(bar_s_full + 8 * w, j & 1, abort_flag, a.status, 7, j, a.wait_ns);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        tc_fence_after();
+        float s[kBNf];
+        tmem_ld64(t_s, s);
+        if constexpr (!C::kAlias) {
+          tc_fence_before();
+          mbar_arrive(bar_s_free + 8 * w);  // the tensor core may write the next scores
+        }
+        const unsigned g_at = s_base + C::kOffG + (j % C::kGDepth) * kBNf * 4;
+#pragma unroll
+        for (int i = 0; i < kBNf; i += 4) {
+          const float4 g = ld_shared_f4(g_at + i * 4);
+          const float2 x0 = fmul2(make_float2(s[i], s[i + 1]), make_float2(g.x, g.y));
+          const float2 x1 = fmul2(make_float2(s[i + 2], s[i + 3]), make_float2(g.z, g.w));
+          s[i] = x0.x, s[i + 1] = x0.y, s[i + 2] = x1.x, s[i + 3] = x1.y;
+        }
+        if (!full) {
+#pragma unroll
+          for (int i = 0; i < kBNf; ++i) s[i] = (i >= c_lo && i < c_hi) ? s[i] : -INFINITY;
+        }
+
+        // unit of this tile's P: 2^p_exp at the reference point, so that P * V lands in O's unit
+        const int ev = v_exp[j & 15];
+        bool slow = false;
+        float v_alpha = 1.f;  // O moves to a new unit
+        if (ev != 127) {
+          if (v_ref == 127) {
+            v_ref = ev;  // nothing but zeros in O so far
+          } else if (ev < v_ref - kVSlack) {
+            v_alpha = pow2i(max(ev - v_ref, -126));
+            v_ref = ev;
+            slow = true;
+          }
+        }
+        const int p_exp = kPBits + ((ev == 127) ? 0 : max(v_ref - ev, -40));  // (smaller V adds nothing to O)
+        // Wait for P.V of the previous tile: its P buffer is about to be written. (With P over S the
+        // scores of this tile, issued behind it, stand for that.)
+        if (!C::kAlias && j > 0) {
+          ok = mbar_wait(bar_o_done + 8 * w, (j - 1) & 1, abort_flag, a.status, 10, j, a.wait_ns);
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
+          tc_fence_after();
+        }
+        const float2 f2 = make_float2(row_f, row_f);
+        float row_sum = 0.f, oct_max = 0.f;
+        // P = 2^(s * f - m_ref + p_exp) as hi + lo in tensor memory, 32 columns at a time; the sums
+        // of eight columns each bound every P and add up to the row sum
+        auto exponentials = [&](float neg_m) {
+          const float2 n2 = make_float2(neg_m, neg_m);
+          float2 sum[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) sum[i] = make_float2(0.f, 0.f);
+#pragma unroll
+          for (int c = 0; c < kBNf / 32; ++c) {
+            unsigned hi[16], lo[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+              const float2 x = ffma2(make_float2(s[32 * c + 2 * i], s[32 * c + 2 * i + 1]), f2, n2);
+              const float2 p = make_float2(ex2(x.x), ex2(x.y));
+              sum[i & 3] = fadd2(sum[i & 3], p);
+              split_pair(p.x, p.y, hi[i], lo[i]);
+            }
+            tmem_st16(t_p + 16 * c, hi);
+            tmem_st16(t_p + 32 + 16 * c, lo);
+          }
+          const float2 s01 = fadd2(sum[0], sum[1]), s23 = fadd2(sum[2], sum[3]);
+          const float2 all = fadd2(s01, s23);
+          oct_max = fmaxf(max3(fmaxf(sum[0].x, sum[0].y), sum[1].x, sum[1].y),
+                          max3(fmaxf(sum[2].x, sum[2].y), sum[3].x, sum[3].y));
+          row_sum = all.x + all.y;
+        };
+        slow = slow || __any_sync(0xffffffffu, m_ref == -INFINITY && c_hi > c_lo) != 0;
+        const float pe = static_cast<float>(p_exp);
+        if (!slow) {
+          exponentials(m_ref == -INFINITY ? 0.f : pe - m_ref);
+          slow = __any_sync(0xffffffffu, !(oct_max <= kPSumLimit) || !(row_sum == row_sum)) != 0;
+        }
+        if (slow) {
+          float mx = s[0];
+#pragma unroll
+          for (int i = 1; i < kBNf - 1; i += 2) mx = max3(mx, s[i], s[i + 1]);
+          mx = fmaxf(mx, s[kBNf - 1]);
+          const float tile_max = mx * row_f;  // -inf stays -inf
+          float alpha = 1.f;
+          if (tile_max > m_ref) {
+            if (m_ref > -INFINITY) alpha = ex2(m_ref - tile_max);
+            m_ref = tile_max;
+          }
+          if (j > 0 && __any_sync(0xffffffffu, alpha != 1.f || v_alpha != 1.f)) {
+            // O is at rest: P.V of tile j - 1 has completed
+            l_run *= alpha;
+            const float oa = alpha * v_alpha;
+#pragma unroll 1
+            for (int c = 0; c < DR / 32; ++c) {
+              float o[32];
+              tmem_ld32(t_o + c * 32, o);
+#pragma unroll
+              for (int i = 0; i < 32; ++i) o[i] *= oa;
+              tmem_st32(t_o + c * 32, o);
+            }
+          }
+          exponentials(m_ref == -INFINITY ? 0.f : pe - m_ref);
+        }
+        l_run += row_sum * pow2i(-p_exp);
+        tmem_wait_st();
+        tc_fence_before();
+        mbar_arrive(bar_p_full + 8 * w);
+      }
+    }
+
+    // ---------------------------------------------------------------- epilogue ----
+    if (ok && mine)
+      ok = mbar_wait(bar_o_done + 8 * w, (n_tiles - 1) & 1, abort_flag, a.status, 8, n_tiles, a.wait_ns);
+    ok = __all_sync(0xffffffffu, ok);
+    if (ok && mine) tc_fence_after();
+    const float o_unit = pow2i(v_ref == 127 ? 0 : -(kPBits + v_ref));
+    if constexpr (kSplit) {
+      merge_key_split<C, DR>(a, smem, s_base, t_o, w, row, row_valid, grow0, ok && mine, m_ref, l_run, o_unit,
+                             cta_rank, fresh, finalize);
+    } else if (ok) {
+      float* o_g = a.out + grow * DR;
+      const bool have = row_valid && mine && m_ref > -INFINITY;
+      float m_old = -INFINITY, l_old = 0.f;
+      if (!fresh && row_valid) {
+        m_old = a.m[grow];
+        l_old = a.l[grow];
+      }
+      const float m_new = have ? m_ref * kLn2 : -INFINITY;  // natural-log units
+      const float m_fin = fmaxf(m_old, m_new);
+      const float ca = (m_old == -INFINITY) ? 0.f : expf(m_old - m_fin);
+      const float cb = have ? expf(m_new - m_fin) : 0.f;
+      const float l_fin = ca * l_old + cb * l_run;
+      const float inv = finalize ? (l_fin > 0.f ? 1.f / l_fin : 0.f) : 1.f;
+      const bool touch = row_valid && (have || fresh || finalize);
+      const float fo = cb * o_unit;
+#pragma unroll 1
+      for (int c = 0; c < DR / 32; ++c) {
+        float o[32];
+        if (mine) {  // warp-uniform: the tensor-memory load is warp-collective
+          tmem_ld32(t_o + c * 32, o);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) o[i] = 0.f;
+        }
+        if (touch) {
+          float4* dst = reinterpret_cast<float4*>(o_g + c * 32);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            float4 old = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (!fresh) old = dst[i];
+            float4 r;
+            r.x = (ca * old.x + (have ? fo * o[4 * i] : 0.f)) * inv;
+            r.y = (ca * old.y + (have ? fo * o[4 * i + 1] : 0.f)) * inv;
+            r.z = (ca * old.z + (have ? fo * o[4 * i + 2] : 0.f)) * inv;
+            r.w = (ca * old.w + (have ? fo * o[4 * i + 3] : 0.f)) * inv;
+            dst[i] = r;
+          }
+        }
+      }
+      if (touch) {
+        a.m[grow] = m_fin;
+        a.l[grow] = l_fin;
+      }
+    }
+  }
+
+  // ---------------------------------------------------------------- teardown ----
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    if (*abort_flag) {
+      // give copies and MMAs still in flight time to land before tensor memory is released
+      const unsigned long long t0 = global_ns();
+      while (global_ns() - t0 < 1000000ull) __nanosleep(1000);
+    }
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem_base)
+                 : "memory");
+  }
+}
+
+// ---- host side ----------------------------------------------------------------------
+
+template <int DR, bool kSplit>
+int launch_f32(const StepArgs& a, cudaStream_t stream, int key_split) {
+  using C = F32Cfg<DR, kSplit>;
+  CUtensorMap mk, mv;
+  int rc = make_map(&mk, RA_F32, a.k, a.D, a.k_rows, a.k_heads_total, a.kv_head_stride, kBNf);
+  if (rc != RA_OK) return rc;
+  rc = make_map(&mv, RA_F32, a.v, a.D, a.k_rows, a.k_heads_total, a.kv_head_stride, kBNf);
+  if (rc != RA_OK) return rc;
+  TcArgs t;
+  t.kv_per_wave = 0;
+  t.key_split = key_split;
+  t.out = a.out;
+  t.m = a.m;
+  t.l = a.l;
+  t.H = a.H;
+  t.kvH = a.kvH;
+  t.Sq = a.Sq;
+  t.n_qblocks_per_seg = (a.qmap.seg_len + 2 * kBM - 1) / (2 * kBM);
+  t.qmap = a.qmap;
+  t.kmap = a.kmap;
+  for (int i = 0; i < RA_MAX_SEG; ++i) {
+    t.kseg_head[i] = a.kseg_head[i];
+    t.kseg_row[i] = a.kseg_row[i];
+  }
+  t.stride = a.stride;
+  t.flags = a.flags;
+  t.doc_len = a.doc_len;
+  t.status = a.status;
+  t.wait_ns = tc_wait_limit_ns();
+  t.stall_after = tc_stall_after();
+  const long long n_qblocks = static_cast<long long>(t.n_qblocks_per_seg) * a.qmap.n_seg;
+  RAB_REQUIRE(n_qblocks <= 65535, RA_ERR_INVALID, "attention step: too many query blocks (%lld)",
+              n_qblocks);
+  auto kern = step_f32_kernel<DR, kSplit>;
+  static std::atomic<unsigned long long> smem_set{0};  // once per device, see step_tc.cu
+  int dev = 0;
+  RAB_CUDA(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 64 || !(smem_set.load(std::memory_order_acquire) >> dev & 1ull)) {
+    RAB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes));
+    if (dev >= 0 && dev < 64) smem_set.fetch_or(1ull << dev, std::memory_order_release);
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(a.B) * a.H * (kSplit ? key_split : 1),
+                     static_cast<unsigned>(n_qblocks));
+  cfg.blockDim = dim3(kThreadsF);
+  cfg.dynamicSmemBytes = C::kSmemBytes;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = key_split;
+  attr.val.clusterDim.y = 1;
+  attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = kSplit ? 1 : 0;
+  RAB_CUDA(cudaLaunchKernelEx(&cfg, kern, mk, mv, static_cast<const float*>(a.q), t));
+  RAB_CUDA(cudaGetLastError());
+  return RA_OK;
+}
+
+template <int DR>
+int launch_f32_d(const StepArgs& a, cudaStream_t stream) {
+  const int split = pick_key_split<kBNf>(a, 2 * kBM, 1.5, 0);
+  return split > 1 ? launch_f32<DR, true>(a, stream, split) : launch_f32<DR, false>(a, stream, 1);
+}
+
+}  // namespace
+
+bool step_f32_supported(int dtype, const StepArgs& a) {
+  if (dtype != RA_F32) return false;
+  if (a.D != 32 && a.D != 64 && a.D != 128) return false;
+  if (a.Sq <= 0 || a.Sk <= 0) return false;
+  if (a.qmap.n_seg * a.qmap.seg_len != a.Sq || a.kmap.n_seg * a.kmap.seg_len != a.Sk) return false;
+  if ((reinterpret_cast<uintptr_t>(a.q) | reinterpret_cast<uintptr_t>(a.k) |
+       reinterpret_cast<uintptr_t>(a.v) | reinterpret_cast<uintptr_t>(a.out)) & 15u)
+    return false;
+  return true;
+}
+
+int launch_step_f32(const StepArgs& a, cudaStream_t stream) {
+  RAB_REQUIRE(a.status != nullptr, RA_ERR_CUDA, "attention step: no device status word");
+  if (a.D == 32) return launch_f32_d<32>(a, stream);
+  if (a.D == 64) return launch_f32_d<64>(a, stream);
+  return launch_f32_d<128>(a, stream);
+}
+
+}  // namespace rab

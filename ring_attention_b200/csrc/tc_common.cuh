@@ -1,5 +1,5 @@
 // Device-side building blocks shared by the tcgen05 step kernels (step_tc.cu: fp16 / bf16,
-// step_tf32.cu: fp32 through split TF32 operands): mbarrier / TMA / tcgen05 wrappers with bounded
+// step_f32.cu: fp32 through split fp16 operands): mbarrier / TMA / tcgen05 wrappers with bounded
 // waits, shared-memory and instruction descriptors, the visible key-tile range of a query
 // block, the kernel argument block and the host-side tensor-map encoder.
 #pragma once
@@ -273,6 +273,27 @@ __device__ inline void tmem_ld128(unsigned taddr, float (&r)[128]) {
 #pragma unroll
   for (int i = 0; i < 128; ++i) r[i] = __uint_as_float(u[i]);
 }
+// 64 columns of a row: two loads in flight and one wait.
+__device__ inline void tmem_ld64(unsigned taddr, float (&r)[64]) {
+  unsigned u[64];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%64];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%32, %33, %34, %35, %36, %37, %38, %39, %40, %41, %42, %43, %44, %45, %46, %47, %48, %49, %50, %51, %52, %53, %54, %55, %56, %57, %58, %59, %60, %61, %62, %63}, [%65];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7]),
+        "=r"(u[8]), "=r"(u[9]), "=r"(u[10]), "=r"(u[11]), "=r"(u[12]), "=r"(u[13]), "=r"(u[14]),
+        "=r"(u[15]), "=r"(u[16]), "=r"(u[17]), "=r"(u[18]), "=r"(u[19]), "=r"(u[20]), "=r"(u[21]),
+        "=r"(u[22]), "=r"(u[23]), "=r"(u[24]), "=r"(u[25]), "=r"(u[26]), "=r"(u[27]), "=r"(u[28]),
+        "=r"(u[29]), "=r"(u[30]), "=r"(u[31]), "=r"(u[32]), "=r"(u[33]), "=r"(u[34]), "=r"(u[35]),
+        "=r"(u[36]), "=r"(u[37]), "=r"(u[38]), "=r"(u[39]), "=r"(u[40]), "=r"(u[41]), "=r"(u[42]),
+        "=r"(u[43]), "=r"(u[44]), "=r"(u[45]), "=r"(u[46]), "=r"(u[47]), "=r"(u[48]), "=r"(u[49]),
+        "=r"(u[50]), "=r"(u[51]), "=r"(u[52]), "=r"(u[53]), "=r"(u[54]), "=r"(u[55]), "=r"(u[56]),
+        "=r"(u[57]), "=r"(u[58]), "=r"(u[59]), "=r"(u[60]), "=r"(u[61]), "=r"(u[62]), "=r"(u[63])
+      : "r"(taddr), "r"(taddr + 32)
+      : "memory");
+#pragma unroll
+  for (int i = 0; i < 64; ++i) r[i] = __uint_as_float(u[i]);
+}
 __device__ inline void tmem_st32(unsigned taddr, const float (&r)[32]) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
@@ -360,16 +381,6 @@ __device__ inline unsigned long long desc_mnmajor(unsigned saddr, unsigned lbo_b
                                                unsigned sbo_bytes) {
   const unsigned lo = ((saddr & 0x3FFFFu) >> 4) | (((lbo_bytes >> 4) & 0x3FFFu) << 16);
   const unsigned hi = ((sbo_bytes >> 4) & 0x3FFFu) | (1u << 14) | (2u << 29);
-  return (static_cast<unsigned long long>(hi) << 32) | lo;
-}
-
-// MN-major operand of 32-bit elements (TF32): the 128B swizzle that moves 32-byte pieces (TMA's
-// SWIZZLE_128B_ATOM_32B), four rows of the contraction index per swizzle atom. Leading byte
-// offset = distance between 32-element N blocks, stride = between 4-row groups (512 B).
-__device__ inline unsigned long long desc_mnmajor_32b(unsigned saddr, unsigned lbo_bytes,
-                                                      unsigned sbo_bytes) {
-  const unsigned lo = ((saddr & 0x3FFFFu) >> 4) | (((lbo_bytes >> 4) & 0x3FFFu) << 16);
-  const unsigned hi = ((sbo_bytes >> 4) & 0x3FFFu) | (1u << 14) | (1u << 29);
   return (static_cast<unsigned long long>(hi) << 32) | lo;
 }
 
@@ -557,8 +568,7 @@ inline EncodeTiledFn encode_fn() {
 // the tensor (head_dim 32 in 16 bits) the upper elements of every row are out of bounds and
 // arrive as zeros, which is exactly a head_dim 64 tile whose upper half is zero.
 inline int make_map(CUtensorMap* map, int dtype, const void* base, int D, long long rows,
-                    long long heads, long long head_stride_elems, int box_rows = 128,
-                    bool swizzle_32b_atoms = false) {
+                    long long heads, long long head_stride_elems, int box_rows = 128) {
   EncodeTiledFn fn = encode_fn();
   RAB_REQUIRE(fn != nullptr, RA_ERR_CUDA, "cuTensorMapEncodeTiled is unavailable");
   const cuuint64_t es = dtype == RA_F32 ? 4 : 2;
@@ -572,8 +582,7 @@ inline int make_map(CUtensorMap* map, int dtype, const void* base, int D, long l
                                    : dtype == RA_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
                                                       : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
   const CUresult r = fn(map, type, 3, const_cast<void*>(base), dims, strides, box, estr,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE,
-                        swizzle_32b_atoms ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   RAB_REQUIRE(r == CUDA_SUCCESS, RA_ERR_CUDA, "cuTensorMapEncodeTiled failed with code %d",
               static_cast<int>(r));

@@ -1,8 +1,9 @@
 """GPU parity of the forms that a call's shape selects: the key-split form of the step kernels (the
-blocks of a cluster share a query block's keys).
+blocks of a cluster share a query block's keys) and the scaled fp16 splitting of the fp32 step.
 
 Tolerances are those of the other step and decode tests: 1e-5 for fp32 and 1e-3 / 8e-3 for fp16 /
-bf16 P, absolute and relative, against the oracle on the same rounded inputs."""
+bf16 P, absolute and relative, against the oracle on the same rounded inputs. Where values are
+scaled by 2^e the absolute part scales with V."""
 import ctypes as C
 
 import numpy as np
@@ -71,3 +72,50 @@ def test_key_split_leaves_rows_without_a_visible_key_alone():
         step(dev(q, dtype), dev(k, dtype), dev(v, dtype), state, api.AttentionShape(B, H, Sq, Sk, D),
              SegMap.make([0], Sq), SegMap.make([1000], Sk), CAUSAL, 4)
     assert (state[0] == 3.0).all() and (state[1] == 0.5).all() and (state[2] == 2.0).all()
+
+
+@pytest.mark.parametrize("D", [32, 64, 128])
+@pytest.mark.parametrize("case", ["small", "large", "tiny_keys", "outlier_key", "growing_v", "zero_v_tiles", "shrinking_v"])
+def test_fp32_step_holds_its_precision_over_the_range_of_fp32(D, case):
+    # magnitudes that fp16 cannot hold have to come through the scaling of Q rows, keys and V tiles
+    B, H, Sq, Sk = 1, 2, 140, 400
+    q, k, v = normal_inputs(8, B, H, H, Sq, Sk, D)
+    if case == "small":
+        q, k, v = q * 2.0 ** 20, k * 2.0 ** -20, v * 2.0 ** -30
+    elif case == "large":
+        q, k, v = q * 2.0 ** -40, k * 2.0 ** 40, v * 2.0 ** 60
+    elif case == "tiny_keys":
+        k *= 2.0 ** -60
+    elif case == "outlier_key":  # hides itself behind a hugely negative score
+        q = np.abs(q)
+        k[:, :, 37] = -1e9
+    elif case == "growing_v":
+        v *= 2.0 ** (np.arange(Sk, dtype=np.float32) // 64 * 9)[None, None, :, None]
+    elif case == "shrinking_v":
+        v *= 2.0 ** -(np.arange(Sk, dtype=np.float32) // 64 * 9)[None, None, :, None]
+    else:
+        v[:, :, :130] = 0.0
+        v[:, :, 256:320] = 0.0
+    q, k, v = (x.astype(np.float32) for x in (q, k, v))
+    want, want_lse = oracle.cpu_attention(q, k, v, False, want_lse=True)
+    state = poisoned(B, H, Sq, D)
+    step(dev(q), dev(k), dev(v), state, api.AttentionShape(B, H, Sq, Sk, D), SegMap.make([0], Sq),
+         SegMap.make([0], Sk), FRESH | FINALIZE)
+    lse = api.attention_lse(state[1], state[2]).cpu().numpy()
+    unit = float(np.abs(want).max())  # errors of a weighted sum of V scale with the largest V
+    assert_close(state[0].cpu().numpy() / unit, want / unit, 1e-5, 1e-5, "out")
+    assert_close(lse, want_lse, 1e-5, 1e-5, "lse")
+
+
+def test_fp32_step_passes_on_nan_and_infinity_of_visible_values_only():
+    B, H, S, D = 1, 1, 200, 64
+    q, k, v = normal_inputs(9, B, H, H, S, S, D)
+    v[0, 0, 150, 7] = np.inf
+    k[0, 0, 190, 3] = np.nan
+    state = poisoned(B, H, S, D)
+    step(dev(q), dev(k), dev(v), state, api.AttentionShape(B, H, S, S, D), SegMap.make([0], S),
+         SegMap.make([0], S), FRESH | FINALIZE | CAUSAL)
+    got = state[0].cpu().numpy()[0, 0]
+    want = oracle.cpu_attention(q[:, :, :128], k[:, :, :128], v[:, :, :128], True)[0, 0]
+    assert_close(got[:128], want, 1e-5, 1e-5, "rows whose key tiles are finite")
+    assert not np.isfinite(got[160, 7]) and np.isnan(got[195]).all()
