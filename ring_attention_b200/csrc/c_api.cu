@@ -270,9 +270,7 @@ int ra_flash_attention(const float* q, const float* k, const float* v, float* ou
   __half* qh = reinterpret_cast<__half*>(hp);
   __half* kh = qh + ((qn + 7) & ~static_cast<size_t>(7));
   __half* vh = kh + ((kn + 7) & ~static_cast<size_t>(7));
-  int rc = ra_float_to_half(q, qh, qn, stream_);
-  if (rc == RA_OK) rc = ra_float_to_half(k, kh, kn, stream_);
-  if (rc == RA_OK) rc = ra_float_to_half(v, vh, kn, stream_);
+  const int rc = launch_narrow_qkv(q, k, v, qh, kh, vh, qn, kn, stream);
   if (rc != RA_OK) return rc;
   return step_ex(RA_F16, qh, kh, vh, out, m, l, *s, qmap, kmap, 1, flags, 0, 0, stream);
 }
@@ -467,6 +465,19 @@ void ra_kv_cache_reset(ra_kv_cache* c) {
   if (c) c->current_len = 0;
 }
 
+// Whether a kernel on the current device can read elements of `es` bytes at p (a copy can also
+// reach memory that is not mapped here).
+static bool readable_here(const void* p, size_t es) {
+  cudaPointerAttributes at;
+  int dev = 0;
+  if (reinterpret_cast<uintptr_t>(p) % es != 0 || cudaGetDevice(&dev) != cudaSuccess) return false;
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return at.type == cudaMemoryTypeDevice && at.device == dev;
+}
+
 // Strided copy of `rows` rows per (batch, kv head) into the cache starting at row `at`
 // (reference: cudaMemcpy2DAsync with pitch s_max * D * sizeof(T), src/kv_cache.cu:41-44,60-63).
 static int cache_copy(ra_kv_cache* c, const void* k_src, const void* v_src, int rows, int at,
@@ -477,6 +488,10 @@ static int cache_copy(ra_kv_cache* c, const void* k_src, const void* v_src, int 
   const size_t height = static_cast<size_t>(c->batch) * c->kv_heads;
   const size_t off = static_cast<size_t>(at) * c->head_dim * es;
   if (width == 0) return RA_OK;
+  if (rows == 1 && height <= 65535 && readable_here(k_src, es) && readable_here(v_src, es))
+    return launch_cache_row(k_src, v_src, static_cast<unsigned char*>(c->k) + off,
+                            static_cast<unsigned char*>(c->v) + off, width, dpitch,
+                            static_cast<int>(height), stream);
   RAB_CUDA(cudaMemcpy2DAsync(static_cast<unsigned char*>(c->k) + off, dpitch, k_src, width, width,
                              height, cudaMemcpyDeviceToDevice, stream));
   RAB_CUDA(cudaMemcpy2DAsync(static_cast<unsigned char*>(c->v) + off, dpitch, v_src, width, width,

@@ -136,6 +136,12 @@ int decode_step(int dtype, const void* q, const void* k, const void* v, float* o
 int launch_init(float* out, float* m, float* l, size_t out_count, size_t m_count,
                 cudaStream_t stream);
 int launch_finalize(float* out, const float* l, size_t rows, int D, cudaStream_t stream);
+// fp32 Q, K and V to fp16 in one launch.
+int launch_narrow_qkv(const float* q, const float* k, const float* v, void* qh, void* kh, void* vh, size_t qn,
+                      size_t kn, cudaStream_t stream);
+// One row per (batch, kv head) of K and V into a cache whose rows are dst_pitch_bytes apart.
+int launch_cache_row(const void* k_src, const void* v_src, void* k_dst, void* v_dst, size_t row_bytes,
+                     size_t dst_pitch_bytes, int rows, cudaStream_t stream);
 // Merge up to 8 online-softmax states of the same rows ([O | m | l] blocks part_stride floats
 // apart, rows * D + rows even multiples of 4 floats so every O stays 16-byte aligned).
 int launch_state_merge(const float* parts, size_t part_stride, int n_parts, size_t rows, int D,

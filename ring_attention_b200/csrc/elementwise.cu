@@ -90,8 +90,8 @@ __device__ inline __nv_bfloat16 cvt_from_float<__nv_bfloat16>(float x) {
 // fp32 -> 16-bit, 8 elements (32 B in, 16 B out) per thread per trip when both pointers are
 // 16-byte aligned (reference: src/attention_step_fp16.cu:217-224).
 template <typename Dst>
-__global__ void narrow_kernel(const float* __restrict__ src, Dst* __restrict__ dst, size_t n,
-                              int vec_ok) {
+__device__ inline void narrow_range(const float* __restrict__ src, Dst* __restrict__ dst, size_t n,
+                                    int vec_ok) {
   const size_t tid = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
   const size_t nth = static_cast<size_t>(gridDim.x) * blockDim.x;
   size_t done = 0;
@@ -118,6 +118,22 @@ __global__ void narrow_kernel(const float* __restrict__ src, Dst* __restrict__ d
     done = n8 * 8;
   }
   for (size_t i = done + tid; i < n; i += nth) dst[i] = cvt_from_float<Dst>(src[i]);
+}
+
+template <typename Dst>
+__global__ void narrow_kernel(const float* __restrict__ src, Dst* __restrict__ dst, size_t n,
+                              int vec_ok) {
+  narrow_range(src, dst, n, vec_ok);
+}
+
+// Q, K and V in one launch (blockIdx.y): three launches of a few microseconds of work each cost
+// the host more than the GPU.
+__global__ void narrow_qkv_kernel(const float* __restrict__ q, __half* __restrict__ qh, size_t qn,
+                                  const float* __restrict__ k, const float* __restrict__ v,
+                                  __half* __restrict__ kh, __half* __restrict__ vh, size_t kn, int vec_ok) {
+  if (blockIdx.y == 0) narrow_range(q, qh, qn, vec_ok);
+  else if (blockIdx.y == 1) narrow_range(k, kh, kn, vec_ok);
+  else narrow_range(v, vh, kn, vec_ok);
 }
 
 // fp16 -> fp32 (reference: src/attention_step_fp16.cu:226-233).
@@ -242,6 +258,18 @@ __global__ void state_merge_kernel(const float* __restrict__ parts, size_t part_
   }
 }
 
+// The K and V rows of one decode token into their cache slots: piece i of (batch, kv head) row
+// blockIdx.y of tensor blockIdx.z. One launch where two strided device copies were two driver calls
+// of several microseconds each on the host.
+template <typename V>
+__global__ void cache_row_kernel(const V* __restrict__ k_src, const V* __restrict__ v_src,
+                                 V* __restrict__ k_dst, V* __restrict__ v_dst, int pieces,
+                                 size_t dst_pitch) {
+  const V* src = (blockIdx.z == 0 ? k_src : v_src) + static_cast<size_t>(blockIdx.y) * pieces;
+  V* dst = (blockIdx.z == 0 ? k_dst : v_dst) + blockIdx.y * dst_pitch;
+  for (int i = threadIdx.x; i < pieces; i += blockDim.x) dst[i] = src[i];
+}
+
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 }  // namespace
@@ -252,6 +280,37 @@ int launch_init(float* out, float* m, float* l, size_t out_count, size_t m_count
   const size_t o_work = vec_ok ? out_count / 4 : out_count;
   const size_t work = o_work > m_count ? o_work : m_count;
   init_kernel<<<grid_for(work, 256), 256, 0, stream>>>(out, m, l, out_count, m_count, vec_ok);
+  RAB_CUDA(cudaGetLastError());
+  return RA_OK;
+}
+
+int launch_narrow_qkv(const float* q, const float* k, const float* v, void* qh, void* kh, void* vh, size_t qn,
+                      size_t kn, cudaStream_t stream) {
+  const size_t most = qn > kn ? qn : kn;
+  if (most == 0) return RA_OK;
+  const int vec = aligned16(q) && aligned16(k) && aligned16(v) && aligned16(qh) && aligned16(kh) && aligned16(vh);
+  narrow_qkv_kernel<<<dim3(grid_for(most / 8 + 1, 256), 3), 256, 0, stream>>>(
+      q, static_cast<__half*>(qh), qn, k, v, static_cast<__half*>(kh), static_cast<__half*>(vh), kn, vec);
+  RAB_CUDA(cudaGetLastError());
+  return RA_OK;
+}
+
+int launch_cache_row(const void* k_src, const void* v_src, void* k_dst, void* v_dst, size_t row_bytes,
+                     size_t dst_pitch_bytes, int rows, cudaStream_t stream) {
+  RAB_REQUIRE(rows <= 65535 && row_bytes % 2 == 0, RA_ERR_INVALID, "cache row: bad sizes");
+  const bool vec = aligned16(k_src) && aligned16(v_src) && aligned16(k_dst) && aligned16(v_dst) &&
+                   row_bytes % 16 == 0 && dst_pitch_bytes % 16 == 0;
+  const dim3 grid(1, rows, 2);
+  if (vec) {
+    cache_row_kernel<uint4><<<grid, 32, 0, stream>>>(
+        static_cast<const uint4*>(k_src), static_cast<const uint4*>(v_src), static_cast<uint4*>(k_dst),
+        static_cast<uint4*>(v_dst), static_cast<int>(row_bytes / 16), dst_pitch_bytes / 16);
+  } else {
+    cache_row_kernel<unsigned short><<<grid, 128, 0, stream>>>(
+        static_cast<const unsigned short*>(k_src), static_cast<const unsigned short*>(v_src),
+        static_cast<unsigned short*>(k_dst), static_cast<unsigned short*>(v_dst),
+        static_cast<int>(row_bytes / 2), dst_pitch_bytes / 2);
+  }
   RAB_CUDA(cudaGetLastError());
   return RA_OK;
 }

@@ -1,5 +1,6 @@
 """GPU parity of the forms that a call's shape selects: the key-split form of the step kernels (the
-blocks of a cluster share a query block's keys) and the scaled fp16 splitting of the fp32 step.
+blocks of a cluster share a query block's keys), the scaled fp16 splitting of the fp32 step and the
+one-launch cache append.
 
 Tolerances are those of the other step and decode tests: 1e-5 for fp32 and 1e-3 / 8e-3 for fp16 /
 bf16 P, absolute and relative, against the oracle on the same rounded inputs. Where values are
@@ -119,3 +120,15 @@ def test_fp32_step_passes_on_nan_and_infinity_of_visible_values_only():
     want = oracle.cpu_attention(q[:, :, :128], k[:, :, :128], v[:, :, :128], True)[0, 0]
     assert_close(got[:128], want, 1e-5, 1e-5, "rows whose key tiles are finite")
     assert not np.isfinite(got[160, 7]) and np.isnan(got[195]).all()
+
+
+@pytest.mark.parametrize("dtype,D", [(torch.float32, 1), (torch.float16, 3), (torch.bfloat16, 8), (torch.float16, 128)])
+def test_cache_append_of_any_row_size_and_alignment(dtype, D):
+    B, kvH, s_max = 2, 3, 5
+    cache = api.DeviceKVCache(B, kvH, s_max, D, dtype)
+    flat = torch.randn(2 * s_max * B * kvH * D + 1, device="cuda").to(dtype)[1:]  # not 16-byte aligned
+    rows = flat.view(2, s_max, B, kvH, 1, D)
+    for t in range(s_max):
+        cache.append(rows[0, t], rows[1, t])
+    assert torch.equal(cache.k_view(), rows[0, :, :, :, 0].permute(1, 2, 0, 3))
+    assert torch.equal(cache.v_view(), rows[1, :, :, :, 0].permute(1, 2, 0, 3))
