@@ -3,28 +3,33 @@
 //
 // What bounds it: every K and V row of the local shard is read exactly once from HBM, so
 // the kernels are built around bytes in flight, not arithmetic.
-//  - One block per (split, KV head, batch row) serves ALL query heads that map to that KV
+//  - A block serves ALL query heads that map to that KV
 //    head (h % kv_heads), so grouped-query attention reads each cached row once instead of
 //    once per query head (the reference re-reads it per head, src/attention_decode.cu:88).
-//  - The split count is chosen so the grid is about three waves of the SM count.
+//  - How the cached rows are dealt to blocks: see Deal.
 //  - decode_mma_kernel (fp16 / bf16 caches, head_dim >= 64) is the fast path: K/V rows stream
-//    through a 5-8-stage shared-memory ring of 64-key stages filled with 16-byte cp.async
+//    through a 3-6-stage shared-memory ring of 64-key stages filled with 16-byte cp.async
 //    copies (fully coalesced, XOR-swizzled), and per 16-key block a warp does both
 //    contractions on mma.sync m16n8k16 with the up to 16 grouped query heads as M rows
 //    (ldmatrix / ldmatrix.trans), online softmax with warp-shuffle row maxima and a lazy
 //    rescale; warps are merged through shared memory. The tensor cores are there to get under
 //    the instruction-issue bound (about 5 instead of about 80 warp instructions per cached
-//    row), the kernel is bound by the copy (0.87 of the measured HBM copy bandwidth).
+//    row), the kernel is bound by the copy. Two blocks of 96 KB of ring per SM: the loads of one
+//    run on through the barriers and the arithmetic of the other (B4 H32/kvH8 D128, 262144 rows:
+//    one block of 160 KB 799 us, two of 96 KB 591-635 us = 6.8-7.25 TB/s).
 //  - decode_split_kernel (fp32 caches, head_dim 32) is the SIMT form of the same structure
 //    with a 4-stage ring: a group of `LPR` lanes owns a row, each lane keeps its slice of q
 //    (pre-scaled) for every head of the group, the dot product finishes with log2(LPR)
 //    shuffles, each lane group carries its own running (m, l, out), and a warp-shuffle
 //    log-sum-exp merge plus one shared-memory pass combine lane groups and warps.
-// Partials (m, l, out) per (split, batch, head) go to a workspace; a second tiny kernel
-// folds them into the persistent state (src/attention_decode.cu:228-277 does the same for
-// its fixed 8 splits).
+// Partials (m, l, out) go to a workspace and a second small kernel folds them into the persistent
+// state (src/attention_decode.cu:228-277 does the same for its fixed 8 splits); short calls merge
+// them inside a cluster instead.
 #include <algorithm>
+#include <atomic>
+#include <cmath>
 #include <mutex>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -97,44 +102,240 @@ struct Piece<__nv_bfloat16> {
   }
 };
 
-template <typename T, int D>
+template <typename T, int D, int GB = 1>
 struct DecodeCfg {
   static constexpr int kRowBytes = D * static_cast<int>(sizeof(T));
   static constexpr int kPieces = kRowBytes / 16;  // 16-byte pieces per row
-  // lanes per row: every lane owns 1..4 pieces
-  static constexpr int kLPR = kPieces >= 32 ? 16 : (kPieces >= 8 ? 8 : 4);
+  // Lanes per row: every lane owns 1..4 pieces. A lane keeps its slice of q and of the accumulator
+  // for GB heads; where those would take 128 registers and leave an SM a single block (eight heads,
+  // or four at 1 KB rows), twice the lanes share a row (B1 H64/kvH8 D128, 45344 rows: 248 -> 133 us,
+  // 174 with the fixed splits and one block per SM that this replaces).
+  static constexpr int kLPRNarrow = kPieces >= 32 ? 16 : (kPieces >= 8 ? 8 : 4);
+  static constexpr bool kWide =
+      GB * (kPieces / kLPRNarrow) * Piece<T>::kElems >= 64 && 2 * kLPRNarrow <= kPieces;
+  static constexpr int kLPR = kWide ? 2 * kLPRNarrow : kLPRNarrow;
   static constexpr int kVPT = kPieces / kLPR;               // pieces per lane
   static constexpr int kEPL = kVPT * Piece<T>::kElems;      // elements per lane
   static constexpr int kRowsPerWarpStep = 32 / kLPR;
   static constexpr int kRowsPerStep = kWarps * kRowsPerWarpStep;
-  static constexpr int kSteps =
-      (8192 / (kRowsPerStep * kRowBytes)) > 0 ? (8192 / (kRowsPerStep * kRowBytes)) : 1;
+  static constexpr int steps_for(int rows) {  // 8 KB per tensor and stage
+    return 8192 / (rows * kRowBytes) > 0 ? 8192 / (rows * kRowBytes) : 1;
+  }
+  static constexpr int kSteps = steps_for(kRowsPerStep);
   static constexpr int kRowsPerStage = kRowsPerStep * kSteps;
+  static constexpr int kPlanRows =  // see fixed_splits
+      kWarps * (32 / kLPRNarrow) * steps_for(kWarps * (32 / kLPRNarrow));
   static constexpr int kStageBytes = kRowsPerStage * kRowBytes;  // per tensor
   static constexpr int kSmemBytes = 2 * kStages * kStageBytes;
 };
 
-// grid = (n_split, kv_heads * head_batches, batch). GB = query heads handled per block.
-template <typename T, int D, int GB>
+// ---- how the keys are dealt to blocks ----------------------------------------------------
+//
+// A group is one (batch row, KV head, batch of query heads); its visible rows are `stages` ring
+// stages. Three forms of the same kernels:
+//  * balanced: one block per resident slot of the GPU, block i takes the stages
+//    [i T / G, (i + 1) T / G) of all T = groups * stages, whatever groups they belong to (one or
+//    two, more when groups are short). Every block moves the same bytes, so there is no last wave:
+//    with a fixed number of splits per group the long-context shape (B4 kvH8, 262144 rows) made
+//    448 blocks for 148 SMs, three waves and four blocks. A block leaves one partial per
+//    group it touches in the workspace and a second kernel folds them. Measured with 160 KB rings
+//    it made no difference by itself (799 against 769 us); with two blocks per SM 1, 3 or 6 times as
+//    many blocks were no faster either, and the B1 H8 D128 fp32 call on 16384 rows slower (37 us
+//    against 31).
+//  * fixed: `splits` blocks per group, about three waves, partials and fold as above. For the
+//    kernel whose registers leave room for one block per SM only, where the loop over shares
+//    gains them nothing (eight fp32 heads of 256).
+//  * cluster: the blocks of a cluster take equal shares of ONE group and merge
+//    their partials through distributed shared memory into the state. No workspace and no second
+//    launch: for calls that one wave finishes in a few microseconds (B1 H32/kvH8 D128 fp16 on 1061
+//    rows 11.5 -> 9.3 us per call, most of it host time).
+enum DealForm { kBalanced, kFixed, kCluster };
+struct Deal {
+  int stages;          // per group
+  int groups;
+  int head_batches;
+  int cap;             // partial slots per (batch, head) row
+  int splits;          // fixed form: blocks per group
+  int ring;            // ring slots (no more than a block's stages)
+  unsigned flags;      // cluster form: RA_STEP_FRESH / RA_STEP_FINALIZE
+};
+// The block that owns stage x of the balanced form: the largest i with floor(i T / G) <= x.
+__host__ __device__ inline int deal_owner(long long x, long long total, int ctas) {
+  return static_cast<int>(((x + 1) * ctas - 1) / total);
+}
+
+__device__ inline unsigned cluster_rank() {
+  unsigned r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ inline void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ inline float ld_cluster(const float* p, unsigned rank) {
+  unsigned addr;
+  float v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+               : "=r"(addr)
+               : "r"(static_cast<unsigned>(__cvta_generic_to_shared(p))), "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr));
+  return v;
+}
+
+constexpr int kMaxCluster = 8;
+constexpr double kFoldUs = 3.0, kMergeUs = 1.0;  // see make_plan
+
+// End of a block's share of a group: the warps' partials (red_*: [warps][ROWS], red_o [..][D]) of
+// the ROWS query heads h = kvh + kvH * (hb * ROWS + r) become the block's, which goes to slot
+// `part` of the workspace or is merged over the cluster and folded into the state.
+template <int ROWS, int D, int NWARPS, DealForm kForm>
+__device__ inline void finish_group(float* red_m, float* red_l, float* red_o, int b, int kvh, int hb, int H,
+                                    int kvH, int part, const Deal& deal, float* __restrict__ Mp,
+                                    float* __restrict__ Lp, float* __restrict__ Op) {
+  constexpr int kThr = NWARPS * 32;
+  const int tid = threadIdx.x;
+  const int first = kvh + kvH * hb * ROWS;
+  const int live = first < H ? min(ROWS, (H - first + kvH - 1) / kvH) : 0;
+  float* blk_m = red_o + NWARPS * ROWS * D;  // [ROWS], [ROWS], [ROWS][D]: cluster form
+  float* blk_l = blk_m + ROWS;
+  float* blk_o = blk_l + ROWS;
+  for (int idx = tid; idx < live * D; idx += kThr) {
+    const int r = idx / D;
+    const int d = idx - r * D;
+    float m_n = -INFINITY;
+#pragma unroll
+    for (int w = 0; w < NWARPS; ++w) m_n = fmaxf(m_n, red_m[w * ROWS + r]);
+    float o_acc = 0.f, l_acc = 0.f;
+#pragma unroll
+    for (int w = 0; w < NWARPS; ++w) {
+      const float mw = red_m[w * ROWS + r];
+      const float sc = (mw == -INFINITY) ? 0.f : ex2(mw - m_n);
+      o_acc += sc * red_o[(w * ROWS + r) * D + d];
+      l_acc += sc * red_l[w * ROWS + r];
+    }
+    // natural-log units, the unit of the persistent state
+    if constexpr (kForm == kCluster) {
+      blk_o[idx] = o_acc;
+      if (d == 0) {
+        blk_m[r] = m_n * kLn2;
+        blk_l[r] = l_acc;
+      }
+    } else {
+      const size_t slot = (static_cast<size_t>(b) * H + first + kvH * r) * deal.cap + part;
+      Op[slot * D + d] = o_acc;
+      if (d == 0) {
+        Mp[slot] = m_n * kLn2;
+        Lp[slot] = l_acc;
+      }
+    }
+  }
+  if constexpr (kForm == kCluster) {
+    // Mp / Lp / Op are the state itself here
+    const bool fresh = (deal.flags & RA_STEP_FRESH) != 0, finalize = (deal.flags & RA_STEP_FINALIZE) != 0;
+    const int n = static_cast<int>(gridDim.x), rank = static_cast<int>(cluster_rank());
+    cluster_barrier();  // every block's partial is staged
+    for (int idx = rank * kThr + tid; idx < live * D; idx += n * kThr) {
+      const int r = idx / D;
+      const size_t row = static_cast<size_t>(b) * H + first + kvH * r;
+      float mp[kMaxCluster], lp[kMaxCluster], op[kMaxCluster];
+#pragma unroll
+      for (int i = 0; i < kMaxCluster; ++i) {
+        mp[i] = i < n ? ld_cluster(blk_m + r, i) : -INFINITY;
+        lp[i] = i < n ? ld_cluster(blk_l + r, i) : 0.f;
+        op[i] = i < n ? ld_cluster(blk_o + idx, i) : 0.f;
+      }
+      const float m_old = fresh ? -INFINITY : Mp[row];
+      float m_n = m_old;
+#pragma unroll
+      for (int i = 0; i < kMaxCluster; ++i) m_n = fmaxf(m_n, mp[i]);
+      if (m_n == -INFINITY) {
+        // nothing visible anywhere: the state stays as it is (or is written empty)
+        if (fresh || finalize) Op[row * D + (idx - r * D)] = 0.f;
+        continue;
+      }
+      const float a = (m_old == -INFINITY) ? 0.f : expf(m_old - m_n);
+      float o_acc = (m_old == -INFINITY) ? 0.f : a * Op[row * D + (idx - r * D)];
+      float l_acc = (m_old == -INFINITY) ? 0.f : a * Lp[row];
+#pragma unroll
+      for (int i = 0; i < kMaxCluster; ++i) {
+        const float sc = (mp[i] == -INFINITY) ? 0.f : expf(mp[i] - m_n);
+        o_acc += sc * op[i];
+        l_acc += sc * lp[i];
+      }
+      if (finalize) o_acc *= l_acc > 0.f ? 1.f / l_acc : 0.f;
+      Op[row * D + (idx - r * D)] = o_acc;
+    }
+    // (m, l) of a row once every block has read the old ones and nobody needs this block any more
+    float m_n = -INFINITY, l_acc = 0.f;
+    const bool owner = rank == 0 && tid < live;
+    size_t row = 0;
+    if (owner) {
+      row = static_cast<size_t>(b) * H + first + kvH * tid;
+      const float m_old = fresh ? -INFINITY : Mp[row];
+      m_n = m_old;
+      for (int i = 0; i < n; ++i) m_n = fmaxf(m_n, ld_cluster(blk_m + tid, i));
+      l_acc = (m_old == -INFINITY) ? 0.f : expf(m_old - m_n) * Lp[row];
+      for (int i = 0; i < n; ++i) {
+        const float mi = ld_cluster(blk_m + tid, i);
+        if (mi > -INFINITY) l_acc += expf(mi - m_n) * ld_cluster(blk_l + tid, i);
+      }
+    }
+    cluster_barrier();
+    if (owner && (m_n > -INFINITY || m_n != m_n || fresh)) {
+      Mp[row] = m_n;
+      Lp[row] = l_acc;
+    }
+  }
+}
+
+// A block's shares around both kernels' bodies: stages [stage_beg, stage_end) of the group
+// (b, kvh, hb), partial slot `part`. Only the balanced form loops.
+#define RAB_DECODE_LOOP_BEGIN                                                                      \
+  constexpr bool kLoop = kForm == kBalanced;                                                       \
+  const int n_share = kForm == kFixed ? deal.splits : static_cast<int>(gridDim.x);                 \
+  const int i_share = static_cast<int>(kForm == kFixed ? blockIdx.x % deal.splits : blockIdx.x);   \
+  const long long total = static_cast<long long>(deal.groups) * deal.stages;                       \
+  long long at = kLoop ? total * i_share / n_share : 0;                                            \
+  const long long at_end = kLoop ? total * (i_share + 1ll) / n_share : 1;                          \
+  if (kForm != kCluster) asm volatile("griddepcontrol.launch_dependents;");                        \
+  while (at < at_end) {                                                                            \
+    const int group = static_cast<int>(kLoop             ? at / deal.stages                        \
+                                       : kForm == kFixed ? blockIdx.x / deal.splits                \
+                                                         : blockIdx.y);                            \
+    const int stage_beg =                                                                          \
+        kLoop ? static_cast<int>(at - static_cast<long long>(group) * deal.stages)                 \
+              : static_cast<int>(static_cast<long long>(deal.stages) * i_share / n_share);         \
+    const int stage_end =                                                                          \
+        kLoop ? static_cast<int>(min(static_cast<long long>(deal.stages), stage_beg + (at_end - at))) \
+              : static_cast<int>(static_cast<long long>(deal.stages) * (i_share + 1ll) / n_share); \
+    const int part =                                                                               \
+        kLoop ? i_share - deal_owner(static_cast<long long>(group) * deal.stages, total, n_share)  \
+              : i_share;                                                                           \
+    at += kLoop ? stage_end - stage_beg : 1;                                                       \
+    const int hb = group % deal.head_batches;                                                      \
+    const int kvh = (group / deal.head_batches) % kvH;                                             \
+    const int b = group / (deal.head_batches * kvH);
+#define RAB_DECODE_LOOP_END                                                                        \
+    if (kLoop) __syncthreads(); /* the ring is free again */                                       \
+  }
+
+// GB = query heads handled per block. Grid: see Deal.
+template <typename T, int D, int GB, DealForm kForm>
 __global__ void __launch_bounds__(kThreads)
     decode_split_kernel(const T* __restrict__ Q, const T* __restrict__ K, const T* __restrict__ V,
-                        float* __restrict__ Mp, float* __restrict__ Lp, float* __restrict__ Op,
-                        int B, int H, int kvH, int sk_eff, long long kv_head_stride,
-                        int rows_per_split, int head_batches, float scale_log2) {
-  using C = DecodeCfg<T, D>;
+                        float* __restrict__ Mp, float* __restrict__ Lp, float* __restrict__ Op, int H,
+                        int kvH, int sk_eff, long long kv_head_stride, const Deal deal, float scale_log2) {
+  using C = DecodeCfg<T, D, GB>;
   extern __shared__ __align__(16) unsigned char smem[];
   unsigned char* k_ring = smem;
-  unsigned char* v_ring = smem + kStages * C::kStageBytes;
+  unsigned char* v_ring = smem + deal.ring * C::kStageBytes;
 
   const int tid = threadIdx.x;
   const int lane = tid & 31;
   const int warp = tid >> 5;
   const int lr = lane % C::kLPR;       // lane within the row group
   const int grp = lane / C::kLPR;      // row group within the warp
-  const int split = blockIdx.x;
-  const int kvh = blockIdx.y / head_batches;
-  const int hb = blockIdx.y % head_batches;
-  const int b = blockIdx.z;
+  RAB_DECODE_LOOP_BEGIN
 
   // Query heads of this block: h = kvh + kvH * (hb * GB + g), while h < H.
   float q_reg[GB][C::kEPL];
@@ -165,10 +366,10 @@ __global__ void __launch_bounds__(kThreads)
     }
   }
 
-  const int row_begin = split * rows_per_split;
-  const int row_end = min(sk_eff, row_begin + rows_per_split);
-  const int n_rows = max(0, row_end - row_begin);
-  const int n_stages = (n_rows + C::kRowsPerStage - 1) / C::kRowsPerStage;
+  const int row_begin = stage_beg * C::kRowsPerStage;
+  const int row_end = min(static_cast<long long>(sk_eff), static_cast<long long>(stage_end) * C::kRowsPerStage);
+  const int n_rows = row_end - row_begin;
+  const int n_stages = stage_end - stage_beg;
   const unsigned char* k_base = reinterpret_cast<const unsigned char*>(
       K + (static_cast<size_t>(b) * kvH + kvh) * kv_head_stride);
   const unsigned char* v_base = reinterpret_cast<const unsigned char*>(
@@ -294,29 +495,8 @@ __global__ void __launch_bounds__(kThreads)
     }
   }
   __syncthreads();
-  for (int idx = tid; idx < GB * D; idx += kThreads) {
-    const int g = idx / D;
-    const int d = idx - g * D;
-    const int h = kvh + kvH * (hb * GB + g);
-    if (h >= H) continue;
-    float m_n = -INFINITY;
-#pragma unroll
-    for (int w = 0; w < kWarps; ++w) m_n = fmaxf(m_n, red_m[w * GB + g]);
-    float o_acc = 0.f, l_acc = 0.f;
-#pragma unroll
-    for (int w = 0; w < kWarps; ++w) {
-      const float mw = red_m[w * GB + g];
-      const float sc = (mw == -INFINITY) ? 0.f : ex2(mw - m_n);
-      o_acc += sc * red_o[(w * GB + g) * D + d];
-      l_acc += sc * red_l[w * GB + g];
-    }
-    const size_t prow = (static_cast<size_t>(split) * B + b) * H + h;
-    Op[prow * D + d] = o_acc;
-    if (d == 0) {
-      Mp[prow] = m_n * kLn2;  // back to natural-log units, the unit of the persistent state
-      Lp[prow] = l_acc;
-    }
-  }
+  finish_group<GB, D, kWarps, kForm>(red_m, red_l, red_o, b, kvh, hb, H, kvH, part, deal, Mp, Lp, Op);
+  RAB_DECODE_LOOP_END
 }
 
 // ---- tensor-core variant for 16-bit caches ---------------------------------------------
@@ -329,10 +509,7 @@ __global__ void __launch_bounds__(kThreads)
 // K/V rows go to shared memory with the same 16-byte cp.async copies, but each 16-byte
 // piece c of row r is stored at piece c ^ (r & 7), so that the ldmatrix reads (8 rows at a
 // fixed column) touch all banks once.
-constexpr int kMmaWarps = 4;
-constexpr int kMmaThreads = kMmaWarps * 32;
 constexpr int kMmaKeysPerWarp = 16;
-constexpr int kMmaStageRows = kMmaWarps * kMmaKeysPerWarp;  // 64 keys per stage
 
 template <typename T>
 __device__ inline void mma16816(float (&c)[4], const unsigned (&a)[4], unsigned b0, unsigned b1);
@@ -381,34 +558,34 @@ template <int D>
 struct MmaCfg {
   static constexpr int kRowBytes = D * 2;
   static constexpr int kPieces = kRowBytes / 16;
-  static constexpr int kStageBytes = kMmaStageRows * kRowBytes;  // per tensor
-  static constexpr int kStagesRaw = (160 * 1024) / (2 * kStageBytes);
-  static constexpr int kStages = kStagesRaw > 8 ? 8 : (kStagesRaw < 3 ? 3 : kStagesRaw);
+  // head_dim 256: two warps and 32-key stages, so that three stages are 96 KB as well and two
+  // blocks fit an SM (B3 kvH4 bf16, 34876 rows: 86 us with four warps and 192 KB, 74 so)
+  static constexpr int kWarps = D == 256 ? 2 : 4;
+  static constexpr int kThreads = kWarps * 32;
+  static constexpr int kStageRows = kWarps * kMmaKeysPerWarp;
+  static constexpr int kStageBytes = kStageRows * kRowBytes;  // per tensor
+  static constexpr int kStages = (96 * 1024) / (2 * kStageBytes);
   static constexpr int kSmemBytes = 2 * kStages * kStageBytes;
 };
 
-// grid = (n_split, kv_heads * head_batches, batch); a block serves up to 16 query heads of one
-// KV head (rows of the MMA tile; row r is head kvh + kv_heads * (16 * hb + r)).
-template <typename T, int D>
-__global__ void __launch_bounds__(kMmaThreads)
+// A block serves up to 16 query heads of one KV head (rows of the MMA tile; row r is head
+// kvh + kv_heads * (16 * hb + r)). Grid: see Deal.
+template <typename T, int D, DealForm kForm>
+__global__ void __launch_bounds__(MmaCfg<D>::kThreads)
     decode_mma_kernel(const T* __restrict__ Q, const T* __restrict__ K, const T* __restrict__ V,
-                      float* __restrict__ Mp, float* __restrict__ Lp, float* __restrict__ Op, int B,
-                      int H, int kvH, int sk_eff, long long kv_head_stride, int rows_per_split,
-                      int head_batches, float scale_log2) {
+                      float* __restrict__ Mp, float* __restrict__ Lp, float* __restrict__ Op, int H,
+                      int kvH, int sk_eff, long long kv_head_stride, const Deal deal, float scale_log2) {
   using C = MmaCfg<D>;
-  extern __shared__ __align__(128) unsigned char smem[];
+  extern __shared__ __align__(16) unsigned char smem[];
   unsigned char* k_ring = smem;
-  unsigned char* v_ring = smem + C::kStages * C::kStageBytes;
+  unsigned char* v_ring = smem + deal.ring * C::kStageBytes;
 
   const int tid = threadIdx.x;
   const int lane = tid & 31;
   const int warp = tid >> 5;
   const int g = lane >> 2;   // fragment row (and row + 8)
   const int tq = lane & 3;   // fragment column pair
-  const int split = blockIdx.x;
-  const int kvh = blockIdx.y / head_batches;
-  const int hb = blockIdx.y % head_batches;
-  const int b = blockIdx.z;
+  RAB_DECODE_LOOP_BEGIN
 
   // Q as A fragments: reg0 (row g, k 2tq..), reg1 (row g+8, same k), reg2 / reg3 the same at k+8.
   const int h0 = kvh + kvH * (hb * 16 + g);
@@ -431,10 +608,10 @@ __global__ void __launch_bounds__(kMmaThreads)
   float m_run[2] = {-INFINITY, -INFINITY};
   float l_run[2] = {0.f, 0.f};  // this lane's share of the row sums (its four columns per block)
 
-  const int row_begin = split * rows_per_split;
-  const int row_end = min(sk_eff, row_begin + rows_per_split);
-  const int n_rows = max(0, row_end - row_begin);
-  const int n_stages = (n_rows + kMmaStageRows - 1) / kMmaStageRows;
+  const int row_begin = stage_beg * C::kStageRows;
+  const int row_end = min(static_cast<long long>(sk_eff), static_cast<long long>(stage_end) * C::kStageRows);
+  const int n_rows = row_end - row_begin;
+  const int n_stages = stage_end - stage_beg;
   const unsigned char* k_base = reinterpret_cast<const unsigned char*>(
       K + (static_cast<size_t>(b) * kvH + kvh) * kv_head_stride);
   const unsigned char* v_base = reinterpret_cast<const unsigned char*>(
@@ -443,10 +620,10 @@ __global__ void __launch_bounds__(kMmaThreads)
   auto issue = [&](int st) {
     if (st < n_stages) {
       const int slot = st % C::kStages;
-      const long long first = static_cast<long long>(row_begin) + st * kMmaStageRows;
+      const long long first = static_cast<long long>(row_begin) + st * C::kStageRows;
       const long long valid_bytes = (static_cast<long long>(row_end) - first) * C::kRowBytes;
       const size_t goff = static_cast<size_t>(first) * C::kRowBytes;
-      for (int p = tid; p < C::kStageBytes / 16; p += kMmaThreads) {
+      for (int p = tid; p < C::kStageBytes / 16; p += C::kThreads) {
         const int r = p / C::kPieces;
         const int c = p - r * C::kPieces;
         const long long off = static_cast<long long>(p) * 16;
@@ -473,7 +650,7 @@ __global__ void __launch_bounds__(kMmaThreads)
     __syncthreads();
     issue(st + C::kStages - 1);
     const int slot = st % C::kStages;
-    const int n_valid = n_rows - (st * kMmaStageRows + key0);  // valid keys of this warp's block
+    const int n_valid = n_rows - (st * C::kStageRows + key0);  // valid keys of this warp's block
     if (n_valid <= 0) continue;
     const unsigned kt = static_cast<unsigned>(__cvta_generic_to_shared(k_ring + slot * C::kStageBytes));
     const unsigned vt = static_cast<unsigned>(__cvta_generic_to_shared(v_ring + slot * C::kStageBytes));
@@ -551,8 +728,8 @@ __global__ void __launch_bounds__(kMmaThreads)
   }
   __syncthreads();
   float* red_m = reinterpret_cast<float*>(smem);  // [warps][16]
-  float* red_l = red_m + kMmaWarps * 16;          // [warps][16]
-  float* red_o = red_l + kMmaWarps * 16;          // [warps][16][D]
+  float* red_l = red_m + C::kWarps * 16;          // [warps][16]
+  float* red_o = red_l + C::kWarps * 16;          // [warps][16][D]
   if (tq == 0) {
     red_m[warp * 16 + g] = m_run[0];
     red_m[warp * 16 + g + 8] = m_run[1];
@@ -569,48 +746,53 @@ __global__ void __launch_bounds__(kMmaThreads)
     r1[1] = o[n][3];
   }
   __syncthreads();
-  for (int idx = tid; idx < 16 * D; idx += kMmaThreads) {
-    const int r = idx / D;
-    const int d = idx - r * D;
-    const int h = kvh + kvH * (hb * 16 + r);
-    if (h >= H) continue;
-    float m_n = -INFINITY;
-#pragma unroll
-    for (int w = 0; w < kMmaWarps; ++w) m_n = fmaxf(m_n, red_m[w * 16 + r]);
-    float o_acc = 0.f, l_acc = 0.f;
-#pragma unroll
-    for (int w = 0; w < kMmaWarps; ++w) {
-      const float mw = red_m[w * 16 + r];
-      const float sc = (mw == -INFINITY) ? 0.f : ex2(mw - m_n);
-      o_acc += sc * red_o[(w * 16 + r) * D + d];
-      l_acc += sc * red_l[w * 16 + r];
-    }
-    const size_t prow = (static_cast<size_t>(split) * B + b) * H + h;
-    Op[prow * D + d] = o_acc;
-    if (d == 0) {
-      Mp[prow] = m_n * kLn2;
-      Lp[prow] = l_acc;
-    }
-  }
+  finish_group<16, D, C::kWarps, kForm>(red_m, red_l, red_o, b, kvh, hb, H, kvH, part, deal, Mp, Lp, Op);
+  RAB_DECODE_LOOP_END
 }
 
-// Fold n_split partials into the persistent (out, m, l). grid = (H, B), block = D threads.
+#undef RAB_DECODE_LOOP_BEGIN
+#undef RAB_DECODE_LOOP_END
+
+// Fold the partials of the balanced and fixed forms into the persistent (out, m, l). grid = (H, B), block =
+// D x kFoldThreads / D threads: the partials are dealt to the thread groups (a single group walked up
+// to 57 partials one after the other, twice: 8 of the 36 us of the B1 H8 D128 fp32 call on 16384
+// rows) and (m, l) are read by lanes. Launched while the split kernel still runs (programmatic
+// dependent launch); everything it reads comes after griddepcontrol.wait.
 // RA_STEP_FRESH: the state is known to be empty (it is written, never read, which saves the
 // caller an init launch); RA_STEP_FINALIZE: divide by l after folding (saves the finalize
 // launch).
-__global__ void decode_reduce_kernel(const float* __restrict__ Mp, const float* __restrict__ Lp,
-                                     const float* __restrict__ Op, float* __restrict__ M,
-                                     float* __restrict__ L, float* __restrict__ O, int B, int H,
-                                     int D, int n_split, unsigned flags) {
-  const int h = blockIdx.x, b = blockIdx.y, d = threadIdx.x;
+constexpr int kFoldThreads = 512;
+__global__ void __launch_bounds__(kFoldThreads)
+    decode_reduce_kernel(const float* __restrict__ Mp, const float* __restrict__ Lp,
+                         const float* __restrict__ Op, float* __restrict__ M, float* __restrict__ L,
+                         float* __restrict__ O, int H, int kvH, int D, int head_rows, int ctas,
+                         const Deal deal) {
+  __shared__ float sc[kMaxSplits];
+  __shared__ float part_o[kFoldThreads];
+  const int h = blockIdx.x, b = blockIdx.y;
+  const int d = threadIdx.x % D, grp = threadIdx.x / D, n_grp = blockDim.x / D;
+  const int lane = threadIdx.x & 31;
   const size_t row = static_cast<size_t>(b) * H + h;
-  const bool fresh = (flags & RA_STEP_FRESH) != 0, finalize = (flags & RA_STEP_FINALIZE) != 0;
+  const bool fresh = (deal.flags & RA_STEP_FRESH) != 0, finalize = (deal.flags & RA_STEP_FINALIZE) != 0;
+  const long long total = static_cast<long long>(deal.groups) * deal.stages;
+  const long long group =
+      (static_cast<long long>(b) * kvH + h % kvH) * deal.head_batches + (h / kvH) / head_rows;
+  const int n = deal.splits > 0 ? deal.splits
+                                : deal_owner((group + 1) * deal.stages - 1, total, ctas) -
+                                      deal_owner(group * deal.stages, total, ctas) + 1;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const float* mp = Mp + row * deal.cap;
+  const float* lp = Lp + row * deal.cap;
+  const float* op = Op + row * deal.cap * D;
+  // every warp works out the same maximum and sum; the scales go to shared memory once
   const float m_old = fresh ? -INFINITY : M[row];
   float m_n = m_old;
-  for (int s = 0; s < n_split; ++s) m_n = fmaxf(m_n, Mp[(static_cast<size_t>(s) * B + b) * H + h]);
+  for (int s = lane; s < n; s += 32) m_n = fmaxf(m_n, mp[s]);
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) m_n = fmaxf(m_n, __shfl_xor_sync(0xffffffffu, m_n, off));
   if (m_n == -INFINITY) {
     // nothing visible anywhere: the state stays as it is (or is written empty)
-    if (fresh || finalize) {
+    if ((fresh || finalize) && grp == 0) {
       O[row * D + d] = 0.f;
       if (fresh && d == 0) {
         M[row] = -INFINITY;
@@ -619,31 +801,33 @@ __global__ void decode_reduce_kernel(const float* __restrict__ Mp, const float* 
     }
     return;
   }
-  const float a = (m_old == -INFINITY) ? 0.f : expf(m_old - m_n);
-  float o_acc = (m_old == -INFINITY) ? 0.f : a * O[row * D + d];
-  float l_acc = (m_old == -INFINITY) ? 0.f : a * L[row];
-  for (int s = 0; s < n_split; ++s) {
-    const size_t prow = (static_cast<size_t>(s) * B + b) * H + h;
-    const float ms = Mp[prow];
-    const float sc = (ms == -INFINITY) ? 0.f : expf(ms - m_n);
-    o_acc += sc * Op[prow * D + d];
-    l_acc += sc * Lp[prow];
+  float l_acc = 0.f;
+  for (int s = lane; s < n; s += 32) {
+    const float ms = mp[s];
+    const float f = (ms == -INFINITY) ? 0.f : expf(ms - m_n);
+    l_acc += f * lp[s];
+    if (threadIdx.x < 32) sc[s] = f;
   }
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) l_acc += __shfl_xor_sync(0xffffffffu, l_acc, off);
+  const float a = (m_old == -INFINITY) ? 0.f : expf(m_old - m_n);
+  if (m_old > -INFINITY) l_acc += a * L[row];
+  __syncthreads();
+  float o_acc = 0.f;
+#pragma unroll 4
+  for (int s = grp; s < n; s += n_grp) o_acc += sc[s] * op[static_cast<size_t>(s) * D + d];
+  part_o[threadIdx.x] = o_acc;
+  __syncthreads();
+  if (grp > 0) return;
+  for (int i = 1; i < n_grp; ++i) o_acc += part_o[i * D + d];
+  if (m_old > -INFINITY) o_acc += a * O[row * D + d];
   if (finalize) o_acc *= l_acc > 0.f ? 1.f / l_acc : 0.f;
   O[row * D + d] = o_acc;
-  __syncthreads();  // every thread has read M/L before thread 0 overwrites them
-  if (d == 0) {
+  if (d == 0) {  // every thread has read M / L: two block barriers ago
     M[row] = m_n;
     L[row] = l_acc;
   }
 }
-
-struct Plan {
-  int n_split;
-  int rows_per_split;
-  int gb;
-  int head_batches;
-};
 
 int sm_count() {
   int dev = 0, v = 148;
@@ -652,21 +836,51 @@ int sm_count() {
   return v > 0 ? v : 148;
 }
 
-Plan make_plan(int B, int H, int kvH, int sk_eff, int rows_per_stage, int sms,
-               int split_cap = kMaxSplits) {
-  Plan p;
-  const int group = (H + kvH - 1) / kvH;  // query heads per KV head (largest group)
-  p.gb = group > 4 ? 8 : (group > 2 ? 4 : (group > 1 ? 2 : 1));  // smallest of 1/2/4/8 that fits
-  p.head_batches = (group + p.gb - 1) / p.gb;
-  const int blocks_per_split = B * kvH * p.head_batches;
-  int want = (3 * sms + blocks_per_split - 1) / blocks_per_split;
-  const int max_by_rows = std::max(1, sk_eff / (2 * rows_per_stage));
-  want = std::max(1, std::min(std::min(want, max_by_rows), split_cap));
-  int rps = (sk_eff + want - 1) / want;
-  rps = ((rps + rows_per_stage - 1) / rows_per_stage) * rows_per_stage;
-  if (rps < rows_per_stage) rps = rows_per_stage;
-  p.rows_per_split = rps;
-  p.n_split = std::max(1, (sk_eff + rps - 1) / rps);
+struct DecodePlan {
+  int cluster;  // > 0: the cluster form with this many blocks per group
+  int ctas;     // balanced form: blocks
+  Deal deal;
+};
+
+// Which form, and how many blocks. `per_sm`: resident blocks per SM; `cap`: partial slots per row
+// that the workspace holds. Estimates in microseconds from a stage's bytes: 6.5 TB/s for the whole
+// GPU, 0.1 MB/us for one SM, and what the fold (launch and kernel) or the merge adds.
+DecodePlan make_plan(int groups, int stages, size_t stage_bytes, int per_sm, int cap, int ring_max,
+                     int fixed) {
+  DecodePlan p;
+  const int sms = sm_count();
+  const double total = static_cast<double>(groups) * stages;
+  const double whole = total * stage_bytes / 6.5e6, one = stage_bytes / 0.1e6;
+  const int slots = sms * per_sm;
+  // no more partials than the workspace holds: a group meets at most ceil(ctas / groups) + 1 blocks,
+  // exactly one each when there are as many blocks as groups
+  long long ctas = std::min<long long>(slots, static_cast<long long>(total));
+  ctas = cap > 1 ? std::min(ctas, (cap - 1ll) * groups) : groups;
+  fixed = std::min(std::min(fixed, cap), stages);
+  const double waves_f = std::ceil(static_cast<double>(groups) * fixed / slots);
+  const double share = fixed ? waves_f * std::ceil(static_cast<double>(stages) / fixed) : std::ceil(total / ctas);
+  const double t_bal = std::max(whole, share * one * per_sm) + kFoldUs;
+  p.cluster = 0;
+  p.ctas = static_cast<int>(ctas);
+  double best = t_bal;
+  for (int c = 1; c <= kMaxCluster; c *= 2) {
+    if (c > 1 && c > stages) break;
+    const double waves = std::ceil(static_cast<double>(groups) * c / slots);
+    const double t = std::max(whole, waves * std::ceil(static_cast<double>(stages) / c) * one * per_sm) +
+                     (c > 1 ? kMergeUs : 0.0);
+    if (t < best && groups <= 65535) {
+      best = t;
+      p.cluster = c;
+    }
+  }
+  p.deal.stages = stages;
+  p.deal.groups = groups;
+  p.deal.splits = fixed;
+  p.deal.cap = fixed ? fixed : (p.ctas + groups - 1) / groups + (p.ctas == groups ? 0 : 1);
+  const long long most = p.cluster ? (stages + p.cluster - 1) / p.cluster
+                         : fixed   ? (stages + fixed - 1) / fixed
+                                   : std::min<long long>(stages, (static_cast<long long>(total) + ctas - 1) / ctas);
+  p.deal.ring = static_cast<int>(std::max<long long>(1, std::min<long long>(ring_max, most)));
   return p;
 }
 
@@ -719,93 +933,163 @@ int decode_ml_scratch(size_t floats, float** out) {
 
 namespace {
 
+// Workspace of the balanced form: [row][slot] of O, m and l.
+int partial_space(size_t rows, int D, int cap, void* workspace, float** Op, float** Mp, float** Lp) {
+  const size_t need = rows * cap * (D + 2) * sizeof(float);
+  if (workspace == nullptr) {
+    const int rc = ensure_workspace(need, &workspace);
+    if (rc != RA_OK) return rc;
+  }
+  *Op = static_cast<float*>(workspace);
+  *Mp = *Op + rows * cap * D;
+  *Lp = *Mp + rows * cap;
+  return RA_OK;
+}
+
+// Everything both kernels' launches share: plan, workspace, dynamic shared memory, the fold.
+// launch(cluster form?, config, deal, Mp, Lp, Op) sets the attribute and launches the kernel.
+template <int D, int ROWS, typename Launch>
+int run_plan(const ra_shape& s, int head_batches, int stages, size_t stage_bytes, int ring_max, int per_sm,
+             size_t red_bytes, int old_splits, bool fixed, float* out, float* m, float* l, void* workspace,
+             size_t workspace_bytes, int split_cap, unsigned flags, cudaStream_t stream, Launch launch) {
+  const int kvH = kv_heads_of(s);
+  const size_t rows = static_cast<size_t>(s.batch) * s.heads;
+  const size_t slot_bytes = rows * (D + 2) * sizeof(float);
+  int cap = split_cap;
+  if (workspace != nullptr) {
+    RAB_REQUIRE(workspace_bytes >= old_splits * slot_bytes, RA_ERR_OVERFLOW,
+                "decode workspace too small: %zu < %zu bytes", workspace_bytes, old_splits * slot_bytes);
+    cap = static_cast<int>(std::min<size_t>(cap, workspace_bytes / slot_bytes));
+  }
+  DecodePlan p = make_plan(s.batch * kvH * head_batches, stages, stage_bytes, per_sm, cap, ring_max,
+                           fixed ? old_splits : 0);
+  p.deal.head_batches = head_batches;
+  p.deal.flags = flags;
+  cudaLaunchConfig_t cfg = {};
+  cfg.stream = stream;
+  cfg.dynamicSmemBytes = std::max(p.deal.ring * stage_bytes, red_bytes);
+  cudaLaunchAttribute attr;
+  cfg.attrs = &attr;
+  if (p.cluster) {
+    cfg.gridDim = dim3(p.cluster, p.deal.groups);
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = p.cluster;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.numAttrs = 1;
+    return launch(true, cfg, p.deal, m, l, out);
+  }
+  float *Op, *Mp, *Lp;
+  int rc = partial_space(rows, D, p.deal.cap, workspace, &Op, &Mp, &Lp);
+  if (rc != RA_OK) return rc;
+  cfg.gridDim = fixed ? dim3(static_cast<unsigned>(p.deal.splits) * p.deal.groups) : dim3(p.ctas);
+  rc = launch(false, cfg, p.deal, Mp, Lp, Op);
+  if (rc != RA_OK) return rc;
+  cudaLaunchConfig_t fold = {};
+  fold.gridDim = dim3(s.heads, s.batch);
+  fold.blockDim = dim3(kFoldThreads / D * D);
+  fold.stream = stream;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  fold.attrs = &attr;
+  fold.numAttrs = 1;
+  RAB_CUDA(cudaLaunchKernelEx(&fold, decode_reduce_kernel, static_cast<const float*>(Mp),
+                              static_cast<const float*>(Lp), static_cast<const float*>(Op), m, l, out,
+                              s.heads, kvH, D, ROWS, p.ctas, p.deal));
+  RAB_CUDA(cudaGetLastError());
+  return RA_OK;
+}
+
+// Splits per group of the fixed-split plan, which a caller's workspace has always been held to.
+int fixed_splits(int blocks_per_split, int sk_eff, int rows_per_stage, int split_cap) {
+  int want = (3 * sm_count() + blocks_per_split - 1) / blocks_per_split;
+  want = std::max(1, std::min(std::min(want, std::max(1, sk_eff / (2 * rows_per_stage))), split_cap));
+  long long rps = (sk_eff + want - 1ll) / want;
+  rps = ((rps + rows_per_stage - 1) / rows_per_stage) * rows_per_stage;
+  return static_cast<int>(std::max(1ll, (sk_eff + rps - 1) / rps));
+}
+
+template <typename K>
+int resident_blocks(K kern, int threads, size_t smem) {
+  int n = 0;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) !=
+          cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, threads, smem) != cudaSuccess)
+    cudaGetLastError();
+  return n > 0 ? n : 1;
+}
+
 template <typename T, int D>
 int launch_decode_typed(const void* q, const void* k, const void* v, float* out, float* m,
                         float* l, const ra_shape& s, int sk_eff, long long kv_head_stride,
                         void* workspace, size_t workspace_bytes, cudaStream_t stream,
                         int split_cap = kMaxSplits, unsigned flags = 0) {
-  if constexpr (sizeof(T) == 2 && D >= 64) {
-    // 16-bit caches: the tensor-core kernel (16 query heads per block, 64-key stages)
-    using M = MmaCfg<D>;
-    const int kvH = kv_heads_of(s);
-    const int group = (s.heads + kvH - 1) / kvH;
-    const int head_batches = (group + 15) / 16;
-    const int blocks_per_split = s.batch * kvH * head_batches;
-    int want = (3 * sm_count() + blocks_per_split - 1) / blocks_per_split;
-    want = std::max(1, std::min(std::min(want, std::max(1, sk_eff / (2 * kMmaStageRows))),
-                                split_cap));
-    int rps = (sk_eff + want - 1) / want;
-    rps = ((rps + kMmaStageRows - 1) / kMmaStageRows) * kMmaStageRows;
-    const int n_split = std::max(1, (sk_eff + rps - 1) / rps);
-    const size_t prow = static_cast<size_t>(n_split) * s.batch * s.heads;
-    const size_t need = prow * (D + 2) * sizeof(float);
-    if (workspace == nullptr) {
-      const int rc = ensure_workspace(need, &workspace);
-      if (rc != RA_OK) return rc;
-    } else {
-      RAB_REQUIRE(workspace_bytes >= need, RA_ERR_OVERFLOW,
-                  "decode workspace too small: %zu < %zu bytes", workspace_bytes, need);
-    }
-    float* Mp = static_cast<float*>(workspace);
-    float* Lp = Mp + prow;
-    float* Op = Lp + prow;
-    const float scale_log2 = kLog2e / sqrtf(static_cast<float>(D));
-    const size_t red_bytes = static_cast<size_t>(kMmaWarps) * 16 * (D + 2) * sizeof(float);
-    const size_t smem = std::max(static_cast<size_t>(M::kSmemBytes), red_bytes);
-    auto kern = decode_mma_kernel<T, D>;
-    RAB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  static_cast<int>(smem)));
-    kern<<<dim3(n_split, kvH * head_batches, s.batch), kMmaThreads, smem, stream>>>(
-        static_cast<const T*>(q), static_cast<const T*>(k), static_cast<const T*>(v), Mp, Lp, Op,
-        s.batch, s.heads, kvH, sk_eff, kv_head_stride, rps, head_batches, scale_log2);
-    RAB_CUDA(cudaGetLastError());
-    decode_reduce_kernel<<<dim3(s.heads, s.batch), D, 0, stream>>>(Mp, Lp, Op, m, l, out, s.batch,
-                                                                   s.heads, D, n_split, flags);
-    RAB_CUDA(cudaGetLastError());
-    return RA_OK;
-  }
-  using C = DecodeCfg<T, D>;
   const int kvH = kv_heads_of(s);
-  const Plan p =
-      make_plan(s.batch, s.heads, kvH, sk_eff, C::kRowsPerStage, sm_count(), split_cap);
-  const size_t prow = static_cast<size_t>(p.n_split) * s.batch * s.heads;
-  const size_t need = prow * (D + 2) * sizeof(float);
-  if (workspace == nullptr) {
-    const int rc = ensure_workspace(need, &workspace);
-    if (rc != RA_OK) return rc;
-  } else {
-    RAB_REQUIRE(workspace_bytes >= need, RA_ERR_OVERFLOW,
-                "decode workspace too small: %zu < %zu bytes", workspace_bytes, need);
-  }
-  float* Mp = static_cast<float*>(workspace);
-  float* Lp = Mp + prow;
-  float* Op = Lp + prow;
+  const int group = (s.heads + kvH - 1) / kvH;  // query heads per KV head (largest group)
   const float scale_log2 = kLog2e / sqrtf(static_cast<float>(D));
-  const dim3 grid(p.n_split, kvH * p.head_batches, s.batch);
-  const size_t red_bytes = static_cast<size_t>(kWarps) * 8 * (D + 2) * sizeof(float);
-  const size_t smem = std::max(static_cast<size_t>(C::kSmemBytes), red_bytes);
-#define RAB_DECODE_GB(GBV)                                                                     \
-  case GBV: {                                                                                  \
-    auto kern = decode_split_kernel<T, D, GBV>;                                                \
-    RAB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,           \
-                                  static_cast<int>(smem)));                                    \
-    kern<<<grid, kThreads, smem, stream>>>(static_cast<const T*>(q), static_cast<const T*>(k), \
-                                           static_cast<const T*>(v), Mp, Lp, Op, s.batch,      \
-                                           s.heads, kvH, sk_eff, kv_head_stride,               \
-                                           p.rows_per_split, p.head_batches, scale_log2);      \
-  } break;
-  switch (p.gb) {
-    RAB_DECODE_GB(1)
-    RAB_DECODE_GB(2)
-    RAB_DECODE_GB(4)
-    RAB_DECODE_GB(8)
+  const T *qt = static_cast<const T*>(q), *kt = static_cast<const T*>(k), *vt = static_cast<const T*>(v);
+  auto launch_with = [&](auto kern, size_t smem_max, std::atomic<unsigned long long>& smem_set,
+                         cudaLaunchConfig_t& cfg, int threads, const Deal& deal, float* Mp, float* Lp,
+                         float* Op) -> int {
+    // once per device and instantiation
+    int dev = 0;
+    RAB_CUDA(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64 || !(smem_set.load(std::memory_order_acquire) >> dev & 1ull)) {
+      RAB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    static_cast<int>(smem_max)));
+      if (dev >= 0 && dev < 64) smem_set.fetch_or(1ull << dev, std::memory_order_release);
+    }
+    cfg.blockDim = dim3(threads);
+    RAB_CUDA(cudaLaunchKernelEx(&cfg, kern, qt, kt, vt, Mp, Lp, Op, s.heads, kvH, sk_eff, kv_head_stride,
+                                deal, scale_log2));
+    return RA_OK;
+  };
+  if constexpr (sizeof(T) == 2 && D >= 64) {
+    // 16-bit caches: the tensor-core kernel (16 query heads per block)
+    using M = MmaCfg<D>;
+    constexpr size_t kRed = static_cast<size_t>(M::kWarps + 1) * 16 * (D + 2) * sizeof(float);
+    constexpr size_t kSmem = M::kSmemBytes > kRed ? M::kSmemBytes : kRed;
+    const int head_batches = (group + 15) / 16;
+    const int stages = (sk_eff + M::kStageRows - 1) / M::kStageRows;
+    static const int per_sm = resident_blocks(decode_mma_kernel<T, D, kBalanced>, M::kThreads, kSmem);
+    return run_plan<D, 16>(
+        s, head_batches, stages, 2 * M::kStageBytes, M::kStages, per_sm, kRed,
+        fixed_splits(s.batch * kvH * head_batches, sk_eff, 64, split_cap), false, out,
+        m, l, workspace, workspace_bytes, split_cap, flags, stream,
+        [&](bool cluster, cudaLaunchConfig_t& cfg, const Deal& deal, float* Mp, float* Lp, float* Op) {
+          static std::atomic<unsigned long long> set_c{0}, set_b{0};
+          return cluster ? launch_with(decode_mma_kernel<T, D, kCluster>, kSmem, set_c, cfg, M::kThreads, deal,
+                                       Mp, Lp, Op)
+                         : launch_with(decode_mma_kernel<T, D, kBalanced>, kSmem, set_b, cfg, M::kThreads, deal,
+                                       Mp, Lp, Op);
+        });
+  } else {
+    auto run = [&](auto gb_tag) {
+      constexpr int GB = decltype(gb_tag)::value;
+      using C = DecodeCfg<T, D, GB>;
+      constexpr DealForm kDealt = GB * C::kEPL >= 64 ? kFixed : kBalanced;  // (see DecodeCfg)
+      constexpr size_t kRed = static_cast<size_t>(kWarps + 1) * GB * (D + 2) * sizeof(float);
+      constexpr size_t kSmem = C::kSmemBytes > kRed ? C::kSmemBytes : kRed;
+      const int head_batches = (group + GB - 1) / GB;
+      const int stages = (sk_eff + C::kRowsPerStage - 1) / C::kRowsPerStage;
+      static const int per_sm = resident_blocks(decode_split_kernel<T, D, GB, kDealt>, kThreads, kSmem);
+      return run_plan<D, GB>(
+          s, head_batches, stages, 2 * C::kStageBytes, kStages, per_sm, kRed,
+          fixed_splits(s.batch * kvH * head_batches, sk_eff, C::kPlanRows, split_cap), kDealt == kFixed,
+          out, m, l, workspace, workspace_bytes, split_cap, flags, stream,
+          [&](bool cluster, cudaLaunchConfig_t& cfg, const Deal& deal, float* Mp, float* Lp, float* Op) {
+            static std::atomic<unsigned long long> set_c{0}, set_b{0};
+            return cluster ? launch_with(decode_split_kernel<T, D, GB, kCluster>, kSmem, set_c, cfg, kThreads,
+                                         deal, Mp, Lp, Op)
+                           : launch_with(decode_split_kernel<T, D, GB, kDealt>, kSmem, set_b, cfg, kThreads,
+                                         deal, Mp, Lp, Op);
+          });
+    };
+    // smallest of 1 / 2 / 4 / 8 that fits the group
+    if (group > 4) return run(std::integral_constant<int, 8>{});
+    if (group > 2) return run(std::integral_constant<int, 4>{});
+    if (group > 1) return run(std::integral_constant<int, 2>{});
+    return run(std::integral_constant<int, 1>{});
   }
-#undef RAB_DECODE_GB
-  RAB_CUDA(cudaGetLastError());
-  decode_reduce_kernel<<<dim3(s.heads, s.batch), D, 0, stream>>>(Mp, Lp, Op, m, l, out, s.batch,
-                                                                 s.heads, D, p.n_split, flags);
-  RAB_CUDA(cudaGetLastError());
-  return RA_OK;
 }
 
 template <typename T>

@@ -1,6 +1,6 @@
 """GPU parity of the forms that a call's shape selects: the key-split form of the step kernels (the
-blocks of a cluster share a query block's keys), the scaled fp16 splitting of the fp32 step and the
-one-launch cache append.
+blocks of a cluster share a query block's keys), the scaled fp16 splitting of the fp32 step, the two
+forms of the decode kernels and the one-launch cache append.
 
 Tolerances are those of the other step and decode tests: 1e-5 for fp32 and 1e-3 / 8e-3 for fp16 /
 bf16 P, absolute and relative, against the oracle on the same rounded inputs. Where values are
@@ -122,6 +122,31 @@ def test_fp32_step_passes_on_nan_and_infinity_of_visible_values_only():
     assert not np.isfinite(got[160, 7]) and np.isnan(got[195]).all()
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+@pytest.mark.parametrize("D", [32, 128, 256])
+@pytest.mark.parametrize("shape", [  # B, H, kvH, Sk: both forms, single stages, ragged ends, several head batches
+    (1, 1, 1, 1), (1, 8, 8, 64), (1, 40, 2, 65), (3, 6, 2, 1023), (1, 4, 4, 30011), (2, 34, 1, 9000), (40, 4, 4, 190)])
+def test_decode_forms_match_the_oracle_with_and_without_a_state(dtype, D, shape):
+    B, H, kvH, Sk = shape
+    q, k, v = (round_to(x, dtype) for x in normal_inputs(11, B, H, kvH, 1, Sk, D))
+    want, want_lse = oracle.cpu_attention(q, k, v, False, kv_heads=kvH, want_lse=True, threads=8)
+    s = api.AttentionShape(B, H, 1, Sk, D, kvH)
+    dq, dk, dv = dev(q, dtype), dev(k, dtype), dev(v, dtype)
+    out, m, l = poisoned(B, H, 1, D)
+    api.launch_attention_init(out, m, l, s)
+    # the least workspace that has always been enough (one partial per row) and the full one
+    one = B * H * (D + 2) * 4
+    spaces = [None, torch.empty(lib().ra_decode_workspace_bytes(C.byref(s.c())), dtype=torch.uint8, device="cuda")]
+    if Sk == 1:
+        spaces.append(torch.empty(one, dtype=torch.uint8, device="cuda"))
+    for ws in spaces:  # folding the same keys again leaves the normalised result as it is
+        api.launch_attention_decode_step(dq, dk, dv, out, m, l, s, 0, 0, False, workspace=ws)
+    lse = api.attention_lse(m, l).cpu().numpy() - np.log(len(spaces))
+    api.launch_attention_finalize(out, l, s)
+    assert_close(out.cpu().numpy(), want, TOL[dtype], TOL[dtype], "out")
+    assert_close(lse, want_lse, TOL[dtype], TOL[dtype], "lse")
+
+
 @pytest.mark.parametrize("dtype,D", [(torch.float32, 1), (torch.float16, 3), (torch.bfloat16, 8), (torch.float16, 128)])
 def test_cache_append_of_any_row_size_and_alignment(dtype, D):
     B, kvH, s_max = 2, 3, 5
@@ -132,3 +157,38 @@ def test_cache_append_of_any_row_size_and_alignment(dtype, D):
         cache.append(rows[0, t], rows[1, t])
     assert torch.equal(cache.k_view(), rows[0, :, :, :, 0].permute(1, 2, 0, 3))
     assert torch.equal(cache.v_view(), rows[1, :, :, :, 0].permute(1, 2, 0, 3))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+@pytest.mark.parametrize("heads,kv_heads,rows,D", [(8, 8, 20000, 128), (16, 2, 6000, 128), (8, 8, 300, 64), (4, 4, 9000, 256)])
+def test_decode_and_key_split_replay_from_a_captured_graph(dtype, heads, kv_heads, rows, D):
+    # the fold of the decode partials is a programmatic dependent launch, the key split a cluster launch
+    g = torch.Generator(device="cuda").manual_seed(3)
+    k = torch.randn((1, kv_heads, rows, D), generator=g, device="cuda").to(dtype)
+    v = torch.randn((1, kv_heads, rows, D), generator=g, device="cuda").to(dtype)
+    cache = api.DeviceKVCache(1, kv_heads, rows + 1, D, dtype)
+    cache.copy_prefill(k, v, rows)
+    q1 = torch.randn((1, heads, 1, D), generator=g, device="cuda").to(dtype)
+    qn = torch.randn((1, heads, 100, D), generator=g, device="cuda").to(dtype)
+    o1 = torch.empty((1, heads, 1, D), device="cuda")
+    on, m, l = poisoned(1, heads, 100, D)
+    shape = api.AttentionShape(1, heads, 100, rows, D, kv_heads)
+    maps = SegMap.make([rows - 100], 100), SegMap.make([0], rows)
+
+    def both():
+        api.run_local_decode_step(q1, cache, heads, rows - 1, 0, True, o1)
+        api.attention_step_ex(qn, k, v, on, m, l, shape, *maps, causal=True, fresh=True, finalize=True)
+
+    both()  # workspaces are made here
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        both()
+    q1.copy_(torch.randn(q1.shape, generator=g, device="cuda").to(dtype))
+    qn.copy_(torch.randn(qn.shape, generator=g, device="cuda").to(dtype))
+    graph.replay()
+    torch.cuda.synchronize()
+    got1, gotn = o1.clone(), on.clone()
+    both()
+    torch.cuda.synchronize()
+    assert torch.equal(got1, o1) and torch.equal(gotn, on) and api.device_status()[0] == 0
