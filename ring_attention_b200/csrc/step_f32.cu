@@ -35,6 +35,11 @@
 //
 // Tensor memory, 256 columns per query tile: S [0,64) P hi [64,96) P lo [96,128) O [128,192) Q hi
 // [192,224) Q lo [224,256); head_dim 128: S and P [0,64) O [64,192) Q hi [192,256).
+// What bounds it: at head_dim 128 the chain scores -> softmax -> P.V of the two query tiles, which take
+// turns on the tensor core (tensor pipe 44 %, issue slots 34 %). Measured, us per call, against one
+// 128-row tile per block on TF32 pairs: B1 H4 S16384 D128 causal 960 (2700), B1 H8 S1024 D64 dense 23
+// (37), H4/kvH1 8231 x 9075 rows D64 causal 164 (272).
+//
 // Every wait on an mbarrier is bounded (see tc_common.cuh); a wait that runs out reports into
 // the device status word and the block unwinds.
 #include <atomic>
