@@ -56,8 +56,9 @@ constexpr int kBNf = 64;          // keys per tile
 constexpr int kThreadsF = 640;
 constexpr int kSplitThreads = 256;
 constexpr int kTopExp = 14;       // scaled values have their largest magnitude in [2^14, 2^15)
-constexpr int kPBits = 8;         // P at the row's reference point is 2^8
-constexpr int kVSlack = 2;        // a V tile may exceed the accumulator's unit by 2^2
+constexpr int kPBits = 8;         // the largest P of a tile that sets a row's unit is 2^8
+constexpr int kNoUnit = 1 << 20;  // nothing in O yet, or (as a tile's exponent) nothing but zeros in V
+constexpr int kHeadroom = 60;     // how far O may be scaled up over the unit it was accumulated in
 constexpr float kPSumLimit = 65000.f;  // of eight P: none of them then leaves fp16's range
 
 template <int DR, bool kSplit>
@@ -435,8 +436,7 @@ __global__ void __launch_bounds__(kThreadsF, 1)
 #pragma unroll
           for (int i = 0; i < 8; ++i) mx = max(mx, red[par * 8 + i]);
           e = scale_exp(mx);
-          // (an all-zero tile sets no unit: marked with an exponent no other tile has)
-          if (sw == 0 && lane == 0) v_exp[(it >> 1) & 15] = mx == 0 ? 127 : e;
+          if (sw == 0 && lane == 0) v_exp[(it >> 1) & 15] = mx == 0 ? kNoUnit : e;
         }
         const float sc = pow2i(e);
 #pragma unroll
@@ -514,7 +514,8 @@ __global__ void __launch_bounds__(kThreadsF, 1)
 
     float m_ref = -INFINITY;  // reference point of P, O and l, log2 units
     float l_run = 0.f;
-    int v_ref = 127;          // O is in units of 2^-(kPBits + v_ref); 127: no V seen yet
+    int unit = kNoUnit;       // O is in units of 2^-unit
+    int raised = 0;           // how far O has been scaled up over the unit it was accumulated in
     bool ok = true;
     int j = 0;
     const int n_seg = mine ? a.kmap.n_seg : 0;
@@ -576,20 +577,16 @@ __global__ void __launch_bounds__(kThreadsF, 1)
           for (int i = 0; i < kBNf; ++i) s[i] = (i >= c_lo && i < c_hi) ? s[i] : -INFINITY;
         }
 
-        // unit of this tile's P: 2^p_exp at the reference point, so that P * V lands in O's unit
+        // P of this tile is 2^p_exp at the reference point, so that P * V (scaled by 2^ev) lands in
+        // the row's unit. The unit is the row's own and follows what the row adds to O: a V tile it sees no
+        // key of says nothing, and one of larger values only once a P that it meets would leave fp16. The
+        // two terms of P have an absolute floor of 2^-25, so a tile of much smaller values (p_exp < 0) moves
+        // the unit as well.
         const int ev = v_exp[j & 15];
-        bool slow = false;
-        float v_alpha = 1.f;  // O moves to a new unit
-        if (ev != 127) {
-          if (v_ref == 127) {
-            v_ref = ev;  // nothing but zeros in O so far
-          } else if (ev < v_ref - kVSlack) {
-            v_alpha = pow2i(max(ev - v_ref, -126));
-            v_ref = ev;
-            slow = true;
-          }
-        }
-        const int p_exp = kPBits + ((ev == 127) ? 0 : max(v_ref - ev, -40));  // (smaller V adds nothing to O)
+        const bool adds = c_hi > c_lo && ev != kNoUnit;
+        if (adds && unit == kNoUnit) unit = kPBits + ev;
+        int p_exp = adds ? unit - ev : kPBits;
+        bool slow = __any_sync(0xffffffffu, p_exp < 0 || p_exp > 100 || (m_ref == -INFINITY && c_hi > c_lo)) != 0;
         // Wait for P.V of the previous tile: its P buffer is about to be written. (With P over S the
         // scores of this tile, issued behind it, stand for that.)
         if (!C::kAlias && j > 0) {
@@ -602,8 +599,9 @@ __global__ void __launch_bounds__(kThreadsF, 1)
         float row_sum = 0.f, oct_max = 0.f;
         // P = 2^(s * f - m_ref + p_exp) as hi + lo in tensor memory, 32 columns at a time; the sums
         // of eight columns each bound every P and add up to the row sum
-        auto exponentials = [&](float neg_m) {
-          const float2 n2 = make_float2(neg_m, neg_m);
+        auto exponentials = [&]() {
+          const float n = m_ref == -INFINITY ? 0.f : static_cast<float>(p_exp) - m_ref;
+          const float2 n2 = make_float2(n, n);
           float2 sum[4];
 #pragma unroll
           for (int i = 0; i < 4; ++i) sum[i] = make_float2(0.f, 0.f);
@@ -626,10 +624,8 @@ __global__ void __launch_bounds__(kThreadsF, 1)
                           max3(fmaxf(sum[2].x, sum[2].y), sum[3].x, sum[3].y));
           row_sum = all.x + all.y;
         };
-        slow = slow || __any_sync(0xffffffffu, m_ref == -INFINITY && c_hi > c_lo) != 0;
-        const float pe = static_cast<float>(p_exp);
         if (!slow) {
-          exponentials(m_ref == -INFINITY ? 0.f : pe - m_ref);
+          exponentials();
           slow = __any_sync(0xffffffffu, !(oct_max <= kPSumLimit) || !(row_sum == row_sum)) != 0;
         }
         if (slow) {
@@ -639,14 +635,28 @@ __global__ void __launch_bounds__(kThreadsF, 1)
           mx = fmaxf(mx, s[kBNf - 1]);
           const float tile_max = mx * row_f;  // -inf stays -inf
           float alpha = 1.f;
+          const float m_old = m_ref;
           if (tile_max > m_ref) {
-            if (m_ref > -INFINITY) alpha = ex2(m_ref - tile_max);
+            if (m_old > -INFINITY) alpha = ex2(m_old - tile_max);
             m_ref = tile_max;
           }
-          if (j > 0 && __any_sync(0xffffffffu, alpha != 1.f || v_alpha != 1.f)) {
+          l_run *= alpha;
+          float oa = alpha;  // factor of O
+          if (adds) {
+            // O as it stands is in units of 2^-keep of the new reference point. This tile's largest P,
+            // 2^-low of it, must not exceed 2^kPBits; and if its values are far smaller than the unit,
+            // O is scaled up, as far as it cannot overflow.
+            const int low = static_cast<int>(fminf(m_ref - tile_max, 100.f));
+            const int keep = unit + (m_old > -INFINITY ? static_cast<int>(fminf(m_ref - m_old, 1000.f)) : 0);
+            int to = min(keep, kPBits + ev + low);
+            if (to < ev) to = min(kPBits + ev, keep + kHeadroom - raised);
+            if (m_old > -INFINITY) oa = ex2(m_old - m_ref + static_cast<float>(to - unit));
+            raised = max(0, raised + to - keep);
+            unit = to;
+            p_exp = max(to - ev, -kHeadroom);  // (a P below 2^-25 adds nothing)
+          }
+          if (j > 0 && __any_sync(0xffffffffu, oa != 1.f)) {
             // O is at rest: P.V of tile j - 1 has completed
-            l_run *= alpha;
-            const float oa = alpha * v_alpha;
 #pragma unroll 1
             for (int c = 0; c < DR / 32; ++c) {
               float o[32];
@@ -656,7 +666,7 @@ __global__ void __launch_bounds__(kThreadsF, 1)
               tmem_st32(t_o + c * 32, o);
             }
           }
-          exponentials(m_ref == -INFINITY ? 0.f : pe - m_ref);
+          exponentials();
         }
         l_run += row_sum * pow2i(-p_exp);
         tmem_wait_st();
@@ -670,7 +680,7 @@ __global__ void __launch_bounds__(kThreadsF, 1)
       ok = mbar_wait(bar_o_done + 8 * w, (n_tiles - 1) & 1, abort_flag, a.status, 8, n_tiles, a.wait_ns);
     ok = __all_sync(0xffffffffu, ok);
     if (ok && mine) tc_fence_after();
-    const float o_unit = pow2i(v_ref == 127 ? 0 : -(kPBits + v_ref));
+    const float o_unit = pow2i(unit == kNoUnit ? 0 : -unit);
     if constexpr (kSplit) {
       merge_key_split<C, DR>(a, smem, s_base, t_o, w, row, row_valid, grow0, ok && mine, m_ref, l_run, o_unit,
                              cta_rank, fresh, finalize);

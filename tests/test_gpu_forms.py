@@ -108,6 +108,58 @@ def test_fp32_step_holds_its_precision_over_the_range_of_fp32(D, case):
     assert_close(lse, want_lse, 1e-5, 1e-5, "lse")
 
 
+def _wide_inputs(case, D):
+    """Finite inputs whose parts differ by powers of two: (q, k, v, causal, doc_len, [(rows, columns)]).
+    Every part of the output is held against its own largest value."""
+    S, every = 500, slice(None)
+    q, k, v = (x.astype(np.float64) for x in normal_inputs(21, 1, 2, 2, S, S, D))
+    kind, n = case
+    if kind == "document":  # boundary on a key tile's edge, inside a query block
+        v[:, :, :192] *= 2.0 ** n
+        return q, k, v, True, 192, [(slice(0, 192), every), (slice(192, 384), every), (slice(384, S), every)]
+    if kind == "future":
+        v[:, :, 192:] *= 2.0 ** n
+        return q, k, v, True, 0, [(slice(0, 192), every), (slice(192, S), every)]
+    if kind in ("first tile", "last tile"):  # values 2^n larger under weights about 2^n smaller
+        at = slice(0, 64) if kind == "first tile" else slice(448, S)
+        v[:, :, at] *= 2.0 ** n
+        q[..., 0], k[..., 0] = 4.0, 0.0
+        k[:, :, at] *= 0.1
+        k[:, :, at, 0] = -n * np.log(2.0) / 4.0 * np.sqrt(D)
+        return q, k, v, False, 0, [(every, every)]
+    raise ValueError(kind)
+
+
+@pytest.mark.parametrize("D", [32, 64, 128])
+@pytest.mark.parametrize("split", [1, 3])
+@pytest.mark.parametrize("case", [("document", 20), ("document", 34), ("document", 100), ("document", -40), ("future", 40),
+                                  ("first tile", 20), ("first tile", 34), ("last tile", 20), ("last tile", 34)], ids=str)
+def test_fp32_step_holds_the_precision_of_every_part_of_the_output(D, split, case):
+    # Values that a row cannot see, or sees under a negligible weight, must not cost it bits, nor may
+    # one column cost another. Against 64 bits; 1e-5 of the part's largest value, the fp32 tolerance.
+    q, k, v, causal, doc, parts = _wide_inputs(case, D)
+    q, k, v = (x.astype(np.float32) for x in (q, k, v))
+    B, H, S, _ = q.shape
+    pos = np.arange(S)
+    seen = (pos[None, :] <= pos[:, None]) | (not causal)
+    if doc:
+        seen &= pos[None, :] // doc == pos[:, None] // doc
+    s = np.einsum("bhid,bhjd->bhij", q.astype(np.float64), k.astype(np.float64)) / np.sqrt(D)
+    s = np.where(seen, s, -np.inf)
+    m = s.max(-1, keepdims=True)
+    p = np.exp(s - m)
+    want = np.einsum("bhij,bhjd->bhid", p, v.astype(np.float64)) / p.sum(-1, keepdims=True)
+    want_lse = (m + np.log(p.sum(-1, keepdims=True)))[..., 0]
+    state = poisoned(B, H, S, D)
+    step(dev(q), dev(k), dev(v), state, api.AttentionShape(B, H, S, S, D), SegMap.make([0], S), SegMap.make([0], S),
+         FRESH | FINALIZE | (CAUSAL if causal else 0), split, doc)
+    got, lse = state[0].cpu().numpy(), api.attention_lse(state[1], state[2]).cpu().numpy()
+    assert_close(lse, want_lse, 1e-5, 1e-5, "lse")
+    for rows, cols in parts:
+        unit = np.abs(want[:, :, rows, cols]).max()
+        assert_close(got[:, :, rows, cols] / unit, want[:, :, rows, cols] / unit, 1e-5, 0.0, f"rows {rows} columns {cols}")
+
+
 def test_fp32_step_passes_on_nan_and_infinity_of_visible_values_only():
     B, H, S, D = 1, 1, 200, 64
     q, k, v = normal_inputs(9, B, H, H, S, S, D)
