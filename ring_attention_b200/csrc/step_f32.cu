@@ -101,16 +101,24 @@ struct F32Cfg {
 
 // The power-of-two exponent that brings a largest magnitude (as its bits) to [2^14, 2^15); an
 // infinity or a NaN counts as nothing (it stays what it is under any scale), zero gives zero.
-// Clamped so that the product of two inverse scales is still a normal number.
-__device__ inline int scale_exp(unsigned max_bits) {
-  const int e = static_cast<int>(max_bits >> 23);
-  return e == 0 ? 0 : min(kTopExp + 127 - e, 62);
+// At least -113, at most `limit`. The limits keep the scale and its inverse normal numbers: below 2^-106
+// (K: 2^-98) values lose bits gradually.
+__device__ inline int scale_exp(unsigned max_bits, int limit) {
+  return max_bits == 0 ? 0 : min(kTopExp + 127 - static_cast<int>(max_bits >> 23), limit);
 }
+constexpr int kMaxExp = 120;
+// A score is scaled back in two steps, by 2^-(exponent of the key + kBias) and by 2^-(exponent of the row
+// - kBias): neither factor nor the value between them leaves fp32 where the score does not, unless
+// magnitudes of Q or K exceed 2^118.
+constexpr int kBias = 14, kMaxExpK = 126 - kBias;
 __device__ inline unsigned finite_abs_bits(float x) {
   const unsigned u = __float_as_uint(x) & 0x7fffffffu;
   return u < 0x7f800000u ? u : 0u;
 }
 __device__ inline float pow2i(int e) { return __int_as_float((e + 127) << 23); }  // -126 <= e <= 127
+__device__ inline float pow2_any(int e) {                                          // -149 <= e <= 127
+  return e >= -126 ? pow2i(e) : __int_as_float(1 << (e + 149));
+}
 // Two scaled values as packed hi and lo fp16 pairs.
 __device__ inline void split_pair(float x0, float x1, unsigned& hi, unsigned& lo) {
   const __half2 h = __floats2half2_rn(x0, x1);
@@ -414,10 +422,10 @@ __global__ void __launch_bounds__(kThreadsF, 1)
           // K: by key. The row's pieces sit in the four lanes r8, r8 + 8, ...
           mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
           mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
-          e = scale_exp(mx);
+          e = scale_exp(mx, kMaxExpK);
           if (p4 == 0) {
             const unsigned g = s_base + C::kOffG + (((it >> 1) % C::kGDepth) * kBNf + sw * 8 + r8) * 4;
-            asm volatile("st.shared.f32 [%0], %1;" ::"r"(g), "f"(pow2i(-e)) : "memory");
+            asm volatile("st.shared.f32 [%0], %1;" ::"r"(g), "f"(pow2i(-e - kBias)) : "memory");
           }
           __syncwarp();  // the rows of this warp have been read
         } else {
@@ -435,7 +443,7 @@ __global__ void __launch_bounds__(kThreadsF, 1)
           mx = 0;
 #pragma unroll
           for (int i = 0; i < 8; ++i) mx = max(mx, red[par * 8 + i]);
-          e = scale_exp(mx);
+          e = scale_exp(mx, kMaxExp);
           if (sw == 0 && lane == 0) v_exp[(it >> 1) & 15] = mx == 0 ? kNoUnit : e;
         }
         const float sc = pow2i(e);
@@ -482,9 +490,9 @@ __global__ void __launch_bounds__(kThreadsF, 1)
         mx = max(max(max(mx, finite_abs_bits(v.x)), max(finite_abs_bits(v.y), finite_abs_bits(v.z))),
                  finite_abs_bits(v.w));
       }
-      const int e = scale_exp(mx);
+      const int e = scale_exp(mx, kMaxExp);
       const float sc = pow2i(e);
-      row_f = rsqrtf(static_cast<float>(DR)) * kLog2e * pow2i(-e);
+      row_f = rsqrtf(static_cast<float>(DR)) * kLog2e * pow2i(kBias - e);
 #pragma unroll
       for (int g = 0; g < DR / 32; ++g) {  // 32 columns at a time (second read: L1 / L2)
         unsigned hi[16], lo[16];
@@ -680,7 +688,7 @@ __global__ void __launch_bounds__(kThreadsF, 1)
       ok = mbar_wait(bar_o_done + 8 * w, (n_tiles - 1) & 1, abort_flag, a.status, 8, n_tiles, a.wait_ns);
     ok = __all_sync(0xffffffffu, ok);
     if (ok && mine) tc_fence_after();
-    const float o_unit = pow2i(unit == kNoUnit ? 0 : -unit);
+    const float o_unit = pow2_any(unit == kNoUnit ? 0 : -unit);
     if constexpr (kSplit) {
       merge_key_split<C, DR>(a, smem, s_base, t_o, w, row, row_valid, grow0, ok && mine, m_ref, l_run, o_unit,
                              cta_rank, fresh, finalize);
@@ -699,7 +707,6 @@ __global__ void __launch_bounds__(kThreadsF, 1)
       const float l_fin = ca * l_old + cb * l_run;
       const float inv = finalize ? (l_fin > 0.f ? 1.f / l_fin : 0.f) : 1.f;
       const bool touch = row_valid && (have || fresh || finalize);
-      const float fo = cb * o_unit;
 #pragma unroll 1
       for (int c = 0; c < DR / 32; ++c) {
         float o[32];
@@ -716,10 +723,10 @@ __global__ void __launch_bounds__(kThreadsF, 1)
             float4 old = make_float4(0.f, 0.f, 0.f, 0.f);
             if (!fresh) old = dst[i];
             float4 r;
-            r.x = (ca * old.x + (have ? fo * o[4 * i] : 0.f)) * inv;
-            r.y = (ca * old.y + (have ? fo * o[4 * i + 1] : 0.f)) * inv;
-            r.z = (ca * old.z + (have ? fo * o[4 * i + 2] : 0.f)) * inv;
-            r.w = (ca * old.w + (have ? fo * o[4 * i + 3] : 0.f)) * inv;
+            r.x = (ca * old.x + (have ? cb * (o[4 * i] * o_unit) : 0.f)) * inv;
+            r.y = (ca * old.y + (have ? cb * (o[4 * i + 1] * o_unit) : 0.f)) * inv;
+            r.z = (ca * old.z + (have ? cb * (o[4 * i + 2] * o_unit) : 0.f)) * inv;
+            r.w = (ca * old.w + (have ? cb * (o[4 * i + 3] * o_unit) : 0.f)) * inv;
             dst[i] = r;
           }
         }

@@ -496,7 +496,7 @@ __device__ inline void merge_key_split(const TcArgs& a, unsigned char* smem, uns
   const float inv = finalize ? (l_fin > 0.f ? 1.f / l_fin : 0.f) : 1.f;
   const bool touch = row_valid && (any || fresh || finalize);
   fac[rb] = touch ? make_float2(ca * inv, cb * inv) : make_float2(-1.f, 0.f);  // factors are never negative
-  const float scale = have ? ex2(m_ref - m_all) * o_unit : 0.f;
+  const float scale = have ? ex2(m_ref - m_all) : 0.f;
 #pragma unroll 1
   for (int c = 0; c < DR / 32; ++c) {
     float o[32];
@@ -509,8 +509,8 @@ __device__ inline void merge_key_split(const TcArgs& a, unsigned char* smem, uns
     float4* dst = reinterpret_cast<float4*>(o_stage + rb * kStride + c * 32);
 #pragma unroll
     for (int i = 0; i < 8; ++i)
-      dst[i] = have ? make_float4(o[4 * i] * scale, o[4 * i + 1] * scale, o[4 * i + 2] * scale,
-                                  o[4 * i + 3] * scale)
+      dst[i] = have ? make_float4(o[4 * i] * o_unit * scale, o[4 * i + 1] * o_unit * scale,
+                                  o[4 * i + 2] * o_unit * scale, o[4 * i + 3] * o_unit * scale)
                     : make_float4(0.f, 0.f, 0.f, 0.f);
   }
   cluster_sync_threads();  // every block's O is staged, every old (m, l) has been read

@@ -127,13 +127,18 @@ def _wide_inputs(case, D):
         k[:, :, at] *= 0.1
         k[:, :, at, 0] = -n * np.log(2.0) / 4.0 * np.sqrt(D)
         return q, k, v, False, 0, [(every, every)]
+    if kind == "V":
+        return q, k, v * 2.0 ** n, False, 0, [(every, every)]
+    if kind == "Q against K":
+        return q * 2.0 ** n, k * 2.0 ** -n, v, False, 0, [(every, every)]
     raise ValueError(kind)
 
 
 @pytest.mark.parametrize("D", [32, 64, 128])
 @pytest.mark.parametrize("split", [1, 3])
 @pytest.mark.parametrize("case", [("document", 20), ("document", 34), ("document", 100), ("document", -40), ("future", 40),
-                                  ("first tile", 20), ("first tile", 34), ("last tile", 20), ("last tile", 34)], ids=str)
+                                  ("first tile", 20), ("first tile", 34), ("last tile", 20), ("last tile", 34), ("V", -70), ("V", -90), ("V", -104), ("V", 120),
+                                  ("Q against K", 80), ("Q against K", -80), ("Q against K", 104), ("Q against K", -96)], ids=str)
 def test_fp32_step_holds_the_precision_of_every_part_of_the_output(D, split, case):
     # Values that a row cannot see, or sees under a negligible weight, must not cost it bits, nor may
     # one column cost another. Against 64 bits; 1e-5 of the part's largest value, the fp32 tolerance.
