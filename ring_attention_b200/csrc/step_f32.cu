@@ -58,8 +58,14 @@ constexpr int kSplitThreads = 256;
 constexpr int kTopExp = 14;       // scaled values have their largest magnitude in [2^14, 2^15)
 constexpr int kPBits = 8;         // the largest P of a tile that sets a row's unit is 2^8
 constexpr int kNoUnit = 1 << 20;  // nothing in O yet, or (as a tile's exponent) nothing but zeros in V
-constexpr int kHeadroom = 60;     // how far O may be scaled up over the unit it was accumulated in
+constexpr int kOTop = 116;        // O may be scaled up to 2^116
+constexpr int kMinPExp = -60;     // (a P below 2^-25 adds nothing)
 constexpr float kPSumLimit = 65000.f;  // of eight P: none of them then leaves fp16's range
+// A V tile is wide if the largest value of some key (not all zeros) is below 2^-kKeyRange of the tile's, or
+// that of some column among a splitter warp's eight keys below 2^-kColRange: what its elements lose
+// below 2^-40 of the tile's largest (and P below 2^-33) could then show in a row or a column.
+constexpr int kKeyRange = 9, kColRange = 16;
+constexpr int kExpBias = 512, kWide = 1 << 12;  // a tile's exponent as v_exp holds it
 
 template <int DR, bool kSplit>
 struct F32Cfg {
@@ -88,10 +94,11 @@ struct F32Cfg {
   static constexpr int kOffBar = kOffKV + kStages * kSlotBytes;
   static constexpr int kNumBars = 2 + 3 * kStages + 8 + 1;
   static constexpr int kOffSlot = kOffBar + kNumBars * 8;      // tensor-memory address, abort flag
-  static constexpr int kOffRed = kOffSlot + 8;                 // [2][8] tile maxima of V by warp
-  static constexpr int kOffVExp = kOffRed + 64;                // [16] exponents of V tiles
+  static constexpr int kOffRed = kOffSlot + 8;                 // [2][2][8] range of a V tile by warp
+  static constexpr int kOffVExp = kOffRed + 128;               // [16] exponents of V tiles
   static constexpr int kOffG = (kOffVExp + 64 + 15) & ~15;     // [kGDepth][kBNf] factors of K
-  static constexpr int kOffMl = kOffG + kGDepth * kBNf * 4;
+  static constexpr int kOffVKey = kOffG + kGDepth * kBNf * 4;  // [8][kBNf] exponents of V's keys
+  static constexpr int kOffMl = kOffVKey + 8 * kBNf;
   static constexpr int kMlBytes = kSplit ? kTiles * kBM * 8 : 0;
   static constexpr int kSmemBytes = kOffMl + kMlBytes;
   static constexpr int kColS = 0, kColP = kAlias ? 0 : 64, kColO = kAlias ? 64 : 128, kColQ = 192;
@@ -134,6 +141,11 @@ __device__ inline float2 fmul2(float2 a, float2 b) {
       : "l"(*reinterpret_cast<unsigned long long*>(&a)),
         "l"(*reinterpret_cast<unsigned long long*>(&b)));
   return d;
+}
+__device__ inline unsigned ld_shared_u1(unsigned addr) {
+  unsigned v;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
+  return v;
 }
 __device__ inline float4 ld_shared_f4(unsigned addr) {
   float4 v;
@@ -331,14 +343,17 @@ __global__ void __launch_bounds__(kThreadsF, 1)
           // MN-major V: 64 columns per 128-byte row, groups 2 boxes apart, 16 keys per k-step
           const unsigned long long vd =
               desc_mnmajor(s_kv + slot * C::kSlotBytes, 2 * C::kBoxBytes, 1024);
+          const bool wide = (v_exp[t & 15] & kWide) != 0;  // the softmax threads have added it to O
           if (elect_one()) {
+            if (!wide) {
 #pragma unroll
-            for (int term = 0; term < 3; ++term) {
+              for (int term = 0; term < 3; ++term) {
 #pragma unroll
-              for (int ks = 0; ks < kBNf / 16; ++ks)
-                mma_ts(t_o, t_p + ks * 8 + (term == 0 ? 32 : 0),
-                       vd + ks * (2048 >> 4) + (term == 1 ? kLo : 0), idesc_pv,
-                       (t > 0 || term > 0 || ks > 0) ? 1u : 0u);
+                for (int ks = 0; ks < kBNf / 16; ++ks)
+                  mma_ts(t_o, t_p + ks * 8 + (term == 0 ? 32 : 0),
+                         vd + ks * (2048 >> 4) + (term == 1 ? kLo : 0), idesc_pv,
+                         (t > 0 || term > 0 || ks > 0) ? 1u : 0u);
+              }
             }
             tc_commit(b_o_done);
             tc_commit(bar_kv_empty + 8 * slot);
@@ -418,6 +433,7 @@ __global__ void __launch_bounds__(kThreadsF, 1)
             for (int i = 0; i < 8; ++i) mx = max(mx, finite_abs_bits(x[u][i]));
         }
         int e;
+        bool wide = false;
         if ((it & 1) == 0) {
           // K: by key. The row's pieces sit in the four lanes r8, r8 + 8, ...
           mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
@@ -429,11 +445,41 @@ __global__ void __launch_bounds__(kThreadsF, 1)
           }
           __syncwarp();  // the rows of this warp have been read
         } else {
-          // V: by tile
+          // V: by tile. How wide it is: the smallest nonzero maximum of a column among the warp's
+          // eight keys (the upper halves of two magnitudes in a word, each lane ends with its share of the
+          // columns; 1 below, so that none is zero) and of a key.
+          unsigned c2[4 * kUnits];
+#pragma unroll
+          for (int i = 0; i < 4 * kUnits; ++i)
+            c2[i] = __byte_perm(__float_as_uint(x[i / 4][2 * (i & 3)]), __float_as_uint(x[i / 4][2 * (i & 3) + 1]), 0x7632) &
+                    0x7fff7fffu;
+#pragma unroll
+          for (int step = 0; step < 3; ++step) {
+            const bool odd = (lane >> step) & 1;
+            const int n = (4 * kUnits) >> (step + 1);
+            if (n > 0) {
+#pragma unroll
+              for (int i = 0; i < 2 * kUnits; ++i)
+                if (i < n)
+                  c2[i] = __vmaxu2(odd ? c2[i + n] : c2[i],
+                                   __shfl_xor_sync(0xffffffffu, odd ? c2[i] : c2[i + n], 1 << step));
+            } else {
+              c2[0] = __vmaxu2(c2[0], __shfl_xor_sync(0xffffffffu, c2[0], 1 << step));
+            }
+          }
+          unsigned low2 = __vsub2(c2[0], 0x00010001u);
+          if constexpr (kUnits == 4) low2 = __vminu2(low2, __vsub2(c2[1], 0x00010001u));
+          mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
+          mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+          if (p4 == 0) smem[C::kOffVKey + ((it >> 1) & 7) * kBNf + sw * 8 + r8] = static_cast<unsigned char>(mx >> 23);
+          unsigned low = min(low2 & 0xffffu, low2 >> 16) + (kColRange << 7);
+          low = min(low, (mx == 0 ? 0xffffu : mx >> 16) + (kKeyRange << 7));
+          low = __reduce_min_sync(0xffffffffu, low);
           mx = __reduce_max_sync(0xffffffffu, mx);
           const int par = (it >> 1) & 1;
           if (lane == 0) {
-            red[par * 8 + sw] = mx;
+            red[par * 16 + sw] = mx;
+            red[par * 16 + 8 + sw] = low;
             mbar_arrive(bar_v_max);
           }
           // (an mbarrier and not bar.sync: a warp that gives up must not leave the others waiting)
@@ -442,20 +488,23 @@ __global__ void __launch_bounds__(kThreadsF, 1)
           if (!ok) break;
           mx = 0;
 #pragma unroll
-          for (int i = 0; i < 8; ++i) mx = max(mx, red[par * 8 + i]);
+          for (int i = 0; i < 8; ++i) mx = max(mx, red[par * 16 + i]), low = min(low, red[par * 16 + 8 + i]);
           e = scale_exp(mx, kMaxExp);
-          if (sw == 0 && lane == 0) v_exp[(it >> 1) & 15] = mx == 0 ? kNoUnit : e;
+          wide = low < mx >> 16;
+          if (sw == 0 && lane == 0) v_exp[(it >> 1) & 15] = mx == 0 ? kNoUnit : e + kExpBias + (wide ? kWide : 0);
         }
         const float sc = pow2i(e);
+        if (!wide) {  // (a wide tile stays as it is)
 #pragma unroll
-        for (int u = 0; u < kUnits; ++u) {
-          const int piece = p4 + 4 * u;  // split box pair = piece / 8
-          const unsigned hi_at = base + (piece >> 3) * 2 * C::kBoxBytes + (((piece & 7) ^ r8) << 4);
-          unsigned hi[4], lo[4];
+          for (int u = 0; u < kUnits; ++u) {
+            const int piece = p4 + 4 * u;  // split box pair = piece / 8
+            const unsigned hi_at = base + (piece >> 3) * 2 * C::kBoxBytes + (((piece & 7) ^ r8) << 4);
+            unsigned hi[4], lo[4];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) split_pair(x[u][2 * i] * sc, x[u][2 * i + 1] * sc, hi[i], lo[i]);
-          st_shared_u4(hi_at, hi[0], hi[1], hi[2], hi[3]);
-          st_shared_u4(hi_at + C::kBoxBytes, lo[0], lo[1], lo[2], lo[3]);
+            for (int i = 0; i < 4; ++i) split_pair(x[u][2 * i] * sc, x[u][2 * i + 1] * sc, hi[i], lo[i]);
+            st_shared_u4(hi_at, hi[0], hi[1], hi[2], hi[3]);
+            st_shared_u4(hi_at + C::kBoxBytes, lo[0], lo[1], lo[2], lo[3]);
+          }
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         mbar_arrive(bar_kv_full + 8 * slot);
@@ -523,7 +572,6 @@ __global__ void __launch_bounds__(kThreadsF, 1)
     float m_ref = -INFINITY;  // reference point of P, O and l, log2 units
     float l_run = 0.f;
     int unit = kNoUnit;       // O is in units of 2^-unit
-    int raised = 0;           // how far O has been scaled up over the unit it was accumulated in
     bool ok = true;
     int j = 0;
     const int n_seg = mine ? a.kmap.n_seg : 0;
@@ -590,8 +638,9 @@ __global__ void __launch_bounds__(kThreadsF, 1)
         // key of says nothing, and one of larger values only once a P that it meets would leave fp16. The
         // two terms of P have an absolute floor of 2^-25, so a tile of much smaller values (p_exp < 0) moves
         // the unit as well.
-        const int ev = v_exp[j & 15];
-        const bool adds = c_hi > c_lo && ev != kNoUnit;
+        const int ve = v_exp[j & 15], ev = ve - kExpBias;
+        const bool wide = (ve & kWide) != 0;
+        const bool adds = c_hi > c_lo && ve < kWide;
         if (adds && unit == kNoUnit) unit = kPBits + ev;
         int p_exp = adds ? unit - ev : kPBits;
         bool slow = __any_sync(0xffffffffu, p_exp < 0 || p_exp > 100 || (m_ref == -INFINITY && c_hi > c_lo)) != 0;
@@ -649,19 +698,29 @@ __global__ void __launch_bounds__(kThreadsF, 1)
             m_ref = tile_max;
           }
           l_run *= alpha;
+          // O as it stands is in units of 2^-keep of the new reference point. This tile's largest P,
+          // 2^-low of it, must not exceed 2^kPBits; and if its values are far smaller than the unit, O is
+          // scaled up, as far as it cannot overflow.
+          const int low = static_cast<int>(fminf(m_ref - tile_max, 100.f));
+          const int keep = unit + (m_old > -INFINITY ? static_cast<int>(fminf(m_ref - m_old, 1000.f)) : 0);
+          int to = adds ? min(keep, kPBits + ev + low) : unit;
+          if (j > 0 && __any_sync(0xffffffffu, adds && to < ev)) {
+            float top = 0.f;
+#pragma unroll 1
+            for (int c = 0; c < DR / 32; ++c) {
+              float o[32];
+              tmem_ld32(t_o + c * 32, o);
+#pragma unroll
+              for (int i = 0; i < 32; i += 2) top = max3(top, fabsf(o[i]), fabsf(o[i + 1]));
+            }
+            const int room = kOTop + 126 - (__float_as_int(top) >> 23);
+            if (adds && to < ev) to = max(to, min(kPBits + ev, keep + room));
+          }
           float oa = alpha;  // factor of O
           if (adds) {
-            // O as it stands is in units of 2^-keep of the new reference point. This tile's largest P,
-            // 2^-low of it, must not exceed 2^kPBits; and if its values are far smaller than the unit,
-            // O is scaled up, as far as it cannot overflow.
-            const int low = static_cast<int>(fminf(m_ref - tile_max, 100.f));
-            const int keep = unit + (m_old > -INFINITY ? static_cast<int>(fminf(m_ref - m_old, 1000.f)) : 0);
-            int to = min(keep, kPBits + ev + low);
-            if (to < ev) to = min(kPBits + ev, keep + kHeadroom - raised);
             if (m_old > -INFINITY) oa = ex2(m_old - m_ref + static_cast<float>(to - unit));
-            raised = max(0, raised + to - keep);
             unit = to;
-            p_exp = max(to - ev, -kHeadroom);  // (a P below 2^-25 adds nothing)
+            p_exp = max(to - ev, kMinPExp);
           }
           if (j > 0 && __any_sync(0xffffffffu, oa != 1.f)) {
             // O is at rest: P.V of tile j - 1 has completed
@@ -678,6 +737,50 @@ __global__ void __launch_bounds__(kThreadsF, 1)
         }
         l_run += row_sum * pow2i(-p_exp);
         tmem_wait_st();
+        if (wide && __any_sync(0xffffffffu, j == 0 || c_hi > c_lo)) {
+          // P * V of a wide tile in plain fp32: a row per thread, V as it landed in its ring slot (every
+          // lane reads the same 16 bytes). What the P written above says does not matter.
+          const float n = m_ref == -INFINITY ? 0.f : kPBits - m_ref;
+          int c_top = 0;  // biased exponents of P and V of the largest product
+#pragma unroll
+          for (int i = 0; i < kBNf; ++i) {
+            s[i] = ex2(fmaf(s[i], row_f, n));
+            const unsigned word = ld_shared_u1(s_base + C::kOffVKey + (j & 7) * kBNf + (i & ~3));
+            const int vk = (word >> (8 * (i & 3))) & 255;
+            if (s[i] > 0.f && vk > 0) c_top = max(c_top, (__float_as_int(s[i]) >> 23) + vk);
+          }
+          // unit: a product becomes at most 2^22
+          const int to = c_top == 0 ? unit : min(unit, min(kMaxExp, 22 - (c_top - 252 - kPBits)));
+          const float fac = unit == kNoUnit ? 1.f : ex2(static_cast<float>(to - unit));
+          unit = to;
+          const float p_sc = to == kNoUnit ? 0.f : pow2i(to - kPBits);
+#pragma unroll
+          for (int i = 0; i < kBNf; ++i) s[i] *= p_sc;
+          const unsigned v_at = s_kv + (vit % C::kStages) * C::kSlotBytes;
+#pragma unroll 1
+          for (int c = 0; c < DR; c += 8) {
+            const unsigned box = v_at + (c >> 5) * C::kBoxBytes;
+            const int chunk = (c & 31) >> 2;  // 16-byte chunk of the box's rows
+            float acc[8] = {};
+#pragma unroll
+            for (int i = 0; i < kBNf; ++i) {
+              const float4 v0 = ld_shared_f4(box + i * 128 + ((chunk ^ (i & 7)) << 4));
+              const float4 v1 = ld_shared_f4(box + i * 128 + (((chunk + 1) ^ (i & 7)) << 4));
+              acc[0] = fmaf(s[i], v0.x, acc[0]), acc[1] = fmaf(s[i], v0.y, acc[1]);
+              acc[2] = fmaf(s[i], v0.z, acc[2]), acc[3] = fmaf(s[i], v0.w, acc[3]);
+              acc[4] = fmaf(s[i], v1.x, acc[4]), acc[5] = fmaf(s[i], v1.y, acc[5]);
+              acc[6] = fmaf(s[i], v1.z, acc[6]), acc[7] = fmaf(s[i], v1.w, acc[7]);
+            }
+            if (j > 0) {
+              float o[8];
+              tmem_ld8(t_o + c, o);
+#pragma unroll
+              for (int i = 0; i < 8; ++i) acc[i] = fmaf(o[i], fac, acc[i]);
+            }
+            tmem_st8(t_o + c, acc);
+          }
+          tmem_wait_st();
+        }
         tc_fence_before();
         mbar_arrive(bar_p_full + 8 * w);
       }

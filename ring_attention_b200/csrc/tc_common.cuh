@@ -313,6 +313,24 @@ __device__ inline void tmem_st32(unsigned taddr, const float (&r)[32]) {
       "r"(__float_as_uint(r[30])), "r"(__float_as_uint(r[31]))
       : "memory");
 }
+__device__ inline void tmem_ld8(unsigned taddr, float (&r)[8]) {
+  unsigned u[8];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7])
+      : "r"(taddr)
+      : "memory");
+#pragma unroll
+  for (int i = 0; i < 8; ++i) r[i] = __uint_as_float(u[i]);
+}
+__device__ inline void tmem_st8(unsigned taddr, const float (&r)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr),
+               "r"(__float_as_uint(r[0])), "r"(__float_as_uint(r[1])), "r"(__float_as_uint(r[2])),
+               "r"(__float_as_uint(r[3])), "r"(__float_as_uint(r[4])), "r"(__float_as_uint(r[5])),
+               "r"(__float_as_uint(r[6])), "r"(__float_as_uint(r[7]))
+               : "memory");
+}
 __device__ inline void tmem_st16(unsigned taddr, const unsigned (&u)[16]) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "

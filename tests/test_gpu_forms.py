@@ -114,12 +114,35 @@ def _wide_inputs(case, D):
     S, every = 500, slice(None)
     q, k, v = (x.astype(np.float64) for x in normal_inputs(21, 1, 2, 2, S, S, D))
     kind, n = case
-    if kind == "document":  # boundary on a key tile's edge, inside a query block
-        v[:, :, :192] *= 2.0 ** n
-        return q, k, v, True, 192, [(slice(0, 192), every), (slice(192, 384), every), (slice(384, S), every)]
-    if kind == "future":
-        v[:, :, 192:] *= 2.0 ** n
-        return q, k, v, True, 0, [(slice(0, 192), every), (slice(192, S), every)]
+    if kind in ("document", "ragged document"):  # inside a query block, on a key tile's edge or not
+        at = 192 if kind == "document" else 230
+        v[:, :, :at] *= 2.0 ** n
+        return q, k, v, True, at, [(slice(0, at), every), (slice(at, 2 * at), every), (slice(2 * at, S), every)]
+    if kind in ("future", "ragged future"):
+        at = 192 if kind == "future" else 150
+        v[:, :, at:] *= 2.0 ** n
+        return q, k, v, True, 0, [(slice(0, at), every), (slice(at, S), every)]
+    if kind == "column":
+        v[..., 5] *= 2.0 ** n
+        return q, k, v, False, 0, [(every, slice(0, 5)), (every, slice(5, 6)), (every, slice(6, D))]
+    if kind == "element":  # in the first key tile; rows before it do not see it
+        v[:, :, 10, 3] = 2.0 ** n
+        return q, k, v, True, 0, [(slice(0, 10), every), (slice(10, S), slice(3, 4)), (slice(10, S), slice(4, D))]
+    if kind == "key":  # visible, under a weight of e^-40
+        q[..., 0], k[..., 0] = 4.0, 0.0
+        v[:, :, 100] *= 2.0 ** n
+        k[:, :, 100] = 0.0
+        k[:, :, 100, 0] = -10.0 * np.sqrt(D)
+        return q, k, v, False, 0, [(every, every)]
+    if kind == "every other key":  # values 2^n larger under weights about 2^n smaller
+        q[..., 0], k[..., 0] = 4.0, 0.0
+        v[:, :, ::2] *= 2.0 ** n
+        k[:, :, ::2, 0] = -n * np.log(2.0) / 4.0 * np.sqrt(D)
+        return q, k, v, False, 0, [(every, every)]
+    if kind == "small keys":
+        v[:, :, 64:] *= 2.0 ** n
+        v[:, :, 70:80] *= 2.0 ** -n
+        return q, k, v, True, 0, [(slice(0, 64), every), (slice(64, S), every)]
     if kind in ("first tile", "last tile"):  # values 2^n larger under weights about 2^n smaller
         at = slice(0, 64) if kind == "first tile" else slice(448, S)
         v[:, :, at] *= 2.0 ** n
@@ -138,7 +161,10 @@ def _wide_inputs(case, D):
 @pytest.mark.parametrize("split", [1, 3])
 @pytest.mark.parametrize("case", [("document", 20), ("document", 34), ("document", 100), ("document", -40), ("future", 40),
                                   ("first tile", 20), ("first tile", 34), ("last tile", 20), ("last tile", 34), ("V", -70), ("V", -90), ("V", -104), ("V", 120),
-                                  ("Q against K", 80), ("Q against K", -80), ("Q against K", 104), ("Q against K", -96)], ids=str)
+                                  ("ragged document", 12), ("ragged document", 34), ("ragged document", 100), ("ragged document", -100),
+                                  ("ragged future", 40), ("column", 20), ("column", 30), ("column", 100), ("element", 30),
+                                  ("element", 100), ("key", 24), ("key", 34), ("every other key", 20), ("every other key", 30),
+                                  ("small keys", -40), ("Q against K", 80), ("Q against K", -80), ("Q against K", 104), ("Q against K", -96)], ids=str)
 def test_fp32_step_holds_the_precision_of_every_part_of_the_output(D, split, case):
     # Values that a row cannot see, or sees under a negligible weight, must not cost it bits, nor may
     # one column cost another. Against 64 bits; 1e-5 of the part's largest value, the fp32 tolerance.
