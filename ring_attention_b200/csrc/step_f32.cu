@@ -7,12 +7,19 @@
 // Precision. hi + lo carry 22 bits like a pair of TF32 terms, and kind::f16 runs at twice the rate
 // of kind::tf32 with half the operand bytes and half the accumulations per product. What fp16
 // lacks is range, so values are scaled by powers of two first (exact): Q by row, K by key, V by
-// key tile, each so that the largest magnitude sits in [2^14, 2^15). An element keeps all 22 bits
-// down to 2^-17 of that largest one and an absolute 2^-40 of it below. P is fp32 until it is split
-// the same way (unit 2^kPBits), the row sums stay fp32. The dropped lo*lo and the rounding of lo
-// are about 2^-22 of a product; what shows in the output is the tensor core's fp32 accumulation
-// over the key tiles, as in any such kernel. RA_STEP_FORCE_SIMT selects the plain-fp32 kernel;
-// head_dim 256 keeps it (its split Q tiles and key ring exceed shared memory).
+// key tile, each so that the largest magnitude sits in [2^14, 2^15), and P by row and tile (see the unit
+// of O in the softmax). An element keeps 22 bits down to 2^-17 of that largest one and an absolute 2^-40
+// of it below; P keeps them down to 2^-11 of its largest and an absolute 2^-33. The row sums stay
+// fp32. The dropped lo*lo and the rounding of lo are about 2^-22 of a product; what shows in the
+// output is the tensor core's fp32 accumulation over the key tiles, as in any such kernel.
+// Where the shared scales do not hold what single elements need, a tile is marked and taken in plain
+// fp32 by the softmax threads: V tiles with a key or a column far below the tile's largest value, and
+// tiles whose products with Q span too much (kKeyRange, kColRange, kScoreRange). B1 H4 S16384 D128 causal:
+// 20 us for one marked tile in each head, 6.6 ms when a column of V lies 2^20 above the others (every
+// tile), 28 ms when a channel of Q lies 2^24 above and that of K 2^24 below the others (2.6 ms each on
+// TF32 pairs, which need no marks).
+// RA_STEP_FORCE_SIMT selects the plain-fp32 kernel; head_dim 256 keeps it (its split Q tiles and key
+// ring exceed shared memory).
 //
 // Work decomposition: grid = (batch * heads, 256-row query blocks), heavy blocks first; a block
 // owns two 128-row query tiles and walks the visible 64-key tiles of every key segment. Calls with
@@ -28,7 +35,8 @@
 //                 128: the hi term; lo goes as swizzled tiles into shared memory).
 //   warps 12-19   splitters: a landed raw tile is read into registers, scaled, split and written
 //                 back over itself, the hi tiles over the even 32-column boxes and the lo tiles over
-//                 the odd ones, in the layout TMA would give 16-bit data.
+//                 the odd ones, in the layout TMA would give 16-bit data. They also find the range of
+//                 every tile; a marked V tile stays as it landed.
 //   Head_dim 32 / 64: S and P have buffers of their own, so the scores of tile t+1 are computed
 //   while the softmax of tile t runs. Head_dim 128: P is written over S and the two query tiles take
 //   turns on the tensor core.
@@ -37,7 +45,7 @@
 // [192,224) Q lo [224,256); head_dim 128: S and P [0,64) O [64,192) Q hi [192,256).
 // What bounds it: at head_dim 128 the chain scores -> softmax -> P.V of the two query tiles, which take
 // turns on the tensor core (tensor pipe 44 %, issue slots 34 %). Measured, us per call, against one
-// 128-row tile per block on TF32 pairs: B1 H4 S16384 D128 causal 960 (2700), B1 H8 S1024 D64 dense 23
+// 128-row tile per block on TF32 pairs: B1 H4 S16384 D128 causal 830-950 (2700), B1 H8 S1024 D64 dense 23
 // (37), H4/kvH1 8231 x 9075 rows D64 causal 164 (272).
 //
 // Every wait on an mbarrier is bounded (see tc_common.cuh); a wait that runs out reports into
@@ -65,7 +73,12 @@ constexpr float kPSumLimit = 65000.f;  // of eight P: none of them then leaves f
 // that of some column among a splitter warp's eight keys below 2^-kColRange: what its elements lose
 // below 2^-40 of the tile's largest (and P below 2^-33) could then show in a row or a column.
 constexpr int kKeyRange = 9, kColRange = 16;
-constexpr int kExpBias = 512, kWide = 1 << 12;  // a tile's exponent as v_exp holds it
+// The scores of a query block and a key tile whose largest magnitudes multiply to 2^kScoreRange or more are
+// taken in plain fp32: what the terms lose (2^-40 of a row's or a key's largest element each) could
+// reach 2^-20 in a score.
+constexpr int kScoreRange = 17;
+// A tile as v_exp holds it: V's exponent + kExpBias, or kNoUnit, or kWide with or without kPlain.
+constexpr int kExpBias = 512, kWide = 1 << 12, kPlain = 1 << 13;
 
 template <int DR, bool kSplit>
 struct F32Cfg {
@@ -94,11 +107,12 @@ struct F32Cfg {
   static constexpr int kOffBar = kOffKV + kStages * kSlotBytes;
   static constexpr int kNumBars = 2 + 3 * kStages + 8 + 1;
   static constexpr int kOffSlot = kOffBar + kNumBars * 8;      // tensor-memory address, abort flag
-  static constexpr int kOffRed = kOffSlot + 8;                 // [2][2][8] range of a V tile by warp
+  static constexpr int kOffRed = (kOffSlot + 8 + 15) & ~15;    // [2][2][8] range of a V tile by warp
   static constexpr int kOffVExp = kOffRed + 128;               // [16] exponents of V tiles
   static constexpr int kOffG = (kOffVExp + 64 + 15) & ~15;     // [kGDepth][kBNf] factors of K
   static constexpr int kOffVKey = kOffG + kGDepth * kBNf * 4;  // [8][kBNf] exponents of V's keys
-  static constexpr int kOffMl = kOffVKey + 8 * kBNf;
+  static constexpr int kOffQTop = kOffVKey + 8 * kBNf;         // [2][4] exponents of Q by softmax warp
+  static constexpr int kOffMl = kOffQTop + 32;
   static constexpr int kMlBytes = kSplit ? kTiles * kBM * 8 : 0;
   static constexpr int kSmemBytes = kOffMl + kMlBytes;
   static constexpr int kColS = 0, kColP = kAlias ? 0 : 64, kColO = kAlias ? 64 : 128, kColQ = 192;
@@ -147,6 +161,11 @@ __device__ inline unsigned ld_shared_u1(unsigned addr) {
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
   return v;
 }
+__device__ inline uint4 ld_shared_u4(unsigned addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
+  return v;
+}
 __device__ inline float4 ld_shared_f4(unsigned addr) {
   float4 v;
   asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
@@ -163,7 +182,7 @@ template <int DR, bool kSplit>
 __global__ void __launch_bounds__(kThreadsF, 1)
     step_f32_kernel(const __grid_constant__ CUtensorMap tmap_k,
                     const __grid_constant__ CUtensorMap tmap_v, const float* __restrict__ q_g,
-                    const TcArgs a) {
+                    const float* __restrict__ k_g, long long kv_head_stride, const TcArgs a) {
   using C = F32Cfg<DR, kSplit>;
   extern __shared__ __align__(1024) unsigned char smem[];  // 128B-swizzled tiles
   const unsigned s_base = smem_u32(smem);
@@ -183,6 +202,7 @@ __global__ void __launch_bounds__(kThreadsF, 1)
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   volatile unsigned* red = reinterpret_cast<volatile unsigned*>(smem + C::kOffRed);
   volatile int* v_exp = reinterpret_cast<volatile int*>(smem + C::kOffVExp);
+  volatile int* q_tops = reinterpret_cast<volatile int*>(smem + C::kOffQTop);
 
   const int tid = threadIdx.x;
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
@@ -343,7 +363,7 @@ __global__ void __launch_bounds__(kThreadsF, 1)
           // MN-major V: 64 columns per 128-byte row, groups 2 boxes apart, 16 keys per k-step
           const unsigned long long vd =
               desc_mnmajor(s_kv + slot * C::kSlotBytes, 2 * C::kBoxBytes, 1024);
-          const bool wide = (v_exp[t & 15] & kWide) != 0;  // the softmax threads have added it to O
+          const bool wide = (v_exp[t & 15] & kWide) != 0;  // the softmax threads have added this tile to O
           if (elect_one()) {
             if (!wide) {
 #pragma unroll
@@ -404,6 +424,7 @@ __global__ void __launch_bounds__(kThreadsF, 1)
       const int sw = warp - 12, r8 = lane & 7, p4 = lane >> 3;
       const unsigned row_off = (sw * 8 + r8) * 128;
       bool ok = true;
+      int q_top = 0, k_top = 0;  // exponents: of the query block, of the warp's eight keys of the tile
       for (int it = 0; it < 2 * n_tiles && ok; ++it) {
         const int slot = it % C::kStages;
         ok = __all_sync(0xffffffffu, mbar_wait(bar_kv_raw + 8 * slot, (it / C::kStages) & 1, abort_flag,
@@ -443,42 +464,62 @@ __global__ void __launch_bounds__(kThreadsF, 1)
             const unsigned g = s_base + C::kOffG + (((it >> 1) % C::kGDepth) * kBNf + sw * 8 + r8) * 4;
             asm volatile("st.shared.f32 [%0], %1;" ::"r"(g), "f"(pow2i(-e - kBias)) : "memory");
           }
-          __syncwarp();  // the rows of this warp have been read
+          k_top = static_cast<int>(__reduce_max_sync(0xffffffffu, mx) >> 23);  // (the warp's rows have been read)
         } else {
-          // V: by tile. How wide it is: the smallest nonzero maximum of a column among the warp's
-          // eight keys (the upper halves of two magnitudes in a word, each lane ends with its share of the
-          // columns; 1 below, so that none is zero) and of a key.
-          unsigned c2[4 * kUnits];
+          // V: by tile. How wide it is: the smallest nonzero maximum of a key and of a column among the
+          // warp's eight keys. No column lies below the warp's smallest element, which is near enough for
+          // most tiles.
+          float fn = fabsf(x[0][0]);
 #pragma unroll
-          for (int i = 0; i < 4 * kUnits; ++i)
-            c2[i] = __byte_perm(__float_as_uint(x[i / 4][2 * (i & 3)]), __float_as_uint(x[i / 4][2 * (i & 3) + 1]), 0x7632) &
-                    0x7fff7fffu;
+          for (int u = 0; u < kUnits; ++u)
 #pragma unroll
-          for (int step = 0; step < 3; ++step) {
-            const bool odd = (lane >> step) & 1;
-            const int n = (4 * kUnits) >> (step + 1);
-            if (n > 0) {
-#pragma unroll
-              for (int i = 0; i < 2 * kUnits; ++i)
-                if (i < n)
-                  c2[i] = __vmaxu2(odd ? c2[i + n] : c2[i],
-                                   __shfl_xor_sync(0xffffffffu, odd ? c2[i] : c2[i + n], 1 << step));
-            } else {
-              c2[0] = __vmaxu2(c2[0], __shfl_xor_sync(0xffffffffu, c2[0], 1 << step));
-            }
-          }
-          unsigned low2 = __vsub2(c2[0], 0x00010001u);
-          if constexpr (kUnits == 4) low2 = __vminu2(low2, __vsub2(c2[1], 0x00010001u));
+            for (int i = 0; i < 8; i += 2) fn = min3(fn, fabsf(x[u][i]), fabsf(x[u][i + 1]));
           mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
           mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
           if (p4 == 0) smem[C::kOffVKey + ((it >> 1) & 7) * kBNf + sw * 8 + r8] = static_cast<unsigned char>(mx >> 23);
-          unsigned low = min(low2 & 0xffffu, low2 >> 16) + (kColRange << 7);
-          low = min(low, (mx == 0 ? 0xffffu : mx >> 16) + (kKeyRange << 7));
-          low = __reduce_min_sync(0xffffffffu, low);
+          unsigned low = (mx == 0 ? 0xffffu : mx >> 16) + (kKeyRange << 7);
+          const unsigned low_all = (__reduce_min_sync(0xffffffffu, __float_as_uint(fn)) >> 16) + (kColRange << 7);
           mx = __reduce_max_sync(0xffffffffu, mx);
+          if (__builtin_expect(low_all - (1u << 7) >= mx >> 16, 1)) {
+            low = min(low, low_all);
+          } else {
+            // column by column, the upper halves of two magnitudes in a word; each lane ends with its
+            // share of the columns (1 below, so that none is zero)
+            unsigned c2[4 * kUnits];
+#pragma unroll
+            for (int i = 0; i < 4 * kUnits; ++i)
+              c2[i] = __byte_perm(__float_as_uint(x[i / 4][2 * (i & 3)]), __float_as_uint(x[i / 4][2 * (i & 3) + 1]),
+                                  0x7632) & 0x7fff7fffu;
+#pragma unroll
+            for (int step = 0; step < 3; ++step) {
+              const bool odd = (lane >> step) & 1;
+              const int n = (4 * kUnits) >> (step + 1);
+              if (n > 0) {
+#pragma unroll
+                for (int i = 0; i < 2 * kUnits; ++i)
+                  if (i < n)
+                    c2[i] = __vmaxu2(odd ? c2[i + n] : c2[i],
+                                     __shfl_xor_sync(0xffffffffu, odd ? c2[i] : c2[i + n], 1 << step));
+              } else {
+                c2[0] = __vmaxu2(c2[0], __shfl_xor_sync(0xffffffffu, c2[0], 1 << step));
+              }
+            }
+            unsigned low2 = __vsub2(c2[0], 0x00010001u);
+            if constexpr (kUnits == 4) low2 = __vminu2(low2, __vsub2(c2[1], 0x00010001u));
+            low = min(low, min(low2 & 0xffffu, low2 >> 16) + (kColRange << 7));
+          }
+          low = __reduce_min_sync(0xffffffffu, low);
+          if (it == 1) {
+            for (int w = 0; w < live && ok; ++w) {
+              ok = __all_sync(0xffffffffu, mbar_wait(bar_q_full + 8 * w, 0, abort_flag, a.status, 3, w, a.wait_ns)) != 0;
+              if (ok) q_top = max(q_top, max(max(q_tops[4 * w], q_tops[4 * w + 1]), max(q_tops[4 * w + 2], q_tops[4 * w + 3])));
+            }
+            if (!ok) break;
+          }
+          const bool plain = q_top + k_top - 254 >= kScoreRange;
           const int par = (it >> 1) & 1;
           if (lane == 0) {
-            red[par * 16 + sw] = mx;
+            red[par * 16 + sw] = mx | (plain ? 0x80000000u : 0u);
             red[par * 16 + 8 + sw] = low;
             mbar_arrive(bar_v_max);
           }
@@ -486,12 +527,18 @@ __global__ void __launch_bounds__(kThreadsF, 1)
           ok = __all_sync(0xffffffffu,
                           mbar_wait(bar_v_max, par, abort_flag, a.status, 15, it, a.wait_ns)) != 0;
           if (!ok) break;
-          mx = 0;
-#pragma unroll
-          for (int i = 0; i < 8; ++i) mx = max(mx, red[par * 16 + i]), low = min(low, red[par * 16 + 8 + i]);
+          const unsigned red_at = s_base + C::kOffRed + par * 64;
+          const uint4 m0 = ld_shared_u4(red_at), m1 = ld_shared_u4(red_at + 16);
+          const uint4 l0 = ld_shared_u4(red_at + 32), l1 = ld_shared_u4(red_at + 48);
+          const unsigned marks = (m0.x | m0.y | m0.z | m0.w) | (m1.x | m1.y | m1.z | m1.w);
+          constexpr unsigned kMag = 0x7fffffffu;
+          mx = max(max(max(m0.x & kMag, m0.y & kMag), max(m0.z & kMag, m0.w & kMag)),
+                   max(max(m1.x & kMag, m1.y & kMag), max(m1.z & kMag, m1.w & kMag)));
+          low = min(min(min(l0.x, l0.y), min(l0.z, l0.w)), min(min(l1.x, l1.y), min(l1.z, l1.w)));
           e = scale_exp(mx, kMaxExp);
-          wide = low < mx >> 16;
-          if (sw == 0 && lane == 0) v_exp[(it >> 1) & 15] = mx == 0 ? kNoUnit : e + kExpBias + (wide ? kWide : 0);
+          wide = low < mx >> 16 || marks > kMag;
+          if (sw == 0 && lane == 0)
+            v_exp[(it >> 1) & 15] = wide ? (marks > kMag ? kWide | kPlain : kWide) : mx == 0 ? kNoUnit : e + kExpBias;
         }
         const float sc = pow2i(e);
         if (!wide) {  // (a wide tile stays as it is)
@@ -529,6 +576,8 @@ __global__ void __launch_bounds__(kThreadsF, 1)
     const bool mine = w < live && n_tiles > 0;
 
     // ---- this row of Q: scale, split, hand to the MMA warp
+    // 1 / sqrt(head_dim) in log2 units
+    constexpr float kPlainF = (DR == 32 ? 0.17677669529663689f : DR == 64 ? 0.125f : 0.08838834764831845f) * kLog2e;
     float row_f = 0.f;  // turns a scaled score (K factor applied) into log2 units
     if (mine) {
       const float4* q4 = reinterpret_cast<const float4*>(q_g + grow * DR);
@@ -541,7 +590,9 @@ __global__ void __launch_bounds__(kThreadsF, 1)
       }
       const int e = scale_exp(mx, kMaxExp);
       const float sc = pow2i(e);
-      row_f = rsqrtf(static_cast<float>(DR)) * kLog2e * pow2i(kBias - e);
+      mx = __reduce_max_sync(0xffffffffu, mx);
+      if (lane == 0) q_tops[warp - 4] = static_cast<int>(mx >> 23);
+      row_f = kPlainF * pow2i(kBias - e);
 #pragma unroll
       for (int g = 0; g < DR / 32; ++g) {  // 32 columns at a time (second read: L1 / L2)
         unsigned hi[16], lo[16];
@@ -609,18 +660,140 @@ __global__ void __launch_bounds__(kThreadsF, 1)
         // reused before this softmax is done
         const int vit = 2 * j + 1;
         ok = mbar_wait(bar_kv_full + 8 * (vit % C::kStages), (vit / C::kStages) & 1, abort_flag, a.status,
-                       11, j, a.wait_ns) &&
-             mbar_wait(bar_s_full + 8 * w, j & 1, abort_flag, a.status, 7, j, a.wait_ns);
+                       11, j, a.wait_ns);
+        const int ve = v_exp[j & 15];
+        ok = ok && mbar_wait(bar_s_full + 8 * w, j & 1, abort_flag, a.status, 7, j, a.wait_ns);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tc_fence_after();
+        const unsigned g_at = s_base + C::kOffG + (j % C::kGDepth) * kBNf * 4;
+        if (__builtin_expect((ve & kWide) != 0, 0)) {
+          // A marked tile: P * V in plain fp32 from V as it landed in its slot (every lane reads the same
+          // 16 bytes), and the scores too if Q and K ask for it. Short loops over tensor memory, so that
+          // the registers of the common path do not suffer. The issuer only passes the barriers on.
+          if (!C::kAlias && j > 0) {
+            ok = mbar_wait(bar_o_done + 8 * w, (j - 1) & 1, abort_flag, a.status, 10, j, a.wait_ns);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            tc_fence_after();
+          }
+          const bool any = __any_sync(0xffffffffu, c_hi > c_lo) != 0;
+          if (any && (ve & kPlain) != 0) {
+            // eight keys at a time, Q and K from memory (the K slot may have been given back), scaled as
+            // the tensor core's scores are, in their place
+            const float4* q4 = reinterpret_cast<const float4*>(q_g + grow * DR);
+            const float* k_t = k_g + (a.kseg_head[sk] + kv_bh) * kv_head_stride +
+                               static_cast<long long>(a.kseg_row[sk] + t * kBNf) * DR;
+            const int last = min(kBNf, a.kmap.seg_len - t * kBNf) - 1;
+            const float unscale = pow2i((__float_as_int(kPlainF) >> 23) - (__float_as_int(row_f) >> 23));
+#pragma unroll 1
+            for (int i0 = 0; i0 < kBNf; i0 += 8) {
+              float x[8] = {};
+#pragma unroll 1
+              for (int c = 0; c < DR / 4; ++c) {
+                const float4 qv = row_valid ? q4[c] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                  const float4 kv = *reinterpret_cast<const float4*>(k_t + min(i0 + i, last) * DR + 4 * c);
+                  x[i] = fmaf(qv.w, kv.w, fmaf(qv.z, kv.z, fmaf(qv.y, kv.y, fmaf(qv.x, kv.x, x[i]))));
+                }
+              }
+#pragma unroll
+              for (int i = 0; i < 8; ++i)
+                x[i] = x[i] * unscale * pow2i(127 - static_cast<int>(ld_shared_u1(g_at + (i0 + i) * 4) >> 23));
+              tmem_st8(t_s + i0, x);
+            }
+            tmem_wait_st();
+          }
+          auto scores = [&](int i0, float (&x)[8]) {
+            tmem_ld8(t_s + i0, x);
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+              x[i] = i0 + i >= c_lo && i0 + i < c_hi ? x[i] * __uint_as_float(ld_shared_u1(g_at + (i0 + i) * 4)) : -INFINITY;
+          };
+          float alpha = 1.f;
+          int c_top = 0;  // biased exponents of P and V of the largest product
+          if (any) {
+            float mx = -INFINITY, x[8];
+#pragma unroll 1
+            for (int i0 = 0; i0 < kBNf; i0 += 8) {
+              scores(i0, x);
+#pragma unroll
+              for (int i = 0; i < 8; ++i) mx = fmaxf(mx, x[i]);
+            }
+            const float tile_max = mx * row_f;
+            if (tile_max > m_ref) {
+              if (m_ref > -INFINITY) alpha = ex2(m_ref - tile_max);
+              m_ref = tile_max;
+            }
+            const float n = m_ref == -INFINITY ? 0.f : kPBits - m_ref;
+            float sum = 0.f;
+#pragma unroll 1
+            for (int i0 = 0; i0 < kBNf; i0 += 8) {  // P as fp32 over the columns of its terms
+              scores(i0, x);
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {
+                x[i] = ex2(fmaf(x[i], row_f, n));
+                sum += x[i];
+                const int vk = smem[C::kOffVKey + (j & 7) * kBNf + i0 + i];
+                if (x[i] > 0.f && vk > 0) c_top = max(c_top, (__float_as_int(x[i]) >> 23) + vk);
+              }
+              tmem_st8(t_p + i0, x);
+            }
+            tmem_wait_st();
+            l_run = l_run * alpha + sum * pow2i(-kPBits);
+          }
+          if constexpr (!C::kAlias) {
+            tc_fence_before();
+            mbar_arrive(bar_s_free + 8 * w);
+          }
+          if (any || j == 0) {
+            // unit: a product becomes at most 2^22
+            const int to = c_top == 0 ? unit : min(unit, min(kMaxExp, 22 - (c_top - 252 - kPBits)));
+            const float fac = unit == kNoUnit ? alpha : alpha * ex2(static_cast<float>(to - unit));
+            unit = to;
+            const float p_sc = to == kNoUnit ? 0.f : pow2i(to - kPBits);
+            const unsigned v_at = s_kv + (vit % C::kStages) * C::kSlotBytes;
+#pragma unroll 1
+            for (int c = 0; c < DR; c += 16) {
+              const unsigned box = v_at + (c >> 5) * C::kBoxBytes;
+              float acc[16] = {};
+#pragma unroll 1
+              for (int i0 = 0; any && i0 < kBNf; i0 += 8) {
+                float p[8];
+                tmem_ld8(t_p + i0, p);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                  p[i] *= p_sc;
+#pragma unroll
+                  for (int u = 0; u < 4; ++u) {  // 16-byte chunks of the row
+                    const float4 v = ld_shared_f4(box + (i0 + i) * 128 + ((((c & 31) >> 2) + u) ^ i) * 16);
+                    acc[4 * u] = fmaf(p[i], v.x, acc[4 * u]), acc[4 * u + 1] = fmaf(p[i], v.y, acc[4 * u + 1]);
+                    acc[4 * u + 2] = fmaf(p[i], v.z, acc[4 * u + 2]), acc[4 * u + 3] = fmaf(p[i], v.w, acc[4 * u + 3]);
+                  }
+                }
+              }
+#pragma unroll
+              for (int u = 0; u < 16; u += 8) {
+                float o[8] = {};
+                if (j > 0) tmem_ld8(t_o + c + u, o);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) o[i] = fmaf(o[i], fac, acc[u + i]);
+                tmem_st8(t_o + c + u, o);
+              }
+            }
+            tmem_wait_st();
+          }
+          tc_fence_before();
+          mbar_arrive(bar_p_full + 8 * w);
+          continue;
+        }
         float s[kBNf];
         tmem_ld64(t_s, s);
         if constexpr (!C::kAlias) {
           tc_fence_before();
           mbar_arrive(bar_s_free + 8 * w);  // the tensor core may write the next scores
         }
-        const unsigned g_at = s_base + C::kOffG + (j % C::kGDepth) * kBNf * 4;
 #pragma unroll
         for (int i = 0; i < kBNf; i += 4) {
           const float4 g = ld_shared_f4(g_at + i * 4);
@@ -638,8 +811,7 @@ __global__ void __launch_bounds__(kThreadsF, 1)
         // key of says nothing, and one of larger values only once a P that it meets would leave fp16. The
         // two terms of P have an absolute floor of 2^-25, so a tile of much smaller values (p_exp < 0) moves
         // the unit as well.
-        const int ve = v_exp[j & 15], ev = ve - kExpBias;
-        const bool wide = (ve & kWide) != 0;
+        const int ev = ve - kExpBias;
         const bool adds = c_hi > c_lo && ve < kWide;
         if (adds && unit == kNoUnit) unit = kPBits + ev;
         int p_exp = adds ? unit - ev : kPBits;
@@ -737,50 +909,6 @@ __global__ void __launch_bounds__(kThreadsF, 1)
         }
         l_run += row_sum * pow2i(-p_exp);
         tmem_wait_st();
-        if (wide && __any_sync(0xffffffffu, j == 0 || c_hi > c_lo)) {
-          // P * V of a wide tile in plain fp32: a row per thread, V as it landed in its ring slot (every
-          // lane reads the same 16 bytes). What the P written above says does not matter.
-          const float n = m_ref == -INFINITY ? 0.f : kPBits - m_ref;
-          int c_top = 0;  // biased exponents of P and V of the largest product
-#pragma unroll
-          for (int i = 0; i < kBNf; ++i) {
-            s[i] = ex2(fmaf(s[i], row_f, n));
-            const unsigned word = ld_shared_u1(s_base + C::kOffVKey + (j & 7) * kBNf + (i & ~3));
-            const int vk = (word >> (8 * (i & 3))) & 255;
-            if (s[i] > 0.f && vk > 0) c_top = max(c_top, (__float_as_int(s[i]) >> 23) + vk);
-          }
-          // unit: a product becomes at most 2^22
-          const int to = c_top == 0 ? unit : min(unit, min(kMaxExp, 22 - (c_top - 252 - kPBits)));
-          const float fac = unit == kNoUnit ? 1.f : ex2(static_cast<float>(to - unit));
-          unit = to;
-          const float p_sc = to == kNoUnit ? 0.f : pow2i(to - kPBits);
-#pragma unroll
-          for (int i = 0; i < kBNf; ++i) s[i] *= p_sc;
-          const unsigned v_at = s_kv + (vit % C::kStages) * C::kSlotBytes;
-#pragma unroll 1
-          for (int c = 0; c < DR; c += 8) {
-            const unsigned box = v_at + (c >> 5) * C::kBoxBytes;
-            const int chunk = (c & 31) >> 2;  // 16-byte chunk of the box's rows
-            float acc[8] = {};
-#pragma unroll
-            for (int i = 0; i < kBNf; ++i) {
-              const float4 v0 = ld_shared_f4(box + i * 128 + ((chunk ^ (i & 7)) << 4));
-              const float4 v1 = ld_shared_f4(box + i * 128 + (((chunk + 1) ^ (i & 7)) << 4));
-              acc[0] = fmaf(s[i], v0.x, acc[0]), acc[1] = fmaf(s[i], v0.y, acc[1]);
-              acc[2] = fmaf(s[i], v0.z, acc[2]), acc[3] = fmaf(s[i], v0.w, acc[3]);
-              acc[4] = fmaf(s[i], v1.x, acc[4]), acc[5] = fmaf(s[i], v1.y, acc[5]);
-              acc[6] = fmaf(s[i], v1.z, acc[6]), acc[7] = fmaf(s[i], v1.w, acc[7]);
-            }
-            if (j > 0) {
-              float o[8];
-              tmem_ld8(t_o + c, o);
-#pragma unroll
-              for (int i = 0; i < 8; ++i) acc[i] = fmaf(o[i], fac, acc[i]);
-            }
-            tmem_st8(t_o + c, acc);
-          }
-          tmem_wait_st();
-        }
         tc_fence_before();
         mbar_arrive(bar_p_full + 8 * w);
       }
@@ -912,7 +1040,8 @@ int launch_f32(const StepArgs& a, cudaStream_t stream, int key_split) {
   attr.val.clusterDim.z = 1;
   cfg.attrs = &attr;
   cfg.numAttrs = kSplit ? 1 : 0;
-  RAB_CUDA(cudaLaunchKernelEx(&cfg, kern, mk, mv, static_cast<const float*>(a.q), t));
+  RAB_CUDA(cudaLaunchKernelEx(&cfg, kern, mk, mv, static_cast<const float*>(a.q), static_cast<const float*>(a.k),
+                              a.kv_head_stride, t));
   RAB_CUDA(cudaGetLastError());
   return RA_OK;
 }

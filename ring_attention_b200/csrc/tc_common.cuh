@@ -358,6 +358,11 @@ __device__ inline float max3(float a, float b, float c) {
   asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
   return d;
 }
+__device__ inline float min3(float a, float b, float c) {
+  float d;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
 // packed fp32x2 arithmetic: one instruction for two lanes of a float2
 __device__ inline float2 ffma2(float2 a, float2 b, float2 c) {
   float2 d;

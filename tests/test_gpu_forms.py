@@ -150,6 +150,16 @@ def _wide_inputs(case, D):
         k[:, :, at] *= 0.1
         k[:, :, at, 0] = -n * np.log(2.0) / 4.0 * np.sqrt(D)
         return q, k, v, False, 0, [(every, every)]
+    if kind == "channel":  # one element of every Q row far larger, of every key far smaller
+        q[..., 0] *= 2.0 ** n
+        k[..., 0] *= 2.0 ** -n
+        return q, k, v, False, 0, [(every, every)]
+    if kind == "channels apart":  # large elements that do not meet, in some rows and keys
+        q[:, :, ::3, 0] = 2.0 ** n
+        q[..., 1] = 0.0
+        k[..., 0] = 0.0
+        k[:, :, 130::7, 1] = 2.0 ** n
+        return q, k, v, True, 0, [(every, every)]
     if kind == "V":
         return q, k, v * 2.0 ** n, False, 0, [(every, every)]
     if kind == "Q against K":
@@ -164,7 +174,7 @@ def _wide_inputs(case, D):
                                   ("ragged document", 12), ("ragged document", 34), ("ragged document", 100), ("ragged document", -100),
                                   ("ragged future", 40), ("column", 20), ("column", 30), ("column", 100), ("element", 30),
                                   ("element", 100), ("key", 24), ("key", 34), ("every other key", 20), ("every other key", 30),
-                                  ("small keys", -40), ("Q against K", 80), ("Q against K", -80), ("Q against K", 104), ("Q against K", -96)], ids=str)
+                                  ("small keys", -40), ("Q against K", 80), ("Q against K", -80), ("channel", 24), ("channel", 40), ("channels apart", 26), ("Q against K", 104), ("Q against K", -96)], ids=str)
 def test_fp32_step_holds_the_precision_of_every_part_of_the_output(D, split, case):
     # Values that a row cannot see, or sees under a negligible weight, must not cost it bits, nor may
     # one column cost another. Against 64 bits; 1e-5 of the part's largest value, the fp32 tolerance.
