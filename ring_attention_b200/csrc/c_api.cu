@@ -437,7 +437,9 @@ int ra_kv_cache_create(int dtype, int batch, int kv_heads, int s_max, int head_d
               "ra_kv_cache_create: bad sizes");
   RAB_REQUIRE(dtype == RA_F32 || dtype == RA_F16 || dtype == RA_BF16, RA_ERR_INVALID,
               "ra_kv_cache_create: unknown dtype %d", dtype);
-  ra_kv_cache* c = new ra_kv_cache{dtype, batch, kv_heads, s_max, head_dim, 0, nullptr, nullptr};
+  int dev = 0;
+  RAB_CUDA(cudaGetDevice(&dev));
+  ra_kv_cache* c = new ra_kv_cache{dtype, batch, kv_heads, s_max, head_dim, 0, dev, nullptr, nullptr};
   const size_t bytes =
       static_cast<size_t>(batch) * kv_heads * s_max * head_dim * elem_size(dtype);
   if (cudaMalloc(&c->k, bytes) != cudaSuccess || cudaMalloc(&c->v, bytes) != cudaSuccess) {
@@ -465,17 +467,31 @@ void ra_kv_cache_reset(ra_kv_cache* c) {
   if (c) c->current_len = 0;
 }
 
-// Whether a kernel on the current device can read elements of `es` bytes at p (a copy can also
-// reach memory that is not mapped here).
-static bool readable_here(const void* p, size_t es) {
+// A copy reaches memory of every kind and device and may go into a stream of any; a kernel reads and writes
+// only what the current device has mapped, and needs a stream of it. So a token's rows go by the kernel
+// only if sources, cache and stream are all the current device's (-1: not device memory, or not known).
+int ra_debug_append_route(int device, int cache_device, int stream_device, int k_device, int v_device) {
+  return device >= 0 && cache_device == device && stream_device == device && k_device == device && v_device == device;
+}
+
+static int device_of_memory(const void* p, size_t es) {
   cudaPointerAttributes at;
-  int dev = 0;
-  if (reinterpret_cast<uintptr_t>(p) % es != 0 || cudaGetDevice(&dev) != cudaSuccess) return false;
+  if (reinterpret_cast<uintptr_t>(p) % es != 0) return -1;
   if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
     cudaGetLastError();
-    return false;
+    return -1;
   }
-  return at.type == cudaMemoryTypeDevice && at.device == dev;
+  return at.type == cudaMemoryTypeDevice ? at.device : -1;
+}
+
+static int device_of_stream(cudaStream_t stream, int current) {
+  if (stream == nullptr || stream == cudaStreamLegacy || stream == cudaStreamPerThread) return current;
+  int dev = -1;
+  if (cudaStreamGetDevice(stream, &dev) != cudaSuccess) {
+    cudaGetLastError();
+    return -1;
+  }
+  return dev;
 }
 
 // Strided copy of `rows` rows per (batch, kv head) into the cache starting at row `at`
@@ -488,7 +504,11 @@ static int cache_copy(ra_kv_cache* c, const void* k_src, const void* v_src, int 
   const size_t height = static_cast<size_t>(c->batch) * c->kv_heads;
   const size_t off = static_cast<size_t>(at) * c->head_dim * es;
   if (width == 0) return RA_OK;
-  if (rows == 1 && height <= 65535 && readable_here(k_src, es) && readable_here(v_src, es))
+  int dev = 0;
+  RAB_CUDA(cudaGetDevice(&dev));
+  if (rows == 1 && height <= 65535 && c->device == dev &&
+      ra_debug_append_route(dev, c->device, device_of_stream(stream, dev), device_of_memory(k_src, es),
+                            device_of_memory(v_src, es)))
     return launch_cache_row(k_src, v_src, static_cast<unsigned char*>(c->k) + off,
                             static_cast<unsigned char*>(c->v) + off, width, dpitch,
                             static_cast<int>(height), stream);

@@ -15,6 +15,7 @@
 // The cache handle of the C ABI: K and V of shape (batch, kv_heads, s_max, head_dim).
 struct ra_kv_cache {
   int dtype, batch, kv_heads, s_max, head_dim, current_len;
+  int device;  // that k and v are on
   void* k;
   void* v;
 };

@@ -177,3 +177,11 @@ def test_ring2d_data_movement_delivers_the_shard_the_schedule_names(N, G):
         seed = [seed[((r // G - 1) % N) * G + r % G] for r in range(P)]
     for r in range(P):
         assert sorted(seen[r]) == list(range(P))
+
+
+@pytest.mark.parametrize("cache,stream,k,v", [(0, 1, 1, 1), (1, 0, 1, 1), (1, 1, 0, 1), (1, 1, 1, 0), (1, 1, -1, 1),
+                                              (1, 1, 1, -1), (1, -1, 1, 1), (-1, 1, 1, 1)])
+def test_a_cache_append_across_devices_stays_with_the_copies(cache, stream, k, v):
+    # a kernel on device 1 must not touch what only a copy can reach
+    assert lib().ra_debug_append_route(1, 1, 1, 1, 1) == 1
+    assert lib().ra_debug_append_route(1, cache, stream, k, v) == 0

@@ -285,3 +285,21 @@ def test_decode_and_key_split_replay_from_a_captured_graph(dtype, heads, kv_head
     both()
     torch.cuda.synchronize()
     assert torch.equal(got1, o1) and torch.equal(gotn, on) and api.device_status()[0] == 0
+
+
+def test_cache_append_on_a_stream_of_its_own_and_from_a_captured_graph():
+    cache = api.DeviceKVCache(2, 3, 4, 64, torch.float16)
+    rows = torch.randn(4, 2, 2, 3, 1, 64, device="cuda").half()
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        cache.append(rows[0, 0], rows[0, 1])
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        cache.append(rows[1, 0], rows[1, 1])
+    rows[1].copy_(rows[2])
+    graph.replay()
+    torch.cuda.synchronize()
+    for i, src in enumerate((0, 2)):
+        assert torch.equal(cache.k_view()[:, :, i], rows[src, 0, :, :, 0]) and torch.equal(cache.v_view()[:, :, i], rows[src, 1, :, :, 0])
