@@ -486,8 +486,11 @@ static int device_of_memory(const void* p, size_t es) {
 
 static int device_of_stream(cudaStream_t stream, int current) {
   if (stream == nullptr || stream == cudaStreamLegacy || stream == cudaStreamPerThread) return current;
+  // (the question itself would end a capture, so a captured append is two copies)
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
   int dev = -1;
-  if (cudaStreamGetDevice(stream, &dev) != cudaSuccess) {
+  if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone ||
+      cudaStreamGetDevice(stream, &dev) != cudaSuccess) {
     cudaGetLastError();
     return -1;
   }
