@@ -190,8 +190,8 @@ constexpr double kFoldUs = 3.0, kMergeUs = 1.0;  // see make_plan
 // `part` of the workspace or is merged over the cluster and folded into the state.
 template <int ROWS, int D, int NWARPS, DealForm kForm>
 __device__ inline void finish_group(float* red_m, float* red_l, float* red_o, int b, int kvh, int hb, int H,
-                                    int kvH, int part, const Deal& deal, float* __restrict__ Mp,
-                                    float* __restrict__ Lp, float* __restrict__ Op) {
+                                    int kvH, int part, const Deal& deal, float* Mp, float* Lp,
+                                    float* Op) {
   constexpr int kThr = NWARPS * 32;
   const int tid = threadIdx.x;
   const int first = kvh + kvH * hb * ROWS;
@@ -323,7 +323,7 @@ __device__ inline void finish_group(float* red_m, float* red_l, float* red_o, in
 template <typename T, int D, int GB, DealForm kForm>
 __global__ void __launch_bounds__(kThreads)
     decode_split_kernel(const T* __restrict__ Q, const T* __restrict__ K, const T* __restrict__ V,
-                        float* __restrict__ Mp, float* __restrict__ Lp, float* __restrict__ Op, int H,
+                        float* Mp, float* Lp, float* Op, int H,
                         int kvH, int sk_eff, long long kv_head_stride, const Deal deal, float scale_log2) {
   using C = DecodeCfg<T, D, GB>;
   extern __shared__ __align__(16) unsigned char smem[];
@@ -573,7 +573,7 @@ struct MmaCfg {
 template <typename T, int D, DealForm kForm>
 __global__ void __launch_bounds__(MmaCfg<D>::kThreads)
     decode_mma_kernel(const T* __restrict__ Q, const T* __restrict__ K, const T* __restrict__ V,
-                      float* __restrict__ Mp, float* __restrict__ Lp, float* __restrict__ Op, int H,
+                      float* Mp, float* Lp, float* Op, int H,
                       int kvH, int sk_eff, long long kv_head_stride, const Deal deal, float scale_log2) {
   using C = MmaCfg<D>;
   extern __shared__ __align__(16) unsigned char smem[];
@@ -757,16 +757,16 @@ __global__ void __launch_bounds__(MmaCfg<D>::kThreads)
 // D x kFoldThreads / D threads: the partials are dealt to the thread groups (a single group walked up
 // to 57 partials one after the other, twice: 8 of the 36 us of the B1 H8 D128 fp32 call on 16384
 // rows) and (m, l) are read by lanes. Launched while the split kernel still runs (programmatic
-// dependent launch); everything it reads comes after griddepcontrol.wait.
+// dependent launch): everything it reads comes after griddepcontrol.wait and through plain pointers, because
+// the data changes while this kernel runs (const __restrict__ would allow loads through the read-only
+// path and in front of the wait).
 // RA_STEP_FRESH: the state is known to be empty (it is written, never read, which saves the
 // caller an init launch); RA_STEP_FINALIZE: divide by l after folding (saves the finalize
 // launch).
 constexpr int kFoldThreads = 512;
 __global__ void __launch_bounds__(kFoldThreads)
-    decode_reduce_kernel(const float* __restrict__ Mp, const float* __restrict__ Lp,
-                         const float* __restrict__ Op, float* __restrict__ M, float* __restrict__ L,
-                         float* __restrict__ O, int H, int kvH, int D, int head_rows, int ctas,
-                         const Deal deal) {
+    decode_reduce_kernel(const float* Mp, const float* Lp, const float* Op, float* M, float* L, float* O, int H,
+                         int kvH, int D, int head_rows, int ctas, const Deal deal) {
   __shared__ float sc[kMaxSplits];
   __shared__ float part_o[kFoldThreads];
   const int h = blockIdx.x, b = blockIdx.y;

@@ -303,3 +303,40 @@ def test_cache_append_on_a_stream_of_its_own_and_from_a_captured_graph():
     torch.cuda.synchronize()
     for i, src in enumerate((0, 2)):
         assert torch.equal(cache.k_view()[:, :, i], rows[src, 0, :, :, 0]) and torch.equal(cache.v_view()[:, :, i], rows[src, 1, :, :, 0])
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+def test_decode_calls_in_a_row_fold_their_own_partials(dtype):
+    # The fold starts while the split kernel runs and all calls share a workspace: what it reads has to
+    # be this call's partials and this call's state, not what it finds there when it starts.
+    H, Sk, D, calls = 8, 6000, 128, 12
+    shape = api.AttentionShape(1, H, 1, Sk, D, H)
+    g = torch.Generator(device="cuda").manual_seed(4)
+    k, v, q = (torch.randn((calls, 1, H, n, D), generator=g, device="cuda").to(dtype) for n in (Sk, Sk, 1))
+    ws = torch.full((lib().ra_decode_workspace_bytes(C.byref(shape.c())) // 4,), float("nan"), device="cuda")
+    alone, chain = [], poisoned(1, H, 1, D)
+    for i in range(calls):
+        state = poisoned(1, H, 1, D)
+        api.launch_attention_init(*state, shape)
+        api.launch_attention_decode_step(q[i], k[i], v[i], *state, shape, 0, 0, False, workspace=ws)
+        torch.cuda.synchronize()
+        ws.fill_(float("nan"))
+        alone.append(state)
+    api.launch_attention_init(*chain, shape)
+    row = [poisoned(1, H, 1, D) for _ in range(calls)]
+    for state in row:
+        api.launch_attention_init(*state, shape)
+    torch.cuda.synchronize()
+    for i in range(calls):  # nothing waits between these
+        api.launch_attention_decode_step(q[i], k[i], v[i], *row[i], shape, 0, 0, False, workspace=ws)
+        api.launch_attention_decode_step(q[i], k[i], v[i], *chain, shape, 0, 0, False, workspace=ws)
+    torch.cuda.synchronize()
+    for a, b in zip(alone, row):
+        assert all(torch.equal(x, y) for x, y in zip(a, b))
+    # the chained state is the merge of the single ones
+    m = torch.stack([s[1] for s in alone]).double()
+    w = (m - m.max(0).values).exp()
+    l = (torch.stack([s[2] for s in alone]).double() * w).sum(0)
+    o = (torch.stack([s[0] for s in alone]).double() * w[..., None]).sum(0) / l[..., None]
+    api.launch_attention_finalize(chain[0], chain[2], shape)
+    assert_close(chain[0].cpu().numpy(), o.cpu().numpy(), 1e-5, 1e-5, "chained state")
