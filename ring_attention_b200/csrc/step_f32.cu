@@ -921,8 +921,9 @@ __global__ void __launch_bounds__(kThreadsF, 1)
     if (ok && mine) tc_fence_after();
     const float o_unit = pow2_any(unit == kNoUnit ? 0 : -unit);
     if constexpr (kSplit) {
-      merge_key_split<C, DR>(a, smem, s_base, t_o, w, row, row_valid, grow0, ok && mine, m_ref, l_run, o_unit,
-                             cta_rank, fresh, finalize);
+      const bool gave_up = __any_sync(0xffffffffu, !ok || *abort_flag != 0) != 0;
+      merge_key_split<C, DR>(a, smem, s_base, t_o, w, row, row_valid, grow0, gave_up, !gave_up && mine, m_ref, l_run,
+                             o_unit, cta_rank, fresh, finalize);
     } else if (ok) {
       float* o_g = a.out + grow * DR;
       const bool have = row_valid && mine && m_ref > -INFINITY;

@@ -820,9 +820,10 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit>::kThreads),
     ok = __all_sync(0xffffffffu, ok);
     if constexpr (kSplit) {
       tc_fence_after();
+      const bool gave_up = __any_sync(0xffffffffu, !ok || *abort_flag != 0) != 0;
       merge_key_split<C, DR>(a, smem, s_base, t_o, w, row, row_valid,
                              static_cast<size_t>(bh) * a.Sq + static_cast<size_t>(sq) * q_seg_len + row0,
-                             ok && w < live && n_tiles > 0, m_ref, l_run, 1.f, cta_rank, fresh,
+                             gave_up, !gave_up && w < live && n_tiles > 0, m_ref, l_run, 1.f, cta_rank, fresh,
                              finalize);
     } else if (ok) {
       tc_fence_after();

@@ -477,15 +477,15 @@ struct TcArgs {
 // End of a block of the key-split form, run by the softmax threads (one per row; the other threads
 // of the cluster only join the three barriers): the partial (O, m, l) of the cluster's blocks are
 // merged and folded into the state as one step. Every block scales its O to the common reference
-// point (o_unit: what one unit
-// of the accumulator is worth) and stages it in its own shared memory, then each block sums its slice of the elements
-// over all blocks and writes it. 128 KB of staged O per block at head_dim 128 cross the cluster
-// once (about 2 us); no workspace and no second launch.
+// point (o_unit: what one unit of the accumulator is worth) and stages it in its own shared memory,
+// then each block sums its slice of the elements over all blocks and writes it. 128 KB of staged O per
+// block at head_dim 128 cross the cluster once (about 2 us); no workspace and no second launch. A row
+// that some block of the cluster gave up on (a wait ran out) keeps its state, as without a split.
 template <class C, int DR>
 __device__ inline void merge_key_split(const TcArgs& a, unsigned char* smem, unsigned s_base,
-                                       unsigned t_o, int w, int row, bool row_valid, size_t grow0, bool worked,
-                                       float m_ref, float l_run, float o_unit, unsigned rank, bool fresh,
-                                       bool finalize) {
+                                       unsigned t_o, int w, int row, bool row_valid, size_t grow0, bool gave_up,
+                                       bool worked, float m_ref, float l_run, float o_unit, unsigned rank,
+                                       bool fresh, bool finalize) {
   constexpr int kRows = C::kTiles * kBM;
   constexpr int kStride = DR + 4;  // floats: rows 16 bytes apart modulo 128, so float4 stores do not collide
   constexpr int kOffFac = kRows * kStride * 4;
@@ -495,14 +495,16 @@ __device__ inline void merge_key_split(const TcArgs& a, unsigned char* smem, uns
   const int rb = w * kBM + row;
   const int n = a.key_split;
   const bool have = worked && row_valid && m_ref > -INFINITY;
-  ml[rb] = have ? make_float2(m_ref, l_run) : make_float2(-INFINITY, 0.f);
+  ml[rb] = have ? make_float2(m_ref, l_run) : make_float2(-INFINITY, gave_up ? -1.f : 0.f);
   cluster_sync_threads();  // all (m, l) are there, no block reads its Q or ring any more
   const unsigned ml_addr = s_base + C::kOffMl + rb * 8;
   float m_all = -INFINITY, l_all = 0.f;
   for (int r = 0; r < n; ++r) m_all = fmaxf(m_all, ld_cluster_f2(cluster_addr(ml_addr, r)).x);
+  bool lost = false;  // (a sum is never negative)
   for (int r = 0; r < n; ++r) {
     const float2 p = ld_cluster_f2(cluster_addr(ml_addr, r));
     if (p.x > -INFINITY) l_all += p.y * ex2(p.x - m_all);
+    else lost = lost || p.y == -1.f;
   }
   const size_t grow = grow0 + (row_valid ? rb : 0);
   const bool any = row_valid && m_all > -INFINITY;
@@ -517,7 +519,7 @@ __device__ inline void merge_key_split(const TcArgs& a, unsigned char* smem, uns
   const float cb = any ? expf(m_new - m_fin) : 0.f;
   const float l_fin = ca * l_old + cb * l_all;
   const float inv = finalize ? (l_fin > 0.f ? 1.f / l_fin : 0.f) : 1.f;
-  const bool touch = row_valid && (any || fresh || finalize);
+  const bool touch = row_valid && !lost && (any || fresh || finalize);
   fac[rb] = touch ? make_float2(ca * inv, cb * inv) : make_float2(-1.f, 0.f);  // factors are never negative
   const float scale = have ? ex2(m_ref - m_all) : 0.f;
 #pragma unroll 1

@@ -340,3 +340,28 @@ def test_decode_calls_in_a_row_fold_their_own_partials(dtype):
     o = (torch.stack([s[0] for s in alone]).double() * w[..., None]).sum(0) / l[..., None]
     api.launch_attention_finalize(chain[0], chain[2], shape)
     assert_close(chain[0].cpu().numpy(), o.cpu().numpy(), 1e-5, 1e-5, "chained state")
+
+
+@pytest.mark.parametrize("dtype,D", [(torch.float32, 64), (torch.float32, 128), (torch.float16, 64), (torch.float16, 128)])
+@pytest.mark.parametrize("split", [1, 3])
+@pytest.mark.parametrize("finalize", [False, True])
+def test_rows_whose_wait_ran_out_keep_their_state(dtype, D, split, finalize):
+    # The producer stops after so many ring items that with three blocks to a query block the first one or
+    # two finish their share and the last cannot: none of the rows may get a part of the sum.
+    L, S = lib(), 1024
+    q, k, v = (dev(x, dtype) for x in normal_inputs(13, 1, 2, 2, S, S, D))
+    state = [torch.full((1, 2, S, D), 3.0, device="cuda"), torch.full((1, 2, S), 0.5, device="cuda"),
+             torch.full((1, 2, S), 2.0, device="cuda")]
+    assert api.device_status()[0] == 0
+    L.ra_debug_set_wait_limit_ns(5_000_000)
+    L.ra_debug_stall_producer_after(10 if dtype == torch.float32 else 4)
+    try:
+        step(q, k, v, state, api.AttentionShape(1, 2, S, S, D), SegMap.make([0], S), SegMap.make([0], S),
+             FINALIZE if finalize else 0, split)
+        torch.cuda.synchronize()
+    finally:
+        L.ra_debug_stall_producer_after(-1)
+        L.ra_debug_set_wait_limit_ns(0)
+    status = api.device_status()
+    assert status[0] == 5 and status[1] > 0, status
+    assert (state[0] == 3.0).all() and (state[1] == 0.5).all() and (state[2] == 2.0).all()
