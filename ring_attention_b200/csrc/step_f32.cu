@@ -478,10 +478,11 @@ __global__ void __launch_bounds__(kThreadsF, 1)
           mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
           if (p4 == 0) smem[C::kOffVKey + ((it >> 1) & 7) * kBNf + sw * 8 + r8] = static_cast<unsigned char>(mx >> 23);
           unsigned low = (mx == 0 ? 0xffffu : mx >> 16) + (kKeyRange << 7);
-          const unsigned low_all = (__reduce_min_sync(0xffffffffu, __float_as_uint(fn)) >> 16) + (kColRange << 7);
+          const unsigned least = __reduce_min_sync(0xffffffffu, __float_as_uint(fn)) >> 16;
           mx = __reduce_max_sync(0xffffffffu, mx);
-          if (__builtin_expect(low_all - (1u << 7) >= mx >> 16, 1)) {
-            low = min(low, low_all);
+          // (a zero says nothing: the rows behind a ragged end are zeros)
+          if (__builtin_expect(least > 0 && least + ((kColRange - 1) << 7) >= mx >> 16, 1)) {
+            low = min(low, least + (kColRange << 7));
           } else {
             // column by column, the upper halves of two magnitudes in a word; each lane ends with its
             // share of the columns (1 below, so that none is zero)
