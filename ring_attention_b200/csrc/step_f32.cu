@@ -1050,7 +1050,7 @@ int launch_f32(const StepArgs& a, cudaStream_t stream, int key_split) {
 
 template <int DR>
 int launch_f32_d(const StepArgs& a, cudaStream_t stream) {
-  const int split = pick_key_split<kBNf>(a, 2 * kBM, 1.5, 0);
+  const int split = pick_key_split<kBNf>(a, 2 * kBM, 1.5);
   return split > 1 ? launch_f32<DR, true>(a, stream, split) : launch_f32<DR, false>(a, stream, 1);
 }
 

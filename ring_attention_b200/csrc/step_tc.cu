@@ -1029,13 +1029,12 @@ int launch_d(int dtype, const StepArgs& a, cudaStream_t stream) {
   // P stays in tensor memory unless the caller asks for the shared-memory path (kept as a
   // cross-check of the first one; both are tested)
   const bool p_in_tmem = (a.flags & RA_STEP_P_IN_SMEM) == 0;
-  // A key split (not under a forced block order, which is about whole blocks). Head_dim 128 and 256
-  // stay whole up to 16 key tiles, where they equal their cluster-pair form bit for bit; a
-  // merge stages 4 bytes per row and column, so it costs more tiles the wider the head.
+  // A key split (not under a forced block order, which is about whole blocks). A merge stages 4 bytes
+  // per row and column, so it costs more tiles the wider the head.
   const int split = p_in_tmem && (a.flags & RA_STEP_CTA_PAIR) == 0 &&
                             g_block_order.load(std::memory_order_relaxed) < 0
-                        ? pick_key_split<kBN>(a, TcCfg<D, true>::kTiles * kBM, D == 64 ? 1.5 : 2.5,
-                                              D == 64 ? 0 : 16)
+                        ? pick_key_split<kBN>(a, TcCfg<D, true>::kTiles * kBM,
+                                              D == 64 ? 1.5 : D == 128 ? 2.5 : 4.5)
                         : 1;
   // the 64-wide kernel also takes head_dim 32 (DR = 32)
   if constexpr (D == 64) {

@@ -622,13 +622,13 @@ inline int make_map(CUtensorMap* map, int dtype, const void* base, int D, long l
 // block while the blocks with work fit the SMs that clusters of that size can occupy (a cluster
 // lives inside one GPC: cudaOccupancyMaxActiveClusters gives 148, 148, 135, 132, 130, 132, 120 for
 // n = 1, 2, 3, 4, 5, 6, 8), else the total work over them plus half a block for the last wave.
-// `longest_unsplit`: calls whose longest walk is at most this stay whole.
 // Measured, us per call at n = 1 / 2 / 4 / 8 (fp16, causal): 384 rows on 40384 keys H32/kvH8 D128
 // 542 / 296 / 303 / 410 (735 before the second tile of the last block was left out); 64 rows on
 // 65536 keys H8 D128 1077 / 540 / 277 / 146; 1024 x 1024 H8 D64 23 / 19 / 17 / 38; 2048 x 2048 H16
-// D64 (128 blocks) 36 / 38 / 59 / 122.
+// D64 (128 blocks) 36 / 38 / 59 / 122; 1024 x 1024 H8 D128 29 / 25 / 18.5 / 49, H16 29 / 25 / 33 / 80;
+// 1024 x 1024 H8 D256 (64 blocks) 27 / 29 / 39 / 82; 2048 x 2048 H4 D256 41 / 37 / 41 / 86.
 template <int kTileKeys>
-inline int pick_key_split(const StepArgs& a, int q_block_rows, double merge_tiles, int longest_unsplit) {
+inline int pick_key_split(const StepArgs& a, int q_block_rows, double merge_tiles) {
   const int forced = static_cast<int>((a.flags >> RA_STEP_KEY_SPLIT_SHIFT) & 15u);
   if (forced) return forced > 8 ? 8 : forced;
   constexpr int kSms = 148;
@@ -654,7 +654,7 @@ inline int pick_key_split(const StepArgs& a, int q_block_rows, double merge_tile
       longest = tiles > longest ? tiles : longest;
       tiles > 0 ? ++busy : ++idle;
     }
-  if (busy == 0 || longest <= longest_unsplit) return 1;
+  if (busy == 0) return 1;
   const double mean = static_cast<double>(total) / busy;
   constexpr int kSizes[7] = {1, 2, 3, 4, 5, 6, 8}, kSlots[7] = {kSms, kSms, 135, 132, 130, 132, 120};
   int best = 1;

@@ -120,13 +120,13 @@ def test_config1_fp32_noncausal_mha_output_and_lse():
 
 
 def run_ex(q, k, v, qmap, kmap, stride, causal, dtype, kvH, doc_len=0, force_simt=False,
-           p_in_smem=False, cta_pair=False):
+           p_in_smem=False, cta_pair=False, key_split=0):
     B, H, Sq, D = q.shape
     out, m, l = state(B, H, Sq, D, poison=True)
     api.attention_step_ex(dev(q, dtype), dev(k, dtype), dev(v, dtype), out, m, l,
                           api.AttentionShape(B, H, Sq, k.shape[2], D, kvH), qmap, kmap, stride,
                           causal=causal, fresh=True, finalize=True, doc_len=doc_len,
-                          force_simt=force_simt, p_in_smem=p_in_smem, cta_pair=cta_pair)
+                          force_simt=force_simt, p_in_smem=p_in_smem, cta_pair=cta_pair, key_split=key_split)
     torch.cuda.synchronize()
     assert api.device_status()[0] == 0
     return out.cpu().numpy(), api.attention_lse(m, l).cpu().numpy()
@@ -276,7 +276,8 @@ def test_cluster_pair_form_of_the_tensor_core_kernel(D, dtype):
     """M = 256 MMAs over two blocks of a cluster (cta_group::2): each block loads half of every
     K / V tile. Odd numbers of query blocks (the last pair's second block has no rows), a single
     block per segment (falls back to independent blocks), zig-zag segments, GQA, causal and
-    document masks; the result must also equal the independent-block form bit for bit."""
+    document masks; the result must also equal the form of independent blocks, one to a query block,
+    bit for bit."""
     tol = 1e-3 if dtype == torch.float16 else 8e-3
     for seed, (Sq, Sk, causal, doc_len) in enumerate([(640, 1408, True, 0), (1200, 1200, True, 0),
                                                       (130, 700, False, 0), (900, 900, True, 200),
@@ -287,7 +288,7 @@ def test_cluster_pair_form_of_the_tensor_core_kernel(D, dtype):
         want, _ = masked_truth(q, k, v, positions(qmap, 1), positions(kmap, 1), causal, doc_len, 2) \
             if doc_len else (oracle.cpu_attention(q, k, v, causal, kv_heads=2), None)
         pair, lse_pair = run_ex(q, k, v, qmap, kmap, 1, causal, dtype, 2, doc_len=doc_len, cta_pair=True)
-        single, lse_single = run_ex(q, k, v, qmap, kmap, 1, causal, dtype, 2, doc_len=doc_len)
+        single, lse_single = run_ex(q, k, v, qmap, kmap, 1, causal, dtype, 2, doc_len=doc_len, key_split=1)
         assert_close(pair, want, tol, tol, f"D={D} Sq={Sq} Sk={Sk} causal={causal} doc={doc_len}")
         assert np.array_equal(pair, single) and np.array_equal(lse_pair, lse_single)
     # zig-zag: two query segments and four key segments with their own bases
