@@ -127,13 +127,13 @@ __global__ void narrow_kernel(const float* __restrict__ src, Dst* __restrict__ d
 }
 
 // Q, K and V in one launch (blockIdx.y): three launches of a few microseconds of work each cost
-// the host more than the GPU.
+// the host more than the GPU. Bit i of `vec`: tensor i's source and destination are 16-byte aligned.
 __global__ void narrow_qkv_kernel(const float* __restrict__ q, __half* __restrict__ qh, size_t qn,
                                   const float* __restrict__ k, const float* __restrict__ v,
-                                  __half* __restrict__ kh, __half* __restrict__ vh, size_t kn, int vec_ok) {
-  if (blockIdx.y == 0) narrow_range(q, qh, qn, vec_ok);
-  else if (blockIdx.y == 1) narrow_range(k, kh, kn, vec_ok);
-  else narrow_range(v, vh, kn, vec_ok);
+                                  __half* __restrict__ kh, __half* __restrict__ vh, size_t kn, int vec) {
+  if (blockIdx.y == 0) narrow_range(q, qh, qn, vec & 1);
+  else if (blockIdx.y == 1) narrow_range(k, kh, kn, vec & 2);
+  else narrow_range(v, vh, kn, vec & 4);
 }
 
 // fp16 -> fp32 (reference: src/attention_step_fp16.cu:226-233).
@@ -288,7 +288,8 @@ int launch_narrow_qkv(const float* q, const float* k, const float* v, void* qh, 
                       size_t kn, cudaStream_t stream) {
   const size_t most = qn > kn ? qn : kn;
   if (most == 0) return RA_OK;
-  const int vec = aligned16(q) && aligned16(k) && aligned16(v) && aligned16(qh) && aligned16(kh) && aligned16(vh);
+  const int vec = (aligned16(q) && aligned16(qh) ? 1 : 0) | (aligned16(k) && aligned16(kh) ? 2 : 0) |
+                  (aligned16(v) && aligned16(vh) ? 4 : 0);
   narrow_qkv_kernel<<<dim3(grid_for(most / 8 + 1, 256), 3), 256, 0, stream>>>(
       q, static_cast<__half*>(qh), qn, k, v, static_cast<__half*>(kh), static_cast<__half*>(vh), kn, vec);
   RAB_CUDA(cudaGetLastError());

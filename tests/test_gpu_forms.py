@@ -365,3 +365,15 @@ def test_rows_whose_wait_ran_out_keep_their_state(dtype, D, split, finalize):
     status = api.device_status()
     assert status[0] == 5 and status[1] > 0, status
     assert (state[0] == 3.0).all() and (state[1] == 0.5).all() and (state[2] == 2.0).all()
+
+
+@pytest.mark.parametrize("which", [0, 1, 2])
+def test_half_flash_call_with_one_unaligned_source(which):
+    B, H, kvH, S, D = 1, 4, 2, 300, 64
+    x = [dev(t) for t in normal_inputs(14, B, H, kvH, S, S, D)]
+    shape, want, got = api.AttentionShape(B, H, S, S, D, kvH), *(torch.empty(B, H, S, D, device="cuda") for _ in range(2))
+    api.launch_flash_attention_fp16(*x, want, shape, True)
+    flat = torch.empty(x[which].numel() + 1, device="cuda")[1:]
+    x[which] = flat.copy_(x[which].flatten()).view(x[which].shape)
+    api.launch_flash_attention_fp16(*x, got, shape, True)
+    assert torch.equal(got, want)
