@@ -40,7 +40,7 @@ def poisoned(B, H, Sq, D):
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("D", [32, 64, 128, 256])
-@pytest.mark.parametrize("split", [2, 3, 8])
+@pytest.mark.parametrize("split", [1, 2, 3, 8])
 def test_key_split_in_two_steps_matches_the_oracle(dtype, D, split):
     # 300 query rows (a whole block and one of a single short tile), two key chunks of which the
     # second has fewer tiles than blocks; document and causal limits leave some shares empty
@@ -106,6 +106,19 @@ def test_fp32_step_holds_its_precision_over_the_range_of_fp32(D, case):
     unit = float(np.abs(want).max())  # errors of a weighted sum of V scale with the largest V
     assert_close(state[0].cpu().numpy() / unit, want / unit, 1e-5, 1e-5, "out")
     assert_close(lse, want_lse, 1e-5, 1e-5, "lse")
+
+
+def _in_64_bits(q, k, v, qpos, kpos, causal, doc):
+    """(out, log-sum-exp) with one KV head per query head."""
+    seen = (kpos[None, :] <= qpos[:, None]) | (not causal)
+    if doc:
+        seen = seen & (kpos[None, :] // doc == qpos[:, None] // doc)
+    s = np.einsum("bhid,bhjd->bhij", q.astype(np.float64), k.astype(np.float64)) / np.sqrt(q.shape[-1])
+    s = np.where(seen, s, -np.inf)
+    m = s.max(-1, keepdims=True)
+    p = np.exp(s - m)
+    out = np.einsum("bhij,bhjd->bhid", p, v.astype(np.float64)) / p.sum(-1, keepdims=True)
+    return out, (m + np.log(p.sum(-1, keepdims=True)))[..., 0]
 
 
 def _wide_inputs(case, D):
@@ -181,16 +194,7 @@ def test_fp32_step_holds_the_precision_of_every_part_of_the_output(D, split, cas
     q, k, v, causal, doc, parts = _wide_inputs(case, D)
     q, k, v = (x.astype(np.float32) for x in (q, k, v))
     B, H, S, _ = q.shape
-    pos = np.arange(S)
-    seen = (pos[None, :] <= pos[:, None]) | (not causal)
-    if doc:
-        seen &= pos[None, :] // doc == pos[:, None] // doc
-    s = np.einsum("bhid,bhjd->bhij", q.astype(np.float64), k.astype(np.float64)) / np.sqrt(D)
-    s = np.where(seen, s, -np.inf)
-    m = s.max(-1, keepdims=True)
-    p = np.exp(s - m)
-    want = np.einsum("bhij,bhjd->bhid", p, v.astype(np.float64)) / p.sum(-1, keepdims=True)
-    want_lse = (m + np.log(p.sum(-1, keepdims=True)))[..., 0]
+    want, want_lse = _in_64_bits(q, k, v, np.arange(S), np.arange(S), causal, doc)
     state = poisoned(B, H, S, D)
     step(dev(q), dev(k), dev(v), state, api.AttentionShape(B, H, S, S, D), SegMap.make([0], S), SegMap.make([0], S),
          FRESH | FINALIZE | (CAUSAL if causal else 0), split, doc)
@@ -377,3 +381,62 @@ def test_half_flash_call_with_one_unaligned_source(which):
     x[which] = flat.copy_(x[which].flatten()).view(x[which].shape)
     api.launch_flash_attention_fp16(*x, got, shape, True)
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("D", [32, 64, 128])
+@pytest.mark.parametrize("split", [1, 2])
+@pytest.mark.parametrize("case", ["plain", "growing scores", "documents", "marked tiles", "growing v"])
+def test_fp32_step_over_many_key_tiles_into_a_state(D, split, case):
+    # 47 key tiles, 36 of them in one step (18 to a block when two share them): the ring wraps several times, the
+    # 16 tile exponents and 8 sets of key exponents are reused, and the second step folds into the first's state
+    Sq, Sk, cut, doc = 300, 2950, 700, 0
+    q, k, v = (x.astype(np.float64) for x in normal_inputs(17, 1, 2, 2, Sq, Sk, D))
+    if case == "growing scores":  # about 1.5 in the exponent from one key tile to the next
+        q[..., 0], k[..., 0] = 4.0, np.arange(Sk) / 64.0 * 1.5 / 4.0 * np.sqrt(D)
+    elif case == "documents":
+        doc = 1100
+    elif case == "marked tiles":  # single keys and columns, a channel of some keys
+        v[:, :, 100::450] *= 2.0 ** 20
+        v[:, :, 1300:1400, 7] *= 2.0 ** 30
+        q[..., 1], k[..., 1] = q[..., 1] * 2.0 ** 16, k[..., 1] * 2.0 ** -16
+        k[:, :, 2000:2100, 2] = 0.0
+        k[:, :, 2050, 2] = -(2.0 ** 16)
+        q[..., 2] = np.abs(q[..., 2])
+    elif case == "growing v":
+        v *= 2.0 ** (np.arange(Sk) // 64)[None, None, :, None]
+    q, k, v = (x.astype(np.float32) for x in (q, k, v))
+    want, want_lse = _in_64_bits(q, k, v, np.arange(Sq) + Sk - Sq, np.arange(Sk), True, doc)
+    state = poisoned(1, 2, Sq, D)
+    for lo, hi, flags in ((0, cut, FRESH), (cut, Sk, FINALIZE)):
+        step(dev(q), dev(k[:, :, lo:hi]), dev(v[:, :, lo:hi]), state, api.AttentionShape(1, 2, Sq, hi - lo, D),
+             SegMap.make([Sk - Sq], Sq), SegMap.make([lo], hi - lo), flags | CAUSAL, split, doc)
+    lse = api.attention_lse(state[1], state[2]).cpu().numpy()
+    assert api.device_status()[0] == 0
+    # fp32 scores of up to 70 (growing scores) carry 4e-6 each: half an ulp of the score before scaling
+    assert_close(lse, want_lse, 1e-5, 1e-5, "lse")
+    unit = np.abs(want).max()
+    assert_close(state[0].cpu().numpy() / unit, want / unit, 2e-5, 0.0, "out")
+
+
+@pytest.mark.parametrize("dtype,D", [(torch.float16, 64), (torch.float16, 128), (torch.bfloat16, 256), (torch.float32, 64),
+                                     (torch.float32, 128)])
+@pytest.mark.parametrize("split", [1, 3])
+def test_document_mask_and_moving_reference_in_both_forms(dtype, D, split):
+    # scores that climb by about 24 in the exponent per 128 keys, and documents that begin inside tiles
+    S, Sq, doc = 1024, 256, 600
+    rng = np.random.default_rng(12)
+    q, k = rng.standard_normal((1, 2, Sq, D)) * 0.3, rng.standard_normal((1, 2, S, D)) * 0.3
+    q[..., 0] = 4.0
+    k[0, 0, :, 0] = np.arange(S) / 128.0 * 17.0 * np.sqrt(D) / 4.0
+    k[0, 1, :, 0] = -k[0, 0, :, 0]
+    v = rng.standard_normal((1, 2, S, D))
+    q, k, v = (round_to(x.astype(np.float32), dtype) for x in (q, k, v))
+    want, want_lse = _in_64_bits(q, k, v, np.arange(Sq) + S - Sq, np.arange(S), True, doc)
+    state = poisoned(1, 2, Sq, D)
+    step(dev(q, dtype), dev(k, dtype), dev(v, dtype), state, api.AttentionShape(1, 2, Sq, S, D), SegMap.make([S - Sq], Sq),
+         SegMap.make([0], S), FRESH | FINALIZE | CAUSAL, split, doc)
+    lse = api.attention_lse(state[1], state[2]).cpu().numpy()
+    # fp32: raw scores of about 1000, one ulp of which is 1.5e-5 in the exponent after scaling
+    tol = 1e-4 if dtype == torch.float32 else TOL[dtype]
+    assert_close(state[0].cpu().numpy(), want, tol, tol, "out")
+    assert_close(lse, want_lse, tol, tol, "lse")

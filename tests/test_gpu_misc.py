@@ -121,8 +121,8 @@ def test_bounded_wait_runs_out_and_the_context_stays_usable(D, cta_pair):
     first K/V tiles and the limit set to a few milliseconds, the kernel returns by itself, the
     status word says which wait gave up, host entry points that synchronise report
     RA_ERR_DEVICE_WAIT, and after the word is read (which clears it) the same launch is right.
-    Covers the three schedules of the kernel (head_dim 64, 256) and its cluster-pair form, where
-    both blocks of a pair have to give up and meet at the cluster barrier."""
+    Covers two schedules of the kernel (head_dim 64, 256), one block to a query block, and its
+    cluster-pair form, where both blocks of a pair have to give up and meet at the cluster barrier."""
     from ring_attention_b200._lib import RingAttentionError, lib
     L = lib()
     S, H = 1024, 2
