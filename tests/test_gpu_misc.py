@@ -138,7 +138,7 @@ def test_bounded_wait_runs_out_and_the_context_stays_usable(D, cta_pair):
     L.ra_debug_stall_producer_after(2)
     try:
         api.attention_step_ex(dq, dk, dv, out, m, l, shape, one, one, causal=True, fresh=True, finalize=True,
-                              cta_pair=cta_pair)
+                              cta_pair=cta_pair, key_split=1)
         torch.cuda.synchronize()  # returns: nothing waits forever
         # a host-buffer entry point synchronises, so it reports the failure itself
         hq, hk, hv = (torch.from_numpy(x).to(torch.float16).pin_memory() for x in (q, k, v))
@@ -155,7 +155,7 @@ def test_bounded_wait_runs_out_and_the_context_stays_usable(D, cta_pair):
     assert status[0] == 5 and status[1] > 0, status
     assert api.device_status()[0] == 0
     api.attention_step_ex(dq, dk, dv, out, m, l, shape, one, one, causal=True, fresh=True, finalize=True,
-                          cta_pair=cta_pair)
+                          cta_pair=cta_pair, key_split=1)
     torch.cuda.synchronize()
     assert api.device_status()[0] == 0
     assert_close(out.cpu().numpy(), want, 1e-3, 1e-3, "after the status word was cleared")
