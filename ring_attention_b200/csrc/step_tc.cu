@@ -1031,10 +1031,14 @@ int launch_d(int dtype, const StepArgs& a, cudaStream_t stream) {
   const bool p_in_tmem = (a.flags & RA_STEP_P_IN_SMEM) == 0;
   // A key split (not under a forced block order, which is about whole blocks). A merge stages 4 bytes
   // per row and column, so it costs more tiles the wider the head.
+  using S = TcCfg<D, true, false, true>;
+  const int* slots = nullptr;
+  const int rc = cluster_slots(step_tc_kernel<D, false, true, D, false, true>, S::kThreads, S::kSmemBytes, &slots);
+  if (rc != RA_OK) return rc;
   const int split = p_in_tmem && (a.flags & RA_STEP_CTA_PAIR) == 0 &&
                             g_block_order.load(std::memory_order_relaxed) < 0
                         ? pick_key_split<kBN>(a, TcCfg<D, true>::kTiles * kBM,
-                                              D == 64 ? 1.5 : D == 128 ? 2.5 : 4.5)
+                                              D == 64 ? 1.5 : D == 128 ? 2.5 : 4.5, slots)
                         : 1;
   // the 64-wide kernel also takes head_dim 32 (DR = 32)
   if constexpr (D == 64) {
@@ -1092,6 +1096,10 @@ int launch_step_tc(int dtype, const StepArgs& a, cudaStream_t stream) {
 namespace tcgen {
 unsigned long long tc_wait_limit_ns() { return g_wait_ns.load(std::memory_order_relaxed); }
 int tc_stall_after() { return g_stall_after.load(std::memory_order_relaxed); }
+ClusterSlots& cluster_slots_of(int device) {
+  static ClusterSlots tables[64];
+  return tables[device];
+}
 }  // namespace tcgen
 
 void set_tc_wait_limit_ns(unsigned long long ns) {

@@ -614,28 +614,71 @@ inline int make_map(CUtensorMap* map, int dtype, const void* base, int D, long l
   return RA_OK;
 }
 
+// How many blocks the current device holds at once when they come in clusters of n, n = 1..8: asked for
+// once per device, with whichever key-split kernel comes first (all of them hold one block per SM, so the
+// answers are the same; a cluster lives inside one GPC: 148, 148, 135, 132, 130, 132, 126, 120 on a B200).
+struct ClusterSlots {
+  std::once_flag once;
+  int blocks[9];
+};
+ClusterSlots& cluster_slots_of(int device);
+
+template <class Kern>
+inline int cluster_slots(Kern kern, int threads, int smem_bytes, const int** out) {
+  int dev = 0;
+  RAB_CUDA(cudaGetDevice(&dev));
+  RAB_REQUIRE(dev >= 0 && dev < 64, RA_ERR_INVALID, "device index %d out of range", dev);
+  ClusterSlots& t = cluster_slots_of(dev);
+  std::call_once(t.once, [&]() {
+    for (int n = 0; n <= 8; ++n) t.blocks[n] = 0;
+    if (cudaDeviceGetAttribute(&t.blocks[1], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes) != cudaSuccess) {
+      cudaGetLastError();
+      return;  // no split on this device
+    }
+    for (int n = 2; n <= 8; ++n) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(n);
+      cfg.blockDim = dim3(threads);
+      cfg.dynamicSmemBytes = smem_bytes;
+      cudaLaunchAttribute attr;
+      attr.id = cudaLaunchAttributeClusterDimension;
+      attr.val.clusterDim.x = n;
+      attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+      cfg.attrs = &attr;
+      cfg.numAttrs = 1;
+      int clusters = 0;
+      if (cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        clusters = 0;
+      }
+      t.blocks[n] = clusters * n;
+    }
+  });
+  *out = t.blocks;
+  return RA_OK;
+}
+
 // Key split: how many blocks of a cluster share the key tiles of one query block (1: no split).
 // A block walks its key tiles one after the other, so a call with fewer query blocks than SMs
 // leaves SMs idle however many keys there are. Cutting the tile list in n shortens the walk to
 // 1/n and costs every block its own prologue and the merge (kFixed and merge_tiles, in tiles of
 // work; a query block without a visible key costs kEmpty). The estimate is the walk of the longest
-// block while the blocks with work fit the SMs that clusters of that size can occupy (a cluster
-// lives inside one GPC: cudaOccupancyMaxActiveClusters gives 148, 148, 135, 132, 130, 132, 120 for
-// n = 1, 2, 3, 4, 5, 6, 8), else the total work over them plus half a block for the last wave.
+// block while the blocks with work fit the SMs that clusters of that size can occupy (`slots`, see
+// ClusterSlots), else the total work over them plus half a block for the last wave.
 // Measured, us per call at n = 1 / 2 / 4 / 8 (fp16, causal): 384 rows on 40384 keys H32/kvH8 D128
 // 542 / 296 / 303 / 410 (735 before the second tile of the last block was left out); 64 rows on
 // 65536 keys H8 D128 1077 / 540 / 277 / 146; 1024 x 1024 H8 D64 23 / 19 / 17 / 38; 2048 x 2048 H16
 // D64 (128 blocks) 36 / 38 / 59 / 122; 1024 x 1024 H8 D128 29 / 25 / 18.5 / 49, H16 29 / 25 / 33 / 80;
 // 1024 x 1024 H8 D256 (64 blocks) 27 / 29 / 39 / 82; 2048 x 2048 H4 D256 41 / 37 / 41 / 86.
 template <int kTileKeys>
-inline int pick_key_split(const StepArgs& a, int q_block_rows, double merge_tiles) {
+inline int pick_key_split(const StepArgs& a, int q_block_rows, double merge_tiles, const int* slots) {
   const int forced = static_cast<int>((a.flags >> RA_STEP_KEY_SPLIT_SHIFT) & 15u);
   if (forced) return forced > 8 ? 8 : forced;
-  constexpr int kSms = 148;
   constexpr double kFixed = 3, kEmpty = 0.7;
   const int per_seg = (a.qmap.seg_len + q_block_rows - 1) / q_block_rows;
   const long long heads = static_cast<long long>(a.B) * a.H;
-  if (heads * per_seg * a.qmap.n_seg >= kSms) return 1;
+  if (heads * per_seg * a.qmap.n_seg >= slots[1]) return 1;
   const bool causal = (a.flags & RA_STEP_CAUSAL) != 0;
   long long total = 0;
   int longest = 0, busy = 0, idle = 0;  // per head
@@ -656,18 +699,19 @@ inline int pick_key_split(const StepArgs& a, int q_block_rows, double merge_tile
     }
   if (busy == 0) return 1;
   const double mean = static_cast<double>(total) / busy;
-  constexpr int kSizes[7] = {1, 2, 3, 4, 5, 6, 8}, kSlots[7] = {kSms, kSms, 135, 132, 130, 132, 120};
+  constexpr int kSizes[7] = {1, 2, 3, 4, 5, 6, 8};
   int best = 1;
   double best_t = 0;
   for (int i = 0; i < 7; ++i) {
     const int n = kSizes[i];
     if (n > 1 && longest < 2 * n) break;  // at least two tiles to walk
+    if (slots[n] == 0) continue;
     const double fixed = kFixed + (n > 1 ? merge_tiles : 0);
-    const double empties = static_cast<double>(heads * idle) * n * kEmpty / kSlots[i];
+    const double empties = static_cast<double>(heads * idle) * n * kEmpty / slots[n];
     double t = longest / static_cast<double>(n) + fixed + empties;
     const double n_blocks = static_cast<double>(heads * busy) * n;
-    if (n_blocks > kSlots[i]) {
-      const double spread = (n_blocks / kSlots[i] + 0.5) * (mean / n + fixed) + empties;
+    if (n_blocks > slots[n]) {
+      const double spread = (n_blocks / slots[n] + 0.5) * (mean / n + fixed) + empties;
       t = t > spread ? t : spread;
     }
     if (i == 0 || t < best_t) {
