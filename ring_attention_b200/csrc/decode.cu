@@ -182,8 +182,34 @@ __device__ inline float ld_cluster(const float* p, unsigned rank) {
   return v;
 }
 
+__device__ inline float4 ld_cluster4(const float* p, unsigned rank) {
+  unsigned addr;
+  float4 v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+               : "=r"(addr)
+               : "r"(static_cast<unsigned>(__cvta_generic_to_shared(p))), "r"(rank));
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "r"(addr));
+  return v;
+}
+
 constexpr int kMaxCluster = 8;
-constexpr double kFoldUs = 3.0, kMergeUs = 1.0;  // see make_plan
+
+// Four floats of a workspace or a state, which need not be 16-byte aligned.
+__device__ inline float4 ld4(const float* p, bool vec) {
+  return vec ? *reinterpret_cast<const float4*>(p) : make_float4(p[0], p[1], p[2], p[3]);
+}
+__device__ inline void st4(float* p, float4 v, bool vec) {
+  if (vec) *reinterpret_cast<float4*>(p) = v;
+  else p[0] = v.x, p[1] = v.y, p[2] = v.z, p[3] = v.w;
+}
+__device__ inline void add_scaled(float4& a, float f, float4 v) {
+  a.x += f * v.x;
+  a.y += f * v.y;
+  a.z += f * v.z;
+  a.w += f * v.w;
+}
 
 // End of a block's share of a group: the warps' partials (red_*: [warps][ROWS], red_o [..][D]) of
 // the ROWS query heads h = kvh + kvH * (hb * ROWS + r) become the block's, which goes to slot
@@ -198,31 +224,37 @@ __device__ inline void finish_group(float* red_m, float* red_l, float* red_o, in
   const int live = first < H ? min(ROWS, (H - first + kvH - 1) / kvH) : 0;
   float* blk_m = red_o + NWARPS * ROWS * D;  // [ROWS], [ROWS], [ROWS][D]: cluster form
   float* blk_l = blk_m + ROWS;
-  float* blk_o = blk_l + ROWS;
-  for (int idx = tid; idx < live * D; idx += kThr) {
+  float* blk_o = blk_m + ((2 * ROWS + 3) & ~3);
+  for (int idx = 4 * tid; idx < live * D; idx += 4 * kThr) {  // four columns at a time
     const int r = idx / D;
     const int d = idx - r * D;
     float m_n = -INFINITY;
 #pragma unroll
     for (int w = 0; w < NWARPS; ++w) m_n = fmaxf(m_n, red_m[w * ROWS + r]);
-    float o_acc = 0.f, l_acc = 0.f;
+    float4 o_acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    float l_acc = 0.f;
 #pragma unroll
     for (int w = 0; w < NWARPS; ++w) {
       const float mw = red_m[w * ROWS + r];
       const float sc = (mw == -INFINITY) ? 0.f : ex2(mw - m_n);
-      o_acc += sc * red_o[(w * ROWS + r) * D + d];
+      const float4 o = *reinterpret_cast<const float4*>(red_o + (w * ROWS + r) * D + d);
+      o_acc.x += sc * o.x;
+      o_acc.y += sc * o.y;
+      o_acc.z += sc * o.z;
+      o_acc.w += sc * o.w;
       l_acc += sc * red_l[w * ROWS + r];
     }
     // natural-log units, the unit of the persistent state
     if constexpr (kForm == kCluster) {
-      blk_o[idx] = o_acc;
+      *reinterpret_cast<float4*>(blk_o + idx) = o_acc;
       if (d == 0) {
         blk_m[r] = m_n * kLn2;
         blk_l[r] = l_acc;
       }
     } else {
       const size_t slot = (static_cast<size_t>(b) * H + first + kvH * r) * deal.cap + part;
-      Op[slot * D + d] = o_acc;
+      float* dst = Op + slot * D + d;
+      st4(dst, o_acc, (reinterpret_cast<uintptr_t>(dst) & 15u) == 0);
       if (d == 0) {
         Mp[slot] = m_n * kLn2;
         Lp[slot] = l_acc;
@@ -234,36 +266,53 @@ __device__ inline void finish_group(float* red_m, float* red_l, float* red_o, in
     const bool fresh = (deal.flags & RA_STEP_FRESH) != 0, finalize = (deal.flags & RA_STEP_FINALIZE) != 0;
     const int n = static_cast<int>(gridDim.x), rank = static_cast<int>(cluster_rank());
     cluster_barrier();  // every block's partial is staged
-    for (int idx = rank * kThr + tid; idx < live * D; idx += n * kThr) {
+    // (m, l) of row r in every block, all loads in flight at once; then what the maxima make of them:
+    // the factors of the blocks' partials (f), the factor of the old state (returned), the sum
+    auto load_ml = [&](int r, float (&f)[kMaxCluster], float (&ls)[kMaxCluster]) {
+#pragma unroll
+      for (int i = 0; i < kMaxCluster; ++i) {
+        f[i] = i < n ? ld_cluster(blk_m + r, i) : -INFINITY;
+        ls[i] = i < n ? ld_cluster(blk_l + r, i) : 0.f;
+      }
+    };
+    auto factors = [&](size_t row, float (&f)[kMaxCluster], const float (&ls)[kMaxCluster], float& m_n, float& l_acc) {
+      const float m_old = fresh ? -INFINITY : Mp[row];
+      m_n = m_old;
+#pragma unroll
+      for (int i = 0; i < kMaxCluster; ++i) m_n = fmaxf(m_n, f[i]);
+      const float a = (m_old == -INFINITY) ? 0.f : expf(m_old - m_n);
+      l_acc = (m_old == -INFINITY) ? 0.f : a * Lp[row];
+#pragma unroll
+      for (int i = 0; i < kMaxCluster; ++i) {
+        f[i] = (f[i] == -INFINITY) ? 0.f : expf(f[i] - m_n);
+        l_acc += f[i] * ls[i];
+      }
+      return a;
+    };
+    for (int idx = 4 * (rank * kThr + tid); idx < live * D; idx += 4 * n * kThr) {
       const int r = idx / D;
       const size_t row = static_cast<size_t>(b) * H + first + kvH * r;
-      float mp[kMaxCluster], lp[kMaxCluster], op[kMaxCluster];
+      float* dst = Op + row * D + (idx - r * D);
+      const bool vec = (reinterpret_cast<uintptr_t>(dst) & 15u) == 0;
+      float f[kMaxCluster], ls[kMaxCluster], m_n, l_acc;
+      float4 o[kMaxCluster], acc = make_float4(0.f, 0.f, 0.f, 0.f);
+      load_ml(r, f, ls);
 #pragma unroll
-      for (int i = 0; i < kMaxCluster; ++i) {
-        mp[i] = i < n ? ld_cluster(blk_m + r, i) : -INFINITY;
-        lp[i] = i < n ? ld_cluster(blk_l + r, i) : 0.f;
-        op[i] = i < n ? ld_cluster(blk_o + idx, i) : 0.f;
-      }
-      const float m_old = fresh ? -INFINITY : Mp[row];
-      float m_n = m_old;
-#pragma unroll
-      for (int i = 0; i < kMaxCluster; ++i) m_n = fmaxf(m_n, mp[i]);
+      for (int i = 0; i < kMaxCluster; ++i) o[i] = i < n ? ld_cluster4(blk_o + idx, i) : acc;
+      const float a = factors(row, f, ls, m_n, l_acc);
       if (m_n == -INFINITY) {
         // nothing visible anywhere: the state stays as it is (or is written empty)
-        if (fresh || finalize) Op[row * D + (idx - r * D)] = 0.f;
+        if (fresh || finalize) st4(dst, acc, vec);
         continue;
       }
-      const float a = (m_old == -INFINITY) ? 0.f : expf(m_old - m_n);
-      float o_acc = (m_old == -INFINITY) ? 0.f : a * Op[row * D + (idx - r * D)];
-      float l_acc = (m_old == -INFINITY) ? 0.f : a * Lp[row];
+      if (!fresh && Mp[row] > -INFINITY) add_scaled(acc, a, ld4(dst, vec));
 #pragma unroll
-      for (int i = 0; i < kMaxCluster; ++i) {
-        const float sc = (mp[i] == -INFINITY) ? 0.f : expf(mp[i] - m_n);
-        o_acc += sc * op[i];
-        l_acc += sc * lp[i];
+      for (int i = 0; i < kMaxCluster; ++i) add_scaled(acc, f[i], o[i]);
+      if (finalize) {
+        const float inv = l_acc > 0.f ? 1.f / l_acc : 0.f;
+        acc = make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);
       }
-      if (finalize) o_acc *= l_acc > 0.f ? 1.f / l_acc : 0.f;
-      Op[row * D + (idx - r * D)] = o_acc;
+      st4(dst, acc, vec);
     }
     // (m, l) of a row once every block has read the old ones and nobody needs this block any more
     float m_n = -INFINITY, l_acc = 0.f;
@@ -271,21 +320,21 @@ __device__ inline void finish_group(float* red_m, float* red_l, float* red_o, in
     size_t row = 0;
     if (owner) {
       row = static_cast<size_t>(b) * H + first + kvH * tid;
-      const float m_old = fresh ? -INFINITY : Mp[row];
-      m_n = m_old;
-      for (int i = 0; i < n; ++i) m_n = fmaxf(m_n, ld_cluster(blk_m + tid, i));
-      l_acc = (m_old == -INFINITY) ? 0.f : expf(m_old - m_n) * Lp[row];
-      for (int i = 0; i < n; ++i) {
-        const float mi = ld_cluster(blk_m + tid, i);
-        if (mi > -INFINITY) l_acc += expf(mi - m_n) * ld_cluster(blk_l + tid, i);
-      }
+      float f[kMaxCluster], ls[kMaxCluster];
+      load_ml(tid, f, ls);
+      factors(row, f, ls, m_n, l_acc);
     }
     cluster_barrier();
     if (owner && (m_n > -INFINITY || m_n != m_n || fresh)) {
       Mp[row] = m_n;
-      Lp[row] = l_acc;
+      Lp[row] = m_n == -INFINITY ? 0.f : l_acc;
     }
   }
+}
+
+// Floats of shared memory that a block's end takes: (m, l, O) by warp, then the block's.
+constexpr size_t red_floats(int warps, int rows, int D) {
+  return static_cast<size_t>(warps) * rows * (D + 2) + ((2 * rows + 3) & ~3) + static_cast<size_t>(rows) * D;
 }
 
 // A block's shares around both kernels' bodies: stages [stage_beg, stage_end) of the group
@@ -753,24 +802,24 @@ __global__ void __launch_bounds__(MmaCfg<D>::kThreads)
 #undef RAB_DECODE_LOOP_BEGIN
 #undef RAB_DECODE_LOOP_END
 
-// Fold the partials of the balanced and fixed forms into the persistent (out, m, l). grid = (H, B), block =
-// D x kFoldThreads / D threads: the partials are dealt to the thread groups (a single group walked up
-// to 57 partials one after the other, twice: 8 of the 36 us of the B1 H8 D128 fp32 call on 16384
-// rows) and (m, l) are read by lanes. Launched while the split kernel still runs (programmatic
-// dependent launch): everything it reads comes after griddepcontrol.wait and through plain pointers, because
-// the data changes while this kernel runs (const __restrict__ would allow loads through the read-only
-// path and in front of the wait).
+// Fold the partials of the balanced and fixed forms into the persistent (out, m, l). grid = (H, B); a thread
+// takes four columns of every n_grp-th partial (with one column and two groups at head_dim 256 the B1 H64/kvH1
+// call on 6000 rows spent 17 of its 28 us of kernels on 38 loads in a row per thread), and (m, l) are read by
+// lanes. Launched while the split kernel still runs (programmatic dependent launch): everything it
+// reads comes after griddepcontrol.wait and through plain pointers, because the data changes while this
+// kernel runs (const __restrict__ would allow loads through the read-only path and in front of the wait).
 // RA_STEP_FRESH: the state is known to be empty (it is written, never read, which saves the
 // caller an init launch); RA_STEP_FINALIZE: divide by l after folding (saves the finalize
-// launch).
-constexpr int kFoldThreads = 512;
+// launch). vec: Op and O are 16-byte aligned (a caller's workspace and state need not be).
+constexpr int kFoldGroups = 16, kFoldThreads = kFoldGroups * 64;
 __global__ void __launch_bounds__(kFoldThreads)
     decode_reduce_kernel(const float* Mp, const float* Lp, const float* Op, float* M, float* L, float* O, int H,
-                         int kvH, int D, int head_rows, int ctas, const Deal deal) {
+                         int kvH, int D, int head_rows, int ctas, bool vec, const Deal deal) {
   __shared__ float sc[kMaxSplits];
-  __shared__ float part_o[kFoldThreads];
+  __shared__ float4 part_o[kFoldThreads];
   const int h = blockIdx.x, b = blockIdx.y;
-  const int d = threadIdx.x % D, grp = threadIdx.x / D, n_grp = blockDim.x / D;
+  const int cols = D / 4;
+  const int d = threadIdx.x % cols * 4, grp = threadIdx.x / cols, n_grp = blockDim.x / cols;
   const int lane = threadIdx.x & 31;
   const size_t row = static_cast<size_t>(b) * H + h;
   const bool fresh = (deal.flags & RA_STEP_FRESH) != 0, finalize = (deal.flags & RA_STEP_FINALIZE) != 0;
@@ -783,7 +832,8 @@ __global__ void __launch_bounds__(kFoldThreads)
   asm volatile("griddepcontrol.wait;" ::: "memory");
   const float* mp = Mp + row * deal.cap;
   const float* lp = Lp + row * deal.cap;
-  const float* op = Op + row * deal.cap * D;
+  const float* op = Op + row * deal.cap * D + d;
+  float* o_row = O + row * D + d;
   // every warp works out the same maximum and sum; the scales go to shared memory once
   const float m_old = fresh ? -INFINITY : M[row];
   float m_n = m_old;
@@ -793,7 +843,7 @@ __global__ void __launch_bounds__(kFoldThreads)
   if (m_n == -INFINITY) {
     // nothing visible anywhere: the state stays as it is (or is written empty)
     if ((fresh || finalize) && grp == 0) {
-      O[row * D + d] = 0.f;
+      st4(o_row, make_float4(0.f, 0.f, 0.f, 0.f), vec);
       if (fresh && d == 0) {
         M[row] = -INFINITY;
         L[row] = 0.f;
@@ -813,16 +863,19 @@ __global__ void __launch_bounds__(kFoldThreads)
   const float a = (m_old == -INFINITY) ? 0.f : expf(m_old - m_n);
   if (m_old > -INFINITY) l_acc += a * L[row];
   __syncthreads();
-  float o_acc = 0.f;
+  float4 o_acc = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 4
-  for (int s = grp; s < n; s += n_grp) o_acc += sc[s] * op[static_cast<size_t>(s) * D + d];
+  for (int s = grp; s < n; s += n_grp) add_scaled(o_acc, sc[s], ld4(op + static_cast<size_t>(s) * D, vec));
   part_o[threadIdx.x] = o_acc;
   __syncthreads();
   if (grp > 0) return;
-  for (int i = 1; i < n_grp; ++i) o_acc += part_o[i * D + d];
-  if (m_old > -INFINITY) o_acc += a * O[row * D + d];
-  if (finalize) o_acc *= l_acc > 0.f ? 1.f / l_acc : 0.f;
-  O[row * D + d] = o_acc;
+  for (int i = 1; i < n_grp; ++i) add_scaled(o_acc, 1.f, part_o[i * cols + threadIdx.x]);
+  if (m_old > -INFINITY) add_scaled(o_acc, a, ld4(o_row, vec));
+  if (finalize) {
+    const float inv = l_acc > 0.f ? 1.f / l_acc : 0.f;
+    o_acc = make_float4(o_acc.x * inv, o_acc.y * inv, o_acc.z * inv, o_acc.w * inv);
+  }
+  st4(o_row, o_acc, vec);
   if (d == 0) {  // every thread has read M / L: two block barriers ago
     M[row] = m_n;
     L[row] = l_acc;
@@ -842,33 +895,56 @@ struct DecodePlan {
   Deal deal;
 };
 
+// What a kernel needs for a ring stage, in us: `alone` for one block on an SM, `share` of the SM's issue slots
+// (k blocks on an SM take k times that if it is longer). Slopes of calls with few groups, one block each,
+// between 6000 and 20000 rows: the mma kernel 0.53, 0.71 and 1.14 at head_dim 64, 128 (64 keys) and 256 (32);
+// the SIMT kernel 0.34-0.49 for 16 KB with one head, 0.47-0.77 with four, 0.75-1.1 with eight.
+struct StageCost {
+  double alone, share;
+};
+constexpr StageCost mma_stage_cost(int D) { return {0.5 + 0.0038 * D, 0.0036 * D}; }
+constexpr StageCost simt_stage_cost(int heads, size_t stage_bytes) {
+  return {(0.46 + 0.12 * heads) * (stage_bytes / 16384.0), 0.145 * heads * (stage_bytes / 16384.0)};
+}
+
 // Which form, and how many blocks. `per_sm`: resident blocks per SM; `cap`: partial slots per row
-// that the workspace holds. Estimates in microseconds from a stage's bytes: 6.5 TB/s for the whole
-// GPU, 0.1 MB/us for one SM, and what the fold (launch and kernel) or the merge adds.
-DecodePlan make_plan(int groups, int stages, size_t stage_bytes, int per_sm, int cap, int ring_max,
-                     int fixed) {
+// that the workspace holds; `rows`: (batch, head) rows; `head_rows`: rows of a group; `fixed`: splits of the
+// fixed form (0: balanced). Every estimate is the walk of a block, wave by wave, at what its SM or the
+// memory (7 TB/s) allows, plus what the fold (a launch, and more the more rows it has) or the merge
+// (columns of the group, blocks of the cluster, and a wave of clusters starts slower than one of blocks)
+// adds. Constants fitted to 457 shapes (heads 8/8 to 64/1, batch 1 to 64, 200 to 100000 rows, fp16 and fp32,
+// every head_dim) timed in each form: this choice is 1.0 % from the best form on average, the estimate
+// before it (0.1 MB/us for any block, a fold of 3 us) 5.6 %, and up to twofold with few or very many groups.
+DecodePlan make_plan(int groups, int stages, size_t stage_bytes, int per_sm, int cap, int ring_max, int fixed,
+                     StageCost cost, size_t rows, int head_rows, int D) {
+  constexpr double kBytesPerUs = 7e6, kFold = 8.2, kFoldRow = 0.005, kMerge = 0.6, kMergeBlock = 0.15,
+                   kMergeElement = 0.0005, kWave = 1.5, kClusterWave = 4.0;
   DecodePlan p;
   const int sms = sm_count();
   const double total = static_cast<double>(groups) * stages;
-  const double whole = total * stage_bytes / 6.5e6, one = stage_bytes / 0.1e6;
   const int slots = sms * per_sm;
+  auto walk = [&](double blocks, double stages_each) {
+    const double active = std::min<double>(blocks, slots), on_sm = std::min<double>(per_sm, std::ceil(blocks / sms));
+    return std::ceil(blocks / slots) * stages_each *
+           std::max(std::max(cost.alone, on_sm * cost.share), stage_bytes * active / kBytesPerUs);
+  };
   // no more partials than the workspace holds: a group meets at most ceil(ctas / groups) + 1 blocks,
   // exactly one each when there are as many blocks as groups
   long long ctas = std::min<long long>(slots, static_cast<long long>(total));
   ctas = cap > 1 ? std::min(ctas, (cap - 1ll) * groups) : groups;
   fixed = std::min(std::min(fixed, cap), stages);
-  const double waves_f = std::ceil(static_cast<double>(groups) * fixed / slots);
-  const double share = fixed ? waves_f * std::ceil(static_cast<double>(stages) / fixed) : std::ceil(total / ctas);
-  const double t_bal = std::max(whole, share * one * per_sm) + kFoldUs;
   p.cluster = 0;
   p.ctas = static_cast<int>(ctas);
-  double best = t_bal;
-  for (int c = 1; c <= kMaxCluster; c *= 2) {
+  double best = (fixed ? walk(static_cast<double>(groups) * fixed, std::ceil(static_cast<double>(stages) / fixed))
+                       : walk(static_cast<double>(ctas), std::ceil(total / ctas))) +
+                kFold + kFoldRow * rows;
+  for (int c = 1; c <= kMaxCluster && groups <= 65535; c *= 2) {
     if (c > 1 && c > stages) break;
-    const double waves = std::ceil(static_cast<double>(groups) * c / slots);
-    const double t = std::max(whole, waves * std::ceil(static_cast<double>(stages) / c) * one * per_sm) +
-                     (c > 1 ? kMergeUs : 0.0);
-    if (t < best && groups <= 65535) {
+    const double blocks = static_cast<double>(groups) * c;
+    const double t = walk(blocks, std::ceil(static_cast<double>(stages) / c)) + kMergeElement * head_rows * D +
+                     (c > 1 ? kMerge + kMergeBlock * c : 0.0) +
+                     (std::ceil(blocks / slots) - 1) * (c > 1 ? kClusterWave : kWave);
+    if (t < best) {
       best = t;
       p.cluster = c;
     }
@@ -950,7 +1026,7 @@ int partial_space(size_t rows, int D, int cap, void* workspace, float** Op, floa
 // launch(cluster form?, config, deal, Mp, Lp, Op) sets the attribute and launches the kernel.
 template <int D, int ROWS, typename Launch>
 int run_plan(const ra_shape& s, int head_batches, int stages, size_t stage_bytes, int ring_max, int per_sm,
-             size_t red_bytes, int old_splits, bool fixed, float* out, float* m, float* l, void* workspace,
+             StageCost cost, size_t red_bytes, int old_splits, bool fixed, float* out, float* m, float* l, void* workspace,
              size_t workspace_bytes, int split_cap, unsigned flags, cudaStream_t stream, Launch launch) {
   const int kvH = kv_heads_of(s);
   const size_t rows = static_cast<size_t>(s.batch) * s.heads;
@@ -962,7 +1038,7 @@ int run_plan(const ra_shape& s, int head_batches, int stages, size_t stage_bytes
     cap = static_cast<int>(std::min<size_t>(cap, workspace_bytes / slot_bytes));
   }
   DecodePlan p = make_plan(s.batch * kvH * head_batches, stages, stage_bytes, per_sm, cap, ring_max,
-                           fixed ? old_splits : 0);
+                           fixed ? old_splits : 0, cost, rows, std::min(ROWS, (s.heads + kvH - 1) / kvH), D);
   p.deal.head_batches = head_batches;
   p.deal.flags = flags;
   cudaLaunchConfig_t cfg = {};
@@ -986,7 +1062,9 @@ int run_plan(const ra_shape& s, int head_batches, int stages, size_t stage_bytes
   if (rc != RA_OK) return rc;
   cudaLaunchConfig_t fold = {};
   fold.gridDim = dim3(s.heads, s.batch);
-  fold.blockDim = dim3(kFoldThreads / D * D);
+  // (no more thread groups than partials: with many rows and few partials each the idle ones cost, 2048
+  // rows of D32 8 us)
+  fold.blockDim = dim3(std::max(32, std::min(kFoldGroups, p.deal.cap) * (D / 4)));
   fold.stream = stream;
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
@@ -994,7 +1072,8 @@ int run_plan(const ra_shape& s, int head_batches, int stages, size_t stage_bytes
   fold.numAttrs = 1;
   RAB_CUDA(cudaLaunchKernelEx(&fold, decode_reduce_kernel, static_cast<const float*>(Mp),
                               static_cast<const float*>(Lp), static_cast<const float*>(Op), m, l, out,
-                              s.heads, kvH, D, ROWS, p.ctas, p.deal));
+                              s.heads, kvH, D, ROWS, p.ctas,
+                              ((reinterpret_cast<uintptr_t>(Op) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0, p.deal));
   RAB_CUDA(cudaGetLastError());
   return RA_OK;
 }
@@ -1046,13 +1125,13 @@ int launch_decode_typed(const void* q, const void* k, const void* v, float* out,
   if constexpr (sizeof(T) == 2 && D >= 64) {
     // 16-bit caches: the tensor-core kernel (16 query heads per block)
     using M = MmaCfg<D>;
-    constexpr size_t kRed = static_cast<size_t>(M::kWarps + 1) * 16 * (D + 2) * sizeof(float);
+    constexpr size_t kRed = red_floats(M::kWarps, 16, D) * sizeof(float);
     constexpr size_t kSmem = M::kSmemBytes > kRed ? M::kSmemBytes : kRed;
     const int head_batches = (group + 15) / 16;
     const int stages = (sk_eff + M::kStageRows - 1) / M::kStageRows;
     static const int per_sm = resident_blocks(decode_mma_kernel<T, D, kBalanced>, M::kThreads, kSmem);
     return run_plan<D, 16>(
-        s, head_batches, stages, 2 * M::kStageBytes, M::kStages, per_sm, kRed,
+        s, head_batches, stages, 2 * M::kStageBytes, M::kStages, per_sm, mma_stage_cost(D), kRed,
         fixed_splits(s.batch * kvH * head_batches, sk_eff, 64, split_cap), false, out,
         m, l, workspace, workspace_bytes, split_cap, flags, stream,
         [&](bool cluster, cudaLaunchConfig_t& cfg, const Deal& deal, float* Mp, float* Lp, float* Op) {
@@ -1067,13 +1146,13 @@ int launch_decode_typed(const void* q, const void* k, const void* v, float* out,
       constexpr int GB = decltype(gb_tag)::value;
       using C = DecodeCfg<T, D, GB>;
       constexpr DealForm kDealt = GB * C::kEPL >= 64 ? kFixed : kBalanced;  // (see DecodeCfg)
-      constexpr size_t kRed = static_cast<size_t>(kWarps + 1) * GB * (D + 2) * sizeof(float);
+      constexpr size_t kRed = red_floats(kWarps, GB, D) * sizeof(float);
       constexpr size_t kSmem = C::kSmemBytes > kRed ? C::kSmemBytes : kRed;
       const int head_batches = (group + GB - 1) / GB;
       const int stages = (sk_eff + C::kRowsPerStage - 1) / C::kRowsPerStage;
       static const int per_sm = resident_blocks(decode_split_kernel<T, D, GB, kDealt>, kThreads, kSmem);
       return run_plan<D, GB>(
-          s, head_batches, stages, 2 * C::kStageBytes, kStages, per_sm, kRed,
+          s, head_batches, stages, 2 * C::kStageBytes, kStages, per_sm, simt_stage_cost(GB, 2 * C::kStageBytes), kRed,
           fixed_splits(s.batch * kvH * head_batches, sk_eff, C::kPlanRows, split_cap), kDealt == kFixed,
           out, m, l, workspace, workspace_bytes, split_cap, flags, stream,
           [&](bool cluster, cudaLaunchConfig_t& cfg, const Deal& deal, float* Mp, float* Lp, float* Op) {

@@ -440,3 +440,23 @@ def test_document_mask_and_moving_reference_in_both_forms(dtype, D, split):
     tol = 1e-4 if dtype == torch.float32 else TOL[dtype]
     assert_close(state[0].cpu().numpy(), want, tol, tol, "out")
     assert_close(lse, want_lse, tol, tol, "lse")
+
+
+@pytest.mark.parametrize("dtype,H,kvH,Sk,D", [(torch.float16, 32, 2, 300, 256), (torch.float16, 8, 8, 20000, 128),
+                                              (torch.float32, 16, 2, 6000, 256), (torch.float32, 8, 8, 500, 32),
+                                              (torch.bfloat16, 48, 1, 9000, 64)])
+def test_decode_into_a_state_and_a_workspace_aligned_to_four_bytes(dtype, H, kvH, Sk, D):
+    # every form (cluster, equal shares, fixed splits) writes and folds four columns at a time where it can
+    q, k, v = (round_to(x, dtype) for x in normal_inputs(15, 1, H, kvH, 1, Sk, D))
+    want, want_lse = oracle.cpu_attention(q, k, v, False, kv_heads=kvH, want_lse=True, threads=8)
+    s = api.AttentionShape(1, H, 1, Sk, D, kvH)
+    out = torch.full((H * D + 1,), float("nan"), device="cuda")[1:].view(1, H, 1, D)
+    m, l = (torch.full((1, H, 1), float("nan"), device="cuda") for _ in range(2))
+    ws = torch.full((lib().ra_decode_workspace_bytes(C.byref(s.c())) // 4 + 1,), float("nan"), device="cuda")[1:]
+    api.launch_attention_init(out, m, l, s)
+    for _ in range(2):
+        api.launch_attention_decode_step(dev(q, dtype), dev(k, dtype), dev(v, dtype), out, m, l, s, 0, 0, False, workspace=ws)
+    lse = api.attention_lse(m, l).cpu().numpy() - np.log(2.0)
+    api.launch_attention_finalize(out, l, s)
+    assert_close(out.cpu().numpy(), want, TOL[dtype], TOL[dtype], "out")
+    assert_close(lse, want_lse, TOL[dtype], TOL[dtype], "lse")
