@@ -583,7 +583,7 @@ __global__ void __launch_bounds__(kThreadsF, 1)
     if (mine) {
       const float4* q4 = reinterpret_cast<const float4*>(q_g + grow * DR);
       unsigned mx = 0;
-#pragma unroll 4
+#pragma unroll 16
       for (int i = 0; i < DR / 4; ++i) {
         const float4 v = row_valid ? q4[i] : make_float4(0.f, 0.f, 0.f, 0.f);
         mx = max(max(max(mx, finite_abs_bits(v.x)), max(finite_abs_bits(v.y), finite_abs_bits(v.z))),
