@@ -1053,7 +1053,8 @@ int launch_f32_d(const StepArgs& a, cudaStream_t stream) {
   const int* slots = nullptr;
   const int rc = cluster_slots(step_f32_kernel<DR, true>, kThreadsF, F32Cfg<DR, true>::kSmemBytes, &slots);
   if (rc != RA_OK) return rc;
-  const int split = pick_key_split<kBNf>(a, 2 * kBM, 1.5, slots);
+  // (a merge in tiles: those of head_dim 128 take longer)
+  const int split = pick_key_split<kBNf>(a, 2 * kBM, DR == 128 ? 1.5 : 2.5, slots);
   return split > 1 ? launch_f32<DR, true>(a, stream, split) : launch_f32<DR, false>(a, stream, 1);
 }
 

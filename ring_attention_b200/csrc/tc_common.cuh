@@ -671,6 +671,8 @@ inline int cluster_slots(Kern kern, int threads, int smem_bytes, const int** out
 // 65536 keys H8 D128 1077 / 540 / 277 / 146; 1024 x 1024 H8 D64 23 / 19 / 17 / 38; 2048 x 2048 H16
 // D64 (128 blocks) 36 / 38 / 59 / 122; 1024 x 1024 H8 D128 29 / 25 / 18.5 / 49, H16 29 / 25 / 33 / 80;
 // 1024 x 1024 H8 D256 (64 blocks) 27 / 29 / 39 / 82; 2048 x 2048 H4 D256 41 / 37 / 41 / 86.
+// Four tiles at n = 1 / 2 / 4: 512 x 512 H8 D128 20.5 / 20.5 / 16, fp32 200 x 200 H8 D64 18.5 / 19 / 16.5, D128
+// 29 / 28 / 22.6 (so a share may be a single tile); three tiles, fp32 D64: 12.6 at n = 1, 14.4 at 3.
 template <int kTileKeys>
 inline int pick_key_split(const StepArgs& a, int q_block_rows, double merge_tiles, const int* slots) {
   const int forced = static_cast<int>((a.flags >> RA_STEP_KEY_SPLIT_SHIFT) & 15u);
@@ -704,11 +706,11 @@ inline int pick_key_split(const StepArgs& a, int q_block_rows, double merge_tile
   double best_t = 0;
   for (int i = 0; i < 7; ++i) {
     const int n = kSizes[i];
-    if (n > 1 && longest < 2 * n) break;  // at least two tiles to walk
+    if (longest < n) break;
     if (slots[n] == 0) continue;
     const double fixed = kFixed + (n > 1 ? merge_tiles : 0);
     const double empties = static_cast<double>(heads * idle) * n * kEmpty / slots[n];
-    double t = longest / static_cast<double>(n) + fixed + empties;
+    double t = (longest + n - 1) / n + fixed + empties;
     const double n_blocks = static_cast<double>(heads * busy) * n;
     if (n_blocks > slots[n]) {
       const double spread = (n_blocks / slots[n] + 0.5) * (mean / n + fixed) + empties;
