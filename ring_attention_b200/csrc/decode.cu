@@ -31,24 +31,25 @@
 #include <mutex>
 #include <type_traits>
 
-#include "common.cuh"
+#include "tc_common.cuh"
 
 namespace rab {
 
 namespace {
 
+using tcgen::cluster_addr;
+using tcgen::cluster_ctarank;
+using tcgen::cluster_sync_threads;
+using tcgen::ex2;
+using tcgen::kLn2;
+using tcgen::kLog2e;
+using tcgen::ld_cluster_f4;
+using tcgen::smem_u32;
+
 constexpr int kWarps = 8;
 constexpr int kThreads = kWarps * 32;
 constexpr int kStages = 4;
 constexpr int kMaxSplits = 128;
-constexpr float kLog2e = 1.4426950408889634f;
-constexpr float kLn2 = 0.6931471805599453f;
-
-__device__ inline float ex2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
 
 __device__ inline void cp_async16(void* smem_dst, const void* gsrc, int src_bytes) {
   const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(smem_dst));
@@ -142,9 +143,9 @@ struct DecodeCfg {
 //    it made no difference by itself (799 against 769 us); with two blocks per SM 1, 3 or 6 times as
 //    many blocks were no faster either, and the B1 H8 D128 fp32 call on 16384 rows slower (37 us
 //    against 31).
-//  * fixed: `splits` blocks per group, about three waves, partials and fold as above. For the
-//    kernel whose registers leave room for one block per SM only, where the loop over shares
-//    gains them nothing (eight fp32 heads of 256).
+//  * fixed: `splits` blocks per group, about three waves, partials and fold as above. For the SIMT kernels
+//    whose registers leave room for one block per SM only: eight fp32 heads of 256, where the
+//    loop over shares gained nothing, and eight 16-bit heads of 32, which share the rule.
 //  * cluster: the blocks of a cluster take equal shares of ONE group and merge
 //    their partials through distributed shared memory into the state. No workspace and no second
 //    launch: for calls that one wave finishes in a few microseconds (B1 H32/kvH8 D128 fp16 on 1061
@@ -164,33 +165,9 @@ __host__ __device__ inline int deal_owner(long long x, long long total, int ctas
   return static_cast<int>(((x + 1) * ctas - 1) / total);
 }
 
-__device__ inline unsigned cluster_rank() {
-  unsigned r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ inline void cluster_barrier() {
-  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
-}
-__device__ inline float ld_cluster(const float* p, unsigned rank) {
-  unsigned addr;
+__device__ inline float ld_cluster_f1(unsigned addr) {
   float v;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
-               : "=r"(addr)
-               : "r"(static_cast<unsigned>(__cvta_generic_to_shared(p))), "r"(rank));
   asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr));
-  return v;
-}
-
-__device__ inline float4 ld_cluster4(const float* p, unsigned rank) {
-  unsigned addr;
-  float4 v;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
-               : "=r"(addr)
-               : "r"(static_cast<unsigned>(__cvta_generic_to_shared(p))), "r"(rank));
-  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
-               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-               : "r"(addr));
   return v;
 }
 
@@ -264,15 +241,15 @@ __device__ inline void finish_group(float* red_m, float* red_l, float* red_o, in
   if constexpr (kForm == kCluster) {
     // Mp / Lp / Op are the state itself here
     const bool fresh = (deal.flags & RA_STEP_FRESH) != 0, finalize = (deal.flags & RA_STEP_FINALIZE) != 0;
-    const int n = static_cast<int>(gridDim.x), rank = static_cast<int>(cluster_rank());
-    cluster_barrier();  // every block's partial is staged
+    const int n = static_cast<int>(gridDim.x), rank = static_cast<int>(cluster_ctarank());
+    cluster_sync_threads();  // every block's partial is staged
     // (m, l) of row r in every block, all loads in flight at once; then what the maxima make of them:
     // the factors of the blocks' partials (f), the factor of the old state (returned), the sum
     auto load_ml = [&](int r, float (&f)[kMaxCluster], float (&ls)[kMaxCluster]) {
 #pragma unroll
       for (int i = 0; i < kMaxCluster; ++i) {
-        f[i] = i < n ? ld_cluster(blk_m + r, i) : -INFINITY;
-        ls[i] = i < n ? ld_cluster(blk_l + r, i) : 0.f;
+        f[i] = i < n ? ld_cluster_f1(cluster_addr(smem_u32(blk_m + r), i)) : -INFINITY;
+        ls[i] = i < n ? ld_cluster_f1(cluster_addr(smem_u32(blk_l + r), i)) : 0.f;
       }
     };
     auto factors = [&](size_t row, float (&f)[kMaxCluster], const float (&ls)[kMaxCluster], float& m_n, float& l_acc) {
@@ -298,7 +275,7 @@ __device__ inline void finish_group(float* red_m, float* red_l, float* red_o, in
       float4 o[kMaxCluster], acc = make_float4(0.f, 0.f, 0.f, 0.f);
       load_ml(r, f, ls);
 #pragma unroll
-      for (int i = 0; i < kMaxCluster; ++i) o[i] = i < n ? ld_cluster4(blk_o + idx, i) : acc;
+      for (int i = 0; i < kMaxCluster; ++i) o[i] = i < n ? ld_cluster_f4(cluster_addr(smem_u32(blk_o + idx), i)) : acc;
       const float a = factors(row, f, ls, m_n, l_acc);
       if (m_n == -INFINITY) {
         // nothing visible anywhere: the state stays as it is (or is written empty)
@@ -324,7 +301,7 @@ __device__ inline void finish_group(float* red_m, float* red_l, float* red_o, in
       load_ml(tid, f, ls);
       factors(row, f, ls, m_n, l_acc);
     }
-    cluster_barrier();
+    cluster_sync_threads();
     if (owner && (m_n > -INFINITY || m_n != m_n || fresh)) {
       Mp[row] = m_n;
       Lp[row] = m_n == -INFINITY ? 0.f : l_acc;
@@ -337,36 +314,46 @@ constexpr size_t red_floats(int warps, int rows, int D) {
   return static_cast<size_t>(warps) * rows * (D + 2) + ((2 * rows + 3) & ~3) + static_cast<size_t>(rows) * D;
 }
 
-// A block's shares around both kernels' bodies: stages [stage_beg, stage_end) of the group
-// (b, kvh, hb), partial slot `part`. Only the balanced form loops.
-#define RAB_DECODE_LOOP_BEGIN                                                                      \
-  constexpr bool kLoop = kForm == kBalanced;                                                       \
-  const int n_share = kForm == kFixed ? deal.splits : static_cast<int>(gridDim.x);                 \
-  const int i_share = static_cast<int>(kForm == kFixed ? blockIdx.x % deal.splits : blockIdx.x);   \
-  const long long total = static_cast<long long>(deal.groups) * deal.stages;                       \
-  long long at = kLoop ? total * i_share / n_share : 0;                                            \
-  const long long at_end = kLoop ? total * (i_share + 1ll) / n_share : 1;                          \
-  if (kForm != kCluster) asm volatile("griddepcontrol.launch_dependents;");                        \
-  while (at < at_end) {                                                                            \
-    const int group = static_cast<int>(kLoop             ? at / deal.stages                        \
-                                       : kForm == kFixed ? blockIdx.x / deal.splits                \
-                                                         : blockIdx.y);                            \
-    const int stage_beg =                                                                          \
-        kLoop ? static_cast<int>(at - static_cast<long long>(group) * deal.stages)                 \
-              : static_cast<int>(static_cast<long long>(deal.stages) * i_share / n_share);         \
-    const int stage_end =                                                                          \
-        kLoop ? static_cast<int>(min(static_cast<long long>(deal.stages), stage_beg + (at_end - at))) \
-              : static_cast<int>(static_cast<long long>(deal.stages) * (i_share + 1ll) / n_share); \
-    const int part =                                                                               \
-        kLoop ? i_share - deal_owner(static_cast<long long>(group) * deal.stages, total, n_share)  \
-              : i_share;                                                                           \
-    at += kLoop ? stage_end - stage_beg : 1;                                                       \
-    const int hb = group % deal.head_batches;                                                      \
-    const int kvh = (group / deal.head_batches) % kvH;                                             \
-    const int b = group / (deal.head_batches * kvH);
-#define RAB_DECODE_LOOP_END                                                                        \
-    if (kLoop) __syncthreads(); /* the ring is free again */                                       \
+// A block's next share: stages [beg, end) of the group (b, kvh, hb), partial slot `part`. Only the balanced form
+// has more than one.
+struct Share {
+  int beg, end, part, hb, kvh, b;
+};
+template <DealForm kForm>
+struct Shares {
+  long long total, at, at_end;
+  int n, i;
+  __device__ explicit Shares(const Deal& deal) {
+    n = kForm == kFixed ? deal.splits : static_cast<int>(gridDim.x);
+    i = static_cast<int>(kForm == kFixed ? blockIdx.x % deal.splits : blockIdx.x);
+    total = static_cast<long long>(deal.groups) * deal.stages;
+    at = kForm == kBalanced ? total * i / n : 0;
+    at_end = kForm == kBalanced ? total * (i + 1ll) / n : 1;
+    if (kForm != kCluster) asm volatile("griddepcontrol.launch_dependents;");
   }
+  __device__ bool next(const Deal& deal, int kvH, Share& s) {
+    if (at >= at_end) return false;
+    const int group = static_cast<int>(kForm == kBalanced ? at / deal.stages
+                                       : kForm == kFixed  ? blockIdx.x / deal.splits
+                                                          : blockIdx.y);
+    if (kForm == kBalanced) {
+      const long long first = static_cast<long long>(group) * deal.stages;
+      s.beg = static_cast<int>(at - first);
+      s.end = static_cast<int>(min(static_cast<long long>(deal.stages), s.beg + (at_end - at)));
+      s.part = i - deal_owner(first, total, n);
+      at += s.end - s.beg;
+    } else {
+      s.beg = static_cast<int>(static_cast<long long>(deal.stages) * i / n);
+      s.end = static_cast<int>(static_cast<long long>(deal.stages) * (i + 1ll) / n);
+      s.part = i;
+      at = at_end;
+    }
+    s.hb = group % deal.head_batches;
+    s.kvh = (group / deal.head_batches) % kvH;
+    s.b = group / (deal.head_batches * kvH);
+    return true;
+  }
+};
 
 // GB = query heads handled per block. Grid: see Deal.
 template <typename T, int D, int GB, DealForm kForm>
@@ -384,168 +371,172 @@ __global__ void __launch_bounds__(kThreads)
   const int warp = tid >> 5;
   const int lr = lane % C::kLPR;       // lane within the row group
   const int grp = lane / C::kLPR;      // row group within the warp
-  RAB_DECODE_LOOP_BEGIN
+  Shares<kForm> shares(deal);
+  Share share;
+  while (shares.next(deal, kvH, share)) {
+    const int b = share.b, kvh = share.kvh, hb = share.hb;
 
-  // Query heads of this block: h = kvh + kvH * (hb * GB + g), while h < H.
-  float q_reg[GB][C::kEPL];
-  float o_reg[GB][C::kEPL];
-  float m_run[GB], l_run[GB];
+    // Query heads of this block: h = kvh + kvH * (hb * GB + g), while h < H.
+    float q_reg[GB][C::kEPL];
+    float o_reg[GB][C::kEPL];
+    float m_run[GB], l_run[GB];
 #pragma unroll
-  for (int g = 0; g < GB; ++g) {
-    const int h = kvh + kvH * (hb * GB + g);
-    m_run[g] = -INFINITY;
-    l_run[g] = 0.f;
-#pragma unroll
-    for (int v = 0; v < C::kVPT; ++v) {
-      float f[Piece<T>::kElems];
-      if (h < H) {
-        const uint4 u = *reinterpret_cast<const uint4*>(
-            reinterpret_cast<const unsigned char*>(Q + (static_cast<size_t>(b) * H + h) * D) +
-            (v * C::kLPR + lr) * 16);
-        Piece<T>::unpack(u, f);
-      } else {
-#pragma unroll
-        for (int e = 0; e < Piece<T>::kElems; ++e) f[e] = 0.f;
-      }
-#pragma unroll
-      for (int e = 0; e < Piece<T>::kElems; ++e) {
-        q_reg[g][v * Piece<T>::kElems + e] = f[e] * scale_log2;
-        o_reg[g][v * Piece<T>::kElems + e] = 0.f;
-      }
-    }
-  }
-
-  const int row_begin = stage_beg * C::kRowsPerStage;
-  const int row_end = min(static_cast<long long>(sk_eff), static_cast<long long>(stage_end) * C::kRowsPerStage);
-  const int n_rows = row_end - row_begin;
-  const int n_stages = stage_end - stage_beg;
-  const unsigned char* k_base = reinterpret_cast<const unsigned char*>(
-      K + (static_cast<size_t>(b) * kvH + kvh) * kv_head_stride);
-  const unsigned char* v_base = reinterpret_cast<const unsigned char*>(
-      V + (static_cast<size_t>(b) * kvH + kvh) * kv_head_stride);
-
-  auto issue = [&](int st) {
-    if (st < n_stages) {
-      const int slot = st % kStages;
-      const long long first = static_cast<long long>(row_begin) + st * C::kRowsPerStage;
-      const long long valid_bytes =
-          (static_cast<long long>(row_end) - first) * C::kRowBytes;  // > 0
-      const size_t goff = static_cast<size_t>(first) * C::kRowBytes;
-      for (int p = tid; p < C::kStageBytes / 16; p += kThreads) {
-        const long long off = static_cast<long long>(p) * 16;
-        const bool ok = off < valid_bytes;
-        // past the split: src-size 0 zero-fills the destination, the source is not read
-        cp_async16(k_ring + slot * C::kStageBytes + off, ok ? k_base + goff + off : k_base,
-                   ok ? 16 : 0);
-        cp_async16(v_ring + slot * C::kStageBytes + off, ok ? v_base + goff + off : v_base,
-                   ok ? 16 : 0);
-      }
-    }
-    cp_async_commit();
-  };
-
-#pragma unroll
-  for (int s = 0; s < kStages - 1; ++s) issue(s);
-
-  for (int st = 0; st < n_stages; ++st) {
-    cp_async_wait<kStages - 2>();
-    __syncthreads();
-    issue(st + kStages - 1);
-    const int slot = st % kStages;
-    const int stage_row0 = st * C::kRowsPerStage;
-#pragma unroll 1
-    for (int step = 0; step < C::kSteps; ++step) {
-      const int rl = step * C::kRowsPerStep + warp * C::kRowsPerWarpStep + grp;
-      const bool valid = stage_row0 + rl < n_rows;
-      const unsigned char* krow = k_ring + slot * C::kStageBytes + rl * C::kRowBytes;
-      const unsigned char* vrow = v_ring + slot * C::kStageBytes + rl * C::kRowBytes;
-      float kf[C::kEPL];
+    for (int g = 0; g < GB; ++g) {
+      const int h = kvh + kvH * (hb * GB + g);
+      m_run[g] = -INFINITY;
+      l_run[g] = 0.f;
 #pragma unroll
       for (int v = 0; v < C::kVPT; ++v) {
-        const uint4 u = *reinterpret_cast<const uint4*>(krow + (v * C::kLPR + lr) * 16);
-        Piece<T>::unpack(u, &kf[v * Piece<T>::kElems]);
-      }
-      float s[GB];
+        float f[Piece<T>::kElems];
+        if (h < H) {
+          const uint4 u = *reinterpret_cast<const uint4*>(
+              reinterpret_cast<const unsigned char*>(Q + (static_cast<size_t>(b) * H + h) * D) +
+              (v * C::kLPR + lr) * 16);
+          Piece<T>::unpack(u, f);
+        } else {
 #pragma unroll
-      for (int g = 0; g < GB; ++g) {
-        float acc = 0.f;
+          for (int e = 0; e < Piece<T>::kElems; ++e) f[e] = 0.f;
+        }
 #pragma unroll
-        for (int e = 0; e < C::kEPL; ++e) acc = fmaf(q_reg[g][e], kf[e], acc);
-        s[g] = acc;
-      }
-#pragma unroll
-      for (int off = 1; off < C::kLPR; off <<= 1) {
-#pragma unroll
-        for (int g = 0; g < GB; ++g) s[g] += __shfl_xor_sync(0xffffffffu, s[g], off);
-      }
-      float vf[C::kEPL];
-#pragma unroll
-      for (int v = 0; v < C::kVPT; ++v) {
-        const uint4 u = *reinterpret_cast<const uint4*>(vrow + (v * C::kLPR + lr) * 16);
-        Piece<T>::unpack(u, &vf[v * Piece<T>::kElems]);
-      }
-      if (valid) {
-#pragma unroll
-        for (int g = 0; g < GB; ++g) {
-          if (s[g] > m_run[g]) {  // rare after the first rows: rescale only when the max moves
-            const float alpha = ex2(m_run[g] - s[g]);  // ex2(-inf) = 0 on the first row
-            l_run[g] *= alpha;
-#pragma unroll
-            for (int e = 0; e < C::kEPL; ++e) o_reg[g][e] *= alpha;
-            m_run[g] = s[g];
-          }
-          const float p = ex2(s[g] - m_run[g]);
-          l_run[g] += p;
-#pragma unroll
-          for (int e = 0; e < C::kEPL; ++e) o_reg[g][e] = fmaf(p, vf[e], o_reg[g][e]);
+        for (int e = 0; e < Piece<T>::kElems; ++e) {
+          q_reg[g][v * Piece<T>::kElems + e] = f[e] * scale_log2;
+          o_reg[g][v * Piece<T>::kElems + e] = 0.f;
         }
       }
     }
-  }
-  cp_async_wait<0>();
 
-  // Merge the row groups of the warp (log-sum-exp merge through shuffles) ...
-#pragma unroll
-  for (int off = C::kLPR; off < 32; off <<= 1) {
-#pragma unroll
-    for (int g = 0; g < GB; ++g) {
-      const float m_o = __shfl_xor_sync(0xffffffffu, m_run[g], off);
-      const float l_o = __shfl_xor_sync(0xffffffffu, l_run[g], off);
-      const float m_n = fmaxf(m_run[g], m_o);
-      const float a = (m_run[g] == -INFINITY) ? 0.f : ex2(m_run[g] - m_n);
-      const float c = (m_o == -INFINITY) ? 0.f : ex2(m_o - m_n);
-      l_run[g] = a * l_run[g] + c * l_o;
-#pragma unroll
-      for (int e = 0; e < C::kEPL; ++e) {
-        const float o_o = __shfl_xor_sync(0xffffffffu, o_reg[g][e], off);
-        o_reg[g][e] = a * o_reg[g][e] + c * o_o;
+    const int row_begin = share.beg * C::kRowsPerStage;
+    const int row_end = min(static_cast<long long>(sk_eff), static_cast<long long>(share.end) * C::kRowsPerStage);
+    const int n_rows = row_end - row_begin;
+    const int n_stages = share.end - share.beg;
+    const unsigned char* k_base = reinterpret_cast<const unsigned char*>(
+        K + (static_cast<size_t>(b) * kvH + kvh) * kv_head_stride);
+    const unsigned char* v_base = reinterpret_cast<const unsigned char*>(
+        V + (static_cast<size_t>(b) * kvH + kvh) * kv_head_stride);
+
+    auto issue = [&](int st) {
+      if (st < n_stages) {
+        const int slot = st % kStages;
+        const long long first = static_cast<long long>(row_begin) + st * C::kRowsPerStage;
+        const long long valid_bytes =
+            (static_cast<long long>(row_end) - first) * C::kRowBytes;  // > 0
+        const size_t goff = static_cast<size_t>(first) * C::kRowBytes;
+        for (int p = tid; p < C::kStageBytes / 16; p += kThreads) {
+          const long long off = static_cast<long long>(p) * 16;
+          const bool ok = off < valid_bytes;
+          // past the split: src-size 0 zero-fills the destination, the source is not read
+          cp_async16(k_ring + slot * C::kStageBytes + off, ok ? k_base + goff + off : k_base,
+                     ok ? 16 : 0);
+          cp_async16(v_ring + slot * C::kStageBytes + off, ok ? v_base + goff + off : v_base,
+                     ok ? 16 : 0);
+        }
       }
-      m_run[g] = m_n;
-    }
-  }
-  // ... then the warps of the block through shared memory (the ring is idle now).
-  __syncthreads();
-  float* red_m = reinterpret_cast<float*>(smem);            // [kWarps][GB]
-  float* red_l = red_m + kWarps * GB;                        // [kWarps][GB]
-  float* red_o = red_l + kWarps * GB;                        // [kWarps][GB][D]
-  if (grp == 0) {
+      cp_async_commit();
+    };
+
 #pragma unroll
-    for (int g = 0; g < GB; ++g) {
-      if (lr == 0) {
-        red_m[warp * GB + g] = m_run[g];
-        red_l[warp * GB + g] = l_run[g];
+    for (int s = 0; s < kStages - 1; ++s) issue(s);
+
+    for (int st = 0; st < n_stages; ++st) {
+      cp_async_wait<kStages - 2>();
+      __syncthreads();
+      issue(st + kStages - 1);
+      const int slot = st % kStages;
+      const int stage_row0 = st * C::kRowsPerStage;
+#pragma unroll 1
+      for (int step = 0; step < C::kSteps; ++step) {
+        const int rl = step * C::kRowsPerStep + warp * C::kRowsPerWarpStep + grp;
+        const bool valid = stage_row0 + rl < n_rows;
+        const unsigned char* krow = k_ring + slot * C::kStageBytes + rl * C::kRowBytes;
+        const unsigned char* vrow = v_ring + slot * C::kStageBytes + rl * C::kRowBytes;
+        float kf[C::kEPL];
+#pragma unroll
+        for (int v = 0; v < C::kVPT; ++v) {
+          const uint4 u = *reinterpret_cast<const uint4*>(krow + (v * C::kLPR + lr) * 16);
+          Piece<T>::unpack(u, &kf[v * Piece<T>::kElems]);
+        }
+        float s[GB];
+#pragma unroll
+        for (int g = 0; g < GB; ++g) {
+          float acc = 0.f;
+#pragma unroll
+          for (int e = 0; e < C::kEPL; ++e) acc = fmaf(q_reg[g][e], kf[e], acc);
+          s[g] = acc;
+        }
+#pragma unroll
+        for (int off = 1; off < C::kLPR; off <<= 1) {
+#pragma unroll
+          for (int g = 0; g < GB; ++g) s[g] += __shfl_xor_sync(0xffffffffu, s[g], off);
+        }
+        float vf[C::kEPL];
+#pragma unroll
+        for (int v = 0; v < C::kVPT; ++v) {
+          const uint4 u = *reinterpret_cast<const uint4*>(vrow + (v * C::kLPR + lr) * 16);
+          Piece<T>::unpack(u, &vf[v * Piece<T>::kElems]);
+        }
+        if (valid) {
+#pragma unroll
+          for (int g = 0; g < GB; ++g) {
+            if (s[g] > m_run[g]) {  // rare after the first rows: rescale only when the max moves
+              const float alpha = ex2(m_run[g] - s[g]);  // ex2(-inf) = 0 on the first row
+              l_run[g] *= alpha;
+#pragma unroll
+              for (int e = 0; e < C::kEPL; ++e) o_reg[g][e] *= alpha;
+              m_run[g] = s[g];
+            }
+            const float p = ex2(s[g] - m_run[g]);
+            l_run[g] += p;
+#pragma unroll
+            for (int e = 0; e < C::kEPL; ++e) o_reg[g][e] = fmaf(p, vf[e], o_reg[g][e]);
+          }
+        }
       }
-#pragma unroll
-      for (int v = 0; v < C::kVPT; ++v)
-#pragma unroll
-        for (int e = 0; e < Piece<T>::kElems; ++e)
-          red_o[(warp * GB + g) * D + (v * C::kLPR + lr) * Piece<T>::kElems + e] =
-              o_reg[g][v * Piece<T>::kElems + e];
     }
+    cp_async_wait<0>();
+
+    // Merge the row groups of the warp (log-sum-exp merge through shuffles) ...
+#pragma unroll
+    for (int off = C::kLPR; off < 32; off <<= 1) {
+#pragma unroll
+      for (int g = 0; g < GB; ++g) {
+        const float m_o = __shfl_xor_sync(0xffffffffu, m_run[g], off);
+        const float l_o = __shfl_xor_sync(0xffffffffu, l_run[g], off);
+        const float m_n = fmaxf(m_run[g], m_o);
+        const float a = (m_run[g] == -INFINITY) ? 0.f : ex2(m_run[g] - m_n);
+        const float c = (m_o == -INFINITY) ? 0.f : ex2(m_o - m_n);
+        l_run[g] = a * l_run[g] + c * l_o;
+#pragma unroll
+        for (int e = 0; e < C::kEPL; ++e) {
+          const float o_o = __shfl_xor_sync(0xffffffffu, o_reg[g][e], off);
+          o_reg[g][e] = a * o_reg[g][e] + c * o_o;
+        }
+        m_run[g] = m_n;
+      }
+    }
+    // ... then the warps of the block through shared memory (the ring is idle now).
+    __syncthreads();
+    float* red_m = reinterpret_cast<float*>(smem);            // [kWarps][GB]
+    float* red_l = red_m + kWarps * GB;                        // [kWarps][GB]
+    float* red_o = red_l + kWarps * GB;                        // [kWarps][GB][D]
+    if (grp == 0) {
+#pragma unroll
+      for (int g = 0; g < GB; ++g) {
+        if (lr == 0) {
+          red_m[warp * GB + g] = m_run[g];
+          red_l[warp * GB + g] = l_run[g];
+        }
+#pragma unroll
+        for (int v = 0; v < C::kVPT; ++v)
+#pragma unroll
+          for (int e = 0; e < Piece<T>::kElems; ++e)
+            red_o[(warp * GB + g) * D + (v * C::kLPR + lr) * Piece<T>::kElems + e] =
+                o_reg[g][v * Piece<T>::kElems + e];
+      }
+    }
+    __syncthreads();
+    finish_group<GB, D, kWarps, kForm>(red_m, red_l, red_o, b, kvh, hb, H, kvH, share.part, deal, Mp, Lp, Op);
+    if (kForm == kBalanced) __syncthreads();  // the ring is free again
   }
-  __syncthreads();
-  finish_group<GB, D, kWarps, kForm>(red_m, red_l, red_o, b, kvh, hb, H, kvH, part, deal, Mp, Lp, Op);
-  RAB_DECODE_LOOP_END
 }
 
 // ---- tensor-core variant for 16-bit caches ---------------------------------------------
@@ -634,173 +625,174 @@ __global__ void __launch_bounds__(MmaCfg<D>::kThreads)
   const int warp = tid >> 5;
   const int g = lane >> 2;   // fragment row (and row + 8)
   const int tq = lane & 3;   // fragment column pair
-  RAB_DECODE_LOOP_BEGIN
+  Shares<kForm> shares(deal);
+  Share share;
+  while (shares.next(deal, kvH, share)) {
+    const int b = share.b, kvh = share.kvh, hb = share.hb;
 
-  // Q as A fragments: reg0 (row g, k 2tq..), reg1 (row g+8, same k), reg2 / reg3 the same at k+8.
-  const int h0 = kvh + kvH * (hb * 16 + g);
-  const int h1 = kvh + kvH * (hb * 16 + g + 8);
-  unsigned qa[D / 16][4];
-#pragma unroll
-  for (int ks = 0; ks < D / 16; ++ks) {
-    const int d0 = ks * 16 + 2 * tq;
-    const T* q0 = Q + (static_cast<size_t>(b) * H + (h0 < H ? h0 : 0)) * D + d0;
-    const T* q1 = Q + (static_cast<size_t>(b) * H + (h1 < H ? h1 : 0)) * D + d0;
-    qa[ks][0] = h0 < H ? *reinterpret_cast<const unsigned*>(q0) : 0u;
-    qa[ks][1] = h1 < H ? *reinterpret_cast<const unsigned*>(q1) : 0u;
-    qa[ks][2] = h0 < H ? *reinterpret_cast<const unsigned*>(q0 + 8) : 0u;
-    qa[ks][3] = h1 < H ? *reinterpret_cast<const unsigned*>(q1 + 8) : 0u;
-  }
-
-  float o[D / 8][4];
-#pragma unroll
-  for (int n = 0; n < D / 8; ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f;
-  float m_run[2] = {-INFINITY, -INFINITY};
-  float l_run[2] = {0.f, 0.f};  // this lane's share of the row sums (its four columns per block)
-
-  const int row_begin = stage_beg * C::kStageRows;
-  const int row_end = min(static_cast<long long>(sk_eff), static_cast<long long>(stage_end) * C::kStageRows);
-  const int n_rows = row_end - row_begin;
-  const int n_stages = stage_end - stage_beg;
-  const unsigned char* k_base = reinterpret_cast<const unsigned char*>(
-      K + (static_cast<size_t>(b) * kvH + kvh) * kv_head_stride);
-  const unsigned char* v_base = reinterpret_cast<const unsigned char*>(
-      V + (static_cast<size_t>(b) * kvH + kvh) * kv_head_stride);
-
-  auto issue = [&](int st) {
-    if (st < n_stages) {
-      const int slot = st % C::kStages;
-      const long long first = static_cast<long long>(row_begin) + st * C::kStageRows;
-      const long long valid_bytes = (static_cast<long long>(row_end) - first) * C::kRowBytes;
-      const size_t goff = static_cast<size_t>(first) * C::kRowBytes;
-      for (int p = tid; p < C::kStageBytes / 16; p += C::kThreads) {
-        const int r = p / C::kPieces;
-        const int c = p - r * C::kPieces;
-        const long long off = static_cast<long long>(p) * 16;
-        const int dst = slot * C::kStageBytes + r * C::kRowBytes + ((c ^ (r & 7)) << 4);
-        const bool ok = off < valid_bytes;
-        cp_async16(k_ring + dst, ok ? k_base + goff + off : k_base, ok ? 16 : 0);
-        cp_async16(v_ring + dst, ok ? v_base + goff + off : v_base, ok ? 16 : 0);
-      }
-    }
-    cp_async_commit();
-  };
-
-#pragma unroll
-  for (int s = 0; s < C::kStages - 1; ++s) issue(s);
-
-  const int mi = lane >> 3, r8 = lane & 7;
-  const int key0 = warp * kMmaKeysPerWarp;
-  // per-lane row offsets of the ldmatrix addresses (piece index is XORed with r8 = key & 7)
-  const unsigned k_row_off = static_cast<unsigned>((key0 + (mi >> 1) * 8 + r8) * C::kRowBytes);
-  const unsigned v_row_off = static_cast<unsigned>((key0 + (mi & 1) * 8 + r8) * C::kRowBytes);
-
-  for (int st = 0; st < n_stages; ++st) {
-    cp_async_wait<C::kStages - 2>();
-    __syncthreads();
-    issue(st + C::kStages - 1);
-    const int slot = st % C::kStages;
-    const int n_valid = n_rows - (st * C::kStageRows + key0);  // valid keys of this warp's block
-    if (n_valid <= 0) continue;
-    const unsigned kt = static_cast<unsigned>(__cvta_generic_to_shared(k_ring + slot * C::kStageBytes));
-    const unsigned vt = static_cast<unsigned>(__cvta_generic_to_shared(v_ring + slot * C::kStageBytes));
-
-    // S = Q K^T for 16 keys: s0 = keys 0..7, s1 = keys 8..15
-    float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
+    // Q as A fragments: reg0 (row g, k 2tq..), reg1 (row g+8, same k), reg2 / reg3 the same at k+8.
+    const int h0 = kvh + kvH * (hb * 16 + g);
+    const int h1 = kvh + kvH * (hb * 16 + g + 8);
+    unsigned qa[D / 16][4];
 #pragma unroll
     for (int ks = 0; ks < D / 16; ++ks) {
-      unsigned kb[4];
-      ldmatrix_x4(kb, kt + k_row_off + (((2 * ks + (mi & 1)) ^ r8) << 4));
-      mma16816<T>(s0, qa[ks], kb[0], kb[1]);
-      mma16816<T>(s1, qa[ks], kb[2], kb[3]);
+      const int d0 = ks * 16 + 2 * tq;
+      const T* q0 = Q + (static_cast<size_t>(b) * H + (h0 < H ? h0 : 0)) * D + d0;
+      const T* q1 = Q + (static_cast<size_t>(b) * H + (h1 < H ? h1 : 0)) * D + d0;
+      qa[ks][0] = h0 < H ? *reinterpret_cast<const unsigned*>(q0) : 0u;
+      qa[ks][1] = h1 < H ? *reinterpret_cast<const unsigned*>(q1) : 0u;
+      qa[ks][2] = h0 < H ? *reinterpret_cast<const unsigned*>(q0 + 8) : 0u;
+      qa[ks][3] = h1 < H ? *reinterpret_cast<const unsigned*>(q1 + 8) : 0u;
     }
-    // scale, hide the keys past the end, row maxima (rows g and g + 8)
-    float v[8] = {s0[0], s0[1], s1[0], s1[1], s0[2], s0[3], s1[2], s1[3]};
+
+    float o[D / 8][4];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int col = ((i >> 1) & 1) * 8 + 2 * tq + (i & 1);
-      v[i] = (col < n_valid) ? v[i] * scale_log2 : -INFINITY;
-    }
-    float mx0 = fmaxf(fmaxf(v[0], v[1]), fmaxf(v[2], v[3]));
-    float mx1 = fmaxf(fmaxf(v[4], v[5]), fmaxf(v[6], v[7]));
-    mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1));
-    mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1));
-    mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
-    mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
-    const bool moved = mx0 > m_run[0] || mx1 > m_run[1];
-    if (__any_sync(0xffffffffu, moved)) {  // rare after the first blocks
-      const float mn0 = fmaxf(m_run[0], mx0), mn1 = fmaxf(m_run[1], mx1);
-      const float a0 = (m_run[0] == -INFINITY) ? 0.f : ex2(m_run[0] - mn0);
-      const float a1 = (m_run[1] == -INFINITY) ? 0.f : ex2(m_run[1] - mn1);
-      l_run[0] *= a0;
-      l_run[1] *= a1;
-#pragma unroll
-      for (int n = 0; n < D / 8; ++n) {
-        o[n][0] *= a0;
-        o[n][1] *= a0;
-        o[n][2] *= a1;
-        o[n][3] *= a1;
+    for (int n = 0; n < D / 8; ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f;
+    float m_run[2] = {-INFINITY, -INFINITY};
+    float l_run[2] = {0.f, 0.f};  // this lane's share of the row sums (its four columns per block)
+
+    const int row_begin = share.beg * C::kStageRows;
+    const int row_end = min(static_cast<long long>(sk_eff), static_cast<long long>(share.end) * C::kStageRows);
+    const int n_rows = row_end - row_begin;
+    const int n_stages = share.end - share.beg;
+    const unsigned char* k_base = reinterpret_cast<const unsigned char*>(
+        K + (static_cast<size_t>(b) * kvH + kvh) * kv_head_stride);
+    const unsigned char* v_base = reinterpret_cast<const unsigned char*>(
+        V + (static_cast<size_t>(b) * kvH + kvh) * kv_head_stride);
+
+    auto issue = [&](int st) {
+      if (st < n_stages) {
+        const int slot = st % C::kStages;
+        const long long first = static_cast<long long>(row_begin) + st * C::kStageRows;
+        const long long valid_bytes = (static_cast<long long>(row_end) - first) * C::kRowBytes;
+        const size_t goff = static_cast<size_t>(first) * C::kRowBytes;
+        for (int p = tid; p < C::kStageBytes / 16; p += C::kThreads) {
+          const int r = p / C::kPieces;
+          const int c = p - r * C::kPieces;
+          const long long off = static_cast<long long>(p) * 16;
+          const int dst = slot * C::kStageBytes + r * C::kRowBytes + ((c ^ (r & 7)) << 4);
+          const bool ok = off < valid_bytes;
+          cp_async16(k_ring + dst, ok ? k_base + goff + off : k_base, ok ? 16 : 0);
+          cp_async16(v_ring + dst, ok ? v_base + goff + off : v_base, ok ? 16 : 0);
+        }
       }
-      m_run[0] = mn0;
-      m_run[1] = mn1;
-    }
-    const float ms0 = (m_run[0] == -INFINITY) ? 0.f : m_run[0];
-    const float ms1 = (m_run[1] == -INFINITY) ? 0.f : m_run[1];
-    float p[8];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      p[i] = ex2(v[i] - ms0);
-      p[4 + i] = ex2(v[4 + i] - ms1);
-    }
-    l_run[0] += (p[0] + p[1]) + (p[2] + p[3]);
-    l_run[1] += (p[4] + p[5]) + (p[6] + p[7]);
-    // P as the A fragment of the second product
-    unsigned pa[4];
-    pa[0] = pack_pair<T>(p[0], p[1]);  // row g,     keys 2tq, 2tq+1
-    pa[1] = pack_pair<T>(p[4], p[5]);  // row g + 8, same keys
-    pa[2] = pack_pair<T>(p[2], p[3]);  // row g,     keys 8 + 2tq, ...
-    pa[3] = pack_pair<T>(p[6], p[7]);  // row g + 8
-#pragma unroll
-    for (int c2 = 0; c2 < D / 16; ++c2) {
-      unsigned vb[4];
-      ldmatrix_x4_trans(vb, vt + v_row_off + (((2 * c2 + (mi >> 1)) ^ r8) << 4));
-      mma16816<T>(o[2 * c2], pa, vb[0], vb[1]);
-      mma16816<T>(o[2 * c2 + 1], pa, vb[2], vb[3]);
-    }
-  }
-  cp_async_wait<0>();
+      cp_async_commit();
+    };
 
-  // row sums over the four lanes of a row, then the warps of the block through shared memory
 #pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    l_run[i] += __shfl_xor_sync(0xffffffffu, l_run[i], 1);
-    l_run[i] += __shfl_xor_sync(0xffffffffu, l_run[i], 2);
-  }
-  __syncthreads();
-  float* red_m = reinterpret_cast<float*>(smem);  // [warps][16]
-  float* red_l = red_m + C::kWarps * 16;          // [warps][16]
-  float* red_o = red_l + C::kWarps * 16;          // [warps][16][D]
-  if (tq == 0) {
-    red_m[warp * 16 + g] = m_run[0];
-    red_m[warp * 16 + g + 8] = m_run[1];
-    red_l[warp * 16 + g] = l_run[0];
-    red_l[warp * 16 + g + 8] = l_run[1];
-  }
+    for (int s = 0; s < C::kStages - 1; ++s) issue(s);
+
+    const int mi = lane >> 3, r8 = lane & 7;
+    const int key0 = warp * kMmaKeysPerWarp;
+    // per-lane row offsets of the ldmatrix addresses (piece index is XORed with r8 = key & 7)
+    const unsigned k_row_off = static_cast<unsigned>((key0 + (mi >> 1) * 8 + r8) * C::kRowBytes);
+    const unsigned v_row_off = static_cast<unsigned>((key0 + (mi & 1) * 8 + r8) * C::kRowBytes);
+
+    for (int st = 0; st < n_stages; ++st) {
+      cp_async_wait<C::kStages - 2>();
+      __syncthreads();
+      issue(st + C::kStages - 1);
+      const int slot = st % C::kStages;
+      const int n_valid = n_rows - (st * C::kStageRows + key0);  // valid keys of this warp's block
+      if (n_valid <= 0) continue;
+      const unsigned kt = static_cast<unsigned>(__cvta_generic_to_shared(k_ring + slot * C::kStageBytes));
+      const unsigned vt = static_cast<unsigned>(__cvta_generic_to_shared(v_ring + slot * C::kStageBytes));
+
+      // S = Q K^T for 16 keys: s0 = keys 0..7, s1 = keys 8..15
+      float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-  for (int n = 0; n < D / 8; ++n) {
-    float* r0 = red_o + (warp * 16 + g) * D + n * 8 + 2 * tq;
-    float* r1 = red_o + (warp * 16 + g + 8) * D + n * 8 + 2 * tq;
-    r0[0] = o[n][0];
-    r0[1] = o[n][1];
-    r1[0] = o[n][2];
-    r1[1] = o[n][3];
+      for (int ks = 0; ks < D / 16; ++ks) {
+        unsigned kb[4];
+        ldmatrix_x4(kb, kt + k_row_off + (((2 * ks + (mi & 1)) ^ r8) << 4));
+        mma16816<T>(s0, qa[ks], kb[0], kb[1]);
+        mma16816<T>(s1, qa[ks], kb[2], kb[3]);
+      }
+      // scale, hide the keys past the end, row maxima (rows g and g + 8)
+      float v[8] = {s0[0], s0[1], s1[0], s1[1], s0[2], s0[3], s1[2], s1[3]};
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int col = ((i >> 1) & 1) * 8 + 2 * tq + (i & 1);
+        v[i] = (col < n_valid) ? v[i] * scale_log2 : -INFINITY;
+      }
+      float mx0 = fmaxf(fmaxf(v[0], v[1]), fmaxf(v[2], v[3]));
+      float mx1 = fmaxf(fmaxf(v[4], v[5]), fmaxf(v[6], v[7]));
+      mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1));
+      mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1));
+      mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
+      mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
+      const bool moved = mx0 > m_run[0] || mx1 > m_run[1];
+      if (__any_sync(0xffffffffu, moved)) {  // rare after the first blocks
+        const float mn0 = fmaxf(m_run[0], mx0), mn1 = fmaxf(m_run[1], mx1);
+        const float a0 = (m_run[0] == -INFINITY) ? 0.f : ex2(m_run[0] - mn0);
+        const float a1 = (m_run[1] == -INFINITY) ? 0.f : ex2(m_run[1] - mn1);
+        l_run[0] *= a0;
+        l_run[1] *= a1;
+#pragma unroll
+        for (int n = 0; n < D / 8; ++n) {
+          o[n][0] *= a0;
+          o[n][1] *= a0;
+          o[n][2] *= a1;
+          o[n][3] *= a1;
+        }
+        m_run[0] = mn0;
+        m_run[1] = mn1;
+      }
+      const float ms0 = (m_run[0] == -INFINITY) ? 0.f : m_run[0];
+      const float ms1 = (m_run[1] == -INFINITY) ? 0.f : m_run[1];
+      float p[8];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        p[i] = ex2(v[i] - ms0);
+        p[4 + i] = ex2(v[4 + i] - ms1);
+      }
+      l_run[0] += (p[0] + p[1]) + (p[2] + p[3]);
+      l_run[1] += (p[4] + p[5]) + (p[6] + p[7]);
+      // P as the A fragment of the second product
+      unsigned pa[4];
+      pa[0] = pack_pair<T>(p[0], p[1]);  // row g,     keys 2tq, 2tq+1
+      pa[1] = pack_pair<T>(p[4], p[5]);  // row g + 8, same keys
+      pa[2] = pack_pair<T>(p[2], p[3]);  // row g,     keys 8 + 2tq, ...
+      pa[3] = pack_pair<T>(p[6], p[7]);  // row g + 8
+#pragma unroll
+      for (int c2 = 0; c2 < D / 16; ++c2) {
+        unsigned vb[4];
+        ldmatrix_x4_trans(vb, vt + v_row_off + (((2 * c2 + (mi >> 1)) ^ r8) << 4));
+        mma16816<T>(o[2 * c2], pa, vb[0], vb[1]);
+        mma16816<T>(o[2 * c2 + 1], pa, vb[2], vb[3]);
+      }
+    }
+    cp_async_wait<0>();
+
+    // row sums over the four lanes of a row, then the warps of the block through shared memory
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      l_run[i] += __shfl_xor_sync(0xffffffffu, l_run[i], 1);
+      l_run[i] += __shfl_xor_sync(0xffffffffu, l_run[i], 2);
+    }
+    __syncthreads();
+    float* red_m = reinterpret_cast<float*>(smem);  // [warps][16]
+    float* red_l = red_m + C::kWarps * 16;          // [warps][16]
+    float* red_o = red_l + C::kWarps * 16;          // [warps][16][D]
+    if (tq == 0) {
+      red_m[warp * 16 + g] = m_run[0];
+      red_m[warp * 16 + g + 8] = m_run[1];
+      red_l[warp * 16 + g] = l_run[0];
+      red_l[warp * 16 + g + 8] = l_run[1];
+    }
+#pragma unroll
+    for (int n = 0; n < D / 8; ++n) {
+      float* r0 = red_o + (warp * 16 + g) * D + n * 8 + 2 * tq;
+      float* r1 = red_o + (warp * 16 + g + 8) * D + n * 8 + 2 * tq;
+      r0[0] = o[n][0];
+      r0[1] = o[n][1];
+      r1[0] = o[n][2];
+      r1[1] = o[n][3];
+    }
+    __syncthreads();
+    finish_group<16, D, C::kWarps, kForm>(red_m, red_l, red_o, b, kvh, hb, H, kvH, share.part, deal, Mp, Lp, Op);
+    if (kForm == kBalanced) __syncthreads();  // the ring is free again
   }
-  __syncthreads();
-  finish_group<16, D, C::kWarps, kForm>(red_m, red_l, red_o, b, kvh, hb, H, kvH, part, deal, Mp, Lp, Op);
-  RAB_DECODE_LOOP_END
 }
-
-#undef RAB_DECODE_LOOP_BEGIN
-#undef RAB_DECODE_LOOP_END
 
 // Fold the partials of the balanced and fixed forms into the persistent (out, m, l). grid = (H, B); a thread
 // takes four columns of every n_grp-th partial (with one column and two groups at head_dim 256 the B1 H64/kvH1
@@ -1009,7 +1001,7 @@ int decode_ml_scratch(size_t floats, float** out) {
 
 namespace {
 
-// Workspace of the balanced form: [row][slot] of O, m and l.
+// Workspace of the balanced and the fixed form: [row][slot] of O, m and l.
 int partial_space(size_t rows, int D, int cap, void* workspace, float** Op, float** Mp, float** Lp) {
   const size_t need = rows * cap * (D + 2) * sizeof(float);
   if (workspace == nullptr) {
