@@ -574,7 +574,9 @@ def run_profile_case(args):
     quarter of the cached length (65536 tokens, 1 GB of K/V), 1 warm-up + 2 steps.
     prefill-d128 / prefill-d256 / prefill-d256-pair: the step kernel's other head_dims (and its
     cluster-pair form) on B1 H8 S16384 causal (0.4 GB on the device). prefill-gqa /
-    prefill-gqa-heads-fastest: B2 H32/kvH8 S32768 D128 causal in either block order."""
+    prefill-gqa-heads-fastest: B2 H32/kvH8 S32768 D128 causal in either block order. flash-fp32-d64 /
+    flash-fp32-d128: the fp32 step on B1 H8 S8192 causal. chunk: 384 rows on 40384 keys, H32/kvH8 D128
+    fp16, whose query blocks share their keys over clusters (0.2 GB)."""
     import torch
 
     from ring_attention_b200 import api
@@ -610,6 +612,22 @@ def run_profile_case(args):
             api.attention_step_ex(q, k, v, out, m, l, api.AttentionShape(B, H, S, S, D, kvH), one, one, 1,
                                   causal=True, fresh=True, finalize=True)
         api.lib().ra_debug_set_block_order(-1)
+    elif args.profile.startswith("flash-fp32"):
+        B, H, S, D = 1, 8, 8192, 128 if args.profile.endswith("128") else 64
+        q, k, v = (torch.randn((B, H, S, D), generator=g, device=dev) for _ in range(3))
+        out = torch.empty_like(q)
+        for _ in range(3):
+            api.launch_flash_attention(q, k, v, out, api.AttentionShape(B, H, S, S, D), True)
+    elif args.profile == "chunk":
+        H, kvH, Sq, Sk, D = 32, 8, 384, 40384, 128
+        q = torch.randn((1, H, Sq, D), generator=g, device=dev, dtype=torch.float16)
+        k, v = (torch.randn((1, kvH, Sk, D), generator=g, device=dev, dtype=torch.float16) for _ in range(2))
+        out = torch.empty((1, H, Sq, D), device=dev)
+        m = torch.empty((1, H, Sq), device=dev)
+        l = torch.empty_like(m)
+        for _ in range(3):
+            api.attention_step_ex(q, k, v, out, m, l, api.AttentionShape(1, H, Sq, Sk, D, kvH), SegMap.make([Sk - Sq], Sq),
+                                  SegMap.make([0], Sk), 1, causal=True, fresh=True, finalize=True)
     elif args.profile.startswith("prefill-d"):
         D = 128 if "128" in args.profile else 256
         B, H, S = 1, 8, 16384
@@ -749,7 +767,7 @@ def check_decode_rows(torch, dist, dev, cache, lens, q, out, rank, P):
 def main():
     ap = argparse.ArgumentParser()
     ap.add_argument("--profile", default=None, choices=["prefill", "decode", "prefill-d128", "prefill-d256", "prefill-d256-pair", "prefill-gqa",
-                             "prefill-gqa-heads-fastest", "prefill-docs"],
+                             "prefill-gqa-heads-fastest", "prefill-docs", "flash-fp32-d64", "flash-fp32-d128", "chunk"],
                     help="run a small self-ending case for ncu instead of the benchmark")
     ap.add_argument("--gpus", type=int, default=1)
     ap.add_argument("--steps", type=int, default=20)

@@ -48,28 +48,6 @@ def _compile(src, verbose):
     return obj, r.stderr
 
 
-PROBE_SRC = os.path.join(CSRC, "probe")
-PROBE_BIN = os.path.join(PROBE_SRC, "_bin")
-
-
-def build_probes() -> list:
-    """The stand-alone timing probes under csrc/probe (measurement tools behind the design notes;
-    nothing in the library links them) into csrc/probe/_bin/<name>."""
-    os.makedirs(PROBE_BIN, exist_ok=True)
-    outs = []
-    for f in sorted(os.listdir(PROBE_SRC)):
-        if not f.endswith(".cu"):
-            continue
-        src, exe = os.path.join(PROBE_SRC, f), os.path.join(PROBE_BIN, f[:-3])
-        if _stale(exe, [src]):
-            r = subprocess.run([NVCC, "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3",
-                                "-std=c++17", "-o", exe, src], capture_output=True, text=True)
-            if r.returncode != 0:
-                raise RuntimeError(f"nvcc failed on {f}:\n{r.stdout}\n{r.stderr}")
-        outs.append(exe)
-    return outs
-
-
 def build(verbose: bool = False, force: bool = False) -> str:
     os.makedirs(OBJ, exist_ok=True)
     if force:
@@ -94,5 +72,3 @@ def build(verbose: bool = False, force: bool = False) -> str:
 
 if __name__ == "__main__":
     print(build(verbose="-v" in sys.argv, force="-f" in sys.argv))
-    if "--probes" in sys.argv:
-        print("\n".join(build_probes()))
