@@ -460,3 +460,34 @@ def test_decode_into_a_state_and_a_workspace_aligned_to_four_bytes(dtype, H, kvH
     api.launch_attention_finalize(out, l, s)
     assert_close(out.cpu().numpy(), want, TOL[dtype], TOL[dtype], "out")
     assert_close(lse, want_lse, TOL[dtype], TOL[dtype], "lse")
+
+
+@pytest.mark.parametrize("D", [32, 64, 128])
+@pytest.mark.parametrize("split", [1, 2])
+def test_marked_tiles_in_a_cache_with_segments_strides_and_grouped_heads(D, split):
+    # plain scores read K from memory by segment, batch row, KV head and row stride
+    B, H, kvH, Lq, Lk, stride, room = 2, 4, 2, 70, 150, 3, 400
+    rng = np.random.default_rng(23)
+    q = rng.standard_normal((B, H, 2 * Lq, D))
+    k, v = (rng.standard_normal((B, kvH, room, D)) for _ in range(2))
+    q[..., 0] *= 2.0 ** 20
+    k[..., 0] *= 2.0 ** -20
+    k[:, 1, 20:140, 3] = 0.0
+    k[:, 1, 30, 3] = -(2.0 ** 12)  # one KV head has larger keys too
+    q[..., 3] = np.abs(q[..., 3])
+    v[:, :, 40] *= 2.0 ** 15
+    q, k, v = (x.astype(np.float32) for x in (q, k, v))
+    qmap, kmap = SegMap.make([300, 2000], Lq), SegMap.make([0, 1500], Lk)
+    qpos = np.concatenate([b + np.arange(Lq) * stride for b in (300, 2000)])
+    kpos = np.concatenate([b + np.arange(Lk) * stride for b in (0, 1500)])
+    heads = [h % kvH for h in range(H)]
+    want, want_lse = _in_64_bits(q, k[:, heads, :2 * Lk], v[:, heads, :2 * Lk], qpos, kpos, True, 0)
+    out, m, l = poisoned(B, H, 2 * Lq, D)
+    shape = api.AttentionShape(B, H, 2 * Lq, 2 * Lk, D, kvH)
+    api.attention_step_ex(dev(q), dev(k), dev(v), out, m, l, shape, qmap, kmap, pos_stride=stride, causal=True, fresh=True,
+                          finalize=True, kv_row_stride=room, key_split=split)
+    lse = api.attention_lse(m, l).cpu().numpy()
+    assert api.device_status()[0] == 0
+    assert_close(lse, want_lse, 1e-5, 1e-5, "lse")
+    unit = np.abs(want).max()
+    assert_close(out.cpu().numpy() / unit, want / unit, 1e-5, 0.0, "out")
