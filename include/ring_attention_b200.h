@@ -103,9 +103,10 @@ RA_API int ra_attention_init(float* out, float* m, float* l, const ra_shape* sha
 
 /* One ring step, fp32 Q/K/V. Replaces launch_attention_step (src/attention.hpp:92-94,
  * src/attention_step.cu:488-525). Head_dim 32, 64 and 128 run on the tensor cores with every
- * operand scaled by a power of two and split into two fp16 terms (about 2^-22 per product, inside
- * the reference's fp32 tolerance of 1e-5 for its test and benchmark inputs; RA_STEP_FORCE_SIMT of
- * ra_attention_step_ex selects plain fp32), 256 on the SIMT kernel; seq_q == 1 dispatches to the decode kernel exactly as
+ * operand scaled by a power of two and split into two fp16 terms (about 2^-22 per product, and an
+ * absolute 2^-40 of the largest value of a Q row, a key or a 64-key V tile; tiles whose range that
+ * does not hold are taken in plain fp32; inside the reference's fp32 tolerance of 1e-5 for its test
+ * and benchmark inputs; RA_STEP_FORCE_SIMT of ra_attention_step_ex selects plain fp32), 256 on the SIMT kernel; seq_q == 1 dispatches to the decode kernel exactly as
  * the reference does (src/attention_step.cu:494-497). */
 RA_API int ra_attention_step(const float* q, const float* k, const float* v, float* out, float* m,
                              float* l, const ra_shape* shape, int q_offset, int k_offset,

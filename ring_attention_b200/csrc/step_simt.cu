@@ -1,7 +1,7 @@
 // SIMT online-softmax ring step: fp32 arithmetic end to end, for fp32 / fp16 / bf16 inputs
-// and every supported head_dim (32, 64, 128, 256). It is the fp32 path of the library
-// (1e-5 agreement with cpu_attention needs fp32 products, which tensor cores do not give)
-// and the path for the head sizes the tcgen05 kernel does not take.
+// and every supported head_dim (32, 64, 128, 256). It is the fp32 path at head_dim 256 and for
+// tensors that TMA does not take, the form a caller can ask for at every other shape, and what
+// the tensor-core kernels are checked against.
 //
 // Same recurrence and state semantics as the reference's attention_step_kernel
 // (src/attention_step.cu:114-282): per row, m/l/out are read, folded with one K/V chunk and

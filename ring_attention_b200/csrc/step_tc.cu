@@ -6,16 +6,18 @@
 // K tiles no row of the block can see.
 //
 // Work decomposition
-//   grid = (batch * heads, query blocks). A block owns 256 query rows of one segment as two
+//   grid = (batch * heads, query blocks); with a key split (batch * heads * blocks that share a
+//   query block's keys, query blocks). A block owns 256 query rows of one segment as two
 //   128-row tiles (head_dim 256: one tile) and walks the visible 128-key tiles of every key
 //   segment. Heaviest query blocks (largest positions) are launched first; with very many query
 //   blocks per KV head the grid is turned so that all query blocks of the heads sharing one KV
 //   head run before the next KV head (see launch_cfg).
 //
-// Three selectable forms of the same kernel, tested against each other: P in tensor memory
-// (default) or staged through shared memory (RA_STEP_P_IN_SMEM), and cluster pairs
-// (RA_STEP_CTA_PAIR, head_dim 128 / 256): tcgen05.mma.cta_group::2 with M = 256 over the two
-// blocks of a cluster, each block loading half of every K and V tile.
+// Four forms of the same kernel, tested against each other: P in tensor memory (default) or staged
+// through shared memory (RA_STEP_P_IN_SMEM); cluster pairs (RA_STEP_CTA_PAIR, head_dim 128 / 256):
+// tcgen05.mma.cta_group::2 with M = 256 over the two blocks of a cluster, each block loading half of
+// every K and V tile; and the key split (chosen by shape, pick_key_split): 2 to 8 blocks of a cluster
+// share the key tiles of one query block and merge their states (merge_key_split).
 //
 // Roles inside a block (384 threads)
 //   warp 0        TMA producer: Q tiles once, then K_j, V_j, K_j+1, ... into a shared-memory
@@ -42,8 +44,9 @@
 // per M128 N128 K16 instruction (shared-memory operands) and 33 clk at N = 64 with A in tensor
 // memory, i.e. the arithmetic rate; cta_group::2 pairs cost the same per SM. A pair of 128x128
 // tiles therefore needs ~1070 clk of tensor time at head_dim 64 (~2110 at 128) but 2048 clk of
-// the exp unit (16 ex2 per clock per SM) plus the rest of the softmax instructions: the
-// softmax warps, not the MMA issue, set the tile period at head_dim 64.
+// the exp unit (16 ex2 per clock per SM). Measured at head_dim 64: 2650-2700 clk, the exp unit busy 78 %
+// of them, issue slots 40 %, the tensor pipe 39 %, with 0.51 warps eligible per cycle and
+// scheduler: the busiest unit is the exp unit, and it idles while both softmax warps of a scheduler wait.
 //
 // Epilogue: the step's partial (O, m_ref, l) is merged with the persistent state in HBM using
 // the log-sum-exp merge, which is the same recurrence as folding the tiles one by one
