@@ -106,8 +106,9 @@ RA_API int ra_attention_init(float* out, float* m, float* l, const ra_shape* sha
  * operand scaled by a power of two and split into two fp16 terms (about 2^-22 per product, and an
  * absolute 2^-40 of the largest value of a Q row, a key or a 64-key V tile; tiles whose range that
  * does not hold are taken in plain fp32; inside the reference's fp32 tolerance of 1e-5 for its test
- * and benchmark inputs; RA_STEP_FORCE_SIMT of ra_attention_step_ex selects plain fp32), 256 on the SIMT kernel; seq_q == 1 dispatches to the decode kernel exactly as
- * the reference does (src/attention_step.cu:494-497). */
+ * and benchmark inputs; RA_STEP_FORCE_SIMT of ra_attention_step_ex selects plain fp32), 256 on
+ * the SIMT kernel; seq_q == 1 dispatches to the decode kernel exactly as the reference does
+ * (src/attention_step.cu:494-497). */
 RA_API int ra_attention_step(const float* q, const float* k, const float* v, float* out, float* m,
                              float* l, const ra_shape* shape, int q_offset, int k_offset,
                              int causal, ra_stream stream, int pos_stride);
