@@ -44,6 +44,39 @@ const char* last_error();
     }                                 \
   } while (0)
 
+// ---- launches that overlap the kernel before them ---------------------------------------
+// A kernel launched with launch_overlapped may start while the one before it in the stream still
+// runs: its blocks fill the SMs that are free already and do what touches no memory (barriers, tensor
+// memory, index arithmetic). It calls wait_for_previous, in every block, before its first access to
+// memory that an earlier launch may write or read; that returns once everything before it in the stream has
+// completed and is visible. Loads that must stay behind the wait go through plain pointers: the
+// compiler may move those of a const __restrict__ one. let_next_start allows the next overlapped launch
+// to do the same, once every block of this kernel has called it or left: the next one's blocks never take
+// a place that a block of this one still needs. Measured, us a pass back to back, plain launches -> overlapped:
+// four dependent steps and a log-sum-exp (16 heads, shards of 2042 rows, D64) 146 -> 134; casts and a step (24
+// heads, 1531 rows) 43.0 -> 37.9; append + decode, 8 tokens of 5 x 24 heads on 1531 rows (with the prompt's copy)
+// 202 -> 190; passes of 100 us and more are as they were.
+#ifdef __CUDACC__
+__device__ inline void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ inline void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <typename... P, typename... A>
+inline cudaError_t launch_overlapped(void (*kern)(P...), dim3 grid, dim3 block, size_t smem,
+                                     cudaStream_t stream, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+#endif
+
 inline int kv_heads_of(const ra_shape& s) { return s.kv_heads > 0 ? s.kv_heads : s.heads; }
 
 // ---- device status word ----------------------------------------------------------

@@ -329,7 +329,8 @@ struct Shares {
     total = static_cast<long long>(deal.groups) * deal.stages;
     at = kForm == kBalanced ? total * i / n : 0;
     at_end = kForm == kBalanced ? total * (i + 1ll) / n : 1;
-    if (kForm != kCluster) asm volatile("griddepcontrol.launch_dependents;");
+    let_next_start();
+    wait_for_previous();
   }
   __device__ bool next(const Deal& deal, int kvH, Share& s) {
     if (at >= at_end) return false;
@@ -358,7 +359,7 @@ struct Shares {
 // GB = query heads handled per block. Grid: see Deal.
 template <typename T, int D, int GB, DealForm kForm>
 __global__ void __launch_bounds__(kThreads)
-    decode_split_kernel(const T* __restrict__ Q, const T* __restrict__ K, const T* __restrict__ V,
+    decode_split_kernel(const T* Q, const T* K, const T* V,
                         float* Mp, float* Lp, float* Op, int H,
                         int kvH, int sk_eff, long long kv_head_stride, const Deal deal, float scale_log2) {
   using C = DecodeCfg<T, D, GB>;
@@ -612,7 +613,7 @@ struct MmaCfg {
 // kvh + kv_heads * (16 * hb + r)). Grid: see Deal.
 template <typename T, int D, DealForm kForm>
 __global__ void __launch_bounds__(MmaCfg<D>::kThreads)
-    decode_mma_kernel(const T* __restrict__ Q, const T* __restrict__ K, const T* __restrict__ V,
+    decode_mma_kernel(const T* Q, const T* K, const T* V,
                       float* Mp, float* Lp, float* Op, int H,
                       int kvH, int sk_eff, long long kv_head_stride, const Deal deal, float scale_log2) {
   using C = MmaCfg<D>;
@@ -818,10 +819,11 @@ __global__ void __launch_bounds__(kFoldThreads)
   const long long total = static_cast<long long>(deal.groups) * deal.stages;
   const long long group =
       (static_cast<long long>(b) * kvH + h % kvH) * deal.head_batches + (h / kvH) / head_rows;
+  let_next_start();
   const int n = deal.splits > 0 ? deal.splits
                                 : deal_owner((group + 1) * deal.stages - 1, total, ctas) -
                                       deal_owner(group * deal.stages, total, ctas) + 1;
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  wait_for_previous();
   const float* mp = Mp + row * deal.cap;
   const float* lp = Lp + row * deal.cap;
   const float* op = Op + row * deal.cap * D + d;
@@ -1036,14 +1038,17 @@ int run_plan(const ra_shape& s, int head_batches, int stages, size_t stage_bytes
   cudaLaunchConfig_t cfg = {};
   cfg.stream = stream;
   cfg.dynamicSmemBytes = std::max(p.deal.ring * stage_bytes, red_bytes);
-  cudaLaunchAttribute attr;
-  cfg.attrs = &attr;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
   if (p.cluster) {
     cfg.gridDim = dim3(p.cluster, p.deal.groups);
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = p.cluster;
-    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-    cfg.numAttrs = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = p.cluster;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.numAttrs = 2;
     return launch(true, cfg, p.deal, m, l, out);
   }
   float *Op, *Mp, *Lp;
@@ -1052,20 +1057,12 @@ int run_plan(const ra_shape& s, int head_batches, int stages, size_t stage_bytes
   cfg.gridDim = fixed ? dim3(static_cast<unsigned>(p.deal.splits) * p.deal.groups) : dim3(p.ctas);
   rc = launch(false, cfg, p.deal, Mp, Lp, Op);
   if (rc != RA_OK) return rc;
-  cudaLaunchConfig_t fold = {};
-  fold.gridDim = dim3(s.heads, s.batch);
   // (no more thread groups than partials: with many rows and few partials each the idle ones cost, 2048
   // rows of D32 8 us)
-  fold.blockDim = dim3(std::max(32, std::min(kFoldGroups, p.deal.cap) * (D / 4)));
-  fold.stream = stream;
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  fold.attrs = &attr;
-  fold.numAttrs = 1;
-  RAB_CUDA(cudaLaunchKernelEx(&fold, decode_reduce_kernel, static_cast<const float*>(Mp),
-                              static_cast<const float*>(Lp), static_cast<const float*>(Op), m, l, out,
-                              s.heads, kvH, D, ROWS, p.ctas,
-                              ((reinterpret_cast<uintptr_t>(Op) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0, p.deal));
+  RAB_CUDA(launch_overlapped(decode_reduce_kernel, dim3(s.heads, s.batch),
+                             dim3(std::max(32, std::min(kFoldGroups, p.deal.cap) * (D / 4))), 0, stream, Mp, Lp, Op, m, l,
+                             out, s.heads, kvH, D, ROWS, p.ctas,
+                             ((reinterpret_cast<uintptr_t>(Op) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0, p.deal));
   RAB_CUDA(cudaGetLastError());
   return RA_OK;
 }

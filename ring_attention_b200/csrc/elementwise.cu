@@ -71,8 +71,9 @@ __global__ void finalize_scalar_kernel(float* __restrict__ out, const float* __r
   }
 }
 
-__global__ void lse_kernel(const float* __restrict__ m, const float* __restrict__ l,
-                           float* __restrict__ lse, size_t n) {
+__global__ void lse_kernel(const float* m, const float* l, float* lse, size_t n) {
+  let_next_start();
+  wait_for_previous();
   const size_t tid = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
   const size_t nth = static_cast<size_t>(gridDim.x) * blockDim.x;
   for (size_t i = tid; i < n; i += nth) lse[i] = l[i] > 0.f ? m[i] + logf(l[i]) : -INFINITY;
@@ -90,8 +91,7 @@ __device__ inline __nv_bfloat16 cvt_from_float<__nv_bfloat16>(float x) {
 // fp32 -> 16-bit, 8 elements (32 B in, 16 B out) per thread per trip when both pointers are
 // 16-byte aligned (reference: src/attention_step_fp16.cu:217-224).
 template <typename Dst>
-__device__ inline void narrow_range(const float* __restrict__ src, Dst* __restrict__ dst, size_t n,
-                                    int vec_ok) {
+__device__ inline void narrow_range(const float* src, Dst* dst, size_t n, int vec_ok) {
   const size_t tid = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
   const size_t nth = static_cast<size_t>(gridDim.x) * blockDim.x;
   size_t done = 0;
@@ -128,9 +128,10 @@ __global__ void narrow_kernel(const float* __restrict__ src, Dst* __restrict__ d
 
 // Q, K and V in one launch (blockIdx.y): three launches of a few microseconds of work each cost
 // the host more than the GPU. Bit i of `vec`: tensor i's source and destination are 16-byte aligned.
-__global__ void narrow_qkv_kernel(const float* __restrict__ q, __half* __restrict__ qh, size_t qn,
-                                  const float* __restrict__ k, const float* __restrict__ v,
-                                  __half* __restrict__ kh, __half* __restrict__ vh, size_t kn, int vec) {
+__global__ void narrow_qkv_kernel(const float* q, __half* qh, size_t qn, const float* k, const float* v,
+                                  __half* kh, __half* vh, size_t kn, int vec) {
+  let_next_start();
+  wait_for_previous();
   if (blockIdx.y == 0) narrow_range(q, qh, qn, vec & 1);
   else if (blockIdx.y == 1) narrow_range(k, kh, kn, vec & 2);
   else narrow_range(v, vh, kn, vec & 4);
@@ -262,9 +263,10 @@ __global__ void state_merge_kernel(const float* __restrict__ parts, size_t part_
 // blockIdx.y of tensor blockIdx.z. One launch where two strided device copies were two driver calls
 // of several microseconds each on the host.
 template <typename V>
-__global__ void cache_row_kernel(const V* __restrict__ k_src, const V* __restrict__ v_src,
-                                 V* __restrict__ k_dst, V* __restrict__ v_dst, int pieces,
+__global__ void cache_row_kernel(const V* k_src, const V* v_src, V* k_dst, V* v_dst, int pieces,
                                  size_t dst_pitch) {
+  let_next_start();
+  wait_for_previous();
   const V* src = (blockIdx.z == 0 ? k_src : v_src) + static_cast<size_t>(blockIdx.y) * pieces;
   V* dst = (blockIdx.z == 0 ? k_dst : v_dst) + blockIdx.y * dst_pitch;
   for (int i = threadIdx.x; i < pieces; i += blockDim.x) dst[i] = src[i];
@@ -290,8 +292,8 @@ int launch_narrow_qkv(const float* q, const float* k, const float* v, void* qh, 
   if (most == 0) return RA_OK;
   const int vec = (aligned16(q) && aligned16(qh) ? 1 : 0) | (aligned16(k) && aligned16(kh) ? 2 : 0) |
                   (aligned16(v) && aligned16(vh) ? 4 : 0);
-  narrow_qkv_kernel<<<dim3(grid_for(most / 8 + 1, 256), 3), 256, 0, stream>>>(
-      q, static_cast<__half*>(qh), qn, k, v, static_cast<__half*>(kh), static_cast<__half*>(vh), kn, vec);
+  RAB_CUDA(launch_overlapped(narrow_qkv_kernel, dim3(grid_for(most / 8 + 1, 256), 3), dim3(256), 0, stream, q,
+                             static_cast<__half*>(qh), qn, k, v, static_cast<__half*>(kh), static_cast<__half*>(vh), kn, vec));
   RAB_CUDA(cudaGetLastError());
   return RA_OK;
 }
@@ -303,14 +305,14 @@ int launch_cache_row(const void* k_src, const void* v_src, void* k_dst, void* v_
                    row_bytes % 16 == 0 && dst_pitch_bytes % 16 == 0;
   const dim3 grid(1, rows, 2);
   if (vec) {
-    cache_row_kernel<uint4><<<grid, 32, 0, stream>>>(
-        static_cast<const uint4*>(k_src), static_cast<const uint4*>(v_src), static_cast<uint4*>(k_dst),
-        static_cast<uint4*>(v_dst), static_cast<int>(row_bytes / 16), dst_pitch_bytes / 16);
+    RAB_CUDA(launch_overlapped(cache_row_kernel<uint4>, grid, dim3(32), 0, stream, static_cast<const uint4*>(k_src),
+                               static_cast<const uint4*>(v_src), static_cast<uint4*>(k_dst), static_cast<uint4*>(v_dst),
+                               static_cast<int>(row_bytes / 16), dst_pitch_bytes / 16));
   } else {
-    cache_row_kernel<unsigned short><<<grid, 128, 0, stream>>>(
-        static_cast<const unsigned short*>(k_src), static_cast<const unsigned short*>(v_src),
-        static_cast<unsigned short*>(k_dst), static_cast<unsigned short*>(v_dst),
-        static_cast<int>(row_bytes / 2), dst_pitch_bytes / 2);
+    RAB_CUDA(launch_overlapped(cache_row_kernel<unsigned short>, grid, dim3(128), 0, stream,
+                               static_cast<const unsigned short*>(k_src), static_cast<const unsigned short*>(v_src),
+                               static_cast<unsigned short*>(k_dst), static_cast<unsigned short*>(v_dst),
+                               static_cast<int>(row_bytes / 2), dst_pitch_bytes / 2));
   }
   RAB_CUDA(cudaGetLastError());
   return RA_OK;
@@ -362,8 +364,8 @@ int ra_attention_finalize(float* out, const float* l, const ra_shape* shape, ra_
 int ra_attention_lse(const float* m, const float* l, float* lse, size_t count, ra_stream stream) {
   RAB_REQUIRE(m && l && lse, RA_ERR_INVALID, "ra_attention_lse: null argument");
   if (count == 0) return RA_OK;
-  lse_kernel<<<grid_for(count, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(m, l, lse,
-                                                                                   count);
+  RAB_CUDA(launch_overlapped(lse_kernel, dim3(grid_for(count, 256)), dim3(256), 0, static_cast<cudaStream_t>(stream), m, l,
+                             lse, count));
   RAB_CUDA(cudaGetLastError());
   return RA_OK;
 }

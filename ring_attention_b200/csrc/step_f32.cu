@@ -181,8 +181,8 @@ __device__ inline void st_shared_u4(unsigned addr, unsigned a, unsigned b, unsig
 template <int DR, bool kSplit>
 __global__ void __launch_bounds__(kThreadsF, 1)
     step_f32_kernel(const __grid_constant__ CUtensorMap tmap_k,
-                    const __grid_constant__ CUtensorMap tmap_v, const float* __restrict__ q_g,
-                    const float* __restrict__ k_g, long long kv_head_stride, const TcArgs a) {
+                    const __grid_constant__ CUtensorMap tmap_v, const float* q_g,
+                    const float* k_g, long long kv_head_stride, const TcArgs a) {
   using C = F32Cfg<DR, kSplit>;
   extern __shared__ __align__(1024) unsigned char smem[];  // 128B-swizzled tiles
   const unsigned s_base = smem_u32(smem);
@@ -210,11 +210,8 @@ __global__ void __launch_bounds__(kThreadsF, 1)
   unsigned cta_rank = 0;
   if constexpr (kSplit) cta_rank = cluster_ctarank();
 
-  // an earlier block gave up: leave at once; a cluster starts in the aborted state instead and
-  // still meets at its barriers (see step_tc.cu)
-  if constexpr (!kSplit) {
-    if (__syncthreads_or(*reinterpret_cast<volatile int*>(a.status) != 0)) return;
-  }
+  const int gone = tid == 0 ? *reinterpret_cast<volatile int*>(a.status) : 0;
+  let_next_start();
 
   const bool causal = (a.flags & RA_STEP_CAUSAL) != 0;
   const bool fresh = (a.flags & RA_STEP_FRESH) != 0;
@@ -261,7 +258,7 @@ __global__ void __launch_bounds__(kThreadsF, 1)
       mbar_init(bar_kv_full + 8 * s, kSplitThreads);
       mbar_init(bar_kv_empty + 8 * s, live);
     }
-    *abort_flag = (kSplit && *reinterpret_cast<volatile int*>(a.status) != 0) ? 1 : 0;
+    *abort_flag = gone != 0;
     if (s_base & 1023u) {  // the swizzle of TMA and the descriptors below count on it
       *abort_flag = 1;
       atomicCAS(&a.status[0], 0, RA_ERR_DEVICE_WAIT);
@@ -274,10 +271,22 @@ __global__ void __launch_bounds__(kThreadsF, 1)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
+  if (warp == 0 && lane == 0) {
+    prefetch_map(&tmap_k);
+    prefetch_map(&tmap_v);
+  }
   tc_fence_before();
-  __syncthreads();
+  // an earlier block gave up: leave at once; a cluster starts in the aborted state instead and
+  // still meets at its barriers (see step_tc.cu)
+  const bool leave = __syncthreads_or(gone) != 0 && !kSplit;
   tc_fence_after();
   const unsigned tmem_base = *tmem_slot;
+  wait_for_previous();
+  if (leave) {
+    if (warp == 1)
+      asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem_base) : "memory");
+    return;
+  }
 
   // Registers: 640 threads start with 96 each (61440 in all); 128 * 40 + 256 * 144 + 256 * 72 = 60416.
   if (warp < 4) {
@@ -1035,13 +1044,15 @@ int launch_f32(const StepArgs& a, cudaStream_t stream, int key_split) {
   cfg.blockDim = dim3(kThreadsF);
   cfg.dynamicSmemBytes = C::kSmemBytes;
   cfg.stream = stream;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = key_split;
-  attr.val.clusterDim.y = 1;
-  attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = kSplit ? 1 : 0;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = key_split;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = kSplit ? 2 : 1;
   RAB_CUDA(cudaLaunchKernelEx(&cfg, kern, mk, mv, static_cast<const float*>(a.q), static_cast<const float*>(a.k),
                               a.kv_head_stride, t));
   RAB_CUDA(cudaGetLastError());

@@ -210,12 +210,9 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit>::kThreads),
   const bool leader = cta_rank == 0;
   constexpr bool kCluster = kPair || kSplit;
 
-  // An earlier block gave up: leave at once (the vote makes the decision block-uniform). The
-  // blocks of a cluster could decide differently, so a cluster starts in the aborted state instead
-  // (every wait then returns at once) and still meets at the cluster barriers below.
-  if constexpr (!kCluster) {
-    if (__syncthreads_or(*reinterpret_cast<volatile int*>(a.status) != 0)) return;
-  }
+  // The status word (see below) is on its way while the block sets itself up.
+  const int gone = tid == 0 ? *reinterpret_cast<volatile int*>(a.status) : 0;
+  let_next_start();
 
   const bool causal = (a.flags & RA_STEP_CAUSAL) != 0;
   const bool fresh = (a.flags & RA_STEP_FRESH) != 0;
@@ -297,8 +294,13 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit>::kThreads),
       mbar_init(bar_s_free + 8 * w, kPair ? 4 * peers : kBM);
     }
 
-    *abort_flag = (kCluster && *reinterpret_cast<volatile int*>(a.status) != 0) ? 1 : 0;
+    *abort_flag = gone != 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0 && lane == 0) {
+    prefetch_map(&tmap_q);
+    prefetch_map(&tmap_k);
+    prefetch_map(&tmap_v);
   }
   if (warp == 1) {
     if constexpr (kPair) {
@@ -314,11 +316,21 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit>::kThreads),
     }
   }
   tc_fence_before();
-  __syncthreads();
+  // An earlier block gave up: leave at once (the vote makes the decision block-uniform). The
+  // blocks of a cluster could decide differently, so a cluster starts in the aborted state instead
+  // (every wait then returns at once) and still meets at the cluster barriers below.
+  const bool leave = __syncthreads_or(gone) != 0 && !kCluster;
   // no arrival from the peer and no multicast commit before both blocks' barriers exist
   if constexpr (kPair) cluster_sync();
   tc_fence_after();
   const unsigned tmem_base = *tmem_slot;
+  // Everything so far touched no memory but the status word, whose value only ever says to leave.
+  wait_for_previous();
+  if (leave) {
+    if (warp == 1)
+      asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem_base) : "memory");
+    return;
+  }
 
   // Registers follow the work: the producer / MMA warpgroup gives most of its registers back,
   // the two softmax warpgroups (one row of 128 scores per thread) take them.
@@ -1006,16 +1018,18 @@ int launch_cfg(const StepArgs& a, cudaStream_t stream, int key_split = 1) {
     cfg.blockDim = dim3(C::kThreads);
     cfg.dynamicSmemBytes = C::kSmemBytes;
     cfg.stream = stream;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = kSplit ? key_split : 2;
-    attr.val.clusterDim.y = 1;
-    attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = kSplit ? key_split : 2;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
     RAB_CUDA(cudaLaunchKernelEx(&cfg, kern, mq, mk, mv, t));
   } else {
-    kern<<<grid, C::kThreads, C::kSmemBytes, stream>>>(mq, mk, mv, t);
+    RAB_CUDA(launch_overlapped(kern, grid, dim3(C::kThreads), C::kSmemBytes, stream, mq, mk, mv, t));
   }
   RAB_CUDA(cudaGetLastError());
   return RA_OK;

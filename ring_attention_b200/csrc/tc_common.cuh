@@ -122,6 +122,9 @@ __device__ inline void tma_load_3d(unsigned dst, const CUtensorMap* map, unsigne
       : "memory");
 }
 
+__device__ inline void prefetch_map(const CUtensorMap* map) {
+  asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<unsigned long long>(map)) : "memory");
+}
 __device__ inline void tc_fence_before() {
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
 }
