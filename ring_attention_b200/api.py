@@ -34,8 +34,13 @@ class AttentionShape:
         return Shape(self.batch, self.heads, self.seq_q, self.seq_k, self.head_dim, self.kv_heads)
 
 
+# The handle of torch.cuda.current_stream(), without the two objects that call builds around it: they
+# cost more than 1 us of the 9 that a decode call on a short context took.
+_current_device, _raw_stream = torch._C._cuda_getDevice, torch._C._cuda_getCurrentRawStream
+
+
 def _stream():
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return _raw_stream(_current_device())
 
 
 def _ptr(t):
@@ -43,7 +48,7 @@ def _ptr(t):
         return None
     if not t.is_cuda or not t.is_contiguous():
         raise ValueError("expected a contiguous CUDA tensor")
-    return C.c_void_p(t.data_ptr())
+    return t.data_ptr()
 
 
 def _dtype(t):
