@@ -96,7 +96,9 @@ struct F32Cfg {
   static constexpr int kBoxBytes = kBNf * 128;
   static constexpr int kSlotBytes = 2 * kGroups * kBoxBytes;  // raw tile = hi + lo tiles
   static constexpr int kRawBytes = kBoxes * kBoxBytes;
-  static constexpr int kStages = D == 128 ? (kSplit ? 4 : 5) : 10;
+  // (eight slots leave room for the staged rows without taking L1 from the second read of Q: with ten a call with
+  // one key tile at head_dim 64 took 16.4 us, with eight 14.7)
+  static constexpr int kStages = D == 128 ? (kSplit ? 4 : 5) : (kSplit ? 10 : 8);
   // per-key factors of K are read by the softmax of their tile while later tiles are split; the
   // ring holds the producer back far enough for this many copies
   static constexpr int kGDepth = D == 128 ? 4 : 8;
@@ -114,7 +116,11 @@ struct F32Cfg {
   static constexpr int kOffQTop = kOffVKey + 8 * kBNf;         // [2][4] exponents of Q by softmax warp
   static constexpr int kOffMl = kOffQTop + 32;
   static constexpr int kMlBytes = kSplit ? kTiles * kBM * 8 : 0;
-  static constexpr int kSmemBytes = kOffMl + kMlBytes;
+  // where the unsplit form stages its rows (see RowStore): over Q's lo tiles, else in a place of their own
+  static constexpr int kRowStage = 4 * RowStore<DR>::kStageBytes;  // of a query tile
+  static constexpr bool kOwnStage = !kSplit && kQBytes < kRowStage;
+  static constexpr int kOffStage = kOwnStage ? (kOffMl + 15) & ~15 : kOffQ;
+  static constexpr int kSmemBytes = kOwnStage ? kOffStage + kTiles * kRowStage : kOffMl + kMlBytes;
   static constexpr int kColS = 0, kColP = kAlias ? 0 : 64, kColO = kAlias ? 64 : 128, kColQ = 192;
   static_assert(kSmemBytes <= 232448, "shared memory budget");
   static_assert(kTiles * kBM * ((DR + 4) * 4 + 8) <= kOffBar, "staging of the key-split merge");
@@ -925,58 +931,42 @@ __global__ void __launch_bounds__(kThreadsF, 1)
     }
 
     // ---------------------------------------------------------------- epilogue ----
-    if (ok && mine)
-      ok = mbar_wait(bar_o_done + 8 * w, (n_tiles - 1) & 1, abort_flag, a.status, 8, n_tiles, a.wait_ns);
-    ok = __all_sync(0xffffffffu, ok);
-    if (ok && mine) tc_fence_after();
+    auto wait_o = [&]() {
+      if (ok && mine)
+        ok = mbar_wait(bar_o_done + 8 * w, (n_tiles - 1) & 1, abort_flag, a.status, 8, n_tiles, a.wait_ns);
+      ok = __all_sync(0xffffffffu, ok);
+      if (ok && mine) tc_fence_after();
+      return ok;
+    };
     const float o_unit = pow2_any(unit == kNoUnit ? 0 : -unit);
     if constexpr (kSplit) {
+      wait_o();
       const bool gave_up = __any_sync(0xffffffffu, !ok || *abort_flag != 0) != 0;
       merge_key_split<C, DR>(a, smem, s_base, t_o, w, row, row_valid, grow0, gave_up, !gave_up && mine, m_ref, l_run,
                              o_unit, cta_rank, fresh, finalize);
-    } else if (ok) {
-      float* o_g = a.out + grow * DR;
-      const bool have = row_valid && mine && m_ref > -INFINITY;
+    } else {
       float m_old = -INFINITY, l_old = 0.f;
       if (!fresh && row_valid) {
         m_old = a.m[grow];
         l_old = a.l[grow];
       }
-      const float m_new = have ? m_ref * kLn2 : -INFINITY;  // natural-log units
-      const float m_fin = fmaxf(m_old, m_new);
-      const float ca = (m_old == -INFINITY) ? 0.f : expf(m_old - m_fin);
-      const float cb = have ? expf(m_new - m_fin) : 0.f;
-      const float l_fin = ca * l_old + cb * l_run;
-      const float inv = finalize ? (l_fin > 0.f ? 1.f / l_fin : 0.f) : 1.f;
-      const bool touch = row_valid && (have || fresh || finalize);
-#pragma unroll 1
-      for (int c = 0; c < DR / 32; ++c) {
-        float o[32];
-        if (mine) {  // warp-uniform: the tensor-memory load is warp-collective
-          tmem_ld32(t_o + c * 32, o);
-        } else {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) o[i] = 0.f;
-        }
-        if (touch) {
-          float4* dst = reinterpret_cast<float4*>(o_g + c * 32);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            float4 old = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (!fresh) old = dst[i];
-            float4 r;
-            r.x = (ca * old.x + (have ? cb * (o[4 * i] * o_unit) : 0.f)) * inv;
-            r.y = (ca * old.y + (have ? cb * (o[4 * i + 1] * o_unit) : 0.f)) * inv;
-            r.z = (ca * old.z + (have ? cb * (o[4 * i + 2] * o_unit) : 0.f)) * inv;
-            r.w = (ca * old.w + (have ? cb * (o[4 * i + 3] * o_unit) : 0.f)) * inv;
-            dst[i] = r;
-          }
-        }
-      }
-      if (touch) {
-        a.m[grow] = m_fin;
-        a.l[grow] = l_fin;
-      }
+      RowStore<DR>::run(
+          a.out, grow0 + w * kBM + row - lane, __ballot_sync(0xffffffffu, row_valid),
+          s_base + C::kOffStage + w * C::kRowStage + (warp & 3) * RowStore<DR>::kStageBytes, t_o, mine, fresh, wait_o, [&]() {
+            const bool have = row_valid && mine && m_ref > -INFINITY;
+            const float m_new = have ? m_ref * kLn2 : -INFINITY;  // natural-log units
+            const float m_fin = fmaxf(m_old, m_new);
+            const float ca = (m_old == -INFINITY) ? 0.f : expf(m_old - m_fin);
+            const float cb = have ? expf(m_new - m_fin) : 0.f;
+            const float l_fin = ca * l_old + cb * l_run;
+            const float inv = finalize ? (l_fin > 0.f ? 1.f / l_fin : 0.f) : 1.f;
+            const bool touch = row_valid && (have || fresh || finalize);
+            if (touch) {
+              a.m[grow] = m_fin;
+              a.l[grow] = l_fin;
+            }
+            return RowOut{touch, have, ca * inv, cb * inv, o_unit};
+          });
     }
   }
 

@@ -829,65 +829,50 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit>::kThreads),
     }
 
     // ---------------------------------------------------------------- epilogue ----
-    if (ok && n_tiles > 0 && (!kSplit || w < live))
-      ok = mbar_wait(bar_o_done + 8 * w, (C::kEarlyS || C::kDoubleS) ? ((n_tiles - 1) & 1) : 0,
-                     abort_flag, a.status, 8, n_tiles, a.wait_ns);
-    ok = __all_sync(0xffffffffu, ok);
-    if constexpr (kSplit) {
+    auto wait_o = [&]() {
+      if (ok && n_tiles > 0 && (!kSplit || w < live))
+        ok = mbar_wait(bar_o_done + 8 * w, (C::kEarlyS || C::kDoubleS) ? ((n_tiles - 1) & 1) : 0,
+                       abort_flag, a.status, 8, n_tiles, a.wait_ns);
+      ok = __all_sync(0xffffffffu, ok);
       tc_fence_after();
+      return ok;
+    };
+    if constexpr (kSplit) {
+      wait_o();
       const bool gave_up = __any_sync(0xffffffffu, !ok || *abort_flag != 0) != 0;
       merge_key_split<C, DR>(a, smem, s_base, t_o, w, row, row_valid,
                              static_cast<size_t>(bh) * a.Sq + static_cast<size_t>(sq) * q_seg_len + row0,
                              gave_up, !gave_up && w < live && n_tiles > 0, m_ref, l_run, 1.f, cta_rank, fresh,
                              finalize);
-    } else if (ok) {
-      tc_fence_after();
-      const size_t grow = (static_cast<size_t>(bh) * a.Sq + static_cast<size_t>(sq) * q_seg_len +
-                           (row_valid ? r_in_seg : 0));
-      float* o_g = a.out + grow * DR;
-      const bool have = row_valid && n_tiles > 0 && m_ref > -INFINITY;
+    } else {
+      const size_t grow0 = static_cast<size_t>(bh) * a.Sq + static_cast<size_t>(sq) * q_seg_len + r_in_seg - lane;
+      const size_t grow = grow0 + lane;
       float m_old = -INFINITY, l_old = 0.f;
       if (!fresh && row_valid) {
         m_old = a.m[grow];
         l_old = a.l[grow];
       }
-      const float m_new = have ? m_ref * kLn2 : -INFINITY;  // natural-log units
-      const float m_fin = fmaxf(m_old, m_new);
-      const float ca = (m_old == -INFINITY) ? 0.f : expf(m_old - m_fin);
-      // O and l are relative to m_ref; bring them to m_fin
-      const float cb = have ? expf(m_new - m_fin) : 0.f;
-      const float l_fin = ca * l_old + cb * l_run;
-      const float inv = finalize ? (l_fin > 0.f ? 1.f / l_fin : 0.f) : 1.f;
-      // a row that saw nothing keeps its state unless the caller asked to overwrite / normalise
-      const bool touch = row_valid && (have || fresh || finalize);
-#pragma unroll 1
-      for (int c = 0; c < DR / 32; ++c) {
-        float o[32];
-        if (n_tiles > 0) {  // block-uniform: the tensor-memory load is warp-collective
-          tmem_ld32(t_o + c * 32, o);
-        } else {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) o[i] = 0.f;
-        }
-        if (touch) {
-          float4* dst = reinterpret_cast<float4*>(o_g + c * 32);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            float4 old = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (!fresh) old = dst[i];
-            float4 r;
-            r.x = (ca * old.x + (have ? cb * o[4 * i] : 0.f)) * inv;
-            r.y = (ca * old.y + (have ? cb * o[4 * i + 1] : 0.f)) * inv;
-            r.z = (ca * old.z + (have ? cb * o[4 * i + 2] : 0.f)) * inv;
-            r.w = (ca * old.w + (have ? cb * o[4 * i + 3] : 0.f)) * inv;
-            dst[i] = r;
-          }
-        }
-      }
-      if (touch) {
-        a.m[grow] = m_fin;
-        a.l[grow] = l_fin;
-      }
+      // (the rows are staged over their own query tile, which no MMA reads any more; every warp has a quarter)
+      static_assert(4 * RowStore<DR>::kStageBytes <= C::kTileBytes, "staging of the rows");
+      RowStore<DR>::run(
+          a.out, grow0, __ballot_sync(0xffffffffu, row_valid),
+          s_q + w * C::kTileBytes + (warp & 3) * RowStore<DR>::kStageBytes, t_o, n_tiles > 0, fresh, wait_o, [&]() {
+            const bool have = row_valid && n_tiles > 0 && m_ref > -INFINITY;
+            const float m_new = have ? m_ref * kLn2 : -INFINITY;  // natural-log units
+            const float m_fin = fmaxf(m_old, m_new);
+            const float ca = (m_old == -INFINITY) ? 0.f : expf(m_old - m_fin);
+            // O and l are relative to m_ref; bring them to m_fin
+            const float cb = have ? expf(m_new - m_fin) : 0.f;
+            const float l_fin = ca * l_old + cb * l_run;
+            const float inv = finalize ? (l_fin > 0.f ? 1.f / l_fin : 0.f) : 1.f;
+            // a row that saw nothing keeps its state unless the caller asked to overwrite / normalise
+            const bool touch = row_valid && (have || fresh || finalize);
+            if (touch) {
+              a.m[grow] = m_fin;
+              a.l[grow] = l_fin;
+            }
+            return RowOut{touch, have, ca * inv, cb * inv, 1.f};
+          });
     }
   }
 
