@@ -262,7 +262,7 @@ __global__ void __launch_bounds__(kThreadsF, 1)
     for (int s = 0; s < C::kStages; ++s) {
       mbar_init(bar_kv_raw + 8 * s, 1);
       mbar_init(bar_kv_full + 8 * s, kSplitThreads);
-      mbar_init(bar_kv_empty + 8 * s, live);
+      mbar_init(bar_kv_empty + 8 * s, C::kAlias ? 1 : live);
     }
     *abort_flag = gone != 0;
     if (s_base & 1023u) {  // the swizzle of TMA and the descriptors below count on it
@@ -328,21 +328,14 @@ __global__ void __launch_bounds__(kThreadsF, 1)
           }
         }
       }
-    } else if (warp == 1 || (warp == 2 && live == 2)) {
+    } else if (warp == 1 || (!C::kAlias && warp == 2 && live == 2)) {
       // ----------------------------------------------------------- MMA issuers ----
       if (n_tiles > 0) {
-        const int w = warp - 1;
         constexpr unsigned idesc_s = make_idesc(0u, 0, kBNf, kBM);
         constexpr unsigned idesc_pv = make_idesc(0u, 1, DR, kBM);
         constexpr unsigned kQBox = (kBM * 128) >> 4;        // one 64-column box, 16-byte units
         constexpr unsigned kGroup = (2 * C::kBoxBytes) >> 4;  // hi and lo box of a 64-column group
         constexpr unsigned kLo = C::kBoxBytes >> 4;
-        const unsigned t_w = tmem_base + 256 * w;
-        const unsigned t_s = t_w + C::kColS, t_p = t_w + C::kColP, t_o = t_w + C::kColO;
-        const unsigned t_q = t_w + C::kColQ;
-        [[maybe_unused]] const unsigned long long qd = desc_kmajor(s_q + w * C::kQBytes);
-        const unsigned b_s_full = bar_s_full + 8 * w, b_s_free = bar_s_free + 8 * w;
-        const unsigned b_p_full = bar_p_full + 8 * w, b_o_done = bar_o_done + 8 * w;
         auto wait = [&](unsigned bar, unsigned parity, int which, int tile) {
           return __all_sync(0xffffffffu,
                             mbar_wait(bar, parity, abort_flag, a.status, which, tile, a.wait_ns)) != 0;
@@ -351,9 +344,12 @@ __global__ void __launch_bounds__(kThreadsF, 1)
         auto wait_kv = [&](int it, int which, int t) {
           return wait(bar_kv_full + 8 * (it % C::kStages), (it / C::kStages) & 1, which, t);
         };
-        auto issue_s = [&](int t) {
+        // `last`: no other query tile reads the slot after this one
+        auto issue_s = [&](int t, int w, bool last) {
           const int slot = (2 * t) % C::kStages;
           const unsigned long long kd = desc_kmajor(s_kv + slot * C::kSlotBytes);
+          [[maybe_unused]] const unsigned long long qd = desc_kmajor(s_q + w * C::kQBytes);
+          const unsigned t_s = tmem_base + 256 * w + C::kColS, t_q = tmem_base + 256 * w + C::kColQ;
           if (elect_one()) {
             // small terms first: lo*hi, hi*lo, hi*hi
 #pragma unroll
@@ -369,15 +365,16 @@ __global__ void __launch_bounds__(kThreadsF, 1)
                 }
               }
             }
-            tc_commit(b_s_full);
-            tc_commit(bar_kv_empty + 8 * slot);
+            tc_commit(bar_s_full + 8 * w);
+            if (last) tc_commit(bar_kv_empty + 8 * slot);
           }
         };
-        auto issue_pv = [&](int t) {
+        auto issue_pv = [&](int t, int w, bool last) {
           const int slot = (2 * t + 1) % C::kStages;
           // MN-major V: 64 columns per 128-byte row, groups 2 boxes apart, 16 keys per k-step
           const unsigned long long vd =
               desc_mnmajor(s_kv + slot * C::kSlotBytes, 2 * C::kBoxBytes, 1024);
+          const unsigned t_p = tmem_base + 256 * w + C::kColP, t_o = tmem_base + 256 * w + C::kColO;
           const bool wide = (v_exp[t & 15] & kWide) != 0;  // the softmax threads have added this tile to O
           if (elect_one()) {
             if (!wide) {
@@ -390,37 +387,55 @@ __global__ void __launch_bounds__(kThreadsF, 1)
                          (t > 0 || term > 0 || ks > 0) ? 1u : 0u);
               }
             }
-            tc_commit(b_o_done);
-            tc_commit(bar_kv_empty + 8 * slot);
+            tc_commit(bar_o_done + 8 * w);
+            if (last) tc_commit(bar_kv_empty + 8 * slot);
           }
         };
-        bool ok = wait(bar_q_full + 8 * w, 0, 3, w) && wait_kv(0, 5, 0);
-        if (ok) {
-          tc_fence_after();
-          issue_s(0);
-        }
-        for (int t = 0; t < n_tiles && ok; ++t) {
-          const bool more = t + 1 < n_tiles;
-          if constexpr (C::kAlias) {
-            // P.V of tile t and the scores of tile t + 1, which overwrite P, go out together: the
-            // tensor core runs them in order
-            ok = wait_kv(2 * t + 1, 4, t) && (!more || wait_kv(2 * t + 2, 5, t)) &&
-                 wait(b_p_full, t & 1, 6, t);
+        bool ok = true;
+        if constexpr (C::kAlias) {
+          // One warp issues for both query tiles, in turn: P.V of tile t and the scores of tile t + 1, which
+          // overwrite P, of one query tile, then those of the other. The tensor core runs them in that
+          // order, so one tile's softmax works under the other's MMAs. (Two issuing warps end in step:
+          // the tensor core takes their instructions alternately, both batches end together, 3250 clocks
+          // after they began, and both softmax groups run at once while it idles: 6400 clocks a tile.)
+          for (int w = 0; w < live && ok; ++w) {
+            ok = wait(bar_q_full + 8 * w, 0, 3, w) && wait_kv(0, 5, 0);
             if (!ok) break;
             tc_fence_after();
-            issue_pv(t);
-            if (more) issue_s(t + 1);
-          } else {
-            if (more) {
-              ok = wait(b_s_free, t & 1, 9, t) && wait_kv(2 * t + 2, 5, t);
+            issue_s(0, w, w == live - 1);
+          }
+          for (int t = 0; t < n_tiles && ok; ++t) {
+            const bool more = t + 1 < n_tiles;
+            for (int w = 0; w < live && ok; ++w) {
+              ok = wait_kv(2 * t + 1, 4, t) && wait(bar_p_full + 8 * w, t & 1, 6, t);
               if (!ok) break;
               tc_fence_after();
-              issue_s(t + 1);
+              issue_pv(t, w, w == live - 1);
+              if (!more) continue;
+              ok = wait_kv(2 * t + 2, 5, t);
+              if (!ok) break;
+              tc_fence_after();
+              issue_s(t + 1, w, w == live - 1);
             }
-            ok = wait_kv(2 * t + 1, 4, t) && wait(b_p_full, t & 1, 6, t);
+          }
+        } else {
+          const int w = warp - 1;
+          ok = wait(bar_q_full + 8 * w, 0, 3, w) && wait_kv(0, 5, 0);
+          if (ok) {
+            tc_fence_after();
+            issue_s(0, w, true);
+          }
+          for (int t = 0; t < n_tiles && ok; ++t) {
+            if (t + 1 < n_tiles) {
+              ok = wait(bar_s_free + 8 * w, t & 1, 9, t) && wait_kv(2 * t + 2, 5, t);
+              if (!ok) break;
+              tc_fence_after();
+              issue_s(t + 1, w, true);
+            }
+            ok = wait_kv(2 * t + 1, 4, t) && wait(bar_p_full + 8 * w, t & 1, 6, t);
             if (!ok) break;
             tc_fence_after();
-            issue_pv(t);
+            issue_pv(t, w, true);
           }
         }
       }

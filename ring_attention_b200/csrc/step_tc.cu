@@ -142,6 +142,8 @@ struct TcCfg {
   //    one batch when P(t) is written.
   static constexpr bool kDoubleS = kTiles == 1 && kPInTmem;
   static constexpr bool kEarlyS = !kPInTmem || D == 64;
+  // Where P aliases S, one warp issues for both query tiles, in turn (see the issuer).
+  static constexpr bool kOrdered = !kEarlyS && !kDoubleS;
   static constexpr int kColS0 = 0, kColS1 = 128;
   static constexpr int kColO0 = (kTiles == 2 || kDoubleS) ? 256 : 128, kColO1 = 256 + D;
   static constexpr int kColP0 = (kPInTmem && kEarlyS) ? 384 : kColS0;
@@ -285,7 +287,7 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit>::kThreads),
     mbar_init(bar_q_full + 8, peers);
     for (int s = 0; s < C::kStages; ++s) {
       mbar_init(bar_kv_full + 8 * s, peers);
-      mbar_init(bar_kv_empty + 8 * s, live);  // one commit from each issuing warp
+      mbar_init(bar_kv_empty + 8 * s, C::kOrdered ? 1 : live);  // one commit from each issuing warp
     }
     for (int w = 0; w < 2; ++w) {
       mbar_init(bar_s_full + 8 * w, 1);
@@ -443,7 +445,7 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit>::kThreads),
         }
       }
     }
-  } else if (warp == 1 || (warp == 2 && live == 2)) {
+  } else if (warp == 1 || (!C::kOrdered && warp == 2 && live == 2)) {
     // ------------------------------------------------------------- MMA issuers ----
     // One issuing warp per query tile (warp 1: tile 0, warp 2: tile 1). The two tiles are
     // independent instruction streams, so a tile that is still in its exponentials never holds
@@ -453,15 +455,11 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit>::kThreads),
     // warp-uniform; the tcgen05.mma / tcgen05.commit instructions are executed by one elected
     // lane. A K/V ring slot is released when both warps have committed their reads of it.
     if (n_tiles > 0) {
-      const int w = warp - 1;
+      const int w = warp - 1;  // (ordered: the query tile is the loop's, see s_ksteps)
       constexpr unsigned kFmt = kBf16 ? 1u : 0u;
       constexpr unsigned idesc_s = make_idesc(kFmt, 0, kBN, C::kMmaM);
       constexpr unsigned idesc_pv = make_idesc(kFmt, 1, C::kPvN, C::kMmaM);
-      const unsigned t_s = tmem_base + (w == 0 ? C::kColS0 : C::kColS1);
-      const unsigned t_o = tmem_base + (w == 0 ? C::kColO0 : C::kColO1);
-      [[maybe_unused]] const unsigned t_p = tmem_base + (w == 0 ? C::kColP0 : C::kColP1);
-      const unsigned long long qd = desc_kmajor(s_q + w * C::kTileBytes);
-      [[maybe_unused]] const unsigned long long pd = desc_kmajor(s_p + w * C::kPBytes);
+      const unsigned long long qd0 = desc_kmajor(s_q);
       const unsigned long long dkv0_k = desc_kmajor(s_kv);
       const unsigned long long dkv0_v = desc_mnmajor(s_kv, kBN * 128, 1024);
       constexpr unsigned kItemUnits = C::kItemBytes >> 4;  // one ring slot in 16-byte units
@@ -495,7 +493,9 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit>::kThreads),
       };
       // Ring items of key tile t: see ring_pos.
       // The k-steps of one K item of S_w = Q_w K^T (called by the elected lane).
-      auto s_ksteps = [&](int slot, int sub, [[maybe_unused]] int sbuf) {
+      auto s_ksteps = [&](int slot, int sub, [[maybe_unused]] int sbuf, int w) {
+        const unsigned t_s = tmem_base + (w == 0 ? C::kColS0 : C::kColS1);
+        const unsigned long long qd = qd0 + static_cast<unsigned long long>(w * (C::kTileBytes >> 4));
         const unsigned long long kd = dkv0_k + static_cast<unsigned long long>(slot * kItemUnits);
 #pragma unroll
         for (int ks = 0; ks < C::kBoxesPerItem * 4; ++ks) {
@@ -507,7 +507,10 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit>::kThreads),
         }
       };
       // The k-steps of one V item of O_w += P_w V: kPvN output columns.
-      auto pv_ksteps = [&](int slot, int sub, bool acc, [[maybe_unused]] int pbuf) {
+      auto pv_ksteps = [&](int slot, int sub, bool acc, [[maybe_unused]] int pbuf, int w) {
+        const unsigned t_o = tmem_base + (w == 0 ? C::kColO0 : C::kColO1);
+        [[maybe_unused]] const unsigned t_p = tmem_base + (w == 0 ? C::kColP0 : C::kColP1);
+        [[maybe_unused]] const unsigned long long pd = desc_kmajor(s_p + w * C::kPBytes);
         const unsigned long long vd = dkv0_v + static_cast<unsigned long long>(slot * kItemUnits);
 #pragma unroll
         for (int ks = 0; ks < kBN / 16; ++ks) {
@@ -533,7 +536,7 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit>::kThreads),
           tc_fence_after();
           if (elect_one()) {
             const int sbuf = C::kDoubleS ? (t & 1) : 0;
-            s_ksteps(slot, sub, sbuf);
+            s_ksteps(slot, sub, sbuf, w);
             if (sub == kIPT - 1) commit(b_s_full + 8 * sbuf);
             commit(bar_kv_empty + 8 * slot);
           }
@@ -551,14 +554,55 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit>::kThreads),
           if (!good) break;
           tc_fence_after();
           if (elect_one()) {
-            pv_ksteps(slot, sub, t > 0, C::kDoubleS ? (t & 1) : 0);
+            pv_ksteps(slot, sub, t > 0, C::kDoubleS ? (t & 1) : 0, w);
             if (sub == kIPT - 1) commit(b_o_done);
             commit(bar_kv_empty + 8 * slot);
           }
         }
         return good;
       };
-      bool ok = wait(bar_q_full + 8 * w, 0, 3, w) && do_s(0);
+      bool ok = true;
+      if constexpr (C::kOrdered) {
+        // P aliases S (whole tiles are single ring items here): P.V of tile t and the scores of tile t+1
+        // go out in one batch once P_w(t) is written; the scores' completion tells the softmax group that P.V
+        // is done as well. One warp issues the batches of both query tiles in turn, so that each runs
+        // by itself and one tile's softmax works under the other's MMAs; from two warps the tensor core
+        // takes instructions alternately and the two tiles end in step, each waiting for both batches.
+        for (int v = 0; v < live && ok; ++v) {
+          ok = wait(bar_q_full + 8 * v, 0, 3, v) && wait_kv(ring_pos<C>(0, 0, 0), 5, 0);
+          if (!ok) break;
+          tc_fence_after();
+          if (elect_one()) {
+            s_ksteps(ring_pos<C>(0, 0, 0).slot, 0, 0, v);
+            commit(bar_s_full + 8 * v);
+            if (v == live - 1) commit(bar_kv_empty + 8 * ring_pos<C>(0, 0, 0).slot);
+          }
+        }
+        for (int t = 0; t < n_tiles && ok; ++t) {
+          const bool more = t + 1 < n_tiles;
+          const RingPos pos_v = ring_pos<C>(1, t, 0), pos_k = ring_pos<C>(0, t + 1, 0);
+          ok = wait_kv(pos_v, 4, t) && (!more || wait_kv(pos_k, 5, t));
+          for (int v = 0; v < live && ok; ++v) {
+            ok = wait(bar_p_full + 8 * v, t & 1, 6, t);
+            if (!ok) break;
+            tc_fence_after();
+            if (elect_one()) {
+              pv_ksteps(pos_v.slot, 0, t > 0, 0, v);
+              if (more) {
+                s_ksteps(pos_k.slot, 0, 0, v);
+                commit(bar_s_full + 8 * v);
+              } else {
+                commit(bar_o_done + 8 * v);
+              }
+              if (v == live - 1) {
+                commit(bar_kv_empty + 8 * pos_v.slot);
+                if (more) commit(bar_kv_empty + 8 * pos_k.slot);
+              }
+            }
+          }
+        }
+      } else {
+      ok = wait(bar_q_full + 8 * w, 0, 3, w) && do_s(0);
       if constexpr (C::kDoubleS) ok = ok && (n_tiles < 2 || do_s(1));
       for (int t = 0; t < n_tiles && ok; ++t) {
         const bool more = t + 1 < n_tiles;
@@ -573,28 +617,8 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit>::kThreads),
           // while the exponentials of the current tile run.
           if (more) ok = wait(b_s_free, t & 1, 9, t) && do_s(t + 1);
           ok = ok && wait(b_p_full, t & 1, 6, t) && do_pv(t);
-        } else {
-          // P aliases S (whole tiles are single ring items here): P.V of tile t and the scores
-          // of tile t+1 go out in one batch once P_w(t) is written; the scores' completion
-          // tells the softmax group that P.V is done as well.
-          const RingPos pos_v = ring_pos<C>(1, t, 0), pos_k = ring_pos<C>(0, t + 1, 0);
-          const int slot_v = pos_v.slot, slot_k = pos_k.slot;
-          ok = wait_kv(pos_v, 4, t) && (!more || wait_kv(pos_k, 5, t)) && wait(b_p_full, t & 1, 6, t);
-          if (!ok) break;
-          tc_fence_after();
-          if (elect_one()) {
-            pv_ksteps(slot_v, 0, t > 0, 0);
-            if (more) {
-              s_ksteps(slot_k, 0, 0);
-              commit(b_s_full);
-              commit(bar_kv_empty + 8 * slot_v);
-              commit(bar_kv_empty + 8 * slot_k);
-            } else {
-              commit(b_o_done);
-              commit(bar_kv_empty + 8 * slot_v);
-            }
-          }
         }
+      }
       }
     }
   }
