@@ -13,16 +13,17 @@
 //   blocks per KV head the grid is turned so that all query blocks of the heads sharing one KV
 //   head run before the next KV head (see launch_cfg).
 //
-// Four forms of the same kernel, tested against each other: P in tensor memory (default) or staged
+// Five forms of the same kernel, tested against each other: P in tensor memory (default) or staged
 // through shared memory (RA_STEP_P_IN_SMEM); cluster pairs (RA_STEP_CTA_PAIR, head_dim 128 / 256):
 // tcgen05.mma.cta_group::2 with M = 256 over the two blocks of a cluster, each block loading half of
-// every K and V tile; and the key split (chosen by shape, pick_key_split): 2 to 8 blocks of a cluster
-// share the key tiles of one query block and merge their states (merge_key_split).
+// every K and V tile; the key split (chosen by shape, pick_key_split): 2 to 8 blocks of a cluster
+// share the key tiles of one query block and merge their states (merge_key_split); and the fold (chosen by
+// shape, fold_rows): a block's two query tiles are a head's light and heavy ones instead of neighbours.
 //
 // Roles inside a block (384 threads)
 //   warp 0        TMA producer: Q tiles once, then K_j, V_j, K_j+1, ... into a shared-memory
 //                 ring of 128B-swizzled tiles (cp.async.bulk.tensor, no multicast).
-//   warps 1, 2    MMA issuers, one per query tile: S_w = Q_w K_j^T and O_w += P_w V_j with fp32
+//   warps 1, 2    MMA issuers, one per query tile (warp 1 for both where P aliases S): S_w = Q_w K_j^T and O_w += P_w V_j with fp32
 //                 accumulators in tensor memory. The whole warp runs the loop (uniform control
 //                 flow and descriptors), one elected lane executes tcgen05.mma / commit.
 //                 Warp 1 also allocates / frees tensor memory.
@@ -88,7 +89,7 @@ __device__ inline unsigned pack16(float lo, float hi) {
   }
 }
 
-template <int D, bool kPInTmem, bool kPair = false, bool kSplit = false>
+template <int D, bool kPInTmem, bool kPair = false, bool kSplit = false, bool kFold = false>
 struct TcCfg {
   // head_dim 256: O alone takes 256 tensor-memory columns, so a block owns ONE 128-row query
   // tile (one MMA warp, one softmax group), and a 128-key K or V tile (64 KiB) travels through
@@ -176,12 +177,13 @@ __device__ inline RingPos ring_pos(int which, int t, int sub) {
 // DR is the head_dim of the tensors in memory: D, or 32 on the 64-wide kernel (see launch_cfg).
 // kSplit: the blocks of a cluster share the key tiles of ONE query block and merge their partial
 // states through distributed shared memory (see pick_key_split).
-template <int D, bool kBf16, bool kPInTmem, int DR, bool kPair = false, bool kSplit = false>
-__global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit>::kThreads), 1)
+// kFold: the two query tiles of a block are a light and a heavy one of the head (see fold_rows).
+template <int D, bool kBf16, bool kPInTmem, int DR, bool kPair = false, bool kSplit = false, bool kFold = false>
+__global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit, kFold>::kThreads), 1)
     step_tc_kernel(const __grid_constant__ CUtensorMap tmap_q,
                    const __grid_constant__ CUtensorMap tmap_k,
                    const __grid_constant__ CUtensorMap tmap_v, const TcArgs a) {
-  using C = TcCfg<D, kPInTmem, kPair, kSplit>;
+  using C = TcCfg<D, kPInTmem, kPair, kSplit, kFold>;
   extern __shared__ unsigned char smem_raw[];
   // 128B-swizzled tiles need 1024-byte alignment
   unsigned char* smem = reinterpret_cast<unsigned char*>(
@@ -244,13 +246,20 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit>::kThreads),
                          (2 * static_cast<int>(blockIdx.y) + static_cast<int>(blockIdx.x & 1))
                    : static_cast<int>(gridDim.y) - 1 - static_cast<int>(blockIdx.y);
   }
+  // Folded: n_qblocks_per_seg counts tiles; tile 0 is the heavy one, which sees every key that tile 1 does, and
+  // a middle one has no partner. All of the block's code below is about tile 0 unless it names the tile.
+  [[maybe_unused]] int light_lin = 0;
+  if constexpr (kFold) {
+    light_lin = static_cast<int>(blockIdx.y);
+    qb_lin = a.n_qblocks_per_seg * a.qmap.n_seg - 1 - light_lin;
+  }
   const int sq = qb_lin / a.n_qblocks_per_seg;
   const int tq = qb_lin - sq * a.n_qblocks_per_seg;
   const int h = bh % a.H;
   const int b = bh / a.H;
   const int kv_bh = b * a.kvH + (h % a.kvH);
   const int q_seg_len = a.qmap.seg_len;
-  constexpr int kQBlock = C::kTiles * kBM;  // query rows per block
+  constexpr int kQBlock = kFold ? kBM : C::kTiles * kBM;  // consecutive query rows of a block
   const int row0 = tq * kQBlock;            // first row of the block inside its segment
   // The key tiles are chosen for the rows of the block, or of both blocks of a pair (a pair
   // walks one tile list; the second block of the last pair of a segment may have no rows).
@@ -264,13 +273,31 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit>::kThreads),
   // a segment's last block of at most 128 rows leaves its second tile out (384 rows against 40384
   // keys, H32/kvH8 D128: 735 -> 542 us before any split). The other forms run it on zeros: they
   // have many blocks, and the check in their softmax loop costs the D64 pass 2 %.
-  const int live = (kSplit && C::kTiles == 2 && q_seg_len - row0 <= kBM) ? 1 : C::kTiles;
+  const int live = (kSplit && C::kTiles == 2 && q_seg_len - row0 <= kBM) || (kFold && light_lin == qb_lin) ? 1 : C::kTiles;
+
+  // (segment, first row inside it) of query tile w, and tile 1's key tiles of a key segment: the first few of tile 0's
+  [[maybe_unused]] const int light_sq = kFold ? light_lin / a.n_qblocks_per_seg : 0;
+  [[maybe_unused]] const int light_row0 = kFold ? (light_lin - light_sq * a.n_qblocks_per_seg) * kBM : 0;
+  auto tile_sq = [&](int w) { return kFold && w == 1 ? light_sq : sq; };
+  auto tile_row0 = [&](int w) { return kFold ? (w == 1 ? light_row0 : row0) : row0 + w * kBM; };
+  [[maybe_unused]] auto light_range = [&](int sk) {
+    const int q0 = a.qmap.base[light_sq] + light_row0 * a.stride;
+    return tile_range<kBN>(a.kmap, sk, a.stride, causal, a.doc_len, q0,
+                           q0 + (min(kBM, q_seg_len - light_row0) - 1) * a.stride);
+  };
 
   // Tile list: segments in order, tiles [lo, hi) of each; identical in every role.
   int n_tiles = 0;
   for (int sk = 0; sk < a.kmap.n_seg; ++sk) {
     const TileRange r = tile_range<kBN>(a.kmap, sk, a.stride, causal, a.doc_len, qmin, qmax);
     n_tiles += r.hi - r.lo;
+  }
+  [[maybe_unused]] int n_light = 0;
+  if constexpr (kFold) {
+    for (int sk = 0; live == 2 && sk < a.kmap.n_seg; ++sk) {
+      const TileRange r = light_range(sk);
+      n_light += r.hi - r.lo;
+    }
   }
   [[maybe_unused]] int share_beg = 0, share_end = 0;
   if constexpr (kSplit) {  // this block's contiguous share, sizes at most one tile apart
@@ -342,12 +369,12 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit>::kThreads),
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer ----
     if (lane == 0 && n_tiles > 0) {
-      const int q_row = sq * q_seg_len + row0;
       for (int w = 0; w < live; ++w) {
+        const int q_row = tile_sq(w) * q_seg_len + tile_row0(w);
         mbar_expect_tx(bar_q_full + 8 * w, C::kTileBytes);
         for (int bx = 0; bx < C::kBoxes; ++bx)
           tma_load_3d(s_q + w * C::kTileBytes + bx * (kBM * 128), &tmap_q, bar_q_full + 8 * w,
-                      bx * 64, q_row + w * kBM, bh);
+                      bx * 64, q_row, bh);
       }
       int it = 0, jt = 0;  // ring items and key tiles so far
       bool ok = true;
@@ -544,7 +571,7 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit>::kThreads),
         return good;
       };
       // O_w += P_w V_t, one V item at a time.
-      auto do_pv = [&](int t) {
+      auto do_pv = [&](int t, bool acc) {
         bool good = true;
 #pragma unroll
         for (int sub = 0; sub < kIPT && good; ++sub) {
@@ -554,7 +581,7 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit>::kThreads),
           if (!good) break;
           tc_fence_after();
           if (elect_one()) {
-            pv_ksteps(slot, sub, t > 0, C::kDoubleS ? (t & 1) : 0, w);
+            pv_ksteps(slot, sub, acc, C::kDoubleS ? (t & 1) : 0, w);
             if (sub == kIPT - 1) commit(b_o_done);
             commit(bar_kv_empty + 8 * slot);
           }
@@ -562,7 +589,96 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit>::kThreads),
         return good;
       };
       bool ok = true;
-      if constexpr (C::kOrdered) {
+      if constexpr (kFold) {
+        // The walk over tile 0's keys; tile 1 takes part in the first few of every segment.
+        struct Walk {
+          int sk, t, hi, light;  // segment, tile, ends of tile 0's and tile 1's tiles in it
+        };
+        auto settle = [&](Walk& x) {  // on to a segment with tiles; false at the end
+          while (x.t >= x.hi) {
+            if (++x.sk >= a.kmap.n_seg) return false;
+            x.t = 0;
+            x.hi = tile_range<kBN>(a.kmap, x.sk, a.stride, causal, a.doc_len, qmin, qmax).hi;
+            x.light = live == 2 ? light_range(x.sk).hi : 0;
+          }
+          return true;
+        };
+        Walk at{-1, 0, 0, 0};
+        settle(at);
+        if constexpr (C::kOrdered) {
+          // as below, without tile 1 where it takes no part; the last reader of an item gives its slot back
+          int k1 = 0;  // tiles of tile 1 so far
+          auto put_s = [&](int u, int v, bool last) {
+            const int slot = ring_pos<C>(0, u, 0).slot;
+            if (elect_one()) {
+              s_ksteps(slot, 0, 0, v);
+              commit(bar_s_full + 8 * v);
+              if (last) commit(bar_kv_empty + 8 * slot);
+            }
+          };
+          ok = wait(bar_q_full, 0, 3, 0) && (live == 1 || wait(bar_q_full + 8, 0, 3, 1)) &&
+               wait_kv(ring_pos<C>(0, 0, 0), 5, 0);
+          if (ok) {
+            tc_fence_after();
+            put_s(0, 0, at.t >= at.light);
+            if (at.t < at.light) put_s(0, 1, true);
+          }
+          for (int u = 0; u < n_tiles && ok; ++u) {
+            Walk next = at;
+            ++next.t;
+            const bool more = settle(next);
+            const bool part = at.t < at.light, part_next = more && next.t < next.light;
+            const RingPos pos_v = ring_pos<C>(1, u, 0), pos_k = ring_pos<C>(0, u + 1, 0);
+            ok = wait_kv(pos_v, 4, u) && (!more || wait_kv(pos_k, 5, u)) && wait(bar_p_full, u & 1, 6, u);
+            if (!ok) break;
+            tc_fence_after();
+            if (elect_one()) {
+              pv_ksteps(pos_v.slot, 0, u > 0, 0, 0);
+              if (!more) commit(bar_o_done);
+              if (!part) commit(bar_kv_empty + 8 * pos_v.slot);
+            }
+            if (more) put_s(u + 1, 0, !part_next);
+            if (part) {
+              ok = wait(bar_p_full + 8, k1 & 1, 6, u);
+              if (!ok) break;
+              tc_fence_after();
+              if (elect_one()) {
+                pv_ksteps(pos_v.slot, 0, k1 > 0, 0, 1);
+                if (k1 + 1 == n_light) commit(bar_o_done + 8);
+                commit(bar_kv_empty + 8 * pos_v.slot);
+              }
+              ++k1;
+            }
+            if (part_next) put_s(u + 1, 1, true);
+            at = next;
+          }
+        } else {
+          ok = wait(bar_q_full + 8 * w, 0, 3, w);
+          int k = 0;             // tiles of this query tile so far
+          bool issued = false;   // the scores of this tile went out early
+          for (int u = 0; u < n_tiles && ok; ++u) {
+            Walk next = at;
+            ++next.t;
+            const bool more = settle(next);
+            const bool part = w == 0 || at.t < at.light, part_next = more && (w == 0 || next.t < next.light);
+            if (part) {
+              if (!issued) ok = do_s(u);
+              if (part_next) ok = ok && wait(b_s_free, k & 1, 9, u) && do_s(u + 1);
+              issued = part_next;
+              ok = ok && wait(b_p_full, k & 1, 6, u) && do_pv(u, k > 0);
+              ++k;
+            } else {
+              // not this query tile's: its two slots go back unread
+              for (int which = 0; which < 2 && ok; ++which) {
+                const RingPos pos = ring_pos<C>(which, u, 0);
+                ok = wait_kv(pos, 5 - which, u);
+                if (ok && lane == 0) mbar_arrive(bar_kv_empty + 8 * pos.slot);
+              }
+            }
+            at = next;
+          }
+        }
+      } else if constexpr (C::kOrdered) {
         // P aliases S (whole tiles are single ring items here): P.V of tile t and the scores of tile t+1
         // go out in one batch once P_w(t) is written; the scores' completion tells the softmax group that P.V
         // is done as well. One warp issues the batches of both query tiles in turn, so that each runs
@@ -609,14 +725,14 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit>::kThreads),
         if constexpr (C::kDoubleS) {
           // P.V of tile t when its P is written, then the scores of tile t + 2 into the buffer
           // that P(t) leaves (in order behind P.V(t) on the tensor core)
-          ok = wait(b_p_full, t & 1, 6, t) && do_pv(t);
+          ok = wait(b_p_full, t & 1, 6, t) && do_pv(t, t > 0);
           if (t + 2 < n_tiles) ok = ok && do_s(t + 2);
         } else if constexpr (C::kEarlyS) {
           // S_w(t+1) goes out as soon as the softmax threads hold S_w(t) in registers; P.V of
           // tile t follows when its P is written. The tensor core works on the next scores
           // while the exponentials of the current tile run.
           if (more) ok = wait(b_s_free, t & 1, 9, t) && do_s(t + 1);
-          ok = ok && wait(b_p_full, t & 1, 6, t) && do_pv(t);
+          ok = ok && wait(b_p_full, t & 1, 6, t) && do_pv(t, t > 0);
         }
       }
       }
@@ -635,9 +751,10 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit>::kThreads),
     const unsigned t_o = tmem_base + lane_base + (w == 0 ? C::kColO0 : C::kColO1);
     [[maybe_unused]] const unsigned t_p =
         tmem_base + lane_base + (w == 0 ? C::kColP0 : C::kColP1);
-    const int r_in_seg = row0 + w * kBM + row;
-    const bool row_valid = r_in_seg < q_seg_len;
-    const int qpos = a.qmap.base[sq] + r_in_seg * a.stride;
+    const int r_in_seg = tile_row0(w) + row;
+    const bool row_valid = r_in_seg < q_seg_len && (!kFold || w < live);
+    const int qpos = a.qmap.base[tile_sq(w)] + r_in_seg * a.stride;
+    const int n_own = kFold && w == 1 ? n_light : n_tiles;  // key tiles of this query tile
     const long long qdoc = a.doc_len > 0 ? qpos / a.doc_len : 0;
     const float scale_log2 = rsqrtf(static_cast<float>(DR)) * kLog2e;
 
@@ -646,11 +763,14 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit>::kThreads),
     bool ok = true;
 
     int j = 0;
-    const int n_seg = (!kSplit || w < live) ? a.kmap.n_seg : 0;
+    const int n_seg = (!(kSplit || kFold) || w < live) ? a.kmap.n_seg : 0;
     [[maybe_unused]] TileShare share{share_beg, share_end, 0};
     for (int sk = 0; sk < n_seg && ok; ++sk) {
       TileRange tr = tile_range<kBN>(a.kmap, sk, a.stride, causal, a.doc_len, qmin, qmax);
       if constexpr (kSplit) tr = share.clip(tr);
+      if constexpr (kFold) {
+        if (w == 1) tr = light_range(sk);
+      }
       // Keys of this segment the row can see are the local indices [rel_lo, rel_hi): causal
       // and document limits are affine in the key index, so they are worked out once per
       // segment (64-bit divisions) and the per-tile work is two 32-bit clamps.
@@ -854,9 +974,9 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit>::kThreads),
 
     // ---------------------------------------------------------------- epilogue ----
     auto wait_o = [&]() {
-      if (ok && n_tiles > 0 && (!kSplit || w < live))
-        ok = mbar_wait(bar_o_done + 8 * w, (C::kEarlyS || C::kDoubleS) ? ((n_tiles - 1) & 1) : 0,
-                       abort_flag, a.status, 8, n_tiles, a.wait_ns);
+      if (ok && n_own > 0 && (!kSplit || w < live))
+        ok = mbar_wait(bar_o_done + 8 * w, (C::kEarlyS || C::kDoubleS) ? ((n_own - 1) & 1) : 0,
+                       abort_flag, a.status, 8, n_own, a.wait_ns);
       ok = __all_sync(0xffffffffu, ok);
       tc_fence_after();
       return ok;
@@ -869,7 +989,7 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit>::kThreads),
                              gave_up, !gave_up && w < live && n_tiles > 0, m_ref, l_run, 1.f, cta_rank, fresh,
                              finalize);
     } else {
-      const size_t grow0 = static_cast<size_t>(bh) * a.Sq + static_cast<size_t>(sq) * q_seg_len + r_in_seg - lane;
+      const size_t grow0 = static_cast<size_t>(bh) * a.Sq + static_cast<size_t>(tile_sq(w)) * q_seg_len + r_in_seg - lane;
       const size_t grow = grow0 + lane;
       float m_old = -INFINITY, l_old = 0.f;
       if (!fresh && row_valid) {
@@ -880,8 +1000,8 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit>::kThreads),
       static_assert(4 * RowStore<DR>::kStageBytes <= C::kTileBytes, "staging of the rows");
       RowStore<DR>::run(
           a.out, grow0, __ballot_sync(0xffffffffu, row_valid),
-          s_q + w * C::kTileBytes + (warp & 3) * RowStore<DR>::kStageBytes, t_o, n_tiles > 0, fresh, wait_o, [&]() {
-            const bool have = row_valid && n_tiles > 0 && m_ref > -INFINITY;
+          s_q + w * C::kTileBytes + (warp & 3) * RowStore<DR>::kStageBytes, t_o, n_own > 0, fresh, wait_o, [&]() {
+            const bool have = row_valid && n_own > 0 && m_ref > -INFINITY;
             const float m_new = have ? m_ref * kLn2 : -INFINITY;  // natural-log units
             const float m_fin = fmaxf(m_old, m_new);
             const float ca = (m_old == -INFINITY) ? 0.f : expf(m_old - m_fin);
@@ -928,9 +1048,9 @@ std::atomic<unsigned long long> g_wait_ns{kWaitLimitNs};
 std::atomic<int> g_stall_after{-1};
 std::atomic<int> g_block_order{-1};  // -1: by shape, 0: heads fastest, k > 0: waves of k KV heads
 
-template <int D, bool kBf16, bool kPInTmem, int DR, bool kPair = false, bool kSplit = false>
+template <int D, bool kBf16, bool kPInTmem, int DR, bool kPair = false, bool kSplit = false, bool kFold = false>
 int launch_cfg(const StepArgs& a, cudaStream_t stream, int key_split = 1) {
-  using C = TcCfg<D, kPInTmem, kPair, kSplit>;
+  using C = TcCfg<D, kPInTmem, kPair, kSplit, kFold>;
   CUtensorMap mq, mk, mv;
   const int dtype = kBf16 ? RA_BF16 : RA_F16;
   int rc = make_map(&mq, dtype, a.q, a.D, a.Sq, static_cast<long long>(a.B) * a.H,
@@ -948,7 +1068,7 @@ int launch_cfg(const StepArgs& a, cudaStream_t stream, int key_split = 1) {
   t.H = a.H;
   t.kvH = a.kvH;
   t.Sq = a.Sq;
-  constexpr int kQBlock = C::kTiles * kBM;
+  constexpr int kQBlock = kFold ? kBM : C::kTiles * kBM;
   t.n_qblocks_per_seg = (a.qmap.seg_len + kQBlock - 1) / kQBlock;
   if (kPair) t.n_qblocks_per_seg = (t.n_qblocks_per_seg + 1) & ~1;  // whole pairs per segment
   t.qmap = a.qmap;
@@ -963,7 +1083,8 @@ int launch_cfg(const StepArgs& a, cudaStream_t stream, int key_split = 1) {
   t.status = a.status;
   t.wait_ns = g_wait_ns.load(std::memory_order_relaxed);
   t.stall_after = g_stall_after.load(std::memory_order_relaxed);
-  const long long n_qblocks = static_cast<long long>(t.n_qblocks_per_seg) * a.qmap.n_seg;
+  long long n_qblocks = static_cast<long long>(t.n_qblocks_per_seg) * a.qmap.n_seg;
+  if (kFold) n_qblocks = (n_qblocks + 1) / 2;
   // Block order. By default (kv_per_wave = 0) the (batch, head) index runs fastest and the query
   // blocks go heavy first over the whole grid, which balances best - as long as the K and V of
   // all heads stay in L2 together. When they do not (long sequences: 67 MB per KV head at
@@ -999,14 +1120,14 @@ int launch_cfg(const StepArgs& a, cudaStream_t stream, int key_split = 1) {
   }
   const int order = g_block_order.load(std::memory_order_relaxed);  // test hook
   if (order == 0 || (order > 0 && kv_heads_total % order == 0)) kv_per_wave = order;
-  if (kSplit) kv_per_wave = 0;
+  if (kSplit || kFold) kv_per_wave = 0;
   t.kv_per_wave = kv_per_wave;
   t.key_split = key_split;
   const long long bh_total = static_cast<long long>(a.B) * a.H;
   const long long per_x = kv_per_wave > 0 ? static_cast<long long>(a.H / a.kvH) * kv_per_wave : 0;
   RAB_REQUIRE(kv_per_wave > 0 ? n_qblocks * per_x < (1ll << 31) : n_qblocks <= 65535, RA_ERR_INVALID,
               "attention step: grid too large (%lld query blocks, %lld heads)", n_qblocks, bh_total);
-  auto kern = step_tc_kernel<D, kBf16, kPInTmem, DR, kPair, kSplit>;
+  auto kern = step_tc_kernel<D, kBf16, kPInTmem, DR, kPair, kSplit, kFold>;
   // once per device and instantiation: the attribute call costs microseconds that a pass of a
   // few short launches would otherwise pay every time
   static std::atomic<unsigned long long> smem_set{0};
@@ -1050,6 +1171,12 @@ int launch_split(int dtype, const StepArgs& a, cudaStream_t stream, int n) {
                           : launch_cfg<D, false, true, DR, false, true>(a, stream, n);
 }
 
+template <int D, int DR>
+int launch_fold(int dtype, const StepArgs& a, cudaStream_t stream) {
+  return dtype == RA_BF16 ? launch_cfg<D, true, true, DR, false, false, true>(a, stream)
+                          : launch_cfg<D, false, true, DR, false, false, true>(a, stream);
+}
+
 template <int D>
 int launch_d(int dtype, const StepArgs& a, cudaStream_t stream) {
   // P stays in tensor memory unless the caller asks for the shared-memory path (kept as a
@@ -1061,14 +1188,17 @@ int launch_d(int dtype, const StepArgs& a, cudaStream_t stream) {
   const int* slots = nullptr;
   const int rc = cluster_slots(step_tc_kernel<D, false, true, D, false, true>, S::kThreads, S::kSmemBytes, &slots);
   if (rc != RA_OK) return rc;
-  const int split = p_in_tmem && (a.flags & RA_STEP_CTA_PAIR) == 0 &&
-                            g_block_order.load(std::memory_order_relaxed) < 0
-                        ? pick_key_split<kBN>(a, TcCfg<D, true>::kTiles * kBM,
-                                              D == 64 ? 1.5 : D == 128 ? 2.5 : 4.5, slots)
-                        : 1;
+  int split = 1;
+  [[maybe_unused]] bool fold = false;
+  if (p_in_tmem && (a.flags & RA_STEP_CTA_PAIR) == 0 && g_block_order.load(std::memory_order_relaxed) < 0) {
+    double tiles = 0;
+    split = pick_key_split<kBN>(a, TcCfg<D, true>::kTiles * kBM, D == 64 ? 1.5 : D == 128 ? 2.5 : 4.5, slots, &tiles);
+    if constexpr (D <= 128) fold = fold_rows<kBN>(a, D == 64 ? 0.75 : 0.87, tiles);
+  }
   // the 64-wide kernel also takes head_dim 32 (DR = 32)
   if constexpr (D == 64) {
     if (a.D == 32) {
+      if (fold) return launch_fold<64, 32>(dtype, a, stream);
       if (split > 1) return launch_split<64, 32>(dtype, a, stream, split);
       if (dtype == RA_BF16)
         return p_in_tmem ? launch_cfg<64, true, true, 32>(a, stream)
@@ -1076,6 +1206,9 @@ int launch_d(int dtype, const StepArgs& a, cudaStream_t stream) {
       return p_in_tmem ? launch_cfg<64, false, true, 32>(a, stream)
                        : launch_cfg<64, false, false, 32>(a, stream);
     }
+  }
+  if constexpr (D <= 128) {
+    if (fold) return launch_fold<D, D>(dtype, a, stream);
   }
   if (split > 1) return launch_split<D, D>(dtype, a, stream, split);
   if constexpr (D == 128 || D == 256) {

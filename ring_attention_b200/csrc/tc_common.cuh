@@ -765,11 +765,13 @@ inline int cluster_slots(Kern kern, int threads, int smem_bytes, const int** out
 // 1024 x 1024 H8 D256 (64 blocks) 27 / 29 / 39 / 82; 2048 x 2048 H4 D256 41 / 37 / 41 / 86.
 // Four tiles at n = 1 / 2 / 4: 512 x 512 H8 D128 20.5 / 20.5 / 16, fp32 200 x 200 H8 D64 18.5 / 19 / 16.5, D128
 // 29 / 28 / 22.6 (so a share may be a single tile); three tiles, fp32 D64: 12.6 at n = 1, 14.4 at 3.
+constexpr double kBlockTiles = 3;  // start and end of a block, in tiles of work
 template <int kTileKeys>
-inline int pick_key_split(const StepArgs& a, int q_block_rows, double merge_tiles, const int* slots) {
+inline int pick_key_split(const StepArgs& a, int q_block_rows, double merge_tiles, const int* slots,
+                          double* estimate = nullptr) {
   const int forced = static_cast<int>((a.flags >> RA_STEP_KEY_SPLIT_SHIFT) & 15u);
   if (forced) return forced > 8 ? 8 : forced;
-  constexpr double kFixed = 3, kEmpty = 0.7;
+  constexpr double kFixed = kBlockTiles, kEmpty = 0.7;
   const int per_seg = (a.qmap.seg_len + q_block_rows - 1) / q_block_rows;
   const long long heads = static_cast<long long>(a.B) * a.H;
   if (heads * per_seg * a.qmap.n_seg >= slots[1]) return 1;
@@ -813,7 +815,42 @@ inline int pick_key_split(const StepArgs& a, int q_block_rows, double merge_tile
       best_t = t;
     }
   }
+  if (estimate) *estimate = best_t;
   return best;
+}
+
+// Whether to pair a head's query tiles light with heavy (the first with the last, ...) instead of neighbours.
+// For causal calls of one wave or less, whose time is that of the block with the most keys: its two tiles walk
+// all of them, the first block's next to none. A folded block walks the heavy tile's keys, alone where the light one
+// has ended, and a tile alone takes `alone` of the time of two (its MMAs and its softmax have nothing to
+// overlap with); so all blocks take about the same time, but all of them together more: a grid of several
+// waves keeps neighbours. `tiles`: the estimate of the best other form (0: none; see pick_key_split). us per
+// call, neighbours / two blocks a query block / folded, fp16 causal: 2048 rows H16 D64 31.0 / 35.3 / 24.9; 4096 H8 D64
+// 53.0 / 46.2 / 42.1, D128 65.2 / 56.0 / 58.6 (not taken); 1531 B2 H12 D64 29.1 / 34.9 / 27.0, D128 37.1 / 42.4 / 35.0; 512
+// H64 D64 12.8 / 26.7 / 12.0; 8192 H4 D64 (not taken) 95.7 / 67.8. From these `alone`: 0.71 to 0.86 at head_dim 64, 0.84 to
+// 0.89 at 128.
+template <int kTileKeys>
+inline bool fold_rows(const StepArgs& a, double alone, double tiles) {
+  if (tiles <= 0 || (a.flags & RA_STEP_CAUSAL) == 0 || a.doc_len > 0) return false;
+  const int per_seg = (a.qmap.seg_len + kBM - 1) / kBM, n = per_seg * a.qmap.n_seg;
+  for (int s = 1; s < a.qmap.n_seg; ++s)  // later tiles see what earlier ones do
+    if (a.qmap.base[s] < a.qmap.base[s - 1] + (a.qmap.seg_len - 1) * a.stride) return false;
+  auto keys = [&](int lin) {
+    const int s = lin / per_seg, row0 = (lin - s * per_seg) * kBM;
+    const int rows = a.qmap.seg_len - row0 < kBM ? a.qmap.seg_len - row0 : kBM;
+    const int qmin = a.qmap.base[s] + row0 * a.stride;
+    int sum = 0;
+    for (int sk = 0; sk < a.kmap.n_seg; ++sk)
+      sum += tile_range<kTileKeys>(a.kmap, sk, a.stride, true, 0, qmin, qmin + (rows - 1) * a.stride).hi;
+    return sum;
+  };
+  double longest = 0;
+  for (int i = 0; i <= n - 1 - i; ++i) {
+    const int light = n - 1 - i > i ? keys(i) : 0, heavy = keys(n - 1 - i);
+    const double t = light + alone * (heavy - light);
+    longest = t > longest ? t : longest;
+  }
+  return longest + kBlockTiles < 0.95 * tiles;
 }
 
 // Limits set through the test hooks (step_tc.cu owns them).

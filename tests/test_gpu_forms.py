@@ -491,3 +491,33 @@ def test_marked_tiles_in_a_cache_with_segments_strides_and_grouped_heads(D, spli
     assert_close(lse, want_lse, 1e-5, 1e-5, "lse")
     unit = np.abs(want).max()
     assert_close(out.cpu().numpy() / unit, want / unit, 1e-5, 0.0, "out")
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("D", [32, 64, 128])
+@pytest.mark.parametrize("heads,rows,qbases,kbases,seg_k,stride", [
+    (36, 1000, [0], [0], 1000, 1),                    # eight tiles, the last one short
+    (28, 1100, [0], [0], 1100, 1),                    # nine: the middle one alone
+    (16, 1021, [1021, 6126], [1021, 6126], 1021, 1),  # a zig-zag rank's own shard
+    (48, 600, [300], [0], 900, 1),                    # rows behind a cache
+    (40, 700, [0], [350], 700, 1),                    # the first tiles see no key
+    (32, 1000, [1], [0], 1000, 2),                    # striped
+])
+def test_light_and_heavy_query_tiles_share_a_block(dtype, D, heads, rows, qbases, kbases, seg_k, stride):
+    # causal calls of one wave pair a head's tiles light with heavy; asking for an unsplit call gives
+    # neighbours. Every row folds the same tiles in the same order, so the results are the same bits.
+    g = torch.Generator(device="cuda").manual_seed(rows + D)
+    Sq, Sk, kvH = rows * len(qbases), seg_k * len(kbases), heads // 2
+    q, k, v = (torch.randn(1, h, s, D, generator=g, device="cuda").to(dtype) for h, s in ((heads, Sq), (kvH, Sk), (kvH, Sk)))
+    shape = api.AttentionShape(1, heads, Sq, Sk, D, kvH)
+    results = []
+    for split in (0, 1):
+        state = poisoned(1, heads, Sq, D)
+        for i, qi in enumerate((q, -q)):
+            api.attention_step_ex(qi, k, v, *state, shape, SegMap.make(qbases, rows), SegMap.make(kbases, seg_k),
+                                  pos_stride=stride, causal=True, fresh=i == 0, finalize=i == 1, key_split=split)
+        results.append(state)
+    torch.cuda.synchronize()
+    assert api.device_status()[0] == 0
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
