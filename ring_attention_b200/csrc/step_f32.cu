@@ -243,6 +243,12 @@ __global__ void __launch_bounds__(kThreadsF, 1)
     const TileRange r = tile_range<kBNf>(a.kmap, sk, a.stride, causal, a.doc_len, qmin, qmax);
     n_tiles += r.hi - r.lo;
   }
+  if (n_tiles == 0) {  // (the blocks of a cluster agree)
+    wait_for_previous();
+    rows_without_keys<DR>(a, static_cast<size_t>(bh) * a.Sq + static_cast<size_t>(sq) * q_seg_len + row0, rows_in_block,
+                          kSplit ? cta_rank : 0, kSplit ? a.key_split : 1, fresh, finalize);
+    return;
+  }
   int share_beg = 0, share_end = n_tiles;
   if constexpr (kSplit) {
     share_beg = static_cast<int>(static_cast<long long>(n_tiles) * cta_rank / a.key_split);

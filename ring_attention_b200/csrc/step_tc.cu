@@ -292,6 +292,16 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit, kFold>::kTh
     const TileRange r = tile_range<kBN>(a.kmap, sk, a.stride, causal, a.doc_len, qmin, qmax);
     n_tiles += r.hi - r.lo;
   }
+  if (n_tiles == 0) {  // (the blocks of a cluster agree)
+    wait_for_previous();
+    const size_t head0 = static_cast<size_t>(bh) * a.Sq;
+    rows_without_keys<DR>(a, head0 + static_cast<size_t>(sq) * q_seg_len + row0, min(kQBlock, q_seg_len - row0),
+                          kSplit ? cta_rank : 0, kSplit ? a.key_split : 1, fresh, finalize);
+    if (kFold && live == 2)
+      rows_without_keys<DR>(a, head0 + static_cast<size_t>(light_sq) * q_seg_len + light_row0,
+                            min(kBM, q_seg_len - light_row0), 0, 1, fresh, finalize);
+    return;
+  }
   [[maybe_unused]] int n_light = 0;
   if constexpr (kFold) {
     for (int sk = 0; live == 2 && sk < a.kmap.n_seg; ++sk) {

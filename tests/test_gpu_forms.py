@@ -521,3 +521,39 @@ def test_light_and_heavy_query_tiles_share_a_block(dtype, D, heads, rows, qbases
     assert api.device_status()[0] == 0
     for a, b in zip(*results):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("dtype,D", [(torch.float16, 32), (torch.float16, 64), (torch.bfloat16, 128), (torch.float16, 256),
+                                     (torch.float32, 32), (torch.float32, 64), (torch.float32, 128)])
+@pytest.mark.parametrize("split,pair", [(1, False), (3, False), (1, True)])
+@pytest.mark.parametrize("fresh,finalize", [(False, False), (False, True), (True, False), (True, True)])
+def test_blocks_without_keys(dtype, D, split, pair, fresh, finalize):
+    # the second segment's rows see every key, the first one's none: those keep their state bit for bit, or it is
+    # written empty, or divided by l (rows that never saw a key give zeros)
+    if pair and D not in (128, 256):
+        pytest.skip("the pair form is built for head_dim 128 and 256")
+    B, H, kvH, rows, Sk = 2, 4, 2, 333, 200
+    g = torch.Generator(device="cuda").manual_seed(D)
+    q, k, v = (torch.randn(B, h, s, D, generator=g, device="cuda").to(dtype) for h, s in ((H, 2 * rows), (kvH, Sk), (kvH, Sk)))
+    out, m, l = (torch.rand(*s, generator=g, device="cuda") + 0.5 for s in ((B, H, 2 * rows, D), (B, H, 2 * rows), (B, H, 2 * rows)))
+    m[:, :, 5::7] = float("-inf")
+    l[:, :, 5::7] = 0
+    out[:, :, 5::7] = 0
+    before = [t.clone() for t in (out, m, l)]
+    api.attention_step_ex(q, k, v, out, m, l, api.AttentionShape(B, H, 2 * rows, Sk, D, kvH), SegMap.make([0, 1000], rows),
+                          SegMap.make([500], Sk), causal=True, fresh=fresh, finalize=finalize, key_split=split, cta_pair=pair)
+    torch.cuda.synchronize()
+    assert api.device_status()[0] == 0
+    o, mm, ll = (t[:, :, :rows] for t in (out, m, l))
+    wo, wm, wl = (t[:, :, :rows] for t in before)
+    if fresh:
+        assert (o == 0).all() and (mm == float("-inf")).all() and (ll == 0).all()
+    else:
+        assert torch.equal(mm, wm) and torch.equal(ll, wl)
+        if finalize:
+            inv = torch.where(wl > 0, 1 / wl, torch.zeros_like(wl))[..., None]
+            # a product of two roundings on either side
+            assert torch.allclose(o, wo * inv, rtol=3e-7, atol=0)
+        else:
+            assert torch.equal(o, wo)
+    assert torch.isfinite(out).all()
