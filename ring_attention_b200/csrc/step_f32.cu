@@ -300,9 +300,10 @@ __global__ void __launch_bounds__(kThreadsF, 1)
     return;
   }
 
-  // Registers: 640 threads start with 96 each (61440 in all); 128 * 40 + 256 * 144 + 256 * 72 = 60416.
+  // Registers: 640 threads start with 96 each (61440 in all); 128 * 64 + 256 * 152 + 256 * 56 = 61440. (With 40 /
+  // 144 / 72 the issuing warp and the softmax spilled 132 bytes, now 60: B1 H4 S16384 D128 848 -> 828 us.)
   if (warp < 4) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
     if (warp == 0) {
       // ---------------------------------------------------------- TMA producer ----
       if (lane == 0 && n_tiles > 0) {
@@ -450,7 +451,7 @@ __global__ void __launch_bounds__(kThreadsF, 1)
       for (int i = 0; i < 3; ++i) cluster_sync_threads();
     }
   } else if (warp >= 12) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
     // --------------------------------------------------------------- splitters ----
     // A warp owns eight rows of every tile; its lanes own 16-byte pieces of the split rows (8
     // values, 32 raw bytes): lane = (piece, row), so the eight lanes of a phase touch eight rows
@@ -598,7 +599,7 @@ __global__ void __launch_bounds__(kThreadsF, 1)
       for (int i = 0; i < 3; ++i) cluster_sync_threads();
     }
   } else {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 144;");
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 152;");
     // ----------------------------------------------------------------- softmax ----
     const int w = (warp - 4) >> 2;
     const int row = ((warp & 3) << 5) + lane;  // row of the tile = tensor-memory lane
