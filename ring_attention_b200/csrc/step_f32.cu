@@ -28,7 +28,8 @@
 // Roles inside a block (640 threads)
 //   warp 0        TMA producer: K_0, V_0, K_1, ... as 128B-swizzled fp32 tiles into a shared-memory
 //                 ring (no multicast).
-//   warps 1, 2    MMA issuers, one per query tile (converged warp, one elected lane).
+//   warps 1, 2    MMA issuers, one per query tile, at head_dim 128 warp 1 for both in turn (converged
+//                 warp, one elected lane).
 //   warps 4-11    softmax, one thread per row, a warpgroup per query tile. At the start each thread
 //                 reads, scales and splits its row of Q into tensor memory, where the A operand
 //                 costs the scores no shared-memory reads, which bound them otherwise (head_dim
@@ -43,10 +44,10 @@
 //
 // Tensor memory, 256 columns per query tile: S [0,64) P hi [64,96) P lo [96,128) O [128,192) Q hi
 // [192,224) Q lo [224,256); head_dim 128: S and P [0,64) O [64,192) Q hi [192,256).
-// What bounds it: at head_dim 128 the chain scores -> softmax -> P.V of the two query tiles, which take
-// turns on the tensor core (tensor pipe 44 %, issue slots 34 %). Measured, us per call, against one
-// 128-row tile per block on TF32 pairs: B1 H4 S16384 D128 causal 830-950 (2700), B1 H8 S1024 D64 dense 23
-// (37), H4/kvH1 8231 x 9075 rows D64 causal 164 (272).
+// What bounds it: at head_dim 128 a pair of tiles of 64 keys takes 5200 clocks, of which its MMAs need 3400;
+// the two softmax groups (1500 to 1900 clocks a tile) run under the other tile's MMAs, and the issuing warp finds P
+// written when it comes to it. Measured, us per call, against one 128-row tile per block on TF32 pairs:
+// B1 H4 S16384 D128 causal 830 (2700), B1 H8 S1024 D64 dense 20.6 (37), H4/kvH1 8231 x 9075 rows D64 causal 164 (272).
 //
 // Every wait on an mbarrier is bounded (see tc_common.cuh); a wait that runs out reports into
 // the device status word and the block unwinds.
