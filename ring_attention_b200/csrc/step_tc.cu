@@ -987,6 +987,11 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit, kFold>::kTh
       if (ok && n_own > 0 && (!kSplit || w < live))
         ok = mbar_wait(bar_o_done + 8 * w, (C::kEarlyS || C::kDoubleS) ? ((n_own - 1) & 1) : 0,
                        abort_flag, a.status, 8, n_own, a.wait_ns);
+      // a light tile without keys: no MMA has read its Q, whose copy may still be on its way to the place
+      // where the rows are staged
+      if constexpr (kFold) {
+        if (ok && w < live && n_own == 0) ok = mbar_wait(bar_q_full + 8 * w, 0, abort_flag, a.status, 3, w, a.wait_ns);
+      }
       ok = __all_sync(0xffffffffu, ok);
       tc_fence_after();
       return ok;
@@ -1006,7 +1011,8 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit, kFold>::kTh
         m_old = a.m[grow];
         l_old = a.l[grow];
       }
-      // (the rows are staged over their own query tile, which no MMA reads any more; every warp has a quarter)
+      // (the rows are staged over their own query tile, which no copy writes and no MMA reads any more behind wait_o;
+      // every warp has a quarter)
       static_assert(4 * RowStore<DR>::kStageBytes <= C::kTileBytes, "staging of the rows");
       RowStore<DR>::run(
           a.out, grow0, __ballot_sync(0xffffffffu, row_valid),

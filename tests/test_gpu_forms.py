@@ -557,3 +557,37 @@ def test_blocks_without_keys(dtype, D, split, pair, fresh, finalize):
         else:
             assert torch.equal(o, wo)
     assert torch.isfinite(out).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("D", [32, 64, 128])
+@pytest.mark.parametrize("fresh,finalize", [(False, True), (True, False), (True, True)])
+def test_light_query_tiles_without_keys(dtype, D, fresh, finalize):
+    # Keys from position 350 on: two light tiles of a head see none, their blocks' heavy ones do. Such a tile's rows
+    # are staged where the copy of its Q lands, so many calls with the state set anew before each, some right behind
+    # other work and some on an idle GPU.
+    H, kvH, rows = 40, 20, 700
+    g = torch.Generator(device="cuda").manual_seed(D)
+    q, k, v = (torch.randn(1, h, rows, D, generator=g, device="cuda").to(dtype) for h in (H, kvH, kvH))
+    before = [torch.rand(*s, generator=g, device="cuda") + 0.5 for s in ((1, H, rows, D), (1, H, rows), (1, H, rows))]
+    shape = api.AttentionShape(1, H, rows, rows, D, kvH)
+
+    def call(state, split):
+        for t, b in zip(state, before):
+            t.copy_(b)
+        api.attention_step_ex(q, k, v, *state, shape, SegMap.make([0], rows), SegMap.make([350], rows), causal=True,
+                              fresh=fresh, finalize=finalize, key_split=split)
+        return state
+
+    want = call([torch.empty_like(t) for t in before], 1)
+    hidden = torch.zeros_like(before[0][:, :, :350])
+    if not fresh:  # (the product of two roundings on either side)
+        hidden = before[0][:, :, :350] / before[2][:, :, :350, None]
+    assert torch.allclose(want[0][:, :, :350], hidden, rtol=3e-7, atol=0)
+    state = [torch.empty_like(t) for t in before]
+    for i in range(60):
+        call(state, 0)
+        if i % 3 == 0:
+            torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for a, b in zip(state, want)), i
+    assert api.device_status()[0] == 0
