@@ -81,13 +81,13 @@ inline int kv_heads_of(const ra_shape& s) { return s.kv_heads > 0 ? s.kv_heads :
 
 // ---- device status word ----------------------------------------------------------
 // One per device (a __device__ array in status.cu). A kernel whose bounded wait runs out
-// records {code, which wait, block, tile} and every later block of any kernel in this
-// library returns at once, so a protocol bug costs seconds, never a hung GPU.
+// records {code, which wait, block, tile}; every later block of a step kernel returns at once or, if it had
+// already started, leaves its state as it is, so a protocol bug costs seconds, never a hung GPU.
 int* device_status_ptr();  // device address of the 4-int status word of the current device
 int read_device_status(int out[4], bool clear);
 // For entry points that end with a synchronisation of `stream`: enqueue_status_read in front
 // of it, status_after_sync behind it (RA_ERR_DEVICE_WAIT when a wait ran out; the word stays
-// set, so every later launch returns at once, until ra_device_status reads and clears it).
+// set, so every later step leaves its state as it is, until ra_device_status reads and clears it).
 int enqueue_status_read(cudaStream_t stream);
 int status_after_sync();
 // Scratch for the (m, l) of the local decode op, per device, grown on demand.

@@ -954,10 +954,12 @@ __global__ void __launch_bounds__(kThreadsF, 1)
     }
 
     // ---------------------------------------------------------------- epilogue ----
+    // (the status word once more, see step_tc.cu: behind a launch that gave up the state stays as it is)
     auto wait_o = [&]() {
+      const int lost = *reinterpret_cast<volatile int*>(a.status);
       if (ok && mine)
         ok = mbar_wait(bar_o_done + 8 * w, (n_tiles - 1) & 1, abort_flag, a.status, 8, n_tiles, a.wait_ns);
-      ok = __all_sync(0xffffffffu, ok);
+      ok = __all_sync(0xffffffffu, ok && lost == 0);
       if (ok && mine) tc_fence_after();
       return ok;
     };

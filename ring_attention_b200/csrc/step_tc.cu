@@ -58,7 +58,8 @@
 //
 // Every wait on an mbarrier is bounded: when one runs out the block records where in the
 // device status word, all roles leave their loops, tensor memory is freed and the kernel
-// returns; later blocks see the status word and return at once.
+// returns. Later blocks see the status word and return at once; blocks that read it before it was set (those
+// of the next launch, which overlap this one) run, see it at their end and leave the state as it is.
 #include <atomic>
 
 #include "tc_common.cuh"
@@ -363,7 +364,8 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit, kFold>::kTh
   if constexpr (kPair) cluster_sync();
   tc_fence_after();
   const unsigned tmem_base = *tmem_slot;
-  // Everything so far touched no memory but the status word, whose value only ever says to leave.
+  // Everything so far touched no memory but the status word. A word that is set says to leave; one that is not may
+  // yet be set by a launch before this one, so it is read again before the state is written.
   wait_for_previous();
   if (leave) {
     if (warp == 1)
@@ -983,7 +985,10 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit, kFold>::kTh
     }
 
     // ---------------------------------------------------------------- epilogue ----
+    // The status word once more (`gone` was read while an earlier launch may still have been running): behind one
+    // that gave up the state stays as it is. The read runs under the last MMAs.
     auto wait_o = [&]() {
+      const int lost = *reinterpret_cast<volatile int*>(a.status);
       if (ok && n_own > 0 && (!kSplit || w < live))
         ok = mbar_wait(bar_o_done + 8 * w, (C::kEarlyS || C::kDoubleS) ? ((n_own - 1) & 1) : 0,
                        abort_flag, a.status, 8, n_own, a.wait_ns);
@@ -992,7 +997,7 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit, kFold>::kTh
       if constexpr (kFold) {
         if (ok && w < live && n_own == 0) ok = mbar_wait(bar_q_full + 8 * w, 0, abort_flag, a.status, 3, w, a.wait_ns);
       }
-      ok = __all_sync(0xffffffffu, ok);
+      ok = __all_sync(0xffffffffu, ok && lost == 0);
       tc_fence_after();
       return ok;
     };
