@@ -976,7 +976,7 @@ __global__ void __launch_bounds__(kThreadsF, 1)
         l_old = a.l[grow];
       }
       RowStore<DR>::run(
-          a.out, grow0 + w * kBM + row - lane, __ballot_sync(0xffffffffu, row_valid),
+          lane, a.out, grow0 + w * kBM + row - lane, __ballot_sync(0xffffffffu, row_valid),
           s_base + C::kOffStage + w * C::kRowStage + (warp & 3) * RowStore<DR>::kStageBytes, t_o, mine, fresh, wait_o, [&]() {
             const bool have = row_valid && mine && m_ref > -INFINITY;
             const float m_new = have ? m_ref * kLn2 : -INFINITY;  // natural-log units

@@ -1019,8 +1019,14 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit, kFold>::kTh
       // (the rows are staged over their own query tile, which no copy writes and no MMA reads any more behind wait_o;
       // every warp has a quarter)
       static_assert(4 * RowStore<DR>::kStageBytes <= C::kTileBytes, "staging of the rows");
+      // (At head_dim 128 the lane comes from its register, volatile: what hangs on an index from threadIdx the compiler
+      // works out in front of the tile loop and carries through it in registers that the softmax lacks. Spill stores /
+      // loads 72 / 116 -> 64 / 80 bytes; us a pass B2 H32/kvH8 S32768 causal 16318 -> 15891, with one row per lane 16048;
+      // 2048 x 2048 dense H16 54.2 -> 53.0. The other forms spill no less and gain nothing.)
+      int lane_out = lane;
+      if constexpr (D == 128 && !kFold) asm volatile("mov.u32 %0, %%laneid;" : "=r"(lane_out));
       RowStore<DR>::run(
-          a.out, grow0, __ballot_sync(0xffffffffu, row_valid),
+          lane_out, a.out, grow0, __ballot_sync(0xffffffffu, row_valid),
           s_q + w * C::kTileBytes + (warp & 3) * RowStore<DR>::kStageBytes, t_o, n_own > 0, fresh, wait_o, [&]() {
             const bool have = row_valid && n_own > 0 && m_ref > -INFINITY;
             const float m_new = have ? m_ref * kLn2 : -INFINITY;  // natural-log units

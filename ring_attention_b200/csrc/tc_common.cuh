@@ -621,9 +621,8 @@ struct RowStore {
   static constexpr int kBatch = kChunks < 16 ? kChunks : 16;
   static constexpr int kStageBytes = 32 * kCols * 4;
   template <typename Wait, typename Row>
-  __device__ static inline bool run(float* out, size_t grow0, unsigned valid_rows, unsigned stage, unsigned t_o,
+  __device__ static inline bool run(int lane, float* out, size_t grow0, unsigned valid_rows, unsigned stage, unsigned t_o,
                                     bool worked, bool fresh, Wait wait_o, Row row_out) {
-    const int lane = static_cast<int>(threadIdx.x & 31);
     const int sub = lane / kChunks, chunk = lane % kChunks;
     float4 old[kBatch];
     auto row_of = [&](int i) { return i * kRowsPer + sub; };
