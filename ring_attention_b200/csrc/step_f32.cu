@@ -310,6 +310,8 @@ __global__ void __launch_bounds__(kThreadsF, 1)
       if (lane == 0 && n_tiles > 0) {
         int it = 0;
         bool ok = *abort_flag == 0;
+        // (the status word once more, see step_tc.cu: behind a launch that gave up no V comes)
+        const int lost = *reinterpret_cast<volatile int*>(a.status);
         TileShare share{share_beg, share_end, 0};
         for (int sk = 0; sk < a.kmap.n_seg && ok; ++sk) {
           const TileRange r =
@@ -318,6 +320,11 @@ __global__ void __launch_bounds__(kThreadsF, 1)
             const int k_row = a.kseg_row[sk] + t * kBNf;
             const int k_head = a.kseg_head[sk] + kv_bh;
             for (int which = 0; which < 2 && ok; ++which, ++it) {
+              if (which == 1 && lost != 0) {
+                *abort_flag = 1;
+                ok = false;
+                break;
+              }
               const int slot = it % C::kStages;
               if (it >= C::kStages)
                 ok = mbar_wait(bar_kv_empty + 8 * slot, ((it / C::kStages) + 1) & 1, abort_flag,
@@ -954,12 +961,10 @@ __global__ void __launch_bounds__(kThreadsF, 1)
     }
 
     // ---------------------------------------------------------------- epilogue ----
-    // (the status word once more, see step_tc.cu: behind a launch that gave up the state stays as it is)
     auto wait_o = [&]() {
-      const int lost = *reinterpret_cast<volatile int*>(a.status);
       if (ok && mine)
         ok = mbar_wait(bar_o_done + 8 * w, (n_tiles - 1) & 1, abort_flag, a.status, 8, n_tiles, a.wait_ns);
-      ok = __all_sync(0xffffffffu, ok && lost == 0);
+      ok = __all_sync(0xffffffffu, ok);
       if (ok && mine) tc_fence_after();
       return ok;
     };

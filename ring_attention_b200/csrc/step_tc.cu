@@ -59,7 +59,7 @@
 // Every wait on an mbarrier is bounded: when one runs out the block records where in the
 // device status word, all roles leave their loops, tensor memory is freed and the kernel
 // returns. Later blocks see the status word and return at once; blocks that read it before it was set (those
-// of the next launch, which overlap this one) run, see it at their end and leave the state as it is.
+// of the next launch, which overlap this one) see it in front of their first V and leave the state as it is.
 #include <atomic>
 
 #include "tc_common.cuh"
@@ -365,7 +365,7 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit, kFold>::kTh
   tc_fence_after();
   const unsigned tmem_base = *tmem_slot;
   // Everything so far touched no memory but the status word. A word that is set says to leave; one that is not may
-  // yet be set by a launch before this one, so it is read again before the state is written.
+  // yet be set by a launch before this one, so the producer reads it again.
   wait_for_previous();
   if (leave) {
     if (warp == 1)
@@ -381,6 +381,10 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit, kFold>::kTh
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer ----
     if (lane == 0 && n_tiles > 0) {
+      // The status word once more: `gone` was read while an earlier launch may still have been running. Behind one that
+      // gave up no V comes, and the block unwinds without a store. (Read here, looked at in front of a V: nothing waits
+      // for it. Read by the softmax warps under the last MMAs it cost a call 0.15 to 0.4 us.)
+      const int lost = *reinterpret_cast<volatile int*>(a.status);
       for (int w = 0; w < live; ++w) {
         const int q_row = tile_sq(w) * q_seg_len + tile_row0(w);
         mbar_expect_tx(bar_q_full + 8 * w, C::kTileBytes);
@@ -392,6 +396,10 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit, kFold>::kTh
       bool ok = true;
       // all ring items of one operand (which: 0 = K, 1 = V) of key tile `tile`
       auto load_items = [&](int which, int tile, int k_row, int k_head) {
+        if (which == 1 && lost != 0) {
+          *abort_flag = 1;
+          ok = false;
+        }
         for (int sub = 0; sub < C::kItemsPerTile && ok; ++sub, ++it) {
           const RingPos pos = ring_pos<C>(which, tile, sub);
           const int slot = pos.slot;
@@ -985,19 +993,19 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit, kFold>::kTh
     }
 
     // ---------------------------------------------------------------- epilogue ----
-    // The status word once more (`gone` was read while an earlier launch may still have been running): behind one
-    // that gave up the state stays as it is. The read runs under the last MMAs.
     auto wait_o = [&]() {
-      const int lost = *reinterpret_cast<volatile int*>(a.status);
       if (ok && n_own > 0 && (!kSplit || w < live))
         ok = mbar_wait(bar_o_done + 8 * w, (C::kEarlyS || C::kDoubleS) ? ((n_own - 1) & 1) : 0,
                        abort_flag, a.status, 8, n_own, a.wait_ns);
-      // a light tile without keys: no MMA has read its Q, whose copy may still be on its way to the place
-      // where the rows are staged
+      // A light tile without keys: no MMA has read its Q, whose copy may still be on its way to the place where the
+      // rows are staged, and no V has to come, so it looks at the status word itself (see the producer).
       if constexpr (kFold) {
-        if (ok && w < live && n_own == 0) ok = mbar_wait(bar_q_full + 8 * w, 0, abort_flag, a.status, 3, w, a.wait_ns);
+        if (ok && w < live && n_own == 0) {
+          const int lost = *reinterpret_cast<volatile int*>(a.status);
+          ok = mbar_wait(bar_q_full + 8 * w, 0, abort_flag, a.status, 3, w, a.wait_ns) && lost == 0;
+        }
       }
-      ok = __all_sync(0xffffffffu, ok && lost == 0);
+      ok = __all_sync(0xffffffffu, ok);
       tc_fence_after();
       return ok;
     };
