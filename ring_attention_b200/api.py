@@ -34,13 +34,11 @@ class AttentionShape:
         return Shape(self.batch, self.heads, self.seq_q, self.seq_k, self.head_dim, self.kv_heads)
 
 
-# The handle of torch.cuda.current_stream(), without the two objects that call builds around it: they
-# cost more than 1 us of the 9 that a decode call on a short context took.
-_current_device, _raw_stream = torch._C._cuda_getDevice, torch._C._cuda_getCurrentRawStream
-
-
 def _stream():
-    return _raw_stream(_current_device())
+    # The handle of torch.cuda.current_stream(), without the two objects that call builds around it: they cost more
+    # than 1 us of the 9 that a decode call on a short context took. (Looked up at the call: a torch without CUDA
+    # lacks both names, and the partition helpers below ask for no GPU.)
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _ptr(t):

@@ -4,6 +4,8 @@ oracle. No compute call is made here."""
 import ctypes as C
 import os
 import re
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -185,3 +187,15 @@ def test_a_cache_append_across_devices_stays_with_the_copies(cache, stream, k, v
     # a kernel on device 1 must not touch what only a copy can reach
     assert lib().ra_debug_append_route(1, 1, 1, 1, 1) == 1
     assert lib().ra_debug_append_route(1, cache, stream, k, v) == 0
+
+
+def test_the_partition_helpers_need_no_torch_with_cuda():
+    # a CPU build of torch has neither of the two names that the GPU calls get their stream from
+    code = ("import torch\n"
+            "for name in ('_cuda_getDevice', '_cuda_getCurrentRawStream'):\n"
+            "    if hasattr(torch._C, name): delattr(torch._C, name)\n"
+            "from ring_attention_b200 import api\n"
+            "print(api.RingPartition(4, 1, 64, 1, 2).step_maps(0)[2])\n")
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, cwd=ROOT)
+    assert r.returncode == 0, r.stderr
+    assert r.stdout.split() == ["1"]
