@@ -90,6 +90,9 @@ RA_API void ra_debug_stall_producer_after(int items);
  * k; ignored unless k divides batch * kv_heads). Lets a test run every order on a small shape.
  * Process-wide; not for production use. */
 RA_API void ra_debug_set_block_order(int order);
+/* The form that the calling thread's last tensor-core step took: bits 0-3 the blocks that share a
+ * query block's keys, 16 folded query tiles, 32 cluster pairs, 64 P in shared memory. For tests. */
+RA_API int ra_debug_step_form(void);
 /* Whether ra_kv_cache_append takes a token's rows by its kernel (1) or by device copies (0), given the
  * current device and those of the cache, the stream and the two sources (-1: not device memory). */
 RA_API int ra_debug_append_route(int device, int cache_device, int stream_device, int k_device, int v_device);

@@ -12,6 +12,7 @@ namespace rab {
 void set_tc_wait_limit_ns(unsigned long long ns);
 void set_tc_stall_after(int items);
 void set_tc_block_order(int order);
+int step_form();
 
 namespace {
 
@@ -226,6 +227,7 @@ RA_API int ra_attention_step_path(int dtype, int head_dim) {
 RA_API void ra_debug_set_wait_limit_ns(unsigned long long ns) { rab::set_tc_wait_limit_ns(ns); }
 RA_API void ra_debug_stall_producer_after(int items) { rab::set_tc_stall_after(items); }
 RA_API void ra_debug_set_block_order(int order) { rab::set_tc_block_order(order); }
+RA_API int ra_debug_step_form(void) { return rab::step_form(); }
 
 
 /* ------------------------------------------------ whole attention, device buffers ---- */

@@ -1028,6 +1028,7 @@ int launch_f32(const StepArgs& a, cudaStream_t stream, int key_split) {
   TcArgs t;
   t.kv_per_wave = 0;
   t.key_split = key_split;
+  set_step_form(key_split);
   t.out = a.out;
   t.m = a.m;
   t.l = a.l;

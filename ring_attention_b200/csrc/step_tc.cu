@@ -1082,6 +1082,7 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit, kFold>::kTh
 std::atomic<unsigned long long> g_wait_ns{kWaitLimitNs};
 std::atomic<int> g_stall_after{-1};
 std::atomic<int> g_block_order{-1};  // -1: by shape, 0: heads fastest, k > 0: waves of k KV heads
+thread_local int g_form = 0;         // of the calling thread's last launch, see ra_debug_step_form
 
 template <int D, bool kBf16, bool kPInTmem, int DR, bool kPair = false, bool kSplit = false, bool kFold = false>
 int launch_cfg(const StepArgs& a, cudaStream_t stream, int key_split = 1) {
@@ -1158,6 +1159,7 @@ int launch_cfg(const StepArgs& a, cudaStream_t stream, int key_split = 1) {
   if (kSplit || kFold) kv_per_wave = 0;
   t.kv_per_wave = kv_per_wave;
   t.key_split = key_split;
+  set_step_form(key_split | (kFold ? 16 : 0) | (kPair ? 32 : 0) | (kPInTmem ? 0 : 64));
   const long long bh_total = static_cast<long long>(a.B) * a.H;
   const long long per_x = kv_per_wave > 0 ? static_cast<long long>(a.H / a.kvH) * kv_per_wave : 0;
   RAB_REQUIRE(kv_per_wave > 0 ? n_qblocks * per_x < (1ll << 31) : n_qblocks <= 65535, RA_ERR_INVALID,
@@ -1290,6 +1292,7 @@ int launch_step_tc(int dtype, const StepArgs& a, cudaStream_t stream) {
 namespace tcgen {
 unsigned long long tc_wait_limit_ns() { return g_wait_ns.load(std::memory_order_relaxed); }
 int tc_stall_after() { return g_stall_after.load(std::memory_order_relaxed); }
+void set_step_form(int form) { g_form = form; }
 ClusterSlots& cluster_slots_of(int device) {
   static ClusterSlots tables[64];
   return tables[device];
@@ -1301,6 +1304,7 @@ void set_tc_wait_limit_ns(unsigned long long ns) {
 }
 void set_tc_stall_after(int items) { g_stall_after.store(items, std::memory_order_relaxed); }
 void set_tc_block_order(int order) { g_block_order.store(order, std::memory_order_relaxed); }
+int step_form() { return g_form; }
 
 
 }  // namespace rab

@@ -884,6 +884,8 @@ inline bool fold_rows(const StepArgs& a, double alone, double tiles) {
 // Limits set through the test hooks (step_tc.cu owns them).
 unsigned long long tc_wait_limit_ns();
 int tc_stall_after();
+// What ra_debug_step_form answers on this thread.
+void set_step_form(int form);
 
 }  // namespace tcgen
 }  // namespace rab

@@ -533,7 +533,7 @@ def test_marked_tiles_in_a_cache_with_segments_strides_and_grouped_heads(D, spli
     (36, 1000, [0], [0], 1000, 1),                    # eight tiles, the last one short
     (28, 1100, [0], [0], 1100, 1),                    # nine: the middle one alone
     (16, 1021, [1021, 6126], [1021, 6126], 1021, 1),  # a zig-zag rank's own shard
-    (48, 600, [300], [0], 900, 1),                    # rows behind a cache
+    (48, 600, [200], [0], 800, 1),                    # rows behind a cache
     (40, 700, [0], [350], 700, 1),                    # the first tiles see no key
     (32, 1000, [1], [0], 1000, 2),                    # striped
 ])
@@ -550,11 +550,35 @@ def test_light_and_heavy_query_tiles_share_a_block(dtype, D, heads, rows, qbases
         for i, qi in enumerate((q, -q)):
             api.attention_step_ex(qi, k, v, *state, shape, SegMap.make(qbases, rows), SegMap.make(kbases, seg_k),
                                   pos_stride=stride, causal=True, fresh=i == 0, finalize=i == 1, key_split=split)
+            assert lib().ra_debug_step_form() == (1 if split else 1 | 16)
         results.append(state)
     torch.cuda.synchronize()
     assert api.device_status()[0] == 0
     for a, b in zip(*results):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("D", [32, 64, 128])
+@pytest.mark.parametrize("heads,rows,qbases,kbases,seg_k,stride", [
+    (28, 1100, [0], [0], 1100, 1), (16, 1021, [1021, 6126], [1021, 6126], 1021, 1), (32, 1000, [1], [0], 1000, 2)])
+def test_folded_calls_match_64_bits(dtype, D, heads, rows, qbases, kbases, seg_k, stride):
+    kvH = heads // 2
+    Sq, Sk = rows * len(qbases), seg_k * len(kbases)
+    q, k, v = (round_to(x, dtype) for x in normal_inputs(23, 1, heads, kvH, Sq, Sk, D))
+    state = poisoned(1, heads, Sq, D)
+    api.attention_step_ex(dev(q, dtype), dev(k, dtype), dev(v, dtype), *state, api.AttentionShape(1, heads, Sq, Sk, D, kvH),
+                          SegMap.make(qbases, rows), SegMap.make(kbases, seg_k), pos_stride=stride, causal=True, fresh=True,
+                          finalize=True)
+    assert lib().ra_debug_step_form() == 1 | 16
+    lse = api.attention_lse(state[1], state[2]).cpu().numpy()
+    assert api.device_status()[0] == 0
+    qpos, kpos = (np.concatenate([b + stride * np.arange(n) for b in bases]) for bases, n in ((qbases, rows), (kbases, seg_k)))
+    some = [0, heads // 2 + 1]  # (a head of either half; query head h reads KV head h % kvH)
+    kv = [h % kvH for h in some]
+    want, want_lse = _in_64_bits(q[:, some], k[:, kv], v[:, kv], qpos, kpos, True, 0)
+    assert_close(state[0].cpu().numpy()[:, some], want, TOL[dtype], TOL[dtype], "out")
+    assert_close(lse[:, some], want_lse, 1e-5, 1e-5, "lse")
 
 
 @pytest.mark.parametrize("dtype,D", [(torch.float16, 32), (torch.float16, 64), (torch.bfloat16, 128), (torch.float16, 256),
@@ -621,6 +645,7 @@ def test_light_query_tiles_without_keys(dtype, D, fresh, finalize):
     state = [torch.empty_like(t) for t in before]
     for i in range(60):
         call(state, 0)
+        assert lib().ra_debug_step_form() == 1 | 16
         if i % 3 == 0:
             torch.cuda.synchronize()
         assert all(torch.equal(a, b) for a, b in zip(state, want)), i
