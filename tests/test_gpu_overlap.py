@@ -65,3 +65,61 @@ def test_back_to_back_is_what_waiting_gives(dtype, d, rows):
         for a, b in zip(got, want):
             assert torch.equal(a, b)
     assert api.device_status()[0] == 0
+
+
+def dependent_calls(dtype, d, heads, wait):
+    """Calls of which each needs what the one before it wrote (or must not yet overwrite what that one reads),
+    everything prepared beforehand, so that no other kernel stands between two of them. Few blocks that
+    walk long: most SMs are free for the next call's blocks all the while."""
+    def done():
+        if wait:
+            torch.cuda.synchronize()
+
+    B, kvH, rows, keys, n = 1, heads // 2, 300, 3000, 6
+    g = torch.Generator(device="cuda").manual_seed(d + heads)
+
+    def normal(*shape, dt=dtype):
+        return torch.randn(*shape, generator=g, device="cuda").to(dt)
+
+    q, k, v = [normal(B, heads, rows, d) for _ in range(3)], [normal(B, kvH, keys, d) for _ in range(3)], \
+        [normal(B, kvH, keys, d) for _ in range(3)]
+    out = torch.full((B, heads, rows, d), float("nan"), device="cuda")
+    m, l = (torch.full((B, heads, rows), float("nan"), device="cuda") for _ in range(2))
+    shape = api.AttentionShape(B, heads, rows, keys, d, kvH)
+    maps = api.SegMap.make([3 * keys], rows), [api.SegMap.make([i * keys], keys) for i in range(3)]
+    f = [[normal(B, h, s, d, dt=torch.float32) for h, s in ((heads, rows), (kvH, keys), (kvH, keys))] for _ in range(3)]
+    flash = [torch.empty(B, heads, rows, d, device="cuda") for _ in range(3)]
+    cache = api.DeviceKVCache(B, kvH, keys + n, d, dtype)
+    cache.k_view().fill_(float("nan"))
+    cache.v_view().fill_(float("nan"))
+    cache.copy_prefill(k[0], v[0], keys)
+    new = [(normal(B, heads, 1, d), normal(B, kvH, 1, d), normal(B, kvH, 1, d)) for _ in range(n)]
+    tokens = [torch.full((B, heads, 1, d), float("nan"), device="cuda") for _ in range(n)]
+    torch.cuda.synchronize()
+    for i in range(3):
+        api.attention_step_ex(q[i], k[i], v[i], out, m, l, shape, maps[0], maps[1][i], causal=True, fresh=i == 0,
+                              finalize=i == 2)
+        done()
+    lse = api.attention_lse(m, l)
+    done()
+    for i in range(3):  # (the fp16 copies of one call and the next lie in the same memory)
+        api.launch_flash_attention_fp16(*f[i], flash[i], shape, True)
+        done()
+    for i in range(n):
+        cache.append(new[i][1], new[i][2])
+        done()
+        api.run_local_decode_step(new[i][0], cache, heads, keys + i, 0, True, tokens[i])
+        done()
+    torch.cuda.synchronize()
+    return [out, lse, *flash, *tokens]
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("d", [32, 64, 128, 256])
+@pytest.mark.parametrize("heads", [4, 32])
+def test_dependent_calls_with_nothing_between_them(dtype, d, heads):
+    want = dependent_calls(dtype, d, heads, True)
+    assert all(torch.isfinite(t).all() for t in want)
+    for _ in range(3):
+        assert all(torch.equal(a, b) for a, b in zip(dependent_calls(dtype, d, heads, False), want))
+    assert api.device_status()[0] == 0
