@@ -1045,9 +1045,9 @@ int run_plan(const ra_shape& s, int head_batches, int stages, size_t stage_bytes
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   if (p.cluster) {
     // Blocks that start beside those of the kernel before go where there is room, two to an SM while
-    // others stay empty; so only calls whose blocks leave half of the SMs free overlap it. us per call in a
-    // row, launched behind / beside: 64 blocks (B1 kvH8 D128 fp16, 1061 rows) 7.2 / 6.9, 240 blocks (B5 kvH6 D64
-    // bf16, 1531 rows) 7.2 / 8.3.
+    // others stay empty; so only calls whose blocks leave half of the SMs free overlap it. 157 shapes of 1 to 48 KV
+    // heads, 300 to 4000 rows, D64 and D128, fp16 and fp32, calls in a row in a CUDA graph, time beside / behind: up to
+    // 74 blocks 0.94 in the median (0.89 to 1.04), 75 to 148 blocks 1.02 (0.94 to 1.23), more 1.00 (0.96 to 1.18).
     cfg.attrs = attr;
     cfg.numAttrs = 2 * p.deal.groups * p.cluster <= sm_count() ? 2 : 1;
     cfg.gridDim = dim3(p.cluster, p.deal.groups);

@@ -61,6 +61,7 @@
 // returns. Later blocks see the status word and return at once; blocks that read it before it was set (those
 // of the next launch, which overlap this one) see it in front of their first V and leave the state as it is.
 #include <atomic>
+#include <climits>
 
 #include "tc_common.cuh"
 
@@ -778,7 +779,15 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit, kFold>::kTh
     const long long qdoc = a.doc_len > 0 ? qpos / a.doc_len : 0;
     const float scale_log2 = rsqrtf(static_cast<float>(DR)) * kLog2e;
 
-    float m_ref = -INFINITY;  // reference point of P, O and l, log2 units (see the tile loop)
+    // Reference point of P, O and l, log2 units (see the tile loop). A row behind the end of its segment (of a ragged
+    // last tile) is worked as one that sees every key with a reference above all scores, so that its P is 0. With its
+    // keys hidden it took its warp through the masked path in every tile, and the other tile of a folded block, or of
+    // one warp that issues for both, waited for that. us per call: folded 2 x 2226 rows H8 D64 67.7 -> 48.9 (neighbours
+    // 59.5), 1531 rows B2 H12 D64 27.9 -> 21.1; head_dim 128, 951 rows on 3212 keys H32/kvH8 73.1 -> 54.8 (two issuers 69.2),
+    // 2 x 2459 rows H8 112.8 -> 79.9 (103.9). Not in the key split at head_dim 128: 200 rows on 40000 keys H8 would take 86
+    // instead of 108, but short calls 0.5 more (900 rows H2 13.9 / 14.5, 4000 keys 21.2 / 22.1).
+    constexpr bool kAllSee = !(kSplit && D == 128);
+    float m_ref = kAllSee && !row_valid ? 1e30f : -INFINITY;
     float l_run = 0.f;
     bool ok = true;
 
@@ -794,7 +803,7 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit, kFold>::kTh
       // Keys of this segment the row can see are the local indices [rel_lo, rel_hi): causal
       // and document limits are affine in the key index, so they are worked out once per
       // segment (64-bit divisions) and the per-tile work is two 32-bit clamps.
-      int rel_lo = 0, rel_hi = row_valid ? a.kmap.seg_len : 0;
+      int rel_lo = 0, rel_hi = kAllSee || row_valid ? a.kmap.seg_len : 0;
       {
         const long long kb = a.kmap.base[sk];
         if (causal) {
@@ -813,6 +822,7 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit, kFold>::kTh
           }
         }
       }
+      if (kAllSee && !row_valid) rel_lo = 0, rel_hi = INT_MAX;
       for (int t = tr.lo; t < tr.hi && ok; ++t, ++j) {
         // Visible columns of this row in this tile: [c_lo, c_hi), from the segment's bounds.
         int c_lo = min(max(rel_lo - t * kBN, 0), kBN);

@@ -607,40 +607,41 @@ struct RowOut {
 
 // The end of a block that merges with nobody: 32 rows of O from tensor memory into the state, run by one
 // warp (lane = row). A row per lane would touch 32 rows with every load and store, 16 bytes each; so the
-// rows go through shared memory (`stage`: kStageBytes of this warp, swizzled 16-byte chunks, half the
-// columns at a time) and the state is read and written whole 128-byte pieces at a time. The old state
+// rows go through shared memory (`stage`: kStageBytes of this warp, swizzled 16-byte chunks, at most 64
+// columns at a time, 128 take half again as long) and the state is read and written in pieces of 128 bytes and more. The old state
 // does not depend on the MMAs still running: its first loads are issued before wait_o(), which returns whether O is
 // there, and row_out() says what becomes of this lane's row. us per call with one key tile, 128 blocks of 256 rows, a
-// row per lane -> so: head_dim 64 into a new state 8.5 -> 7.7, into an old one 11.3 -> 7.9; head_dim 128 11.9 -> 10.1,
-// 16.9 -> 10.6.
+// row per lane -> so: head_dim 64 into a new state 8.6 -> 7.8, into an old one 11.5 -> 8.2; head_dim 128 12.0 -> 10.1,
+// 17.1 -> 10.7; head_dim 256 (128 rows) 12.4 -> 10.2, 17.9 -> 11.3. With few rows the stores of a row per lane are few too:
+// fp32 head_dim 128, 20 rows into a new state 8.6 -> 9.6, 128 rows 12.6 -> 11.8.
 template <int DR>
 struct RowStore {
-  static constexpr int kCols = DR > 64 ? DR / 2 : 32;   // columns of a pass
+  static constexpr int kCols = DR > 64 ? 64 : 32;       // columns of a pass
   static constexpr int kChunks = kCols / 4;             // 16-byte chunks of a row
   static constexpr int kRowsPer = 32 / kChunks;         // rows that one access of the warp covers
-  static constexpr int kBatch = kChunks < 16 ? kChunks : 16;
   static constexpr int kStageBytes = 32 * kCols * 4;
   template <typename Wait, typename Row>
   __device__ static inline bool run(int lane, float* out, size_t grow0, unsigned valid_rows, unsigned stage, unsigned t_o,
                                     bool worked, bool fresh, Wait wait_o, Row row_out) {
     const int sub = lane / kChunks, chunk = lane % kChunks;
-    float4 old[kBatch];
+    float4 old[kChunks];
     auto row_of = [&](int i) { return i * kRowsPer + sub; };
     auto at = [&](int pass, int i) {
       return reinterpret_cast<float4*>(out + (grow0 + row_of(i)) * DR + pass * kCols + chunk * 4);
     };
-    auto load_old = [&](int pass, int i0) {
+    auto load_old = [&](int pass) {
 #pragma unroll
-      for (int i = 0; i < kBatch; ++i)
-        old[i] = !fresh && (valid_rows >> row_of(i0 + i) & 1u) ? *at(pass, i0 + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int i = 0; i < kChunks; ++i)
+        old[i] = !fresh && (valid_rows >> row_of(i) & 1u) ? *at(pass, i) : make_float4(0.f, 0.f, 0.f, 0.f);
     };
-    load_old(0, 0);
+    load_old(0);
     if (!wait_o()) return false;
     const RowOut ro = row_out();
     const unsigned touched = __ballot_sync(0xffffffffu, ro.touch);
+    if (touched == 0) return true;
 #pragma unroll 1
     for (int pass = 0; pass < DR / kCols; ++pass) {
-      if (pass > 0) load_old(pass, 0);
+      if (pass > 0) load_old(pass);
 #pragma unroll
       for (int c = 0; c < kCols / 32; ++c) {
         float o[32];
@@ -661,25 +662,21 @@ struct RowStore {
         }
       }
       __syncwarp();
-#pragma unroll 1
-      for (int i0 = 0; i0 < kChunks; i0 += kBatch) {
-        if (i0 > 0) load_old(pass, i0);
 #pragma unroll
-        for (int i = 0; i < kBatch; ++i) {
-          const int r = row_of(i0 + i);
-          const float f = __shfl_sync(0xffffffffu, ro.f_old, r);
-          float4 v;
-          asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
-                       : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-                       : "r"(stage + r * (kCols * 4) + ((chunk ^ (r & 7)) << 4)));
-          if (!fresh) {
-            v.x += f * old[i].x;
-            v.y += f * old[i].y;
-            v.z += f * old[i].z;
-            v.w += f * old[i].w;
-          }
-          if (touched >> r & 1u) *at(pass, i0 + i) = v;
+      for (int i = 0; i < kChunks; ++i) {
+        const int r = row_of(i);
+        const float f = __shfl_sync(0xffffffffu, ro.f_old, r);
+        float4 v;
+        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                     : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                     : "r"(stage + r * (kCols * 4) + ((chunk ^ (r & 7)) << 4)));
+        if (!fresh) {
+          v.x += f * old[i].x;
+          v.y += f * old[i].y;
+          v.z += f * old[i].z;
+          v.w += f * old[i].w;
         }
+        if (touched >> r & 1u) *at(pass, i) = v;
       }
       __syncwarp();
     }
