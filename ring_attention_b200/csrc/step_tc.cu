@@ -784,9 +784,10 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit, kFold>::kTh
     // keys hidden it took its warp through the masked path in every tile, and the other tile of a folded block, or of
     // one warp that issues for both, waited for that. us per call: folded 2 x 2226 rows H8 D64 67.7 -> 48.9 (neighbours
     // 59.5), 1531 rows B2 H12 D64 27.9 -> 21.1; head_dim 128, 951 rows on 3212 keys H32/kvH8 73.1 -> 54.8 (two issuers 69.2),
-    // 2 x 2459 rows H8 112.8 -> 79.9 (103.9). Not in the key split at head_dim 128: 200 rows on 40000 keys H8 would take 86
-    // instead of 108, but short calls 0.5 more (900 rows H2 13.9 / 14.5, 4000 keys 21.2 / 22.1).
-    constexpr bool kAllSee = !(kSplit && D == 128);
+    // 2 x 2459 rows H8 112.8 -> 79.9 (103.9). Not in the key split, whose short calls at head_dim 128 it cost 0.5 (900 rows
+    // H2 13.9 / 14.5) and its long ones at head_dim 64 6 % (B5 H16/kvH4, 396 rows on 50774 keys 1098 / 1174), nor at head_dim 64
+    // with neighbours (B1 H8 S32768 causal 1422 / 1474): there the tile loop comes out slower for all rows.
+    constexpr bool kAllSee = !kSplit && kPInTmem && (kFold || D >= 128);
     float m_ref = kAllSee && !row_valid ? 1e30f : -INFINITY;
     float l_run = 0.f;
     bool ok = true;
