@@ -122,6 +122,12 @@ struct F32Cfg {
   static constexpr bool kOwnStage = !kSplit && kQBytes < kRowStage;
   static constexpr int kOffStage = kOwnStage ? (kOffMl + 15) & ~15 : kOffQ;
   static constexpr int kSmemBytes = kOwnStage ? kOffStage + kTiles * kRowStage : kOffMl + kMlBytes;
+  // Registers of a thread of the producer / issuing, the softmax and the splitting warps; 640 threads start with 96
+  // each, 61440 in all. Head_dim 128 spills 60 bytes so and 128 with 40 / 144 / 72: us per call B1 H4 S16384 causal 828 /
+  // 848. The others spill next to nothing either way and gain from registers for the splitters: H8 S8192 D64 242 (247 with
+  // the split of head_dim 128), H16/kvH8 978 rows on 5874 keys D32 93.8 (97.0).
+  static constexpr int kRegsIssue = D == 128 ? 64 : 40, kRegsSoftmax = D == 128 ? 152 : 144, kRegsSplit = D == 128 ? 56 : 72;
+  static_assert(128 * kRegsIssue + 256 * kRegsSoftmax + 256 * kRegsSplit <= 640 * 96, "setmaxnreg draws on the launch's registers");
   static constexpr int kColS = 0, kColP = kAlias ? 0 : 64, kColO = kAlias ? 64 : 128, kColQ = 192;
   static_assert(kSmemBytes <= 232448, "shared memory budget");
   static_assert(kTiles * kBM * ((DR + 4) * 4 + 8) <= kOffBar, "staging of the key-split merge");
@@ -301,10 +307,9 @@ __global__ void __launch_bounds__(kThreadsF, 1)
     return;
   }
 
-  // Registers: 640 threads start with 96 each (61440 in all); 128 * 64 + 256 * 152 + 256 * 56 = 61440. (With 40 /
-  // 144 / 72 the issuing warp and the softmax spilled 132 bytes, now 60: B1 H4 S16384 D128 848 -> 828 us.)
+  // (registers follow the work, see F32Cfg)
   if (warp < 4) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::kRegsIssue));
     if (warp == 0) {
       // ---------------------------------------------------------- TMA producer ----
       if (lane == 0 && n_tiles > 0) {
@@ -459,7 +464,7 @@ __global__ void __launch_bounds__(kThreadsF, 1)
       for (int i = 0; i < 3; ++i) cluster_sync_threads();
     }
   } else if (warp >= 12) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::kRegsSplit));
     // --------------------------------------------------------------- splitters ----
     // A warp owns eight rows of every tile; its lanes own 16-byte pieces of the split rows (8
     // values, 32 raw bytes): lane = (piece, row), so the eight lanes of a phase touch eight rows
@@ -607,7 +612,7 @@ __global__ void __launch_bounds__(kThreadsF, 1)
       for (int i = 0; i < 3; ++i) cluster_sync_threads();
     }
   } else {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 152;");
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(C::kRegsSoftmax));
     // ----------------------------------------------------------------- softmax ----
     const int w = (warp - 4) >> 2;
     const int row = ((warp & 3) << 5) + lane;  // row of the tile = tensor-memory lane
