@@ -34,11 +34,15 @@ class AttentionShape:
         return Shape(self.batch, self.heads, self.seq_q, self.seq_k, self.head_dim, self.kv_heads)
 
 
+# The handle of torch.cuda.current_stream(), without the two objects that call builds around it: they cost more than
+# 1 us of the 9 that a decode call on a short context took. (A torch without CUDA lacks both names, and the
+# partition helpers below ask for no GPU.)
+_current_device = getattr(torch._C, "_cuda_getDevice", None)
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream():
-    # The handle of torch.cuda.current_stream(), without the two objects that call builds around it: they cost more
-    # than 1 us of the 9 that a decode call on a short context took. (Looked up at the call: a torch without CUDA
-    # lacks both names, and the partition helpers below ask for no GPU.)
-    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+    return _raw_stream(_current_device())
 
 
 def _ptr(t):
