@@ -49,7 +49,7 @@ const char* last_error();
 // runs: its blocks fill the SMs that are free already and do what touches no memory (barriers, tensor
 // memory, index arithmetic). It calls wait_for_previous, in every block, before its first access to
 // memory that an earlier launch may write or read; that returns once everything before it in the stream has
-// completed and is visible. Loads that must stay behind the wait go through plain pointers: the
+// completed and is visible. (The step kernels look at the status word before it, and once more behind it.) Loads that must stay behind the wait go through plain pointers: the
 // compiler may move those of a const __restrict__ one. let_next_start allows the next overlapped launch
 // to do the same, once every block of this kernel has called it or left: the next one's blocks never take
 // a place that a block of this one still needs. Measured, us a pass back to back, plain launches -> overlapped:

@@ -44,10 +44,12 @@
 //
 // Tensor memory, 256 columns per query tile: S [0,64) P hi [64,96) P lo [96,128) O [128,192) Q hi
 // [192,224) Q lo [224,256); head_dim 128: S and P [0,64) O [64,192) Q hi [192,256).
-// What bounds it: at head_dim 128 a pair of tiles of 64 keys takes 5200 clocks, of which its MMAs need 3400;
-// the two softmax groups (1500 to 1900 clocks a tile) run under the other tile's MMAs, and the issuing warp finds P
-// written when it comes to it. Measured, us per call, against one 128-row tile per block on TF32 pairs:
-// B1 H4 S16384 D128 causal 830 (2700), B1 H8 S1024 D64 dense 20.6 (37), H4/kvH1 8231 x 9075 rows D64 causal 164 (272).
+// What bounds it: at head_dim 128 a pair of tiles of 64 keys takes 5200 clocks, of which its MMAs need 3400. The
+// two softmax groups (1500 to 1900 clocks a tile) run under the other tile's MMAs, and the issuing warp finds P
+// written when it comes to it, so in the other 1800 clocks the tensor core has no MMA although nothing it
+// waits for is missing: why is not known. Tensor pipe 58 %, issue slots 48 % (B1 H8 S8192 causal). Measured, us per
+// call, against one 128-row tile per block on TF32 pairs: B1 H4 S16384 D128 causal 825 (2700), B1 H8 S1024 D64 dense
+// 20.6 (37), H4/kvH1 8231 x 9075 rows D64 causal 161 (272).
 //
 // Every wait on an mbarrier is bounded (see tc_common.cuh); a wait that runs out reports into
 // the device status word and the block unwinds.

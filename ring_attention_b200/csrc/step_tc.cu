@@ -23,10 +23,10 @@
 // Roles inside a block (384 threads)
 //   warp 0        TMA producer: Q tiles once, then K_j, V_j, K_j+1, ... into a shared-memory
 //                 ring of 128B-swizzled tiles (cp.async.bulk.tensor, no multicast).
-//   warps 1, 2    MMA issuers, one per query tile (warp 1 for both where P aliases S): S_w = Q_w K_j^T and O_w += P_w V_j with fp32
-//                 accumulators in tensor memory. The whole warp runs the loop (uniform control
-//                 flow and descriptors), one elected lane executes tcgen05.mma / commit.
-//                 Warp 1 also allocates / frees tensor memory.
+//   warps 1, 2    MMA issuers, one per query tile, or warp 1 for both in turn where P aliases S
+//                 (head_dim 128): S_w = Q_w K_j^T and O_w += P_w V_j with fp32 accumulators in tensor
+//                 memory. The whole warp runs the loop (uniform control flow and descriptors), one
+//                 elected lane executes tcgen05.mma / commit. Warp 1 also allocates / frees tensor memory.
 //   warps 4-7     softmax for query tile 0: one thread per row reads S from tensor memory,
 //   warps 8-11    (tile 1) writes P = 2^(s * scale - m_ref) as 16-bit back into tensor memory
 //                 (or into shared memory), keeps the row sum, and runs the epilogue. m_ref is
@@ -34,8 +34,8 @@
 //                 sees and moved (with a rescale of O and l) only when a tile's row sum shows
 //                 that some score ran more than 2^15 above it; the common tile needs neither
 //                 a row maximum nor a rescale.
-//   The two query tiles are independent streams (own issuing warp, own barriers): the tensor
-//   core works on one tile's MMAs while the other tile's rows are in their exponentials.
+//   The two query tiles are streams of their own (own barriers and, but where P aliases S, own issuing
+//   warp): the tensor core works on one tile's MMAs while the other tile's rows are in their exponentials.
 //
 // Tensor memory (512 columns): S0 [0,128) S1 [128,256) O0 [256,256+D) O1 [256+D,256+2D), and
 // at head_dim 64 a separate P0 / P1 of 64 columns each behind them (otherwise P overwrites S).
@@ -495,13 +495,14 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit, kFold>::kTh
     }
   } else if (warp == 1 || (!C::kOrdered && warp == 2 && live == 2)) {
     // ------------------------------------------------------------- MMA issuers ----
-    // One issuing warp per query tile (warp 1: tile 0, warp 2: tile 1). The two tiles are
-    // independent instruction streams, so a tile that is still in its exponentials never holds
-    // back the other one and the two softmax groups are free to run out of step (which is what
+    // Where P has a place of its own, one issuing warp per query tile (warp 1: tile 0, warp 2: tile 1). The
+    // two tiles are then independent instruction streams, so a tile that is still in its exponentials never
+    // holds back the other one and the two softmax groups are free to run out of step (which is what
     // keeps the exp unit busy: one group's loads, maxima and stores overlap the other group's
-    // exponentials). The whole warp runs the loop so that descriptors and loop state stay
-    // warp-uniform; the tcgen05.mma / tcgen05.commit instructions are executed by one elected
-    // lane. A K/V ring slot is released when both warps have committed their reads of it.
+    // exponentials); a K/V ring slot is released when both warps have committed their reads of it. Where P
+    // aliases S warp 1 issues for both tiles in turn (see below) and releases a slot behind the last reader. The
+    // whole warp runs the loop so that descriptors and loop state stay warp-uniform; the tcgen05.mma /
+    // tcgen05.commit instructions are executed by one elected lane.
     if (n_tiles > 0) {
       const int w = warp - 1;  // (ordered: the query tile is the loop's, see s_ksteps)
       constexpr unsigned kFmt = kBf16 ? 1u : 0u;
@@ -1261,8 +1262,8 @@ int launch_d(int dtype, const StepArgs& a, cudaStream_t stream) {
   if (split > 1) return launch_split<D, D>(dtype, a, stream, split);
   if constexpr (D == 128 || D == 256) {
     // Cluster pairs with M = 256 MMAs (cta_group::2), on request, wherever a segment has at least
-    // two query blocks to pair up. Measured on B200 the pairs are 5-15 % slower than independent
-    // blocks at both head_dims: each block's operand traffic halves, but neither shared-memory nor
+    // two query blocks to pair up. The pairs are slower than independent blocks (B1 H8 causal, us per call, blocks /
+    // pairs: D128 S8192 138 / 152, S32768 1985 / 2069; D256 296 / 333, 4203 / 4781): each block's operand traffic halves, but neither shared-memory nor
     // L2 bandwidth was the limit, and every tile now crosses between the blocks twice (P written
     // -> leader, commit -> peer).
     const bool want_pair = (a.flags & RA_STEP_CTA_PAIR) != 0;

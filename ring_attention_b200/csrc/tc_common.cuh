@@ -479,7 +479,7 @@ struct TcArgs {
 
 // What a block does whose rows see no key: nothing, or the state of `rows` rows from row0 on is written empty
 // or normalised. Without tensor memory, barriers or a meeting of the cluster, whose blocks take every n-th piece:
-// such a block held its SM for 5 us, and a call that has as many of them as of others, as the ring steps of a zig-zag
+// such a block had held its SM for 5 us, and a call that has as many of them as of others, as the ring steps of a zig-zag
 // shard do, waited for them: 16 heads, 64 blocks of 256 rows with keys and 64 without, us per step 31.4 -> 27.8, the one
 // that normalises 36.7 -> 31.2.
 template <int DR>
@@ -611,9 +611,9 @@ struct RowOut {
 // columns at a time, 128 take half again as long) and the state is read and written in pieces of 128 bytes and more. The old state
 // does not depend on the MMAs still running: its first loads are issued before wait_o(), which returns whether O is
 // there, and row_out() says what becomes of this lane's row. us per call with one key tile, 128 blocks of 256 rows, a
-// row per lane -> so: head_dim 64 into a new state 8.6 -> 7.8, into an old one 11.5 -> 8.2; head_dim 128 12.0 -> 10.1,
-// 17.1 -> 10.7; head_dim 256 (128 rows) 12.4 -> 10.2, 17.9 -> 11.3. With few rows the stores of a row per lane are few too:
-// fp32 head_dim 128, 20 rows into a new state 8.6 -> 9.6, 128 rows 12.6 -> 11.8.
+// row per lane -> so: head_dim 64 into a new state 8.6 -> 7.8, into an old one 11.5 -> 8.0; head_dim 128 12.0 -> 9.5,
+// 17.0 -> 10.0; head_dim 256 (128 rows) 12.4 -> 10.1, 17.8 -> 11.1. With few rows the stores of a row per lane are few too:
+// fp32 head_dim 128, 20 rows into a new state 8.6 -> 9.6, 128 rows 12.5 -> 11.9.
 template <int DR>
 struct RowStore {
   static constexpr int kCols = DR > 64 ? 64 : 32;       // columns of a pass
@@ -626,9 +626,10 @@ struct RowStore {
     const int sub = lane / kChunks, chunk = lane % kChunks;
     float4 old[kChunks];
     auto row_of = [&](int i) { return i * kRowsPer + sub; };
-    auto at = [&](int pass, int i) {
-      return reinterpret_cast<float4*>(out + (grow0 + row_of(i)) * DR + pass * kCols + chunk * 4);
-    };
+    // (one address and offsets known at compile time: an address from every row's index took calls with an old state
+    // 0.4 us more at head_dim 128)
+    float4* const mine = reinterpret_cast<float4*>(out + (grow0 + sub) * DR + chunk * 4);
+    auto at = [&](int pass, int i) { return mine + i * (kRowsPer * DR / 4) + pass * (kCols / 4); };
     auto load_old = [&](int pass) {
 #pragma unroll
       for (int i = 0; i < kChunks; ++i)
@@ -790,6 +791,10 @@ inline int cluster_slots(Kern kern, int threads, int smem_bytes, const int** out
 // 1024 x 1024 H8 D256 (64 blocks) 27 / 29 / 39 / 82; 2048 x 2048 H4 D256 41 / 37 / 41 / 86.
 // Four tiles at n = 1 / 2 / 4: 512 x 512 H8 D128 20.5 / 20.5 / 16, fp32 200 x 200 H8 D64 18.5 / 19 / 16.5, D128
 // 29 / 28 / 22.6 (so a share may be a single tile); three tiles, fp32 D64: 12.6 at n = 1, 14.4 at 3.
+// The figures and constants are from before unsplit blocks stored their rows through shared memory and blocks
+// without keys left at once; both cost less now than kFixed and kEmpty say. Over 195 steps of zig-zag ranks (H8 to H16,
+// 400 to 2048 rows a segment) the choice is 1.2 % off the best of n = 1 to 4 in the mean and 15 % at worst (H16 D64,
+// 400 rows, half of the blocks hidden: 16.2 at the chosen 2, 14.1 at 1).
 constexpr double kBlockTiles = 3;  // start and end of a block, in tiles of work
 template <int kTileKeys>
 inline int pick_key_split(const StepArgs& a, int q_block_rows, double merge_tiles, const int* slots,
@@ -850,10 +855,11 @@ inline int pick_key_split(const StepArgs& a, int q_block_rows, double merge_tile
 // has ended, and a tile alone takes `alone` of the time of two (its MMAs and its softmax have nothing to
 // overlap with); so all blocks take about the same time, but all of them together more: a grid of several
 // waves keeps neighbours. `tiles`: the estimate of the best other form (0: none; see pick_key_split). us per
-// call, neighbours / two blocks a query block / folded, fp16 causal: 2048 rows H16 D64 31.0 / 35.3 / 24.9; 4096 H8 D64
-// 53.0 / 46.2 / 42.1, D128 65.2 / 56.0 / 58.6 (not taken); 1531 B2 H12 D64 29.1 / 34.9 / 27.0, D128 37.1 / 42.4 / 35.0; 512
-// H64 D64 12.8 / 26.7 / 12.0; 8192 H4 D64 (not taken) 95.7 / 67.8. From these `alone`: 0.71 to 0.86 at head_dim 64, 0.84 to
-// 0.89 at 128.
+// call, neighbours / two blocks a query block / folded, fp16 causal: 2048 rows H16 D64 31.2 / 34.7 / 25.4; 4096 H8 D64
+// 53.8 / 45.6 / 42.8, D128 64.4 / 55.9 / 58.6 (not taken); 1531 B2 H12 D64 29.2 / 34.3 / 21.2, D128 30.8 / 42.3 / 27.6; 512
+// H64 D64 12.6 / 26.0 / 12.3; 8192 H4 D64 (not taken) 97.6 / 67.2. From these and 1024 and 1536 rows `alone`: 0.77 to 0.82 at
+// head_dim 64 (512 rows 0.94), 0.86 to 0.87 at 128. Over 60 random causal calls of one wave the folded ones (15) are 0.2 %
+// off the best form in the mean and 2.5 % at worst.
 template <int kTileKeys>
 inline bool fold_rows(const StepArgs& a, double alone, double tiles) {
   if (tiles <= 0 || (a.flags & RA_STEP_CAUSAL) == 0 || a.doc_len > 0) return false;
