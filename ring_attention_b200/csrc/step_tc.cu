@@ -61,6 +61,7 @@
 // returns. Later blocks see the status word and return at once; blocks that read it before it was set (those
 // of the next launch, which overlap this one) see it in front of their first V and leave the state as it is.
 #include <atomic>
+#include <climits>
 
 #include "tc_common.cuh"
 
@@ -780,15 +781,16 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit, kFold>::kTh
     const float scale_log2 = rsqrtf(static_cast<float>(DR)) * kLog2e;
 
     // Reference point of P, O and l, log2 units (see the tile loop). A row behind the end of its segment (of a ragged
-    // last tile) has no vote on whether a tile goes without the mask, and a reference above all scores, so that its P
-    // is 0 either way. With a vote it took its warp through the masked path in every tile, and the other tile of a folded
-    // block, or of one warp that issues for both, waited for that. us per call: folded 2 x 2226 rows H8 D64 67.7 -> 48.9
-    // (neighbours 59.5), 1531 rows B2 H12 D64 27.9 -> 21.1; head_dim 128, 951 rows on 3212 keys H32/kvH8 73.1 -> 53.8 (two
+    // last tile) gets one above all scores, so that its P is 0, and does not take its warp through the masked path in
+    // every tile, for which the other tile of a folded block, or of one warp that issues for both, would wait: it sees
+    // every key, or, in the key split at head_dim 128, has no vote on the mask (where seeing every key cost short
+    // calls 0.5 us; unsplit, no vote costs long passes 0.5 %). us per call: folded 2 x 2226 rows H8 D64 67.7 -> 48.9
+    // (neighbours 59.5), 1531 rows B2 H12 D64 27.9 -> 21.1; head_dim 128, 951 rows on 3212 keys H32/kvH8 73.1 -> 54.0 (two
     // issuers 69.2), 2 x 2459 rows H8 112.8 -> 78.2 (103.9), in the key split 137 rows on 3843 keys H64/kvH16 51.0 -> 42.0 (48.5),
-    // 200 rows on 4000 keys H8 21.2 -> 21.7 (23.8). Not at head_dim 64 without a fold, where nothing waits: with such
-    // rows seeing every key instead, B1 H8 S32768 causal took 1422 -> 1474, the tile loop came out slower for all rows.
-    constexpr bool kNoVote = kPInTmem && (D == 128 || (!kSplit && (kFold || D == 256)));
-    float m_ref = kNoVote && !row_valid ? 1e30f : -INFINITY;
+    // 200 rows on 4000 keys H8 21.2 -> 21.7 (23.8). Not at head_dim 64 without a fold, where nothing waits: there the tile
+    // loop came out slower for all rows (B1 H8 S32768 causal 1422 -> 1474).
+    constexpr bool kAllSee = !kSplit && kPInTmem && (kFold || D >= 128), kNoVote = kSplit && D == 128;
+    float m_ref = (kAllSee || kNoVote) && !row_valid ? 1e30f : -INFINITY;
     float l_run = 0.f;
     bool ok = true;
 
@@ -804,7 +806,7 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit, kFold>::kTh
       // Keys of this segment the row can see are the local indices [rel_lo, rel_hi): causal
       // and document limits are affine in the key index, so they are worked out once per
       // segment (64-bit divisions) and the per-tile work is two 32-bit clamps.
-      int rel_lo = 0, rel_hi = row_valid ? a.kmap.seg_len : 0;
+      int rel_lo = 0, rel_hi = kAllSee || row_valid ? a.kmap.seg_len : 0;
       {
         const long long kb = a.kmap.base[sk];
         if (causal) {
@@ -823,6 +825,7 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit, kFold>::kTh
           }
         }
       }
+      if (kAllSee && !row_valid) rel_lo = 0, rel_hi = INT_MAX;
       for (int t = tr.lo; t < tr.hi && ok; ++t, ++j) {
         // Visible columns of this row in this tile: [c_lo, c_hi), from the segment's bounds.
         int c_lo = min(max(rel_lo - t * kBN, 0), kBN);
