@@ -91,7 +91,8 @@ RA_API void ra_debug_stall_producer_after(int items);
  * Process-wide; not for production use. */
 RA_API void ra_debug_set_block_order(int order);
 /* The form that the calling thread's last tensor-core step took: bits 0-3 the blocks that share a
- * query block's keys, 16 folded query tiles, 32 cluster pairs, 64 P in shared memory. For tests. */
+ * query block's keys, 16 folded query tiles, 32 cluster pairs, 64 P in shared memory, 128 shares in a
+ * workspace. For tests. */
 RA_API int ra_debug_step_form(void);
 /* Whether ra_kv_cache_append takes a token's rows by its kernel (1) or by device copies (0), given the
  * current device and those of the cache, the stream and the two sources (-1: not device memory). */
@@ -155,6 +156,20 @@ RA_API int ra_attention_step_ex(int dtype, const void* q, const void* k, const v
                                 float* m, float* l, const ra_shape* shape, const ra_segmap* qmap,
                                 const ra_segmap* kmap, int pos_stride, unsigned flags,
                                 long long doc_len, int kv_row_stride, ra_stream stream);
+
+/* The same step with device memory for partial results. Calls of few query rows and many keys (a prompt's next
+ * rows against a long cache) then run as shares of the key tiles, one block each, over all SMs, and a second launch folds
+ * the shares; without a workspace the blocks of a cluster share at most eight ways. `workspace`: 16-byte aligned, only
+ * read and written by this call's launches on `stream`, at least ra_attention_step_workspace_bytes(...) bytes (0: the
+ * call does not use one; always 0 below 2048 keys). A smaller one, or NULL, is not an error: it is not used. */
+RA_API size_t ra_attention_step_workspace_bytes(int dtype, const ra_shape* shape, const ra_segmap* qmap,
+                                                const ra_segmap* kmap, int pos_stride, unsigned flags,
+                                                long long doc_len);
+RA_API int ra_attention_step_ws(int dtype, const void* q, const void* k, const void* v, float* out,
+                                float* m, float* l, const ra_shape* shape, const ra_segmap* qmap,
+                                const ra_segmap* kmap, int pos_stride, unsigned flags,
+                                long long doc_len, int kv_row_stride, void* workspace,
+                                size_t workspace_bytes, ra_stream stream);
 
 /* Which kernel the step entry points run for a dtype and head_dim (given 16-byte aligned
  * tensors): 1 = the tcgen05 / TMA / tensor-memory kernel (fp16 and bf16, head_dim 32, 64, 128,

@@ -79,6 +79,11 @@ _SIG = {
     "ra_attention_step_ex": (C.c_int, [C.c_int, _P, _P, _P, _P, _P, _P, C.POINTER(Shape),
                                        C.POINTER(SegMap), C.POINTER(SegMap), C.c_int, C.c_uint,
                                        C.c_longlong, C.c_int, _P]),
+    "ra_attention_step_workspace_bytes": (C.c_size_t, [C.c_int, C.POINTER(Shape), C.POINTER(SegMap), C.POINTER(SegMap),
+                                                       C.c_int, C.c_uint, C.c_longlong]),
+    "ra_attention_step_ws": (C.c_int, [C.c_int, _P, _P, _P, _P, _P, _P, C.POINTER(Shape),
+                                       C.POINTER(SegMap), C.POINTER(SegMap), C.c_int, C.c_uint,
+                                       C.c_longlong, C.c_int, _P, C.c_size_t, _P]),
     "ra_attention_step_stacked": (C.c_int, [C.c_int, _P, _P, _P, _P, _P, _P, C.POINTER(Shape),
                                             C.POINTER(SegMap), C.POINTER(SegMap),
                                             C.POINTER(C.c_int), C.POINTER(C.c_int), C.c_int,

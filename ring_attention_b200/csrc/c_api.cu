@@ -21,8 +21,10 @@ size_t elem_size(int dtype) { return dtype == RA_F32 ? 4 : 2; }
 // Validate and launch one general step (the funnel of every step entry point).
 int step_ex(int dtype, const void* q, const void* k, const void* v, float* out, float* m, float* l,
             const ra_shape& s, const PosMap& qmap, const PosMap& kmap, int pos_stride,
-            unsigned flags, long long doc_len, int kv_row_stride, cudaStream_t stream) {
-  RAB_REQUIRE(q && k && v && out && m && l, RA_ERR_INVALID, "attention step: null argument");
+            unsigned flags, long long doc_len, int kv_row_stride, cudaStream_t stream, void* workspace = nullptr,
+            size_t workspace_bytes = 0, size_t* wanted = nullptr) {
+  // (`wanted`: nothing runs, it gets the size of the workspace that the call would use)
+  RAB_REQUIRE(wanted || (q && k && v && out && m && l), RA_ERR_INVALID, "attention step: null argument");
   RAB_REQUIRE(dtype == RA_F32 || dtype == RA_F16 || dtype == RA_BF16, RA_ERR_INVALID,
               "attention step: unknown dtype %d", dtype);
   RAB_REQUIRE(s.batch > 0 && s.heads > 0 && s.seq_q >= 0 && s.seq_k >= 0, RA_ERR_INVALID,
@@ -38,7 +40,7 @@ int step_ex(int dtype, const void* q, const void* k, const void* v, float* out, 
   RAB_REQUIRE(static_cast<long long>(qmap.n_seg) * qmap.seg_len == s.seq_q &&
                   static_cast<long long>(kmap.n_seg) * kmap.seg_len == s.seq_k,
               RA_ERR_INVALID, "attention step: n_seg * seg_len must equal the sequence length");
-  if (s.seq_q == 0) return RA_OK;
+  if (s.seq_q == 0 || (wanted && s.seq_k == 0)) return RA_OK;
   StepArgs a;
   a.q = q;
   a.k = k;
@@ -66,6 +68,12 @@ int step_ex(int dtype, const void* q, const void* k, const void* v, float* out, 
   a.stride = pos_stride;
   a.flags = flags;
   a.doc_len = doc_len;
+  a.workspace = workspace;
+  a.workspace_bytes = workspace_bytes;
+  if (wanted) {
+    if (!(flags & RA_STEP_FORCE_SIMT) && step_tc_supported(dtype, a)) *wanted = step_tc_workspace_bytes(a);
+    return RA_OK;
+  }
   a.status = device_status_ptr();
   if (s.seq_k == 0) {
     // nothing to fold; honour FRESH / FINALIZE on the state alone
@@ -198,6 +206,25 @@ int ra_attention_step_ex(int dtype, const void* q, const void* k, const void* v,
   RAB_REQUIRE(doc_len >= 0, RA_ERR_INVALID, "attention step: doc_len must be >= 0");
   return step_ex(dtype, q, k, v, out, m, l, *shape, make_posmap(*qmap), make_posmap(*kmap),
                  pos_stride, flags, doc_len, kv_row_stride, static_cast<cudaStream_t>(stream));
+}
+
+size_t ra_attention_step_workspace_bytes(int dtype, const ra_shape* shape, const ra_segmap* qmap, const ra_segmap* kmap,
+                                         int pos_stride, unsigned flags, long long doc_len) {
+  size_t bytes = 0;
+  if (shape && qmap && kmap && doc_len >= 0)
+    step_ex(dtype, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, *shape, make_posmap(*qmap), make_posmap(*kmap),
+            pos_stride, flags, doc_len, 0, nullptr, nullptr, 0, &bytes);
+  return bytes;
+}
+
+int ra_attention_step_ws(int dtype, const void* q, const void* k, const void* v, float* out, float* m, float* l,
+                         const ra_shape* shape, const ra_segmap* qmap, const ra_segmap* kmap, int pos_stride,
+                         unsigned flags, long long doc_len, int kv_row_stride, void* workspace, size_t workspace_bytes,
+                         ra_stream stream) {
+  RAB_REQUIRE(shape && qmap && kmap, RA_ERR_INVALID, "attention step: null argument");
+  RAB_REQUIRE(doc_len >= 0, RA_ERR_INVALID, "attention step: doc_len must be >= 0");
+  return step_ex(dtype, q, k, v, out, m, l, *shape, make_posmap(*qmap), make_posmap(*kmap), pos_stride, flags, doc_len,
+                 kv_row_stride, static_cast<cudaStream_t>(stream), workspace, workspace_bytes);
 }
 
 int ra_attention_step_stacked(int dtype, const void* q, const void* k, const void* v, float* out,

@@ -142,11 +142,14 @@ struct StepArgs {
   unsigned flags;
   long long doc_len;
   int* status;
+  void* workspace = nullptr;  // of the spread form (step_tc.cu); without one the other forms run
+  size_t workspace_bytes = 0;
 };
 
 int launch_step_simt(int dtype, const StepArgs& a, cudaStream_t stream);
 int launch_step_tc(int dtype, const StepArgs& a, cudaStream_t stream);
 bool step_tc_supported(int dtype, const StepArgs& a);
+size_t step_tc_workspace_bytes(const StepArgs& a);  // 0: a workspace would not be used
 // fp32 on the tensor cores through split fp16 operands (step_f32.cu): head_dim 32, 64 and 128
 int launch_step_f32(const StepArgs& a, cudaStream_t stream);
 bool step_f32_supported(int dtype, const StepArgs& a);

@@ -180,7 +180,9 @@ __device__ inline RingPos ring_pos(int which, int t, int sub) {
 // kSplit: the blocks of a cluster share the key tiles of ONE query block and merge their partial
 // states through distributed shared memory (see pick_key_split).
 // kFold: the two query tiles of a block are a light and a heavy one of the head (see fold_rows).
-template <int D, bool kBf16, bool kPInTmem, int DR, bool kPair = false, bool kSplit = false, bool kFold = false>
+// kSpread: a block takes a share of the key tiles of two query tiles of a KV head, into a workspace (see plan_spread).
+template <int D, bool kBf16, bool kPInTmem, int DR, bool kPair = false, bool kSplit = false, bool kFold = false,
+          bool kSpread = false>
 __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit, kFold>::kThreads), 1)
     step_tc_kernel(const __grid_constant__ CUtensorMap tmap_q,
                    const __grid_constant__ CUtensorMap tmap_k,
@@ -255,6 +257,16 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit, kFold>::kTh
     light_lin = static_cast<int>(blockIdx.y);
     qb_lin = a.n_qblocks_per_seg * a.qmap.n_seg - 1 - light_lin;
   }
+  // Spread: x = a share, y = batch * kvH + kv head; qb_lin is the query block, of tiles qb_lin * kTiles and on (here
+  // n_qblocks_per_seg counts tiles), bh the head of its first tile.
+  [[maybe_unused]] int share = 0;
+  [[maybe_unused]] const int group = kSpread ? a.H / a.kvH : 1;
+  if constexpr (kSpread) {
+    qb_lin = 0;
+    while (a.spread.beg[qb_lin + 1] <= blockIdx.x) ++qb_lin;
+    share = static_cast<int>(blockIdx.x) - a.spread.beg[qb_lin];
+    bh = static_cast<int>(blockIdx.y) / a.kvH * a.H + static_cast<int>(blockIdx.y) % a.kvH;
+  }
   const int sq = qb_lin / a.n_qblocks_per_seg;
   const int tq = qb_lin - sq * a.n_qblocks_per_seg;
   const int h = bh % a.H;
@@ -268,20 +280,35 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit, kFold>::kTh
   constexpr int kSpan = kPair ? 2 * kQBlock : kQBlock;
   const int span_row0 = kPair ? (tq & ~1) * kQBlock : row0;
   const int rows_in_span = min(kSpan, q_seg_len - span_row0);
-  const int qmin = a.qmap.base[sq] + span_row0 * a.stride;
-  const int qmax = a.qmap.base[sq] + (span_row0 + rows_in_span - 1) * a.stride;
+  int qmin = 0, qmax = 0;
+  [[maybe_unused]] SpreadTile own[2] = {};
+  [[maybe_unused]] int n_spread = 0;  // query tiles of the block
+  if constexpr (kSpread) {
+    const int i0 = qb_lin * C::kTiles;
+    n_spread = min(C::kTiles, group * a.qmap.n_seg * a.n_qblocks_per_seg - i0);
+    spread_span(a.qmap, a.stride, group, a.n_qblocks_per_seg, i0, i0 + n_spread, &qmin, &qmax);
+    own[0] = spread_tile(i0, group, a.n_qblocks_per_seg);
+    own[1] = spread_tile(i0 + n_spread - 1, group, a.n_qblocks_per_seg);
+  } else {
+    qmin = a.qmap.base[sq] + span_row0 * a.stride;
+    qmax = a.qmap.base[sq] + (span_row0 + rows_in_span - 1) * a.stride;
+  }
 
   // Query tiles of the block that take part. In the key-split form, whose calls have few query rows,
   // a segment's last block of at most 128 rows leaves its second tile out (384 rows against 40384
   // keys, H32/kvH8 D128: 735 -> 542 us before any split). The other forms run it on zeros: they
   // have many blocks, and the check in their softmax loop costs the D64 pass 2 %.
-  const int live = (kSplit && C::kTiles == 2 && q_seg_len - row0 <= kBM) || (kFold && light_lin == qb_lin) ? 1 : C::kTiles;
+  const int live = kSpread ? n_spread
+                   : (kSplit && C::kTiles == 2 && q_seg_len - row0 <= kBM) || (kFold && light_lin == qb_lin) ? 1 : C::kTiles;
 
   // (segment, first row inside it) of query tile w, and tile 1's key tiles of a key segment: the first few of tile 0's
   [[maybe_unused]] const int light_sq = kFold ? light_lin / a.n_qblocks_per_seg : 0;
   [[maybe_unused]] const int light_row0 = kFold ? (light_lin - light_sq * a.n_qblocks_per_seg) * kBM : 0;
-  auto tile_sq = [&](int w) { return kFold && w == 1 ? light_sq : sq; };
-  auto tile_row0 = [&](int w) { return kFold ? (w == 1 ? light_row0 : row0) : row0 + w * kBM; };
+  auto tile_sq = [&](int w) { return kSpread ? (w == 1 ? own[1].seg : own[0].seg) : kFold && w == 1 ? light_sq : sq; };
+  auto tile_row0 = [&](int w) {
+    return kSpread ? (w == 1 ? own[1].row0 : own[0].row0) : kFold ? (w == 1 ? light_row0 : row0) : row0 + w * kBM;
+  };
+  auto tile_bh = [&](int w) { return kSpread ? bh + (w == 1 ? own[1].head : own[0].head) * a.kvH : bh; };
   [[maybe_unused]] auto light_range = [&](int sk) {
     const int q0 = a.qmap.base[light_sq] + light_row0 * a.stride;
     return tile_range<kBN>(a.kmap, sk, a.stride, causal, a.doc_len, q0,
@@ -296,6 +323,11 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit, kFold>::kTh
   }
   if (n_tiles == 0) {  // (the blocks of a cluster agree)
     wait_for_previous();
+    if constexpr (kSpread) {
+      const size_t part = (static_cast<size_t>(blockIdx.y) * a.spread.total + blockIdx.x) * (C::kTiles * kBM);
+      for (int i = tid; i < C::kTiles * kBM; i += C::kThreads) a.part_ml[part + i] = make_float2(-INFINITY, 0.f);
+      return;
+    }
     const size_t head0 = static_cast<size_t>(bh) * a.Sq;
     rows_without_keys<DR>(a, head0 + static_cast<size_t>(sq) * q_seg_len + row0, min(kQBlock, q_seg_len - row0),
                           kSplit ? cta_rank : 0, kSplit ? a.key_split : 1, fresh, finalize);
@@ -315,6 +347,12 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit, kFold>::kTh
   if constexpr (kSplit) {  // this block's contiguous share, sizes at most one tile apart
     share_beg = static_cast<int>(static_cast<long long>(n_tiles) * cta_rank / a.key_split);
     share_end = static_cast<int>(static_cast<long long>(n_tiles) * (cta_rank + 1) / a.key_split);
+    n_tiles = share_end - share_beg;
+  }
+  if constexpr (kSpread) {
+    const int n = a.spread.beg[qb_lin + 1] - a.spread.beg[qb_lin];
+    share_beg = static_cast<int>(static_cast<long long>(n_tiles) * share / n);
+    share_end = static_cast<int>(static_cast<long long>(n_tiles) * (share + 1) / n);
     n_tiles = share_end - share_beg;
   }
 
@@ -391,7 +429,7 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit, kFold>::kTh
         mbar_expect_tx(bar_q_full + 8 * w, C::kTileBytes);
         for (int bx = 0; bx < C::kBoxes; ++bx)
           tma_load_3d(s_q + w * C::kTileBytes + bx * (kBM * 128), &tmap_q, bar_q_full + 8 * w,
-                      bx * 64, q_row, bh);
+                      bx * 64, q_row, tile_bh(w));
       }
       int it = 0, jt = 0;  // ring items and key tiles so far
       bool ok = true;
@@ -440,10 +478,10 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit, kFold>::kTh
       // tile t - 1.
       int v_row = 0, v_head = 0;
       bool v_pending = false;
-      [[maybe_unused]] TileShare share{share_beg, share_end, 0};
+      [[maybe_unused]] TileShare cut{share_beg, share_end, 0};
       for (int sk = 0; sk < a.kmap.n_seg && ok; ++sk) {
         TileRange r = tile_range<kBN>(a.kmap, sk, a.stride, causal, a.doc_len, qmin, qmax);
-        if constexpr (kSplit) r = share.clip(r);
+        if constexpr (kSplit || kSpread) r = cut.clip(r);
         for (int t = r.lo; t < r.hi && ok; ++t, ++jt) {
           const int k_row = a.kseg_row[sk] + t * kBN;
           const int k_head = a.kseg_head[sk] + kv_bh;
@@ -774,7 +812,7 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit, kFold>::kTh
     [[maybe_unused]] const unsigned t_p =
         tmem_base + lane_base + (w == 0 ? C::kColP0 : C::kColP1);
     const int r_in_seg = tile_row0(w) + row;
-    const bool row_valid = r_in_seg < q_seg_len && (!kFold || w < live);
+    const bool row_valid = r_in_seg < q_seg_len && (!(kFold || kSpread) || w < live);
     const int qpos = a.qmap.base[tile_sq(w)] + r_in_seg * a.stride;
     const int n_own = kFold && w == 1 ? n_light : n_tiles;  // key tiles of this query tile
     const long long qdoc = a.doc_len > 0 ? qpos / a.doc_len : 0;
@@ -789,17 +827,17 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit, kFold>::kTh
     // issuers 69.2), 2 x 2459 rows H8 112.8 -> 78.2 (103.9), in the key split 137 rows on 3843 keys H64/kvH16 51.0 -> 42.0 (48.5),
     // 200 rows on 4000 keys H8 21.2 -> 21.7 (23.8). Not at head_dim 64 without a fold, where nothing waits: there the tile
     // loop came out slower for all rows (B1 H8 S32768 causal 1422 -> 1474).
-    constexpr bool kAllSee = !kSplit && kPInTmem && (kFold || D >= 128), kNoVote = kSplit && D == 128;
+    constexpr bool kAllSee = !kSplit && kPInTmem && (kFold || kSpread || D >= 128), kNoVote = kSplit && D == 128;
     float m_ref = (kAllSee || kNoVote) && !row_valid ? 1e30f : -INFINITY;
     float l_run = 0.f;
     bool ok = true;
 
     int j = 0;
-    const int n_seg = (!(kSplit || kFold) || w < live) ? a.kmap.n_seg : 0;
-    [[maybe_unused]] TileShare share{share_beg, share_end, 0};
+    const int n_seg = (!(kSplit || kFold || kSpread) || w < live) ? a.kmap.n_seg : 0;
+    [[maybe_unused]] TileShare cut{share_beg, share_end, 0};
     for (int sk = 0; sk < n_seg && ok; ++sk) {
       TileRange tr = tile_range<kBN>(a.kmap, sk, a.stride, causal, a.doc_len, qmin, qmax);
-      if constexpr (kSplit) tr = share.clip(tr);
+      if constexpr (kSplit || kSpread) tr = cut.clip(tr);
       if constexpr (kFold) {
         if (w == 1) tr = light_range(sk);
       }
@@ -1007,7 +1045,7 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit, kFold>::kTh
 
     // ---------------------------------------------------------------- epilogue ----
     auto wait_o = [&]() {
-      if (ok && n_own > 0 && (!kSplit || w < live))
+      if (ok && n_own > 0 && (!(kSplit || kSpread) || w < live))
         ok = mbar_wait(bar_o_done + 8 * w, (C::kEarlyS || C::kDoubleS) ? ((n_own - 1) & 1) : 0,
                        abort_flag, a.status, 8, n_own, a.wait_ns);
       // A light tile without keys: no MMA has read its Q, whose copy may still be on its way to the place where the
@@ -1029,6 +1067,16 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit, kFold>::kTh
                              static_cast<size_t>(bh) * a.Sq + static_cast<size_t>(sq) * q_seg_len + row0,
                              gave_up, !gave_up && w < live && n_tiles > 0, m_ref, l_run, 1.f, cta_rank, fresh,
                              finalize);
+    } else if constexpr (kSpread) {
+      // The share's part of every row as it is: O and l relative to m_ref, in log2 units (a row that saw nothing: no O)
+      const size_t part0 = ((static_cast<size_t>(blockIdx.y) * a.spread.total + blockIdx.x) * C::kTiles + w) * kBM + row - lane;
+      RowStore<DR>::run(
+          lane, a.part_o, part0, __ballot_sync(0xffffffffu, row_valid),
+          s_q + w * C::kTileBytes + (warp & 3) * RowStore<DR>::kStageBytes, t_o, n_tiles > 0 && w < live, true, wait_o, [&]() {
+            const bool have = row_valid && n_tiles > 0 && m_ref > -INFINITY;
+            a.part_ml[part0 + lane] = make_float2(have ? m_ref : -INFINITY, have ? l_run : 0.f);
+            return RowOut{have, have, 0.f, 1.f, 1.f};
+          });
     } else {
       const size_t grow0 = static_cast<size_t>(bh) * a.Sq + static_cast<size_t>(tile_sq(w)) * q_seg_len + r_in_seg - lane;
       const size_t grow = grow0 + lane;
@@ -1089,6 +1137,94 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit, kFold>::kTh
   }
 }
 
+// Spread form: the shares' partial states of every row into the persistent state, with the same merge as the other
+// forms. If a wait ran out no row changes. A row has DR / 4 threads (four columns each) times kSlices, which take every
+// kSlices-th share: a call with few rows has many shares a row, whose loads would follow one another. us per call at one / four
+// slices: 39 rows on 4151 keys H8/kvH4 D128 (18 shares a row) 19.7 / 16.8, 22 rows on 2706 keys B5 H2/kvH1 16.2 / 13.5.
+constexpr int kFoldThreads = 256;
+template <int DR, int kTiles, int kSlices>
+__global__ void __launch_bounds__(kFoldThreads) spread_fold_kernel(const TcArgs a, int rows) {
+  constexpr int kVec = DR / 4, kRowsPer = kFoldThreads / kVec / kSlices;
+  __shared__ float4 acc_of[kSlices > 1 ? kFoldThreads : 1];
+  __shared__ float2 ml_of[kSlices > 1 ? kFoldThreads / kVec : 1];
+  let_next_start();
+  const int col = threadIdx.x % kVec, lane_row = threadIdx.x / kVec, slice = lane_row % kSlices;
+  const int grow = static_cast<int>(blockIdx.x) * kRowsPer + lane_row / kSlices;
+  const bool fresh = (a.flags & RA_STEP_FRESH) != 0, finalize = (a.flags & RA_STEP_FINALIZE) != 0;
+  const int bh = grow / a.Sq, s = grow - bh * a.Sq;
+  const int h = bh % a.H, b = bh / a.H, kv = h % a.kvH, group = a.H / a.kvH;
+  const int seg = s / a.qmap.seg_len, r = s - seg * a.qmap.seg_len;
+  const int tile = (seg * a.n_qblocks_per_seg + r / kBM) * group + h / a.kvH;
+  const int j = min(tile / kTiles, kMaxSpread - 1);
+  const int beg = a.spread.beg[j], n = a.spread.beg[j + 1] - beg;
+  constexpr size_t kStep = static_cast<size_t>(kTiles) * kBM;  // rows from one share's part to the next
+  const size_t part = ((static_cast<size_t>(b) * a.kvH + kv) * a.spread.total + beg) * kStep + (tile % kTiles) * kBM + r % kBM;
+  wait_for_previous();
+  const bool mine = grow < rows && *reinterpret_cast<volatile int*>(a.status) == 0;
+  const int end = mine ? n : 0;
+  float m_all = -INFINITY;
+#pragma unroll 4
+  for (int i = slice; i < end; i += kSlices) m_all = fmaxf(m_all, a.part_ml[part + i * kStep].x);
+  float l_all = 0.f;
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+  for (int i = slice; i < end; i += kSlices) {
+    const float2 ml = a.part_ml[part + i * kStep];
+    const bool have = ml.x > -INFINITY;
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (have) o = reinterpret_cast<const float4*>(a.part_o)[(part + i * kStep) * kVec + col];
+    const float f = have ? ex2(ml.x - m_all) : 0.f;
+    l_all += f * ml.y;
+    acc.x += f * o.x;
+    acc.y += f * o.y;
+    acc.z += f * o.z;
+    acc.w += f * o.w;
+  }
+  if constexpr (kSlices > 1) {
+    acc_of[threadIdx.x] = acc;
+    if (col == 0) ml_of[lane_row] = make_float2(m_all, l_all);
+    __syncthreads();
+    if (slice == 0) {
+      const float2 own = make_float2(m_all, l_all);
+#pragma unroll
+      for (int i = 1; i < kSlices; ++i) m_all = fmaxf(m_all, ml_of[lane_row + i].x);
+      const float f0 = own.x > -INFINITY ? ex2(own.x - m_all) : 0.f;
+      l_all = f0 * own.y;
+      acc = make_float4(f0 * acc.x, f0 * acc.y, f0 * acc.z, f0 * acc.w);
+#pragma unroll
+      for (int i = 1; i < kSlices; ++i) {
+        const float2 ml = ml_of[lane_row + i];
+        const float4 o = acc_of[threadIdx.x + i * kVec];
+        const float f = ml.x > -INFINITY ? ex2(ml.x - m_all) : 0.f;
+        l_all += f * ml.y;
+        acc.x += f * o.x;
+        acc.y += f * o.y;
+        acc.z += f * o.z;
+        acc.w += f * o.w;
+      }
+    }
+  }
+  const bool any = m_all > -INFINITY, touch = mine && slice == 0 && (any || fresh || finalize);
+  const bool old_state = touch && !fresh;
+  const float m_old = old_state ? a.m[grow] : -INFINITY, l_old = old_state ? a.l[grow] : 0.f;
+  const float m_new = any ? m_all * kLn2 : -INFINITY;  // natural-log units
+  const float m_fin = fmaxf(m_old, m_new);
+  const float ca = m_old == -INFINITY ? 0.f : expf(m_old - m_fin);
+  const float cb = any ? expf(m_new - m_fin) : 0.f;
+  const float l_fin = ca * l_old + cb * l_all;
+  const float inv = finalize ? (l_fin > 0.f ? 1.f / l_fin : 0.f) : 1.f;
+  const float fa = ca * inv, fb = cb * inv;
+  float4* const dst = reinterpret_cast<float4*>(a.out) + static_cast<size_t>(grow) * kVec + col;
+  float4 old = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (old_state) old = *dst;
+  if (touch) *dst = make_float4(fa * old.x + fb * acc.x, fa * old.y + fb * acc.y, fa * old.z + fb * acc.z, fa * old.w + fb * acc.w);
+  __syncthreads();  // every thread of a row has read its old (m, l)
+  if (touch && col == 0) {
+    a.m[grow] = m_fin;
+    a.l[grow] = l_fin;
+  }
+}
+
 // ---- host side ----------------------------------------------------------------------
 
 // Test hooks (see ra_debug_set_wait_limit_ns / ra_debug_stall_producer_after).
@@ -1097,8 +1233,9 @@ std::atomic<int> g_stall_after{-1};
 std::atomic<int> g_block_order{-1};  // -1: by shape, 0: heads fastest, k > 0: waves of k KV heads
 thread_local int g_form = 0;         // of the calling thread's last launch, see ra_debug_step_form
 
-template <int D, bool kBf16, bool kPInTmem, int DR, bool kPair = false, bool kSplit = false, bool kFold = false>
-int launch_cfg(const StepArgs& a, cudaStream_t stream, int key_split = 1) {
+template <int D, bool kBf16, bool kPInTmem, int DR, bool kPair = false, bool kSplit = false, bool kFold = false,
+          bool kSpread = false>
+int launch_cfg(const StepArgs& a, cudaStream_t stream, int key_split = 1, const Spread* spread = nullptr) {
   using C = TcCfg<D, kPInTmem, kPair, kSplit, kFold>;
   CUtensorMap mq, mk, mv;
   const int dtype = kBf16 ? RA_BF16 : RA_F16;
@@ -1117,7 +1254,7 @@ int launch_cfg(const StepArgs& a, cudaStream_t stream, int key_split = 1) {
   t.H = a.H;
   t.kvH = a.kvH;
   t.Sq = a.Sq;
-  constexpr int kQBlock = kFold ? kBM : C::kTiles * kBM;
+  constexpr int kQBlock = kFold || kSpread ? kBM : C::kTiles * kBM;
   t.n_qblocks_per_seg = (a.qmap.seg_len + kQBlock - 1) / kQBlock;
   if (kPair) t.n_qblocks_per_seg = (t.n_qblocks_per_seg + 1) & ~1;  // whole pairs per segment
   t.qmap = a.qmap;
@@ -1169,15 +1306,22 @@ int launch_cfg(const StepArgs& a, cudaStream_t stream, int key_split = 1) {
   }
   const int order = g_block_order.load(std::memory_order_relaxed);  // test hook
   if (order == 0 || (order > 0 && kv_heads_total % order == 0)) kv_per_wave = order;
-  if (kSplit || kFold) kv_per_wave = 0;
+  if (kSplit || kFold || kSpread) kv_per_wave = 0;
   t.kv_per_wave = kv_per_wave;
   t.key_split = key_split;
-  set_step_form(key_split | (kFold ? 16 : 0) | (kPair ? 32 : 0) | (kPInTmem ? 0 : 64));
+  set_step_form(key_split | (kFold ? 16 : 0) | (kPair ? 32 : 0) | (kPInTmem ? 0 : 64) | (kSpread ? 128 : 0));
+  const long long rows_total = static_cast<long long>(a.B) * a.H * a.Sq;
+  if constexpr (kSpread) {
+    t.spread = *spread;
+    const size_t parts = static_cast<size_t>(kv_heads_total) * spread->total * C::kTiles * kBM;
+    t.part_o = static_cast<float*>(a.workspace);
+    t.part_ml = reinterpret_cast<float2*>(t.part_o + parts * DR);
+  }
   const long long bh_total = static_cast<long long>(a.B) * a.H;
   const long long per_x = kv_per_wave > 0 ? static_cast<long long>(a.H / a.kvH) * kv_per_wave : 0;
   RAB_REQUIRE(kv_per_wave > 0 ? n_qblocks * per_x < (1ll << 31) : n_qblocks <= 65535, RA_ERR_INVALID,
               "attention step: grid too large (%lld query blocks, %lld heads)", n_qblocks, bh_total);
-  auto kern = step_tc_kernel<D, kBf16, kPInTmem, DR, kPair, kSplit, kFold>;
+  auto kern = step_tc_kernel<D, kBf16, kPInTmem, DR, kPair, kSplit, kFold, kSpread>;
   // once per device and instantiation: the attribute call costs microseconds that a pass of a
   // few short launches would otherwise pay every time
   static std::atomic<unsigned long long> smem_set{0};
@@ -1188,6 +1332,7 @@ int launch_cfg(const StepArgs& a, cudaStream_t stream, int key_split = 1) {
     if (dev >= 0 && dev < 64) smem_set.fetch_or(1ull << dev, std::memory_order_release);
   }
   dim3 grid(static_cast<unsigned>(a.B) * a.H, static_cast<unsigned>(n_qblocks));
+  if (kSpread) grid = dim3(static_cast<unsigned>(t.spread.total), static_cast<unsigned>(kv_heads_total));
   if (kv_per_wave > 0)
     grid = dim3(static_cast<unsigned>(n_qblocks * per_x), static_cast<unsigned>(kv_heads_total / kv_per_wave));
   if constexpr (kPair || kSplit) {
@@ -1211,6 +1356,18 @@ int launch_cfg(const StepArgs& a, cudaStream_t stream, int key_split = 1) {
   } else {
     RAB_CUDA(launch_overlapped(kern, grid, dim3(C::kThreads), C::kSmemBytes, stream, mq, mk, mv, t));
   }
+  if constexpr (kSpread) {
+    // four slices where some row has more than six shares
+    int most = 0;
+    for (int j = 0; j < kMaxSpread; ++j) most = std::max(most, spread->beg[j + 1] - spread->beg[j]);
+    auto fold = [&](auto kern, int slices) {
+      const int per = kFoldThreads / (DR / 4) / slices;
+      return launch_overlapped(kern, dim3(static_cast<unsigned>((rows_total + per - 1) / per)), dim3(kFoldThreads), 0,
+                               stream, t, static_cast<int>(rows_total));
+    };
+    if (most > 6) RAB_CUDA(fold(spread_fold_kernel<DR, C::kTiles, 4>, 4));
+    else RAB_CUDA(fold(spread_fold_kernel<DR, C::kTiles, 1>, 1));
+  }
   RAB_CUDA(cudaGetLastError());
   return RA_OK;
 }
@@ -1227,23 +1384,57 @@ int launch_fold(int dtype, const StepArgs& a, cudaStream_t stream) {
                           : launch_cfg<D, false, true, DR, false, false, true>(a, stream);
 }
 
+template <int D, int DR>
+int launch_spread(int dtype, const StepArgs& a, cudaStream_t stream, const Spread& spread) {
+  return dtype == RA_BF16 ? launch_cfg<D, true, true, DR, false, false, false, true>(a, stream, 1, &spread)
+                          : launch_cfg<D, false, true, DR, false, false, false, true>(a, stream, 1, &spread);
+}
+
+// The spread form's workspace: 4 (head_dim + 2) bytes for every row of every share.
 template <int D>
-int launch_d(int dtype, const StepArgs& a, cudaStream_t stream) {
-  // P stays in tensor memory unless the caller asks for the shared-memory path (kept as a
-  // cross-check of the first one; both are tested)
-  const bool p_in_tmem = (a.flags & RA_STEP_P_IN_SMEM) == 0;
+size_t spread_bytes(const StepArgs& a, const Spread& spread) {
+  return static_cast<size_t>(a.B) * a.kvH * spread.total * TcCfg<D, true>::kTiles * kBM * (a.D + 2) * sizeof(float);
+}
+
+// The form of a call that may choose: blocks that share a query block's keys, folded tiles, or (`spread` not null) the spread form.
+struct Form {
+  int split = 1;
+  bool fold = false, spread = false;
+};
+template <int D>
+int pick_form(const StepArgs& a, Form* form, Spread* spread) {
   // A key split (not under a forced block order, which is about whole blocks). A merge stages 4 bytes
   // per row and column, so it costs more tiles the wider the head.
   using S = TcCfg<D, true, false, true>;
   const int* slots = nullptr;
   const int rc = cluster_slots(step_tc_kernel<D, false, true, D, false, true>, S::kThreads, S::kSmemBytes, &slots);
   if (rc != RA_OK) return rc;
-  int split = 1;
-  [[maybe_unused]] bool fold = false;
-  if (p_in_tmem && (a.flags & RA_STEP_CTA_PAIR) == 0 && g_block_order.load(std::memory_order_relaxed) < 0) {
+  if ((a.flags & (RA_STEP_P_IN_SMEM | RA_STEP_CTA_PAIR)) == 0 && g_block_order.load(std::memory_order_relaxed) < 0) {
     double tiles = 0;
-    split = pick_key_split<kBN>(a, TcCfg<D, true>::kTiles * kBM, D == 64 ? 1.5 : D == 128 ? 2.5 : 4.5, slots, &tiles);
-    if constexpr (D <= 128) fold = fold_rows<kBN>(a, D == 64 ? 0.75 : 0.87, tiles);
+    form->split = pick_key_split<kBN>(a, TcCfg<D, true>::kTiles * kBM, D == 64 ? 1.5 : D == 128 ? 2.5 : 4.5, slots, &tiles);
+    if constexpr (D <= 128) form->fold = fold_rows<kBN>(a, D == 64 ? 0.75 : 0.87, tiles);
+    form->spread = !form->fold && plan_spread<kBN>(a, TcCfg<D, true>::kTiles, D <= 128 ? 4 : 6, slots[1], tiles, spread);
+  }
+  return RA_OK;
+}
+
+template <int D>
+int launch_d(int dtype, const StepArgs& a, cudaStream_t stream) {
+  // P stays in tensor memory unless the caller asks for the shared-memory path (kept as a
+  // cross-check of the first one; both are tested)
+  const bool p_in_tmem = (a.flags & RA_STEP_P_IN_SMEM) == 0;
+  Form form;
+  Spread spread;
+  const int rc = pick_form<D>(a, &form, &spread);
+  if (rc != RA_OK) return rc;
+  const int split = form.split;
+  [[maybe_unused]] const bool fold = form.fold;
+  if (form.spread && a.workspace != nullptr && a.workspace_bytes >= spread_bytes<D>(a, spread) &&
+      (reinterpret_cast<uintptr_t>(a.workspace) & 15u) == 0) {
+    if constexpr (D == 64) {
+      if (a.D == 32) return launch_spread<64, 32>(dtype, a, stream, spread);
+    }
+    return launch_spread<D, D>(dtype, a, stream, spread);
   }
   // the 64-wide kernel also takes head_dim 32 (DR = 32)
   if constexpr (D == 64) {
@@ -1290,6 +1481,14 @@ bool step_tc_supported(int dtype, const StepArgs& a) {
        reinterpret_cast<uintptr_t>(a.v) | reinterpret_cast<uintptr_t>(a.out)) & 15u)
     return false;
   return true;
+}
+
+size_t step_tc_workspace_bytes(const StepArgs& a) {
+  Form form;
+  Spread spread;
+  if (a.D == 32 || a.D == 64) return pick_form<64>(a, &form, &spread) == RA_OK && form.spread ? spread_bytes<64>(a, spread) : 0;
+  if (a.D == 128) return pick_form<128>(a, &form, &spread) == RA_OK && form.spread ? spread_bytes<128>(a, spread) : 0;
+  return pick_form<256>(a, &form, &spread) == RA_OK && form.spread ? spread_bytes<256>(a, spread) : 0;
 }
 
 int launch_step_tc(int dtype, const StepArgs& a, cudaStream_t stream) {

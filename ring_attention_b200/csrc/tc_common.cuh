@@ -446,6 +446,28 @@ __host__ __device__ inline TileRange tile_range(const PosMap& kmap, int sk, int 
   return {static_cast<int>(j_lo / kTileKeys), static_cast<int>(j_hi / kTileKeys) + 1};
 }
 
+// Query tile i of a KV head in the spread form: by position, then by query head of the group.
+struct SpreadTile {
+  int head, seg, row0;  // head inside the group, query segment, first row inside it
+};
+__host__ __device__ inline SpreadTile spread_tile(int i, int group, int per_seg) {
+  const int pos = i / group;
+  return {i - pos * group, pos / per_seg, (pos % per_seg) * kBM};
+}
+// Positions [qmin, qmax] that the rows of tiles [i0, i1) span.
+__host__ __device__ inline void spread_span(const PosMap& qmap, int stride, int group, int per_seg, int i0, int i1, int* qmin,
+                                            int* qmax) {
+  *qmin = 0x7fffffff;
+  *qmax = -0x7fffffff;
+  for (int i = i0; i < i1; ++i) {
+    const SpreadTile t = spread_tile(i, group, per_seg);
+    const int rows = qmap.seg_len - t.row0 < kBM ? qmap.seg_len - t.row0 : kBM;
+    const int first = qmap.base[t.seg] + t.row0 * stride, last = first + (rows - 1) * stride;
+    *qmin = first < *qmin ? first : *qmin;
+    *qmax = last > *qmax ? last : *qmax;
+  }
+}
+
 // A block's share of its query block's tile list when the list is cut across the blocks of a
 // cluster: list entries [beg, end). clip() is called once per key segment, in order.
 struct TileShare {
@@ -456,6 +478,14 @@ struct TileShare {
     seen += n;
     return {r.lo + lo, r.lo + max(lo, hi)};
   }
+};
+
+// Spread form: the key tiles of every query block of a KV head are cut into shares, a block each, whose partial
+// states go to a workspace (see plan_spread).
+constexpr int kMaxSpread = 160;  // blocks of one KV head, at most (a B200 has 148 SMs)
+struct Spread {
+  int total;                             // blocks of one KV head
+  unsigned char beg[kMaxSpread + 1];     // first block of query block j; beg[number of query blocks] = total
 };
 
 struct TcArgs {
@@ -475,6 +505,9 @@ struct TcArgs {
   int stall_after;             // test hook: the producer stops after this many ring items (< 0: off)
   int kv_per_wave;             // block order: waves of this many KV heads (0: heads fastest)
   int key_split;               // blocks of a cluster that share one query block's key tiles
+  Spread spread;               // spread form: the shares, and where their partial states go
+  float* part_o;
+  float2* part_ml;
 };
 
 // What a block does whose rows see no key: nothing, or the state of `rows` rows from row0 on is written empty
@@ -882,6 +915,65 @@ inline bool fold_rows(const StepArgs& a, double alone, double tiles) {
     longest = t > longest ? t : longest;
   }
   return longest + kBlockTiles < 0.95 * tiles;
+}
+
+// Spread: the same for a call with a workspace, without clusters. All 128-row query tiles of the query heads that share
+// a KV head are paired into blocks (by position, then by head, so that the tiles of a block see about the same keys),
+// and block j's key tiles are cut into n_j contiguous shares, a thread block each, for the smallest longest share whose
+// blocks all fit the SMs at once. A share writes its partial (O, m, l) to the workspace and a second launch folds the
+// shares into the state. Against the key split: no SM is left out because clusters do not fit (135 of 148 in threes), a
+// block may have more than eight shares, grouped heads fill up each other's blocks, and blocks may differ in their number of
+// shares; against that stand a launch and the way of the partial states through L2 (`fold_tiles`, in tiles of work).
+// Chosen where the estimate is 5 %, and four tiles, below that of the best other form (the workspace and the second launch
+// cost the host 5 to 7 us, which a call that is waited for shows). Only from kSpreadKeys keys on: shorter
+// calls never gain, and a caller need not ask for a workspace. us per call, key split / spread (16 bits, causal, CUDA
+// graphs): 384 rows on 40384 keys H32/kvH8 D128 285 / 211, D64 261 / 177; 64 rows on 65536 keys H8 D128 109 / 62; 16 rows on
+// 100000 keys H16/kvH2 D128 211 / 90; 144 rows on 32376 keys H2 D64 71 / 28; 700 rows on 9000 keys H8/kvH2 D256 86 / 62; 337
+// rows on 8336 keys H16/kvH8 D64 39 / 34. Over 104 random calls (16 to 2048 rows on 1000 to 40000 keys more) that gain by
+// more than 5 % in the estimate 0.69 in the mean, 1.05 at worst (19.7 / 20.7, a call that the four tiles now keep out).
+constexpr int kSpreadKeys = 2048;
+template <int kTileKeys>
+inline bool plan_spread(const StepArgs& a, int tiles_per_block, double fold_tiles, int sms, double best_other, Spread* out) {
+  if (a.Sk < kSpreadKeys || a.Sq < 2 || best_other <= 0 || a.H % a.kvH != 0) return false;
+  const long long heads = static_cast<long long>(a.B) * a.kvH;
+  const int cap = static_cast<int>(heads < sms ? sms / heads : 0) < kMaxSpread ? static_cast<int>(heads < sms ? sms / heads : 0) : kMaxSpread;
+  const int group = a.H / a.kvH;
+  const int per_seg = (a.qmap.seg_len + kBM - 1) / kBM;
+  const long long tiles = static_cast<long long>(group) * a.qmap.n_seg * per_seg;
+  const long long n_blocks = (tiles + tiles_per_block - 1) / tiles_per_block;
+  if (n_blocks > cap) return false;
+  int keys[kMaxSpread], longest = 1;
+  for (int j = 0; j < n_blocks; ++j) {
+    int qmin, qmax;
+    spread_span(a.qmap, a.stride, group, per_seg, j * tiles_per_block,
+                static_cast<int>((j + 1) * tiles_per_block < tiles ? (j + 1) * tiles_per_block : tiles), &qmin, &qmax);
+    keys[j] = 0;
+    for (int sk = 0; sk < a.kmap.n_seg; ++sk) {
+      const TileRange r = tile_range<kTileKeys>(a.kmap, sk, a.stride, (a.flags & RA_STEP_CAUSAL) != 0, a.doc_len, qmin, qmax);
+      keys[j] += r.hi - r.lo;
+    }
+    longest = keys[j] > longest ? keys[j] : longest;
+  }
+  auto blocks = [&](int share) {
+    int n = 0;
+    for (int j = 0; j < n_blocks; ++j) n += keys[j] > share ? (keys[j] + share - 1) / share : 1;
+    return n;
+  };
+  int lo = 1, hi = longest;  // the smallest share that fits is in [lo, hi]
+  while (lo < hi) {
+    const int mid = (lo + hi) / 2;
+    if (blocks(mid) <= cap) hi = mid;
+    else lo = mid + 1;
+  }
+  const double gain = best_other - (lo + kBlockTiles + fold_tiles);
+  if (gain < 4 || gain < 0.05 * best_other) return false;
+  out->total = 0;
+  for (int j = 0; j < n_blocks; ++j) {
+    out->beg[j] = static_cast<unsigned char>(out->total);
+    out->total += keys[j] > lo ? (keys[j] + lo - 1) / lo : 1;
+  }
+  for (int j = static_cast<int>(n_blocks); j <= kMaxSpread; ++j) out->beg[j] = static_cast<unsigned char>(out->total);
+  return true;
 }
 
 // Limits set through the test hooks (step_tc.cu owns them).
