@@ -92,7 +92,7 @@ RA_API void ra_debug_stall_producer_after(int items);
 RA_API void ra_debug_set_block_order(int order);
 /* The form that the calling thread's last tensor-core step took: bits 0-3 the blocks that share a
  * query block's keys, 16 folded query tiles, 32 cluster pairs, 64 P in shared memory, 128 shares in a
- * workspace. For tests. */
+ * workspace, 256 K and V split ahead (fp32). For tests. */
 RA_API int ra_debug_step_form(void);
 /* Whether ra_kv_cache_append takes a token's rows by its kernel (1) or by device copies (0), given the
  * current device and those of the cache, the stream and the two sources (-1: not device memory). */
@@ -157,11 +157,12 @@ RA_API int ra_attention_step_ex(int dtype, const void* q, const void* k, const v
                                 const ra_segmap* kmap, int pos_stride, unsigned flags,
                                 long long doc_len, int kv_row_stride, ra_stream stream);
 
-/* The same step with device memory for partial results. Calls of few query rows and many keys (a prompt's next
- * rows against a long cache) then run as shares of the key tiles, one block each, over all SMs, and a second launch folds
- * the shares; without a workspace the blocks of a cluster share at most eight ways. `workspace`: 16-byte aligned, only
- * read and written by this call's launches on `stream`, at least ra_attention_step_workspace_bytes(...) bytes (0: the
- * call does not use one; always 0 below 2048 keys). A smaller one, or NULL, is not an error: it is not used. */
+/* The same step with device memory of its own. 16-bit calls of few query rows and many keys (a prompt's next rows against a
+ * long cache) then run as shares of the key tiles, one block each, over all SMs, and a second launch folds the shares;
+ * without a workspace the blocks of a cluster share at most eight ways. Long fp32 calls have K and V split into their fp16
+ * terms once, by a launch ahead, instead of by every block (the results are the same bits). `workspace`: 128-byte aligned,
+ * only read and written by this call's launches on `stream`, at least ra_attention_step_workspace_bytes(...) bytes (0: the
+ * call does not use one). A smaller one, or NULL, is not an error: it is not used. */
 RA_API size_t ra_attention_step_workspace_bytes(int dtype, const ra_shape* shape, const ra_segmap* qmap,
                                                 const ra_segmap* kmap, int pos_stride, unsigned flags,
                                                 long long doc_len);
@@ -215,7 +216,8 @@ RA_API int ra_int8_to_float(const signed char* src, float* dst, size_t n, ra_str
 /* Whole single-GPU attention, fp32 in and out, end-aligned causal mask
  * (j <= i + seq_k - seq_q). Replaces launch_flash_attention and launch_flash_attention_fp16
  * (src/attention.hpp:48-65). `workspace` must hold
- * ra_flash_workspace_bytes(shape, half_precision) bytes of device memory. */
+ * ra_flash_workspace_bytes(shape, half_precision) bytes of device memory. (The size includes what
+ * ra_attention_step_ws would use; a workspace without that part is accepted.) */
 RA_API size_t ra_flash_workspace_bytes(const ra_shape* shape, int half_precision);
 RA_API int ra_flash_attention(const float* q, const float* k, const float* v, float* out,
                               const ra_shape* shape, int causal, int half_precision,

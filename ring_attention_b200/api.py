@@ -106,8 +106,8 @@ def attention_step_ex(q, k, v, out, m, l, shape, qmap, kmap, pos_stride=1, causa
              (_lib.RA_STEP_P_IN_SMEM if p_in_smem else 0) |
              (_lib.RA_STEP_CTA_PAIR if cta_pair else 0) | key_split << _lib.RA_STEP_KEY_SPLIT_SHIFT)
     dt, s = _dtype(q), shape.c()
-    # (below 2048 keys no call uses a workspace, and the question would cost a short call a microsecond)
-    need = 0 if dt == RA_F32 or s.seq_k < 2048 else lib().ra_attention_step_workspace_bytes(
+    # (below 2048 keys it has little or nothing to gain, and the question costs a short call a microsecond)
+    need = 0 if s.seq_k < 2048 else lib().ra_attention_step_workspace_bytes(
         dt, C.byref(s), C.byref(qmap), C.byref(kmap), pos_stride, flags, doc_len)
     ws = torch.empty(need, dtype=torch.uint8, device=q.device) if need else None
     check(lib().ra_attention_step_ws(dt, _ptr(q), _ptr(k), _ptr(v), _ptr(out), _ptr(m), _ptr(l), C.byref(s),

@@ -71,7 +71,9 @@ int step_ex(int dtype, const void* q, const void* k, const void* v, float* out, 
   a.workspace = workspace;
   a.workspace_bytes = workspace_bytes;
   if (wanted) {
-    if (!(flags & RA_STEP_FORCE_SIMT) && step_tc_supported(dtype, a)) *wanted = step_tc_workspace_bytes(a);
+    if (flags & RA_STEP_FORCE_SIMT) return RA_OK;
+    if (step_tc_supported(dtype, a)) *wanted = step_tc_workspace_bytes(a);
+    else if (step_f32_supported(dtype, a)) *wanted = step_f32_workspace_bytes(a);
     return RA_OK;
   }
   a.status = device_status_ptr();
@@ -259,17 +261,37 @@ RA_API int ra_debug_step_form(void) { return rab::step_form(); }
 
 /* ------------------------------------------------ whole attention, device buffers ---- */
 
-size_t ra_flash_workspace_bytes(const ra_shape* s, int half_precision) {
-  if (!s) return 0;
-  const size_t rows = static_cast<size_t>(s->batch) * s->heads * s->seq_q;
-  size_t bytes = 2 * rows * sizeof(float);  // m, l
+// m, l and, where they are rounded first, Q, K and V; what the step itself can use comes behind it (a caller that
+// brings only this much is served without)
+static size_t flash_bytes(const ra_shape& s, int half_precision) {
+  const size_t rows = static_cast<size_t>(s.batch) * s.heads * s.seq_q;
+  size_t bytes = 2 * rows * sizeof(float);
   if (half_precision) {
-    const int kvH = s->kv_heads > 0 ? s->kv_heads : s->heads;
-    const size_t qn = rows * s->head_dim;
-    const size_t kn = static_cast<size_t>(s->batch) * kvH * s->seq_k * s->head_dim;
+    const size_t qn = rows * s.head_dim;
+    const size_t kn = static_cast<size_t>(s.batch) * kv_heads_of(s) * s.seq_k * s.head_dim;
     bytes += (qn + 2 * kn) * 2 + 64;
   }
   return bytes + 256;
+}
+// end-aligned causal mask: key j visible to query i iff j <= i + (seq_k - seq_q)
+// (src/cpu_attention.cpp:32-34) == global positions q_offset = seq_k - seq_q, k_offset = 0
+static int flash_step(int dtype, const void* q, const void* k, const void* v, float* out, float* m, float* l, const ra_shape& s,
+                      int causal, void* workspace, size_t workspace_bytes, cudaStream_t stream, size_t* wanted = nullptr) {
+  return step_ex(dtype, q, k, v, out, m, l, s, affine_posmap(s.seq_k - s.seq_q, s.seq_q), affine_posmap(0, s.seq_k), 1,
+                 (causal ? RA_STEP_CAUSAL : 0u) | RA_STEP_FRESH | RA_STEP_FINALIZE, 0, 0, stream, workspace, workspace_bytes,
+                 wanted);
+}
+
+size_t ra_flash_workspace_bytes(const ra_shape* s, int half_precision) {
+  if (!s) return 0;
+  size_t most = 0;
+  for (int causal = 0; causal < 2; ++causal) {
+    size_t step = 0;
+    flash_step(half_precision ? RA_F16 : RA_F32, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, *s, causal, nullptr, 0,
+               nullptr, &step);
+    most = std::max(most, step);
+  }
+  return flash_bytes(*s, half_precision) + (most ? most + 256 : 0);
 }
 
 int ra_flash_attention(const float* q, const float* k, const float* v, float* out,
@@ -277,31 +299,27 @@ int ra_flash_attention(const float* q, const float* k, const float* v, float* ou
                        size_t workspace_bytes, ra_stream stream_) {
   RAB_REQUIRE(q && k && v && out && s && workspace, RA_ERR_INVALID,
               "ra_flash_attention: null argument");
-  RAB_REQUIRE(workspace_bytes >= ra_flash_workspace_bytes(s, half_precision), RA_ERR_OVERFLOW,
+  RAB_REQUIRE(workspace_bytes >= flash_bytes(*s, half_precision), RA_ERR_OVERFLOW,
               "ra_flash_attention: workspace too small");
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
-  const int kvH = kv_heads_of(*s);
   const size_t rows = static_cast<size_t>(s->batch) * s->heads * s->seq_q;
   uintptr_t p = (reinterpret_cast<uintptr_t>(workspace) + 255) & ~static_cast<uintptr_t>(255);
   float* m = reinterpret_cast<float*>(p);
   float* l = m + rows;
-  // end-aligned causal mask: key j visible to query i iff j <= i + (seq_k - seq_q)
-  // (src/cpu_attention.cpp:32-34) == global positions q_offset = seq_k - seq_q, k_offset = 0
-  const PosMap qmap = affine_posmap(s->seq_k - s->seq_q, s->seq_q);
-  const PosMap kmap = affine_posmap(0, s->seq_k);
-  const unsigned flags = (causal ? RA_STEP_CAUSAL : 0u) | RA_STEP_FRESH | RA_STEP_FINALIZE;
-  if (!half_precision) {
-    return step_ex(RA_F32, q, k, v, out, m, l, *s, qmap, kmap, 1, flags, 0, 0, stream);
-  }
+  const uintptr_t rest = (reinterpret_cast<uintptr_t>(workspace) + flash_bytes(*s, half_precision) + 255) & ~static_cast<uintptr_t>(255);
+  const uintptr_t end = reinterpret_cast<uintptr_t>(workspace) + workspace_bytes;
+  void* const step_ws = rest < end ? reinterpret_cast<void*>(rest) : nullptr;
+  const size_t step_bytes = rest < end ? end - rest : 0;
+  if (!half_precision) return flash_step(RA_F32, q, k, v, out, m, l, *s, causal, step_ws, step_bytes, stream);
   const size_t qn = rows * s->head_dim;
-  const size_t kn = static_cast<size_t>(s->batch) * kvH * s->seq_k * s->head_dim;
+  const size_t kn = static_cast<size_t>(s->batch) * kv_heads_of(*s) * s->seq_k * s->head_dim;
   uintptr_t hp = (reinterpret_cast<uintptr_t>(l + rows) + 15) & ~static_cast<uintptr_t>(15);
   __half* qh = reinterpret_cast<__half*>(hp);
   __half* kh = qh + ((qn + 7) & ~static_cast<size_t>(7));
   __half* vh = kh + ((kn + 7) & ~static_cast<size_t>(7));
   const int rc = launch_narrow_qkv(q, k, v, qh, kh, vh, qn, kn, stream);
   if (rc != RA_OK) return rc;
-  return step_ex(RA_F16, qh, kh, vh, out, m, l, *s, qmap, kmap, 1, flags, 0, 0, stream);
+  return flash_step(RA_F16, qh, kh, vh, out, m, l, *s, causal, step_ws, step_bytes, stream);
 }
 
 /* --------------------------------------------------- whole attention, host buffers ---- */

@@ -142,7 +142,7 @@ struct StepArgs {
   unsigned flags;
   long long doc_len;
   int* status;
-  void* workspace = nullptr;  // of the spread form (step_tc.cu); without one the other forms run
+  void* workspace = nullptr;  // of the spread form (step_tc.cu) or for split K and V (step_f32.cu); other forms need none
   size_t workspace_bytes = 0;
 };
 
@@ -153,6 +153,7 @@ size_t step_tc_workspace_bytes(const StepArgs& a);  // 0: a workspace would not 
 // fp32 on the tensor cores through split fp16 operands (step_f32.cu): head_dim 32, 64 and 128
 int launch_step_f32(const StepArgs& a, cudaStream_t stream);
 bool step_f32_supported(int dtype, const StepArgs& a);
+size_t step_f32_workspace_bytes(const StepArgs& a);  // 0: a workspace would not be used
 
 // One step over key segments that live in several stacked shards (see StepArgs::kseg_head):
 // k / v point at shard 0, every shard is (B * kvH, shard_rows, D) and shard s starts

@@ -38,21 +38,24 @@
 //                 back over itself, the hi tiles over the even 32-column boxes and the lo tiles over
 //                 the odd ones, in the layout TMA would give 16-bit data. They also find the range of
 //                 every tile; a marked V tile stays as it landed.
+//   With a workspace, long calls split K and V once ahead (split_kv_kernel): no splitters, 384 threads.
 //   Head_dim 32 / 64: S and P have buffers of their own, so the scores of tile t+1 are computed
 //   while the softmax of tile t runs. Head_dim 128: P is written over S and the two query tiles take
 //   turns on the tensor core.
 //
 // Tensor memory, 256 columns per query tile: S [0,64) P hi [64,96) P lo [96,128) O [128,192) Q hi
 // [192,224) Q lo [224,256); head_dim 128: S and P [0,64) O [64,192) Q hi [192,256).
-// What bounds it: at head_dim 128 a pair of tiles of 64 keys takes 5200 clocks, of which its MMAs need 3400. The
-// two softmax groups (1500 to 1900 clocks a tile) run under the other tile's MMAs, and the issuing warp finds P
-// written when it comes to it, so in the other 1800 clocks the tensor core has no MMA although nothing it
-// waits for is missing: why is not known. Tensor pipe 58 %, issue slots 48 % (B1 H8 S8192 causal). Measured, us per
-// call, against one 128-row tile per block on TF32 pairs: B1 H4 S16384 D128 causal 825 (2700), B1 H8 S1024 D64 dense
-// 20.6 (37), H4/kvH1 8231 x 9075 rows D64 causal 161 (272).
+// What bounds it: at head_dim 128 the issue of the MMAs. A pair of tiles of 64 keys needs 3330 clocks of the tensor core, in 72
+// instructions of 32 to 64; its queue holds a few of them, so whatever the issuing warp does between two batches is
+// time in which the tensor core is idle (P is always written when the warp comes to it). A satisfied wait costs it 100 to
+// 150 clocks, a sum of 64 bits in a descriptor half as much as an instruction. us, B1 H4 S16384 D128 causal: 824; descriptors
+// as 32-bit words 781; without a wait for V and with one for K 740; K and V split ahead 719; a warp for each query tile then
+// 672. At head_dim 64 it is the softmax (hi and lo of P beside the exponentials). Against one 128-row tile per block on
+// TF32 pairs: B1 H8 S1024 D64 dense 20.6 (37), H4/kvH1 8231 x 9075 rows D64 causal 161 (272).
 //
 // Every wait on an mbarrier is bounded (see tc_common.cuh); a wait that runs out reports into
 // the device status word and the block unwinds.
+#include <algorithm>
 #include <atomic>
 
 #include "tc_common.cuh"
@@ -83,8 +86,20 @@ constexpr int kScoreRange = 17;
 // A tile as v_exp holds it: V's exponent + kExpBias, or kNoUnit, or kWide with or without kPlain.
 constexpr int kExpBias = 512, kWide = 1 << 12, kPlain = 1 << 13;
 
-template <int DR, bool kSplit>
+// What the softmax needs to know of a key tile besides its split K and V, as the form with split operands keeps it in
+// the workspace and copies it with the tile: factors of the keys, exponents of V's keys, the V tile's as v_exp holds it,
+// and the exponent of the largest magnitude of K.
+constexpr int kMetaG = 0, kMetaVKey = kBNf * 4, kMetaVExp = kMetaVKey + kBNf, kMetaKTop = kMetaVExp + 4, kMetaBytes = 384;
+// The split operands of a call in its workspace, by KV head (as the tensor map counts them) and tile.
+struct SplitKV {
+  unsigned char *k, *v, *meta;
+  int tiles;               // of all key segments of a head
+  int beg[RA_MAX_SEG];     // first tile of a segment
+};
+
+template <int DR, bool kSplit, bool kPre = false>
 struct F32Cfg {
+  static constexpr int kThreads = kPre ? 384 : kThreadsF;
   static constexpr int kTiles = 2;
   static constexpr int D = DR < 64 ? 64 : DR;           // columns of a split tile row
   // Where Q's terms go. Head_dim 32 / 64: both into tensor memory, beside S, P and O. Head_dim 128:
@@ -94,6 +109,9 @@ struct F32Cfg {
   // slot that P.V of the tile before last frees.)
   static constexpr bool kQLoInTmem = D == 64;
   static constexpr bool kAlias = D == 128;
+  // There one warp issues for both query tiles in turn, or, where no splitters take issue slots, a warp for each (B1 H4
+  // S16384 D128 causal: 672 against 719 with split operands, 770 against 740 us without).
+  static constexpr bool kTurns = kAlias && kPre;
   static constexpr int kBoxes = DR / 32;                // raw boxes: 32 fp32 = 128 bytes of a row
   static constexpr int kGroups = D / 64;                // 64-column groups of a split tile
   static constexpr int kBoxBytes = kBNf * 128;
@@ -110,13 +128,13 @@ struct F32Cfg {
   static constexpr int kOffQ = 0;
   static constexpr int kOffKV = kTiles * kQBytes;
   static constexpr int kOffBar = kOffKV + kStages * kSlotBytes;
-  static constexpr int kNumBars = 2 + 3 * kStages + 8 + 1;
+  static constexpr int kNumBars = 2 + 3 * kStages + 8 + 3;
   static constexpr int kOffSlot = kOffBar + kNumBars * 8;      // tensor-memory address, abort flag
   static constexpr int kOffRed = (kOffSlot + 8 + 15) & ~15;    // [2][2][8] range of a V tile by warp
   static constexpr int kOffVExp = kOffRed + 128;               // [16] exponents of V tiles
   static constexpr int kOffG = (kOffVExp + 64 + 15) & ~15;     // [kGDepth][kBNf] factors of K
-  static constexpr int kOffVKey = kOffG + kGDepth * kBNf * 4;  // [8][kBNf] exponents of V's keys
-  static constexpr int kOffQTop = kOffVKey + 8 * kBNf;         // [2][4] exponents of Q by softmax warp
+  static constexpr int kOffVKey = kOffG + kGDepth * (kPre ? kMetaBytes : kBNf * 4);  // [8][kBNf] exponents of V's keys
+  static constexpr int kOffQTop = kOffVKey + (kPre ? 0 : 8 * kBNf);  // [2][4] exponents of Q by softmax warp
   static constexpr int kOffMl = kOffQTop + 32;
   static constexpr int kMlBytes = kSplit ? kTiles * kBM * 8 : 0;
   // where the unsplit form stages its rows (see RowStore): over Q's lo tiles, else in a place of their own
@@ -128,8 +146,9 @@ struct F32Cfg {
   // each, 61440 in all. Head_dim 128 spills 60 bytes so and 128 with 40 / 144 / 72: us per call B1 H4 S16384 causal 828 /
   // 848. The others spill next to nothing either way and gain from registers for the splitters: H8 S8192 D64 242 (247 with
   // the split of head_dim 128), H16/kvH8 978 rows on 5874 keys D32 93.8 (97.0).
-  static constexpr int kRegsIssue = D == 128 ? 64 : 40, kRegsSoftmax = D == 128 ? 152 : 144, kRegsSplit = D == 128 ? 56 : 72;
-  static_assert(128 * kRegsIssue + 256 * kRegsSoftmax + 256 * kRegsSplit <= 640 * 96, "setmaxnreg draws on the launch's registers");
+  static constexpr int kRegsIssue = kPre ? 72 : D == 128 ? 64 : 40, kRegsSoftmax = kPre ? 216 : D == 128 ? 152 : 144,
+                       kRegsSplit = kPre ? 0 : D == 128 ? 56 : 72;
+  static_assert(128 * kRegsIssue + 256 * kRegsSoftmax + 256 * kRegsSplit <= (kPre ? 384 * 168 : 640 * 96), "setmaxnreg draws on the launch's registers");
   static constexpr int kColS = 0, kColP = kAlias ? 0 : 64, kColO = kAlias ? 64 : 128, kColQ = 192;
   static_assert(kSmemBytes <= 232448, "shared memory budget");
   static_assert(kTiles * kBM * ((DR + 4) * 4 + 8) <= kOffBar, "staging of the key-split merge");
@@ -193,12 +212,62 @@ __device__ inline void st_shared_u4(unsigned addr, unsigned a, unsigned b, unsig
                : "memory");
 }
 
-template <int DR, bool kSplit>
-__global__ void __launch_bounds__(kThreadsF, 1)
+// The range of a splitter warp's eight rows of V (x: this lane's pieces of one of them, mx: the largest magnitude
+// among them, out: of all eight rows): returns what their tile's largest must not exceed, as the upper half of
+// its bits, or the tile is wide. Also writes the exponents of the keys. The smallest nonzero maximum of a key and of
+// a column count. No column lies below the warp's smallest element, which is near enough for most tiles.
+template <int kUnits>
+__device__ inline unsigned v_range(const float (&x)[kUnits][8], unsigned& mx, int lane, unsigned char* v_key) {
+  const int r8 = lane & 7, p4 = lane >> 3;
+  float fn = fabsf(x[0][0]);
+#pragma unroll
+  for (int u = 0; u < kUnits; ++u)
+#pragma unroll
+    for (int i = 0; i < 8; i += 2) fn = min3(fn, fabsf(x[u][i]), fabsf(x[u][i + 1]));
+  mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
+  mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+  if (p4 == 0) v_key[r8] = static_cast<unsigned char>(mx >> 23);
+  unsigned low = (mx == 0 ? 0xffffu : mx >> 16) + (kKeyRange << 7);
+  const unsigned least = __reduce_min_sync(0xffffffffu, __float_as_uint(fn)) >> 16;
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  // (a zero says nothing: the rows behind a ragged end are zeros)
+  if (__builtin_expect(least > 0 && least + ((kColRange - 1) << 7) >= mx >> 16, 1)) {
+    low = min(low, least + (kColRange << 7));
+  } else {
+    // column by column, the upper halves of two magnitudes in a word; each lane ends with its
+    // share of the columns (1 below, so that none is zero)
+    unsigned c2[4 * kUnits];
+#pragma unroll
+    for (int i = 0; i < 4 * kUnits; ++i)
+      c2[i] = __byte_perm(__float_as_uint(x[i / 4][2 * (i & 3)]), __float_as_uint(x[i / 4][2 * (i & 3) + 1]),
+                          0x7632) & 0x7fff7fffu;
+#pragma unroll
+    for (int step = 0; step < 3; ++step) {
+      const bool odd = (lane >> step) & 1;
+      const int n = (4 * kUnits) >> (step + 1);
+      if (n > 0) {
+#pragma unroll
+        for (int i = 0; i < 2 * kUnits; ++i)
+          if (i < n)
+            c2[i] = __vmaxu2(odd ? c2[i + n] : c2[i],
+                             __shfl_xor_sync(0xffffffffu, odd ? c2[i] : c2[i + n], 1 << step));
+      } else {
+        c2[0] = __vmaxu2(c2[0], __shfl_xor_sync(0xffffffffu, c2[0], 1 << step));
+      }
+    }
+    unsigned low2 = __vsub2(c2[0], 0x00010001u);
+    if constexpr (kUnits == 4) low2 = __vminu2(low2, __vsub2(c2[1], 0x00010001u));
+    low = min(low, min(low2 & 0xffffu, low2 >> 16) + (kColRange << 7));
+  }
+  return __reduce_min_sync(0xffffffffu, low);
+}
+
+template <int DR, bool kSplit, bool kPre>
+__global__ void __launch_bounds__((F32Cfg<DR, kSplit, kPre>::kThreads), 1)
     step_f32_kernel(const __grid_constant__ CUtensorMap tmap_k,
                     const __grid_constant__ CUtensorMap tmap_v, const float* q_g,
-                    const float* k_g, long long kv_head_stride, const TcArgs a) {
-  using C = F32Cfg<DR, kSplit>;
+                    const float* k_g, long long kv_head_stride, const TcArgs a, const __grid_constant__ SplitKV pre) {
+  using C = F32Cfg<DR, kSplit, kPre>;
   extern __shared__ __align__(1024) unsigned char smem[];  // 128B-swizzled tiles
   const unsigned s_base = smem_u32(smem);
   const unsigned s_q = s_base + C::kOffQ;
@@ -213,6 +282,7 @@ __global__ void __launch_bounds__(kThreadsF, 1)
   const unsigned bar_p_full = bar_s_free + 16;                   // [2]
   const unsigned bar_o_done = bar_p_full + 16;                   // [2] P.V done
   const unsigned bar_v_max = bar_o_done + 16;                    // a V tile's maxima by warp written
+  const unsigned bar_turn = bar_v_max + 8;                       // [2] the MMAs of this query tile may go out
   unsigned* tmem_slot = reinterpret_cast<unsigned*>(smem + C::kOffSlot);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   volatile unsigned* red = reinterpret_cast<volatile unsigned*>(smem + C::kOffRed);
@@ -272,11 +342,12 @@ __global__ void __launch_bounds__(kThreadsF, 1)
       mbar_init(bar_s_free + 8 * w, kBM);
       mbar_init(bar_p_full + 8 * w, kBM);
       mbar_init(bar_o_done + 8 * w, 1);
+      mbar_init(bar_turn + 8 * w, 1);
     }
     mbar_init(bar_v_max, kSplitThreads / 32);
     for (int s = 0; s < C::kStages; ++s) {
       mbar_init(bar_kv_raw + 8 * s, 1);
-      mbar_init(bar_kv_full + 8 * s, kSplitThreads);
+      mbar_init(bar_kv_full + 8 * s, kPre ? 1 : kSplitThreads);
       mbar_init(bar_kv_empty + 8 * s, C::kAlias ? 1 : live);
     }
     *abort_flag = gone != 0;
@@ -309,6 +380,23 @@ __global__ void __launch_bounds__(kThreadsF, 1)
     return;
   }
 
+  // Split operands come as they are: the block's largest magnitude of Q meets each tile's of K where the tile is used.
+  [[maybe_unused]] auto wait_q = [&](int* q_top) {
+    bool ok = true;
+    *q_top = 0;
+    for (int w = 0; w < live && ok; ++w) {
+      ok = mbar_wait(bar_q_full + 8 * w, 0, abort_flag, a.status, 3, w, a.wait_ns);
+      if (ok) *q_top = max(*q_top, max(max(q_tops[4 * w], q_tops[4 * w + 1]), max(q_tops[4 * w + 2], q_tops[4 * w + 3])));
+    }
+    return ok;
+  };
+  [[maybe_unused]] const unsigned char* const meta_ring = smem + C::kOffG;
+  [[maybe_unused]] auto tile_exp = [&](int j, int q_top) {  // as v_exp would hold it
+    const unsigned char* const m = meta_ring + (j % C::kGDepth) * kMetaBytes;
+    const int ve = *reinterpret_cast<const volatile int*>(m + kMetaVExp), k_top = *reinterpret_cast<const volatile int*>(m + kMetaKTop);
+    return q_top + k_top - 254 >= kScoreRange ? kWide | kPlain : ve;
+  };
+
   // (registers follow the work, see F32Cfg)
   if (warp < 4) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::kRegsIssue));
@@ -316,6 +404,7 @@ __global__ void __launch_bounds__(kThreadsF, 1)
       // ---------------------------------------------------------- TMA producer ----
       if (lane == 0 && n_tiles > 0) {
         int it = 0;
+        [[maybe_unused]] int k_top = 0, q_top = 0;
         bool ok = *abort_flag == 0;
         // (the status word once more, see step_tc.cu: behind a launch that gave up no V comes)
         const int lost = *reinterpret_cast<volatile int*>(a.status);
@@ -341,16 +430,38 @@ __global__ void __launch_bounds__(kThreadsF, 1)
                 ok = false;
                 break;
               }
-              mbar_expect_tx(bar_kv_raw + 8 * slot, C::kRawBytes);
               const CUtensorMap* map = which == 0 ? &tmap_k : &tmap_v;
-              for (int bx = 0; bx < C::kBoxes; ++bx)
-                tma_load_3d(s_kv + slot * C::kSlotBytes + bx * C::kBoxBytes, map, bar_kv_raw + 8 * slot,
-                            bx * 32, k_row, k_head);
+              auto raw = [&](unsigned bar) {
+                for (int bx = 0; bx < C::kBoxes; ++bx)
+                  tma_load_3d(s_kv + slot * C::kSlotBytes + bx * C::kBoxBytes, map, bar, bx * 32, k_row, k_head);
+              };
+              if constexpr (kPre) {
+                const unsigned bar = bar_kv_full + 8 * slot;
+                const size_t tile = static_cast<size_t>(kv_bh) * pre.tiles + pre.beg[sk] + t;
+                const unsigned char* const meta = pre.meta + tile * kMetaBytes;
+                if (which == 0) {
+                  mbar_expect_tx(bar, C::kSlotBytes);
+                  bulk_load(s_kv + slot * C::kSlotBytes, pre.k + tile * C::kSlotBytes, C::kSlotBytes, bar);
+                  k_top = *reinterpret_cast<const volatile int*>(meta + kMetaKTop);  // (used with V)
+                } else {
+                  // The meta data come with V, whose slot, other than K's, is not loaded again before the softmax of the
+                  // tile is done: a wait for V's barrier can stand for them.
+                  if (it == 1 && !(ok = wait_q(&q_top))) break;
+                  const bool plain = q_top + k_top - 254 >= kScoreRange;  // P * V will be taken in plain fp32
+                  mbar_expect_tx(bar, (plain ? C::kRawBytes : C::kSlotBytes) + kMetaBytes);
+                  if (plain) raw(bar);
+                  else bulk_load(s_kv + slot * C::kSlotBytes, pre.v + tile * C::kSlotBytes, C::kSlotBytes, bar);
+                  bulk_load(s_base + C::kOffG + ((it >> 1) % C::kGDepth) * kMetaBytes, meta, kMetaBytes, bar);
+                }
+              } else {
+                mbar_expect_tx(bar_kv_raw + 8 * slot, C::kRawBytes);
+                raw(bar_kv_raw + 8 * slot);
+              }
             }
           }
         }
       }
-    } else if (warp == 1 || (!C::kAlias && warp == 2 && live == 2)) {
+    } else if (warp == 1 || ((!C::kAlias || C::kTurns) && warp == 2 && live == 2)) {
       // ----------------------------------------------------------- MMA issuers ----
       if (n_tiles > 0) {
         constexpr unsigned idesc_s = make_idesc(0u, 0, kBNf, kBM);
@@ -362,15 +473,17 @@ __global__ void __launch_bounds__(kThreadsF, 1)
           return __all_sync(0xffffffffu,
                             mbar_wait(bar, parity, abort_flag, a.status, which, tile, a.wait_ns)) != 0;
         };
-        // ring item of K_t: 2t, of V_t: 2t + 1
+        [[maybe_unused]] int q_top = 0;
+        if constexpr (kPre) wait_q(&q_top);  // (one that runs out is met again below)
+        // ring item of K_t: 2t, of V_t: 2t + 1 (which the softmax has waited for when its P is written: no wait here)
         auto wait_kv = [&](int it, int which, int t) {
           return wait(bar_kv_full + 8 * (it % C::kStages), (it / C::kStages) & 1, which, t);
         };
         // `last`: no other query tile reads the slot after this one
         auto issue_s = [&](int t, int w, bool last) {
           const int slot = (2 * t) % C::kStages;
-          const unsigned long long kd = desc_kmajor(s_kv + slot * C::kSlotBytes);
-          [[maybe_unused]] const unsigned long long qd = desc_kmajor(s_q + w * C::kQBytes);
+          const unsigned kd = static_cast<unsigned>(desc_kmajor(s_kv + slot * C::kSlotBytes));
+          [[maybe_unused]] const unsigned qd = static_cast<unsigned>(desc_kmajor(s_q + w * C::kQBytes));
           const unsigned t_s = tmem_base + 256 * w + C::kColS, t_q = tmem_base + 256 * w + C::kColQ;
           if (elect_one()) {
             // small terms first: lo*hi, hi*lo, hi*hi
@@ -381,9 +494,9 @@ __global__ void __launch_bounds__(kThreadsF, 1)
                 const unsigned off_k = (ks / 4) * kGroup + (ks % 4) * 2 + (term == 1 ? kLo : 0);
                 const unsigned acc = (term > 0 || ks > 0) ? 1u : 0u;
                 if (C::kQLoInTmem || term > 0) {
-                  mma_ts(t_s, t_q + ks * 8 + (term == 0 ? 32 : 0), kd + off_k, idesc_s, acc);
+                  mma_ts_lo(t_s, t_q + ks * 8 + (term == 0 ? 32 : 0), kd + off_k, kDescHi, idesc_s, acc);
                 } else {
-                  mma_ss(t_s, qd + (ks / 4) * kQBox + (ks % 4) * 2, kd + off_k, idesc_s, acc);
+                  mma_ss_lo(t_s, qd + (ks / 4) * kQBox + (ks % 4) * 2, kd + off_k, kDescHi, idesc_s, acc);
                 }
               }
             }
@@ -394,19 +507,19 @@ __global__ void __launch_bounds__(kThreadsF, 1)
         auto issue_pv = [&](int t, int w, bool last) {
           const int slot = (2 * t + 1) % C::kStages;
           // MN-major V: 64 columns per 128-byte row, groups 2 boxes apart, 16 keys per k-step
-          const unsigned long long vd =
-              desc_mnmajor(s_kv + slot * C::kSlotBytes, 2 * C::kBoxBytes, 1024);
+          const unsigned vd = static_cast<unsigned>(desc_mnmajor(s_kv + slot * C::kSlotBytes, 2 * C::kBoxBytes, 1024));
           const unsigned t_p = tmem_base + 256 * w + C::kColP, t_o = tmem_base + 256 * w + C::kColO;
-          const bool wide = (v_exp[t & 15] & kWide) != 0;  // the softmax threads have added this tile to O
+          // (marked: the softmax threads have added this tile to O)
+          const bool wide = ((kPre ? tile_exp(t, q_top) : v_exp[t & 15]) & kWide) != 0;
           if (elect_one()) {
             if (!wide) {
 #pragma unroll
               for (int term = 0; term < 3; ++term) {
 #pragma unroll
                 for (int ks = 0; ks < kBNf / 16; ++ks)
-                  mma_ts(t_o, t_p + ks * 8 + (term == 0 ? 32 : 0),
-                         vd + ks * (2048 >> 4) + (term == 1 ? kLo : 0), idesc_pv,
-                         (t > 0 || term > 0 || ks > 0) ? 1u : 0u);
+                  mma_ts_lo(t_o, t_p + ks * 8 + (term == 0 ? 32 : 0),
+                            vd + ks * (2048 >> 4) + (term == 1 ? kLo : 0), kDescHi, idesc_pv,
+                            (t > 0 || term > 0 || ks > 0) ? 1u : 0u);
               }
             }
             tc_commit(bar_o_done + 8 * w);
@@ -414,7 +527,30 @@ __global__ void __launch_bounds__(kThreadsF, 1)
           }
         };
         bool ok = true;
-        if constexpr (C::kAlias) {
+        if constexpr (C::kTurns) {
+          // As below, but with a warp for each query tile, whose turn comes with the end of the other's batch: it has done its
+          // waits by then. The tensor core's queue holds a few instructions, so a batch that follows at once leaves no gap.
+          const int w = warp - 1;
+          auto turn = [&](int n) { return live == 1 || wait(bar_turn + 8 * w, n & 1, 12, n); };
+          auto pass = [&]() {
+            if (live == 2 && elect_one()) mbar_arrive(bar_turn + 8 * (1 - w));
+          };
+          ok = wait(bar_q_full + 8 * w, 0, 3, w) && wait_kv(0, 5, 0) && (w == 0 || turn(0));
+          if (ok) {
+            tc_fence_after();
+            issue_s(0, w, w == live - 1);
+            pass();
+          }
+          for (int t = 0; t < n_tiles && ok; ++t) {
+            const bool more = t + 1 < n_tiles;
+            ok = (!more || wait_kv(2 * t + 2, 5, t)) && wait(bar_p_full + 8 * w, t & 1, 6, t) && turn(t + w);
+            if (!ok) break;
+            tc_fence_after();
+            issue_pv(t, w, w == live - 1);
+            if (more) issue_s(t + 1, w, w == live - 1);
+            pass();
+          }
+        } else if constexpr (C::kAlias) {
           // One warp issues for both query tiles, in turn: P.V of tile t and the scores of tile t + 1, which
           // overwrite P, of one query tile, then those of the other. The tensor core runs them in that
           // order, so one tile's softmax works under the other's MMAs. (Two issuing warps end in step:
@@ -428,16 +564,13 @@ __global__ void __launch_bounds__(kThreadsF, 1)
           }
           for (int t = 0; t < n_tiles && ok; ++t) {
             const bool more = t + 1 < n_tiles;
+            ok = !more || wait_kv(2 * t + 2, 5, t);
             for (int w = 0; w < live && ok; ++w) {
-              ok = wait_kv(2 * t + 1, 4, t) && wait(bar_p_full + 8 * w, t & 1, 6, t);
+              ok = wait(bar_p_full + 8 * w, t & 1, 6, t);
               if (!ok) break;
               tc_fence_after();
               issue_pv(t, w, w == live - 1);
-              if (!more) continue;
-              ok = wait_kv(2 * t + 2, 5, t);
-              if (!ok) break;
-              tc_fence_after();
-              issue_s(t + 1, w, w == live - 1);
+              if (more) issue_s(t + 1, w, w == live - 1);
             }
           }
         } else {
@@ -454,7 +587,7 @@ __global__ void __launch_bounds__(kThreadsF, 1)
               tc_fence_after();
               issue_s(t + 1, w, true);
             }
-            ok = wait_kv(2 * t + 1, 4, t) && wait(bar_p_full + 8 * w, t & 1, 6, t);
+            ok = wait(bar_p_full + 8 * w, t & 1, 6, t);
             if (!ok) break;
             tc_fence_after();
             issue_pv(t, w, true);
@@ -465,7 +598,8 @@ __global__ void __launch_bounds__(kThreadsF, 1)
     if constexpr (kSplit) {  // the three meetings of merge_key_split
       for (int i = 0; i < 3; ++i) cluster_sync_threads();
     }
-  } else if (warp >= 12) {
+  } else if (!kPre && warp >= 12) {
+    if constexpr (!kPre) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::kRegsSplit));
     // --------------------------------------------------------------- splitters ----
     // A warp owns eight rows of every tile; its lanes own 16-byte pieces of the split rows (8
@@ -518,50 +652,8 @@ __global__ void __launch_bounds__(kThreadsF, 1)
           }
           k_top = static_cast<int>(__reduce_max_sync(0xffffffffu, mx) >> 23);  // (the warp's rows have been read)
         } else {
-          // V: by tile. How wide it is: the smallest nonzero maximum of a key and of a column among the
-          // warp's eight keys. No column lies below the warp's smallest element, which is near enough for
-          // most tiles.
-          float fn = fabsf(x[0][0]);
-#pragma unroll
-          for (int u = 0; u < kUnits; ++u)
-#pragma unroll
-            for (int i = 0; i < 8; i += 2) fn = min3(fn, fabsf(x[u][i]), fabsf(x[u][i + 1]));
-          mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
-          mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
-          if (p4 == 0) smem[C::kOffVKey + ((it >> 1) & 7) * kBNf + sw * 8 + r8] = static_cast<unsigned char>(mx >> 23);
-          unsigned low = (mx == 0 ? 0xffffu : mx >> 16) + (kKeyRange << 7);
-          const unsigned least = __reduce_min_sync(0xffffffffu, __float_as_uint(fn)) >> 16;
-          mx = __reduce_max_sync(0xffffffffu, mx);
-          // (a zero says nothing: the rows behind a ragged end are zeros)
-          if (__builtin_expect(least > 0 && least + ((kColRange - 1) << 7) >= mx >> 16, 1)) {
-            low = min(low, least + (kColRange << 7));
-          } else {
-            // column by column, the upper halves of two magnitudes in a word; each lane ends with its
-            // share of the columns (1 below, so that none is zero)
-            unsigned c2[4 * kUnits];
-#pragma unroll
-            for (int i = 0; i < 4 * kUnits; ++i)
-              c2[i] = __byte_perm(__float_as_uint(x[i / 4][2 * (i & 3)]), __float_as_uint(x[i / 4][2 * (i & 3) + 1]),
-                                  0x7632) & 0x7fff7fffu;
-#pragma unroll
-            for (int step = 0; step < 3; ++step) {
-              const bool odd = (lane >> step) & 1;
-              const int n = (4 * kUnits) >> (step + 1);
-              if (n > 0) {
-#pragma unroll
-                for (int i = 0; i < 2 * kUnits; ++i)
-                  if (i < n)
-                    c2[i] = __vmaxu2(odd ? c2[i + n] : c2[i],
-                                     __shfl_xor_sync(0xffffffffu, odd ? c2[i] : c2[i + n], 1 << step));
-              } else {
-                c2[0] = __vmaxu2(c2[0], __shfl_xor_sync(0xffffffffu, c2[0], 1 << step));
-              }
-            }
-            unsigned low2 = __vsub2(c2[0], 0x00010001u);
-            if constexpr (kUnits == 4) low2 = __vminu2(low2, __vsub2(c2[1], 0x00010001u));
-            low = min(low, min(low2 & 0xffffu, low2 >> 16) + (kColRange << 7));
-          }
-          low = __reduce_min_sync(0xffffffffu, low);
+          // V: by tile
+          unsigned low = v_range<kUnits>(x, mx, lane, smem + C::kOffVKey + ((it >> 1) & 7) * kBNf + sw * 8);
           if (it == 1) {
             for (int w = 0; w < live && ok; ++w) {
               ok = __all_sync(0xffffffffu, mbar_wait(bar_q_full + 8 * w, 0, abort_flag, a.status, 3, w, a.wait_ns)) != 0;
@@ -612,6 +704,7 @@ __global__ void __launch_bounds__(kThreadsF, 1)
     }
     if constexpr (kSplit) {
       for (int i = 0; i < 3; ++i) cluster_sync_threads();
+    }
     }
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(C::kRegsSoftmax));
@@ -680,6 +773,8 @@ __global__ void __launch_bounds__(kThreadsF, 1)
     int j = 0;
     const int n_seg = mine ? a.kmap.n_seg : 0;
     TileShare share{share_beg, share_end, 0};
+    [[maybe_unused]] int q_top = 0;
+    if constexpr (kPre) ok = __all_sync(0xffffffffu, !mine || wait_q(&q_top)) != 0;
     for (int sk = 0; sk < n_seg && ok; ++sk) {
       const TileRange tr =
           share.clip(tile_range<kBNf>(a.kmap, sk, a.stride, causal, a.doc_len, qmin, qmax));
@@ -714,12 +809,12 @@ __global__ void __launch_bounds__(kThreadsF, 1)
         const int vit = 2 * j + 1;
         ok = mbar_wait(bar_kv_full + 8 * (vit % C::kStages), (vit / C::kStages) & 1, abort_flag, a.status,
                        11, j, a.wait_ns);
-        const int ve = v_exp[j & 15];
+        const int ve = kPre ? tile_exp(j, q_top) : v_exp[j & 15];
         ok = ok && mbar_wait(bar_s_full + 8 * w, j & 1, abort_flag, a.status, 7, j, a.wait_ns);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tc_fence_after();
-        const unsigned g_at = s_base + C::kOffG + (j % C::kGDepth) * kBNf * 4;
+        const unsigned g_at = s_base + C::kOffG + (j % C::kGDepth) * (kPre ? kMetaBytes : kBNf * 4);
         if (__builtin_expect((ve & kWide) != 0, 0)) {
           // A marked tile: P * V in plain fp32 from V as it landed in its slot (every lane reads the same
           // 16 bytes), and the scores too if Q and K ask for it. Short loops over tensor memory, so that
@@ -788,7 +883,8 @@ __global__ void __launch_bounds__(kThreadsF, 1)
               for (int i = 0; i < 8; ++i) {
                 x[i] = ex2(fmaf(x[i], row_f, n));
                 sum += x[i];
-                const int vk = smem[C::kOffVKey + (j & 7) * kBNf + i0 + i];
+                const int vk = kPre ? meta_ring[(j % C::kGDepth) * kMetaBytes + kMetaVKey + i0 + i]
+                                    : smem[C::kOffVKey + (j & 7) * kBNf + i0 + i];
                 if (x[i] > 0.f && vk > 0) c_top = max(c_top, (__float_as_int(x[i]) >> 23) + vk);
               }
               tmem_st8(t_p + i0, x);
@@ -1022,11 +1118,131 @@ __global__ void __launch_bounds__(kThreadsF, 1)
   }
 }
 
+// Splits K and V once for all query blocks of a call: a block per key tile and KV head writes, to the workspace, what the
+// splitter warps leave in a ring slot, byte for byte, and the tile's meta data. The step then copies whole slots, and has
+// neither splitter warps (two thirds of its issue slots at head_dim 64) nor their traffic in shared memory. Bound by
+// memory: H4 S16384 D128, 67 MB read and as many written, 27 us.
+template <int DR>
+__global__ void __launch_bounds__(kSplitThreads) split_kv_kernel(const float* k, const float* v, long long kv_head_stride,
+                                                                const __grid_constant__ TcArgs a,
+                                                                const __grid_constant__ SplitKV pre, int k_rows) {
+  using C = F32Cfg<DR, false, true>;
+  constexpr int kUnits = DR / 32;
+  __shared__ unsigned red[3][8];
+  let_next_start();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r8 = lane & 7, p4 = lane >> 3;
+  int sk = 0;
+  while (sk + 1 < a.kmap.n_seg && pre.beg[sk + 1] <= static_cast<int>(blockIdx.x)) ++sk;
+  const int row = a.kseg_row[sk] + (static_cast<int>(blockIdx.x) - pre.beg[sk]) * kBNf + warp * 8 + r8;
+  const size_t tile = static_cast<size_t>(blockIdx.y) * pre.tiles + blockIdx.x;
+  const long long src = (a.kseg_head[sk] + static_cast<long long>(blockIdx.y)) * kv_head_stride + static_cast<long long>(row) * DR;
+  const unsigned row_off = (warp * 8 + r8) * 128;
+  unsigned char* const meta = pre.meta + tile * kMetaBytes;
+  wait_for_previous();
+  float x[2][kUnits][8];
+  unsigned mx[2];
+#pragma unroll
+  for (int which = 0; which < 2; ++which) {
+    const float4* const p = reinterpret_cast<const float4*>((which == 0 ? k : v) + src);
+#pragma unroll
+    for (int u = 0; u < kUnits; ++u) {
+      const int piece = p4 + 4 * u;
+      const float4 v0 = row < k_rows ? p[2 * piece] : make_float4(0.f, 0.f, 0.f, 0.f);
+      const float4 v1 = row < k_rows ? p[2 * piece + 1] : make_float4(0.f, 0.f, 0.f, 0.f);
+      x[which][u][0] = v0.x, x[which][u][1] = v0.y, x[which][u][2] = v0.z, x[which][u][3] = v0.w;
+      x[which][u][4] = v1.x, x[which][u][5] = v1.y, x[which][u][6] = v1.z, x[which][u][7] = v1.w;
+    }
+  }
+#pragma unroll
+  for (int which = 0; which < 2; ++which) {
+    mx[which] = 0;
+#pragma unroll
+    for (int u = 0; u < kUnits; ++u)
+#pragma unroll
+      for (int i = 0; i < 8; ++i) mx[which] = max(mx[which], finite_abs_bits(x[which][u][i]));
+  }
+  // K: by key
+  unsigned key = max(mx[0], __shfl_xor_sync(0xffffffffu, mx[0], 8));
+  key = max(key, __shfl_xor_sync(0xffffffffu, key, 16));
+  const int ek = scale_exp(key, kMaxExpK);
+  if (p4 == 0) reinterpret_cast<float*>(meta + kMetaG)[warp * 8 + r8] = pow2i(-ek - kBias);
+  const unsigned k_max = __reduce_max_sync(0xffffffffu, mx[0]);
+  // V: by tile
+  const unsigned low_w = v_range<kUnits>(x[1], mx[1], lane, meta + kMetaVKey + warp * 8);
+  if (lane == 0) red[0][warp] = k_max, red[1][warp] = mx[1], red[2][warp] = low_w;
+  __syncthreads();
+  unsigned k_all = 0, v_all = 0, low = 0xffffffffu;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    k_all = max(k_all, red[0][i]);
+    v_all = max(v_all, red[1][i]);
+    low = min(low, red[2][i]);
+  }
+  const int e = scale_exp(v_all, kMaxExp);
+  const bool wide = low < v_all >> 16;
+  if (threadIdx.x == 0) {
+    *reinterpret_cast<int*>(meta + kMetaVExp) = wide ? kWide : v_all == 0 ? kNoUnit : e + kExpBias;
+    *reinterpret_cast<int*>(meta + kMetaKTop) = static_cast<int>(k_all >> 23);
+  }
+#pragma unroll
+  for (int which = 0; which < 2; ++which) {
+    unsigned char* const base = (which == 0 ? pre.k : pre.v) + tile * C::kSlotBytes + row_off;
+    const float sc = pow2i(which == 0 ? ek : e);
+#pragma unroll
+    for (int u = 0; u < kUnits; ++u) {
+      const int piece = p4 + 4 * u;
+      if (which == 1 && wide) {  // as it is, in the layout in which the copy of an fp32 tile lands
+        unsigned char* const box = base + (piece >> 2) * C::kBoxBytes;
+        const int c = (piece & 3) * 2;
+        *reinterpret_cast<float4*>(box + ((c ^ r8) << 4)) = make_float4(x[1][u][0], x[1][u][1], x[1][u][2], x[1][u][3]);
+        *reinterpret_cast<float4*>(box + (((c + 1) ^ r8) << 4)) = make_float4(x[1][u][4], x[1][u][5], x[1][u][6], x[1][u][7]);
+        continue;
+      }
+      unsigned char* const hi_at = base + (piece >> 3) * 2 * C::kBoxBytes + (((piece & 7) ^ r8) << 4);
+      unsigned hi[4], lo[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) split_pair(x[which][u][2 * i] * sc, x[which][u][2 * i + 1] * sc, hi[i], lo[i]);
+      *reinterpret_cast<uint4*>(hi_at) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+      *reinterpret_cast<uint4*>(hi_at + C::kBoxBytes) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+    }
+  }
+}
+
 // ---- host side ----------------------------------------------------------------------
 
-template <int DR, bool kSplit>
+// Tiles of all key segments of a head, and the workspace of the form with split operands.
+int split_tiles(const StepArgs& a) { return (a.kmap.seg_len + kBNf - 1) / kBNf * a.kmap.n_seg; }
+template <int DR>
+size_t split_bytes(const StepArgs& a) {
+  using C = F32Cfg<DR, false, true>;
+  return static_cast<size_t>(a.B) * a.kvH * split_tiles(a) * (2 * C::kSlotBytes + kMetaBytes);
+}
+// Whether K and V are split ahead, given a workspace: a pair of query tiles saves 0.3 us a key tile (0.35 at head_dim 128), and the
+// launch ahead costs 5 us and the way of K, V and their terms through memory. us per call, split by every block / ahead:
+// B1 H4 S16384 D128 causal 753 / 674, H8 S8192 D64 causal 241 / 217, H16/kvH8 B2 1000 rows on 6000 keys D32 168 / 152,
+// H8/kvH1 3810 rows dense D64 117 / 101; not so H8 2048 rows causal D128 75 / 81, H8 1024 rows dense D64 21 / 27. Over 130
+// random calls (300 to 16384 rows) the 53 taken ones 0.87 in the mean, 0.96 at worst.
+template <int DR>
+bool split_ahead(const StepArgs& a) {
+  long long steps = 0;  // of one head
+  const int per_seg = (a.qmap.seg_len + 2 * kBM - 1) / (2 * kBM);
+  for (int sq = 0; sq < a.qmap.n_seg; ++sq)
+    for (int tq = 0; tq < per_seg; ++tq) {
+      const int row0 = tq * 2 * kBM, rows = std::min(2 * kBM, a.qmap.seg_len - row0);
+      const int qmin = a.qmap.base[sq] + row0 * a.stride;
+      for (int sk = 0; sk < a.kmap.n_seg; ++sk) {
+        const TileRange r = tile_range<kBNf>(a.kmap, sk, a.stride, (a.flags & RA_STEP_CAUSAL) != 0, a.doc_len, qmin,
+                                             qmin + (rows - 1) * a.stride);
+        steps += r.hi - r.lo;
+      }
+    }
+  constexpr double kSms = 148, kSaves = DR == 128 ? 0.35 : 0.3, kLaunch = 5, kBytesPerUs = 5e6;
+  const double bytes = 16.0 * a.B * a.kvH * split_tiles(a) * kBNf * DR;  // read and written
+  return kSaves * a.B * a.H * steps / kSms > kLaunch + bytes / kBytesPerUs;
+}
+template <int DR, bool kSplit, bool kPre>
 int launch_f32(const StepArgs& a, cudaStream_t stream, int key_split) {
-  using C = F32Cfg<DR, kSplit>;
+  using C = F32Cfg<DR, kSplit, kPre>;
   CUtensorMap mk, mv;
   int rc = make_map(&mk, RA_F32, a.k, a.D, a.k_rows, a.k_heads_total, a.kv_head_stride, kBNf);
   if (rc != RA_OK) return rc;
@@ -1035,7 +1251,7 @@ int launch_f32(const StepArgs& a, cudaStream_t stream, int key_split) {
   TcArgs t;
   t.kv_per_wave = 0;
   t.key_split = key_split;
-  set_step_form(key_split);
+  set_step_form(key_split | (kPre ? 256 : 0));
   t.out = a.out;
   t.m = a.m;
   t.l = a.l;
@@ -1058,7 +1274,18 @@ int launch_f32(const StepArgs& a, cudaStream_t stream, int key_split) {
   const long long n_qblocks = static_cast<long long>(t.n_qblocks_per_seg) * a.qmap.n_seg;
   RAB_REQUIRE(n_qblocks <= 65535, RA_ERR_INVALID, "attention step: too many query blocks (%lld)",
               n_qblocks);
-  auto kern = step_f32_kernel<DR, kSplit>;
+  SplitKV pre = {};
+  if constexpr (kPre) {
+    pre.tiles = split_tiles(a);
+    const size_t n = static_cast<size_t>(a.B) * a.kvH * pre.tiles;
+    pre.k = static_cast<unsigned char*>(a.workspace);
+    pre.v = pre.k + n * C::kSlotBytes;
+    pre.meta = pre.v + n * C::kSlotBytes;
+    for (int i = 0; i < a.kmap.n_seg; ++i) pre.beg[i] = i * (pre.tiles / a.kmap.n_seg);
+    RAB_CUDA(launch_overlapped(split_kv_kernel<DR>, dim3(pre.tiles, a.B * a.kvH), dim3(kSplitThreads), 0, stream,
+                               static_cast<const float*>(a.k), static_cast<const float*>(a.v), a.kv_head_stride, t, pre, a.k_rows));
+  }
+  auto kern = step_f32_kernel<DR, kSplit, kPre>;
   static std::atomic<unsigned long long> smem_set{0};  // once per device, see step_tc.cu
   int dev = 0;
   RAB_CUDA(cudaGetDevice(&dev));
@@ -1069,7 +1296,7 @@ int launch_f32(const StepArgs& a, cudaStream_t stream, int key_split) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(a.B) * a.H * (kSplit ? key_split : 1),
                      static_cast<unsigned>(n_qblocks));
-  cfg.blockDim = dim3(kThreadsF);
+  cfg.blockDim = dim3(C::kThreads);
   cfg.dynamicSmemBytes = C::kSmemBytes;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
@@ -1082,7 +1309,7 @@ int launch_f32(const StepArgs& a, cudaStream_t stream, int key_split) {
   cfg.attrs = attr;
   cfg.numAttrs = kSplit ? 2 : 1;
   RAB_CUDA(cudaLaunchKernelEx(&cfg, kern, mk, mv, static_cast<const float*>(a.q), static_cast<const float*>(a.k),
-                              a.kv_head_stride, t));
+                              a.kv_head_stride, t, pre));
   RAB_CUDA(cudaGetLastError());
   return RA_OK;
 }
@@ -1090,11 +1317,14 @@ int launch_f32(const StepArgs& a, cudaStream_t stream, int key_split) {
 template <int DR>
 int launch_f32_d(const StepArgs& a, cudaStream_t stream) {
   const int* slots = nullptr;
-  const int rc = cluster_slots(step_f32_kernel<DR, true>, kThreadsF, F32Cfg<DR, true>::kSmemBytes, &slots);
+  const int rc = cluster_slots(step_f32_kernel<DR, true, false>, kThreadsF, F32Cfg<DR, true>::kSmemBytes, &slots);
   if (rc != RA_OK) return rc;
   // (a merge in tiles: those of head_dim 128 take longer)
   const int split = pick_key_split<kBNf>(a, 2 * kBM, DR == 128 ? 1.5 : 2.5, slots);
-  return split > 1 ? launch_f32<DR, true>(a, stream, split) : launch_f32<DR, false>(a, stream, 1);
+  if (a.workspace != nullptr && a.workspace_bytes >= split_bytes<DR>(a) && (reinterpret_cast<uintptr_t>(a.workspace) & 127u) == 0 &&
+      split_ahead<DR>(a))
+    return split > 1 ? launch_f32<DR, true, true>(a, stream, split) : launch_f32<DR, false, true>(a, stream, 1);
+  return split > 1 ? launch_f32<DR, true, false>(a, stream, split) : launch_f32<DR, false, false>(a, stream, 1);
 }
 
 }  // namespace
@@ -1108,6 +1338,12 @@ bool step_f32_supported(int dtype, const StepArgs& a) {
        reinterpret_cast<uintptr_t>(a.v) | reinterpret_cast<uintptr_t>(a.out)) & 15u)
     return false;
   return true;
+}
+
+size_t step_f32_workspace_bytes(const StepArgs& a) {
+  if (a.D == 32) return split_ahead<32>(a) ? split_bytes<32>(a) : 0;
+  if (a.D == 64) return split_ahead<64>(a) ? split_bytes<64>(a) : 0;
+  return split_ahead<128>(a) ? split_bytes<128>(a) : 0;
 }
 
 int launch_step_f32(const StepArgs& a, cudaStream_t stream) {

@@ -122,6 +122,14 @@ __device__ inline void tma_load_3d(unsigned dst, const CUtensorMap* map, unsigne
       : "memory");
 }
 
+// `bytes` (a multiple of 16) of contiguous memory, both ends 16-byte aligned.
+__device__ inline void bulk_load(unsigned dst, const void* src, unsigned bytes, unsigned bar) {
+  asm volatile(
+      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+      "l"(reinterpret_cast<unsigned long long>(src)), "r"(bytes), "r"(bar)
+      : "memory");
+}
+
 __device__ inline void prefetch_map(const CUtensorMap* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<unsigned long long>(map)) : "memory");
 }
@@ -157,6 +165,27 @@ __device__ inline void mma_ts(unsigned d_tmem, unsigned a_tmem, unsigned long lo
       : "memory");
 }
 
+
+// The same with descriptors as their low words (addresses, in 16-byte units) and a common high word: an instruction of 32
+// clk leaves its issuer no time for sums of 64 bits.
+__device__ inline void mma_ss_lo(unsigned d_tmem, unsigned a_lo, unsigned b_lo, unsigned hi, unsigned idesc,
+                                 unsigned accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+      "setp.ne.b32 p, %5, 0;\n\tmov.b64 da, {%1, %3};\n\tmov.b64 db, {%2, %3};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p;\n\t}" ::"r"(d_tmem),
+      "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ inline void mma_ts_lo(unsigned d_tmem, unsigned a_tmem, unsigned b_lo, unsigned hi, unsigned idesc,
+                                 unsigned accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\t"
+      "setp.ne.b32 p, %5, 0;\n\tmov.b64 db, {%2, %3};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}" ::"r"(d_tmem),
+      "r"(a_tmem), "r"(b_lo), "r"(hi), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
 
 // ---- CTA pairs (cta_group::2): one instruction drives the tensor cores of two CTAs of a cluster,
 // M = 256 (128 rows from each CTA's A operand and into each CTA's tensor memory), each CTA
@@ -395,9 +424,10 @@ __device__ inline float ex2(float x) {
 // Shared-memory matrix descriptors for 128B-swizzled tiles (8-row groups 1024 B apart).
 // K-major operand (rows = M or N index, 64 contiguous 16-bit elements of the contraction
 // dimension per 128-byte row); the leading byte offset is unused for swizzled K-major.
+constexpr unsigned kDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);  // SBO, version 1, SWIZZLE_128B
 __device__ inline unsigned long long desc_kmajor(unsigned saddr) {
   const unsigned lo = ((saddr & 0x3FFFFu) >> 4) | (1u << 16);
-  const unsigned hi = (1024u >> 4) | (1u << 14) | (2u << 29);  // SBO, version 1, SWIZZLE_128B
+  const unsigned hi = kDescHi;
   return (static_cast<unsigned long long>(hi) << 32) | lo;
 }
 // MN-major operand (rows = contraction index, 64 contiguous elements of N per 128-byte row):
