@@ -94,7 +94,7 @@ RA_API void ra_debug_set_block_order(int order);
  * query block's keys, 16 folded query tiles, 32 cluster pairs, 64 P in shared memory, 128 shares in a
  * workspace, 256 K and V split ahead (fp32). For tests. */
 RA_API int ra_debug_step_form(void);
-/* Whether ra_kv_cache_append takes a token's rows by its kernel (1) or by device copies (0), given the
+/* Whether ra_kv_cache_append and ra_kv_cache_copy_prefill take their rows by a kernel (1) or by device copies (0), given the
  * current device and those of the cache, the stream and the two sources (-1: not device memory). */
 RA_API int ra_debug_append_route(int device, int cache_device, int stream_device, int k_device, int v_device);
 

@@ -516,7 +516,7 @@ void ra_kv_cache_reset(ra_kv_cache* c) {
 
 // A copy reaches memory of every kind and device and may go into a stream of any; a kernel reads and writes
 // only what the current device has mapped, and needs a stream of it. So a token's rows go by the kernel
-// only if sources, cache and stream are all the current device's (-1: not device memory, or not known).
+// only if sources, cache and stream are all the current device's (-1: not device memory, or not known). So do a prompt's.
 int ra_debug_append_route(int device, int cache_device, int stream_device, int k_device, int v_device) {
   return device >= 0 && cache_device == device && stream_device == device && k_device == device && v_device == device;
 }
@@ -556,16 +556,14 @@ static int cache_copy(ra_kv_cache* c, const void* k_src, const void* v_src, int 
   if (width == 0) return RA_OK;
   int dev = 0;
   RAB_CUDA(cudaGetDevice(&dev));
-  if (rows == 1 && height <= 65535 && c->device == dev &&
+  unsigned char *const k_dst = static_cast<unsigned char*>(c->k) + off, *const v_dst = static_cast<unsigned char*>(c->v) + off;
+  if ((rows == 1 || cache_rows_supported(k_src, v_src, k_dst, v_dst, width, dpitch)) && height <= 65535 && c->device == dev &&
       ra_debug_append_route(dev, c->device, device_of_stream(stream, dev), device_of_memory(k_src, es),
                             device_of_memory(v_src, es)))
-    return launch_cache_row(k_src, v_src, static_cast<unsigned char*>(c->k) + off,
-                            static_cast<unsigned char*>(c->v) + off, width, dpitch,
-                            static_cast<int>(height), stream);
-  RAB_CUDA(cudaMemcpy2DAsync(static_cast<unsigned char*>(c->k) + off, dpitch, k_src, width, width,
-                             height, cudaMemcpyDeviceToDevice, stream));
-  RAB_CUDA(cudaMemcpy2DAsync(static_cast<unsigned char*>(c->v) + off, dpitch, v_src, width, width,
-                             height, cudaMemcpyDeviceToDevice, stream));
+    return rows == 1 ? launch_cache_row(k_src, v_src, k_dst, v_dst, width, dpitch, static_cast<int>(height), stream)
+                     : launch_cache_rows(k_src, v_src, k_dst, v_dst, width, dpitch, static_cast<int>(height), stream);
+  RAB_CUDA(cudaMemcpy2DAsync(k_dst, dpitch, k_src, width, width, height, cudaMemcpyDeviceToDevice, stream));
+  RAB_CUDA(cudaMemcpy2DAsync(v_dst, dpitch, v_src, width, width, height, cudaMemcpyDeviceToDevice, stream));
   return RA_OK;
 }
 

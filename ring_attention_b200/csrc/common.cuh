@@ -180,6 +180,12 @@ int launch_narrow_qkv(const float* q, const float* k, const float* v, void* qh, 
 // One row per (batch, kv head) of K and V into a cache whose rows are dst_pitch_bytes apart.
 int launch_cache_row(const void* k_src, const void* v_src, void* k_dst, void* v_dst, size_t row_bytes,
                      size_t dst_pitch_bytes, int rows, cudaStream_t stream);
+// The rows of a prompt: head_bytes of every (batch, kv head), one after the other in the sources, dst_pitch_bytes apart in
+// the cache. Everything a multiple of 16 bytes (cache_rows_supported).
+bool cache_rows_supported(const void* k_src, const void* v_src, const void* k_dst, const void* v_dst, size_t head_bytes,
+                          size_t dst_pitch_bytes);
+int launch_cache_rows(const void* k_src, const void* v_src, void* k_dst, void* v_dst, size_t head_bytes,
+                      size_t dst_pitch_bytes, int heads, cudaStream_t stream);
 // Merge up to 8 online-softmax states of the same rows ([O | m | l] blocks part_stride floats
 // apart, rows * D + rows even multiples of 4 floats so every O stays 16-byte aligned).
 int launch_state_merge(const float* parts, size_t part_stride, int n_parts, size_t rows, int D,
