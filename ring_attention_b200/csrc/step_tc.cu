@@ -285,10 +285,11 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit, kFold>::kTh
   [[maybe_unused]] int n_spread = 0;  // query tiles of the block
   if constexpr (kSpread) {
     const int i0 = qb_lin * C::kTiles;
-    n_spread = min(C::kTiles, group * a.qmap.n_seg * a.n_qblocks_per_seg - i0);
-    spread_span(a.qmap, a.stride, group, a.n_qblocks_per_seg, i0, i0 + n_spread, &qmin, &qmax);
-    own[0] = spread_tile(i0, group, a.n_qblocks_per_seg);
-    own[1] = spread_tile(i0 + n_spread - 1, group, a.n_qblocks_per_seg);
+    const int pack = a.spread.pack, n = pack > 1 ? (group + pack - 1) / pack : group * a.qmap.n_seg * a.n_qblocks_per_seg;
+    n_spread = min(C::kTiles, n - i0);
+    spread_span(a.qmap, a.stride, group, a.n_qblocks_per_seg, pack, i0, i0 + n_spread, &qmin, &qmax);
+    own[0] = spread_tile(i0, group, a.n_qblocks_per_seg, pack);
+    own[1] = spread_tile(i0 + n_spread - 1, group, a.n_qblocks_per_seg, pack);
   } else {
     qmin = a.qmap.base[sq] + span_row0 * a.stride;
     qmax = a.qmap.base[sq] + (span_row0 + rows_in_span - 1) * a.stride;
@@ -308,7 +309,7 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit, kFold>::kTh
   auto tile_row0 = [&](int w) {
     return kSpread ? (w == 1 ? own[1].row0 : own[0].row0) : kFold ? (w == 1 ? light_row0 : row0) : row0 + w * kBM;
   };
-  auto tile_bh = [&](int w) { return kSpread ? bh + (w == 1 ? own[1].head : own[0].head) * a.kvH : bh; };
+  [[maybe_unused]] auto tile_head = [&](int w) { return w == 1 ? own[1].head : own[0].head; };
   [[maybe_unused]] auto light_range = [&](int sk) {
     const int q0 = a.qmap.base[light_sq] + light_row0 * a.stride;
     return tile_range<kBN>(a.kmap, sk, a.stride, causal, a.doc_len, q0,
@@ -426,10 +427,17 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit, kFold>::kTh
       const int lost = *reinterpret_cast<volatile int*>(a.status);
       for (int w = 0; w < live; ++w) {
         const int q_row = tile_sq(w) * q_seg_len + tile_row0(w);
-        mbar_expect_tx(bar_q_full + 8 * w, C::kTileBytes);
-        for (int bx = 0; bx < C::kBoxes; ++bx)
-          tma_load_3d(s_q + w * C::kTileBytes + bx * (kBM * 128), &tmap_q, bar_q_full + 8 * w,
-                      bx * 64, q_row, tile_bh(w));
+        if constexpr (kSpread) {
+          const int rows = a.spread.pack > 1 ? a.spread.pack * a.Sq : kBM;  // (rows behind them stay as they are)
+          mbar_expect_tx(bar_q_full + 8 * w, C::kBoxes * rows * 128);
+          for (int bx = 0; bx < C::kBoxes; ++bx)
+            tma_load_5d(s_q + w * C::kTileBytes + bx * (kBM * 128), &tmap_q, bar_q_full + 8 * w, bx * 64, q_row,
+                        static_cast<int>(blockIdx.y) % a.kvH, tile_head(w), b);
+        } else {
+          mbar_expect_tx(bar_q_full + 8 * w, C::kTileBytes);
+          for (int bx = 0; bx < C::kBoxes; ++bx)
+            tma_load_3d(s_q + w * C::kTileBytes + bx * (kBM * 128), &tmap_q, bar_q_full + 8 * w, bx * 64, q_row, bh);
+        }
       }
       int it = 0, jt = 0;  // ring items and key tiles so far
       bool ok = true;
@@ -811,8 +819,15 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit, kFold>::kTh
     const unsigned t_o = tmem_base + lane_base + (w == 0 ? C::kColO0 : C::kColO1);
     [[maybe_unused]] const unsigned t_p =
         tmem_base + lane_base + (w == 0 ? C::kColP0 : C::kColP1);
-    const int r_in_seg = tile_row0(w) + row;
-    const bool row_valid = r_in_seg < q_seg_len && (!(kFold || kSpread) || w < live);
+    int r_in_seg = tile_row0(w) + row;
+    bool row_valid = r_in_seg < q_seg_len && (!(kFold || kSpread) || w < live);
+    if constexpr (kSpread) {
+      if (a.spread.pack > 1) {
+        const int g = row / a.Sq;
+        r_in_seg = row - g * a.Sq;
+        row_valid = w < live && g < a.spread.pack && tile_head(w) + g < group;
+      }
+    }
     const int qpos = a.qmap.base[tile_sq(w)] + r_in_seg * a.stride;
     const int n_own = kFold && w == 1 ? n_light : n_tiles;  // key tiles of this query tile
     const long long qdoc = a.doc_len > 0 ? qpos / a.doc_len : 0;
@@ -967,7 +982,8 @@ __global__ void __launch_bounds__((TcCfg<D, kPInTmem, kPair, kSplit, kFold>::kTh
           half_tile(0, neg_m);
           half_tile(1, neg_m);
           row_sum = (sum_a.x + sum_a.y) + (sum_b.x + sum_b.y);
-          slow = __any_sync(0xffffffffu, !(row_sum <= kRowSumLimit)) != 0;  // also catches NaN
+          // also catches NaN (but not that of rows which only fill a spread tile: nothing was loaded there)
+          slow = __any_sync(0xffffffffu, !(row_sum <= kRowSumLimit) && (!kSpread || row_valid)) != 0;
         }
         else {
           wait_prev_pv(true);
@@ -1154,11 +1170,13 @@ __global__ void __launch_bounds__(kFoldThreads) spread_fold_kernel(const TcArgs 
   const int bh = grow / a.Sq, s = grow - bh * a.Sq;
   const int h = bh % a.H, b = bh / a.H, kv = h % a.kvH, group = a.H / a.kvH;
   const int seg = s / a.qmap.seg_len, r = s - seg * a.qmap.seg_len;
-  const int tile = (seg * a.n_qblocks_per_seg + r / kBM) * group + h / a.kvH;
+  const int pack = a.spread.pack;
+  const int tile = pack > 1 ? h / a.kvH / pack : (seg * a.n_qblocks_per_seg + r / kBM) * group + h / a.kvH;
+  const int row = pack > 1 ? h / a.kvH % pack * a.Sq + s : r % kBM;
   const int j = min(tile / kTiles, kMaxSpread - 1);
   const int beg = a.spread.beg[j], n = a.spread.beg[j + 1] - beg;
   constexpr size_t kStep = static_cast<size_t>(kTiles) * kBM;  // rows from one share's part to the next
-  const size_t part = ((static_cast<size_t>(b) * a.kvH + kv) * a.spread.total + beg) * kStep + (tile % kTiles) * kBM + r % kBM;
+  const size_t part = ((static_cast<size_t>(b) * a.kvH + kv) * a.spread.total + beg) * kStep + (tile % kTiles) * kBM + row;
   wait_for_previous();
   const bool mine = grow < rows && *reinterpret_cast<volatile int*>(a.status) == 0;
   const int end = mine ? n : 0;
@@ -1239,8 +1257,8 @@ int launch_cfg(const StepArgs& a, cudaStream_t stream, int key_split = 1, const 
   using C = TcCfg<D, kPInTmem, kPair, kSplit, kFold>;
   CUtensorMap mq, mk, mv;
   const int dtype = kBf16 ? RA_BF16 : RA_F16;
-  int rc = make_map(&mq, dtype, a.q, a.D, a.Sq, static_cast<long long>(a.B) * a.H,
-                    static_cast<long long>(a.Sq) * a.D);
+  int rc = kSpread ? make_query_map(&mq, dtype, a, spread->pack > 1 ? a.Sq : kBM, spread->pack)
+                   : make_map(&mq, dtype, a.q, a.D, a.Sq, static_cast<long long>(a.B) * a.H, static_cast<long long>(a.Sq) * a.D);
   if (rc != RA_OK) return rc;
   rc = make_map(&mk, dtype, a.k, a.D, a.k_rows, a.k_heads_total, a.kv_head_stride, C::kKRows);
   if (rc != RA_OK) return rc;

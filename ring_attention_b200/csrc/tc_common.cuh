@@ -6,6 +6,7 @@
 
 #include <cuda.h>
 
+#include <algorithm>
 #include <mutex>
 
 #include "common.cuh"
@@ -127,6 +128,14 @@ __device__ inline void bulk_load(unsigned dst, const void* src, unsigned bytes, 
   asm volatile(
       "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
       "l"(reinterpret_cast<unsigned long long>(src)), "r"(bytes), "r"(bar)
+      : "memory");
+}
+
+__device__ inline void tma_load_5d(unsigned dst, const CUtensorMap* map, unsigned bar, int c0, int c1, int c2, int c3, int c4) {
+  asm volatile(
+      "cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, "
+      "{%3, %4, %5, %6, %7}], [%2];" ::"r"(dst),
+      "l"(reinterpret_cast<unsigned long long>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4)
       : "memory");
 }
 
@@ -476,21 +485,23 @@ __host__ __device__ inline TileRange tile_range(const PosMap& kmap, int sk, int 
   return {static_cast<int>(j_lo / kTileKeys), static_cast<int>(j_hi / kTileKeys) + 1};
 }
 
-// Query tile i of a KV head in the spread form: by position, then by query head of the group.
+// Query tile i of a KV head in the spread form: by position, then by query head of the group; or, with `pack` heads to a
+// tile, all rows of heads i * pack and on, one head behind the other.
 struct SpreadTile {
-  int head, seg, row0;  // head inside the group, query segment, first row inside it
+  int head, seg, row0;  // (first) head inside the group, query segment, first row inside it
 };
-__host__ __device__ inline SpreadTile spread_tile(int i, int group, int per_seg) {
+__host__ __device__ inline SpreadTile spread_tile(int i, int group, int per_seg, int pack) {
+  if (pack > 1) return {i * pack, 0, 0};
   const int pos = i / group;
   return {i - pos * group, pos / per_seg, (pos % per_seg) * kBM};
 }
 // Positions [qmin, qmax] that the rows of tiles [i0, i1) span.
-__host__ __device__ inline void spread_span(const PosMap& qmap, int stride, int group, int per_seg, int i0, int i1, int* qmin,
-                                            int* qmax) {
+__host__ __device__ inline void spread_span(const PosMap& qmap, int stride, int group, int per_seg, int pack, int i0, int i1,
+                                            int* qmin, int* qmax) {
   *qmin = 0x7fffffff;
   *qmax = -0x7fffffff;
   for (int i = i0; i < i1; ++i) {
-    const SpreadTile t = spread_tile(i, group, per_seg);
+    const SpreadTile t = spread_tile(i, group, per_seg, pack);
     const int rows = qmap.seg_len - t.row0 < kBM ? qmap.seg_len - t.row0 : kBM;
     const int first = qmap.base[t.seg] + t.row0 * stride, last = first + (rows - 1) * stride;
     *qmin = first < *qmin ? first : *qmin;
@@ -515,6 +526,7 @@ struct TileShare {
 constexpr int kMaxSpread = 160;  // blocks of one KV head, at most (a B200 has 148 SMs)
 struct Spread {
   int total;                             // blocks of one KV head
+  int pack;                              // heads whose rows share a query tile (1: a tile is rows of one head)
   unsigned char beg[kMaxSpread + 1];     // first block of query block j; beg[number of query blocks] = total
 };
 
@@ -795,6 +807,24 @@ inline int make_map(CUtensorMap* map, int dtype, const void* base, int D, long l
   return RA_OK;
 }
 
+// 16-bit queries as (D, rows, kv heads, heads that share one, batch), box = one 128-byte row piece x box_rows x 1 x box_heads x
+// 1: the box lands as box_heads times box_rows rows, swizzled as one tile of them.
+inline int make_query_map(CUtensorMap* map, int dtype, const StepArgs& a, int box_rows, int box_heads) {
+  EncodeTiledFn fn = encode_fn();
+  RAB_REQUIRE(fn != nullptr, RA_ERR_CUDA, "cuTensorMapEncodeTiled is unavailable");
+  const cuuint64_t row = static_cast<cuuint64_t>(a.D) * 2, head = row * a.Sq;
+  const cuuint64_t dims[5] = {static_cast<cuuint64_t>(a.D), static_cast<cuuint64_t>(a.Sq), static_cast<cuuint64_t>(a.kvH),
+                              static_cast<cuuint64_t>(a.H / a.kvH), static_cast<cuuint64_t>(a.B)};
+  const cuuint64_t strides[4] = {row, head, head * a.kvH, head * a.H};
+  const cuuint32_t box[5] = {64, static_cast<cuuint32_t>(box_rows), 1, static_cast<cuuint32_t>(box_heads), 1};
+  const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+  const CUresult r = fn(map, dtype == RA_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 5,
+                        const_cast<void*>(a.q), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                        CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  RAB_REQUIRE(r == CUDA_SUCCESS, RA_ERR_CUDA, "cuTensorMapEncodeTiled failed with code %d", static_cast<int>(r));
+  return RA_OK;
+}
+
 // How many blocks the current device holds at once when they come in clusters of n, n = 1..8: asked for
 // once per device, with whichever key-split kernel comes first (all of them hold one block per SM, so the
 // answers are the same; a cluster lives inside one GPC: 148, 148, 135, 132, 130, 132, 126, 120 on a B200).
@@ -950,7 +980,7 @@ inline bool fold_rows(const StepArgs& a, double alone, double tiles) {
 // Spread: the same for a call with a workspace, without clusters. All 128-row query tiles of the query heads that share
 // a KV head are paired into blocks (by position, then by head, so that the tiles of a block see about the same keys),
 // and block j's key tiles are cut into n_j contiguous shares, a thread block each, for the smallest longest share whose
-// blocks all fit the SMs at once. A share writes its partial (O, m, l) to the workspace and a second launch folds the
+// blocks all fit the SMs at once. Where a head has at most 64 rows, as many heads as fit share a tile. A share writes its partial (O, m, l) to the workspace and a second launch folds the
 // shares into the state. Against the key split: no SM is left out because clusters do not fit (135 of 148 in threes), a
 // block may have more than eight shares, grouped heads fill up each other's blocks, and blocks may differ in their number of
 // shares; against that stand a launch and the way of the partial states through L2 (`fold_tiles`, in tiles of work).
@@ -958,24 +988,27 @@ inline bool fold_rows(const StepArgs& a, double alone, double tiles) {
 // cost the host 5 to 7 us, which a call that is waited for shows). Only from kSpreadKeys keys on: shorter
 // calls never gain, and a caller need not ask for a workspace. us per call, key split / spread (16 bits, causal, CUDA
 // graphs): 384 rows on 40384 keys H32/kvH8 D128 285 / 211, D64 261 / 177; 64 rows on 65536 keys H8 D128 109 / 62; 16 rows on
-// 100000 keys H16/kvH2 D128 211 / 90; 144 rows on 32376 keys H2 D64 71 / 28; 700 rows on 9000 keys H8/kvH2 D256 86 / 62; 337
+// 100000 keys H16/kvH2 D128 212 / 36 (90 with a tile for each head); 144 rows on 32376 keys H2 D64 71 / 28; 700 rows on 9000 keys H8/kvH2 D256 86 / 62; 337
 // rows on 8336 keys H16/kvH8 D64 39 / 34. Over 104 random calls (16 to 2048 rows on 1000 to 40000 keys more) that gain by
-// more than 5 % in the estimate 0.69 in the mean, 1.05 at worst (19.7 / 20.7, a call that the four tiles now keep out).
+// more than 5 % in the estimate 0.69 in the mean, 1.05 at worst (19.7 / 20.7, a call that the four tiles now keep out);
+// over 41 of 16 to 128 rows, with heads that share tiles, 0.47 and 0.77.
 constexpr int kSpreadKeys = 2048;
 template <int kTileKeys>
 inline bool plan_spread(const StepArgs& a, int tiles_per_block, double fold_tiles, int sms, double best_other, Spread* out) {
-  if (a.Sk < kSpreadKeys || a.Sq < 2 || best_other <= 0 || a.H % a.kvH != 0) return false;
+  if (a.Sk < kSpreadKeys || best_other <= 0 || a.H % a.kvH != 0) return false;
   const long long heads = static_cast<long long>(a.B) * a.kvH;
   const int cap = static_cast<int>(heads < sms ? sms / heads : 0) < kMaxSpread ? static_cast<int>(heads < sms ? sms / heads : 0) : kMaxSpread;
   const int group = a.H / a.kvH;
   const int per_seg = (a.qmap.seg_len + kBM - 1) / kBM;
-  const long long tiles = static_cast<long long>(group) * a.qmap.n_seg * per_seg;
+  // (few rows: the tile's place in the tensor core is paid whether rows stand in it or not)
+  const int pack = a.qmap.n_seg == 1 && 2 * a.Sq <= kBM ? std::min(group, kBM / a.Sq) : 1;
+  const long long tiles = pack > 1 ? (group + pack - 1) / pack : static_cast<long long>(group) * a.qmap.n_seg * per_seg;
   const long long n_blocks = (tiles + tiles_per_block - 1) / tiles_per_block;
   if (n_blocks > cap) return false;
   int keys[kMaxSpread], longest = 1;
   for (int j = 0; j < n_blocks; ++j) {
     int qmin, qmax;
-    spread_span(a.qmap, a.stride, group, per_seg, j * tiles_per_block,
+    spread_span(a.qmap, a.stride, group, per_seg, pack, j * tiles_per_block,
                 static_cast<int>((j + 1) * tiles_per_block < tiles ? (j + 1) * tiles_per_block : tiles), &qmin, &qmax);
     keys[j] = 0;
     for (int sk = 0; sk < a.kmap.n_seg; ++sk) {
@@ -998,6 +1031,7 @@ inline bool plan_spread(const StepArgs& a, int tiles_per_block, double fold_tile
   const double gain = best_other - (lo + kBlockTiles + fold_tiles);
   if (gain < 4 || gain < 0.05 * best_other) return false;
   out->total = 0;
+  out->pack = pack;
   for (int j = 0; j < n_blocks; ++j) {
     out->beg[j] = static_cast<unsigned char>(out->total);
     out->total += keys[j] > lo ? (keys[j] + lo - 1) / lo : 1;

@@ -46,6 +46,10 @@ CASES = {  # B, H, kvH, query bases, rows a segment, key bases, keys a segment, 
     "strides": (1, 4, 1, [50001], 140, [0], 20000, 3, True, 0),
     "documents": (1, 3, 1, [20800], 400, [0], 21200, 1, True, 10500),
     "dense": (1, 2, 1, [0], 129, [0], 20000, 1, False, 0),
+    "heads of a tile": (1, 8, 2, [20000], 24, [0], 20024, 1, True, 0),
+    "some heads left over": (2, 6, 2, [30000], 50, [0], 15000, 2, True, 0),
+    "half a tile each": (1, 16, 1, [16000], 64, [0], 16064, 1, True, 0),
+    "single rows": (1, 7, 1, [30000], 1, [0], 30001, 1, True, 16000),
     "blocks without keys": (1, 2, 2, [0, 22000], 200, [2000], 20000, 1, True, 0),
 }
 
@@ -96,11 +100,11 @@ def test_random_spread_calls_match_the_key_split():
     # (both round P to 16 bits under reference points that may differ: two roundings of 2^-11 / 2^-8 of every P, which
     # average out over the keys)
     rng, taken = random.Random(5), 0
-    for n in range(150):
+    for n in range(250):
         kvH = rng.choice([1, 2, 3, 4, 8])
         B, H, D = rng.choice([1, 2]), kvH * rng.choice([1, 2, 3, 4]), rng.choice([32, 64, 128, 256])
         dtype = rng.choice([torch.float16, torch.bfloat16])
-        rows, stride = rng.choice([1, 7, 64, 127, 128, 129, 200, 257, 400]), rng.choice([1, 1, 2])
+        rows, stride = rng.choice([1, 2, 5, 7, 16, 33, 42, 43, 64, 65, 127, 128, 129, 200, 257, 400]), rng.choice([1, 1, 2])
         nq, nk = rng.choice([1, 1, 2, 3]), rng.choice([1, 1, 2])
         keys = rng.randrange(1000, 20000)
         qb = sorted(rng.randrange(0, 30000) for _ in range(nq))
