@@ -17,11 +17,13 @@
 //    row), the kernel is bound by the copy. Two blocks of 96 KB of ring per SM: the loads of one
 //    run on through the barriers and the arithmetic of the other (B4 H32/kvH8 D128, 262144 rows:
 //    one block of 160 KB 799 us, two of 96 KB 591-635 us = 6.8-7.25 TB/s).
-//  - decode_split_kernel (fp32 caches, head_dim 32) is the SIMT form of the same structure
+//  - decode_split_kernel (fp32 caches, head_dim 32; one and two query heads to a KV head) is the SIMT form of the same structure
 //    with a 4-stage ring: a group of `LPR` lanes owns a row, each lane keeps its slice of q
 //    (pre-scaled) for every head of the group, the dot product finishes with log2(LPR)
 //    shuffles, each lane group carries its own running (m, l, out), and a warp-shuffle
 //    log-sum-exp merge plus one shared-memory pass combine lane groups and warps.
+//  - decode_group_kernel: the same caches with more query heads to a KV head, four or eight a block. There the
+//    instructions count, and one butterfly serves the scores of all heads.
 // Partials (m, l, out) go to a workspace and a second small kernel folds them into the persistent
 // state (src/attention_decode.cu:228-277 does the same for its fixed 8 splits); short calls merge
 // them inside a cluster instead.
@@ -41,6 +43,8 @@ using tcgen::cluster_addr;
 using tcgen::cluster_ctarank;
 using tcgen::cluster_sync_threads;
 using tcgen::ex2;
+using tcgen::fadd2;
+using tcgen::ffma2;
 using tcgen::kLn2;
 using tcgen::kLog2e;
 using tcgen::ld_cluster_f4;
@@ -103,37 +107,50 @@ struct Piece<__nv_bfloat16> {
   }
 };
 
-template <typename T, int D, int GB = 1>
+// decode_split_kernel: every lane owns 1..4 pieces of a row.
+template <typename T, int D>
 struct DecodeCfg {
   static constexpr int kRowBytes = D * static_cast<int>(sizeof(T));
   static constexpr int kPieces = kRowBytes / 16;  // 16-byte pieces per row
-  // Lanes per row: every lane owns 1..4 pieces. A lane keeps its slice of q and of the accumulator
-  // for GB heads; where those would take 128 registers and leave an SM a single block (eight heads,
-  // or four at 1 KB rows), twice the lanes share a row (B1 H64/kvH8 D128, 45344 rows: 248 -> 133 us,
-  // 174 with the fixed splits and one block per SM that this replaces).
-  static constexpr int kLPRNarrow = kPieces >= 32 ? 16 : (kPieces >= 8 ? 8 : 4);
-  static constexpr bool kWide =
-      GB * (kPieces / kLPRNarrow) * Piece<T>::kElems >= 64 && 2 * kLPRNarrow <= kPieces;
-  static constexpr int kLPR = kWide ? 2 * kLPRNarrow : kLPRNarrow;
+  static constexpr int kLPR = kPieces >= 32 ? 16 : (kPieces >= 8 ? 8 : 4);
   static constexpr int kVPT = kPieces / kLPR;               // pieces per lane
   static constexpr int kEPL = kVPT * Piece<T>::kElems;      // elements per lane
   static constexpr int kRowsPerWarpStep = 32 / kLPR;
   static constexpr int kRowsPerStep = kWarps * kRowsPerWarpStep;
-  static constexpr int steps_for(int rows) {  // 8 KB per tensor and stage
-    return 8192 / (rows * kRowBytes) > 0 ? 8192 / (rows * kRowBytes) : 1;
-  }
-  static constexpr int kSteps = steps_for(kRowsPerStep);
-  static constexpr int kRowsPerStage = kRowsPerStep * kSteps;
-  static constexpr int kPlanRows =  // see fixed_splits
-      kWarps * (32 / kLPRNarrow) * steps_for(kWarps * (32 / kLPRNarrow));
+  static constexpr int kSteps = 8192 / (kRowsPerStep * kRowBytes) > 0 ? 8192 / (kRowsPerStep * kRowBytes) : 1;
+  static constexpr int kRowsPerStage = kRowsPerStep * kSteps;  // 8 KB per tensor and stage
   static constexpr int kStageBytes = kRowsPerStage * kRowBytes;  // per tensor
   static constexpr int kSmemBytes = 2 * kStages * kStageBytes;
+};
+
+// decode_group_kernel: a lane owns four columns of a row, or eight at head_dim 256, and a warp takes kRows rows of each of
+// its 32 / kLPR lane groups at a time.
+template <typename T, int D, int GB>
+struct GroupCfg {
+  static constexpr int kRowBytes = D * static_cast<int>(sizeof(T));
+  static constexpr int kPieceBytes = 4 * static_cast<int>(sizeof(T));
+  static constexpr int kLPR = D / 4 < 32 ? D / 4 : 32;
+  static constexpr int kVPT = D / 4 / kLPR;
+  static constexpr int kEPL = 4 * kVPT;
+  static constexpr int kRows = D == 256 ? 2 : (kLPR / GB < 4 ? kLPR / GB : 4);
+  static constexpr int kScores = kRows * GB;  // of a lane group; no more than it has lanes
+  static constexpr int kGroups = 32 / kLPR;
+  static constexpr int kRowsPerWarpStep = kGroups * kRows;
+  static constexpr int kWarps =
+      8192 / kRowBytes / kRowsPerWarpStep < 8 ? 8192 / kRowBytes / kRowsPerWarpStep : 8;
+  static constexpr int kThreads = kWarps * 32;
+  static constexpr int kRowsPerStep = kWarps * kRowsPerWarpStep;
+  static constexpr int kSteps = 8192 / (kRowsPerStep * kRowBytes);
+  static constexpr int kRowsPerStage = kRowsPerStep * kSteps;
+  static constexpr int kStageBytes = kRowsPerStage * kRowBytes;  // per tensor
+  static constexpr int kSmemBytes = 2 * kStages * kStageBytes;
+  static_assert(kStageBytes == 8192 && kScores <= kLPR, "8 KB per tensor and stage, a score for each lane");
 };
 
 // ---- how the keys are dealt to blocks ----------------------------------------------------
 //
 // A group is one (batch row, KV head, batch of query heads); its visible rows are `stages` ring
-// stages. Three forms of the same kernels:
+// stages. Two forms of the same kernels:
 //  * balanced: one block per resident slot of the GPU, block i takes the stages
 //    [i T / G, (i + 1) T / G) of all T = groups * stages, whatever groups they belong to (one or
 //    two, more when groups are short). Every block moves the same bytes, so there is no last wave:
@@ -143,20 +160,16 @@ struct DecodeCfg {
 //    it made no difference by itself (799 against 769 us); with two blocks per SM 1, 3 or 6 times as
 //    many blocks were no faster either, and the B1 H8 D128 fp32 call on 16384 rows slower (37 us
 //    against 31).
-//  * fixed: `splits` blocks per group, about three waves, partials and fold as above. For the SIMT kernels
-//    whose registers leave room for one block per SM only: eight fp32 heads of 256, where the
-//    loop over shares gained nothing, and eight 16-bit heads of 32, which share the rule.
 //  * cluster: the blocks of a cluster take equal shares of ONE group and merge
 //    their partials through distributed shared memory into the state. No workspace and no second
 //    launch: for calls that one wave finishes in a few microseconds (B1 H32/kvH8 D128 fp16 on 1061
 //    rows 11.5 -> 9.3 us per call, most of it host time).
-enum DealForm { kBalanced, kFixed, kCluster };
+enum DealForm { kBalanced, kCluster };
 struct Deal {
   int stages;          // per group
   int groups;
   int head_batches;
   int cap;             // partial slots per (batch, head) row
-  int splits;          // fixed form: blocks per group
   int ring;            // ring slots (no more than a block's stages)
   unsigned flags;      // cluster form: RA_STEP_FRESH / RA_STEP_FINALIZE
 };
@@ -324,8 +337,8 @@ struct Shares {
   long long total, at, at_end;
   int n, i;
   __device__ explicit Shares(const Deal& deal) {
-    n = kForm == kFixed ? deal.splits : static_cast<int>(gridDim.x);
-    i = static_cast<int>(kForm == kFixed ? blockIdx.x % deal.splits : blockIdx.x);
+    n = static_cast<int>(gridDim.x);
+    i = static_cast<int>(blockIdx.x);
     total = static_cast<long long>(deal.groups) * deal.stages;
     at = kForm == kBalanced ? total * i / n : 0;
     at_end = kForm == kBalanced ? total * (i + 1ll) / n : 1;
@@ -334,9 +347,7 @@ struct Shares {
   }
   __device__ bool next(const Deal& deal, int kvH, Share& s) {
     if (at >= at_end) return false;
-    const int group = static_cast<int>(kForm == kBalanced ? at / deal.stages
-                                       : kForm == kFixed  ? blockIdx.x / deal.splits
-                                                          : blockIdx.y);
+    const int group = static_cast<int>(kForm == kBalanced ? at / deal.stages : blockIdx.y);
     if (kForm == kBalanced) {
       const long long first = static_cast<long long>(group) * deal.stages;
       s.beg = static_cast<int>(at - first);
@@ -362,7 +373,7 @@ __global__ void __launch_bounds__(kThreads)
     decode_split_kernel(const T* Q, const T* K, const T* V,
                         float* Mp, float* Lp, float* Op, int H,
                         int kvH, int sk_eff, long long kv_head_stride, const Deal deal, float scale_log2) {
-  using C = DecodeCfg<T, D, GB>;
+  using C = DecodeCfg<T, D>;
   extern __shared__ __align__(16) unsigned char smem[];
   unsigned char* k_ring = smem;
   unsigned char* v_ring = smem + deal.ring * C::kStageBytes;
@@ -536,6 +547,262 @@ __global__ void __launch_bounds__(kThreads)
     }
     __syncthreads();
     finish_group<GB, D, kWarps, kForm>(red_m, red_l, red_o, b, kvh, hb, H, kvH, share.part, deal, Mp, Lp, Op);
+    if (kForm == kBalanced) __syncthreads();  // the ring is free again
+  }
+}
+
+// ---- four and eight query heads to a KV head ---------------------------------------------------
+//
+// The kernel above finishes every head's dot product with a butterfly of its own and works out the
+// softmax of every head in every lane. Here a lane's kRows x GB partial sums go through ONE butterfly that halves their
+// number at each exchange and leaves one (row, head) score a lane. No value is selected on the way: register j of a
+// lane holds head j ^ (lane % GB) and row i is row i ^ (lane / GB % kRows), so what a lane keeps and what it
+// gives away are the same registers in all of them. The softmax is one exponential a lane, the
+// weights go to all lanes through shared memory, both contractions are packed FMAs, and a step's rows are added up before they
+// reach the accumulators (without that the error against 64 bits grew from 2.4e-7 to 2.9e-7 on 40000 rows: an SM has fewer
+// warps than before, so each adds more rows). With eight heads of 128 about 80 instead of 180 instructions a row and warp, 16
+// instead of 40 of them shuffles. fp32, eight heads, before / now (floor of the copy): B1 H64/kvH8 D256 135081 rows 939 / 332 us
+// (338), B3 H48/kvH6 D128 179592 rows 1073 / 508 (505), B1 H32/kvH4 D128 16049 rows 31 / 20 (10); bf16 rows of 32, B2 H32/kvH4
+// 225843 rows 179 / 96 (35). Four heads were near the copy in long calls (B3 H64/kvH16 D64 162905 rows 578 / 548);
+// short ones are 3 to 25 % faster (B2 H12/kvH4 D128 683 rows 8.2 / 6.9). 110 random calls: 0.85 in the mean, 0.99 at worst.
+// One and two heads stay with the kernel above: a row costs it 17 to 35 instructions there, below what its copy takes.
+template <typename T>
+__device__ inline void load_four(const unsigned char* p, float (&f)[4]) {
+  if constexpr (sizeof(T) == 4) {
+    const float4 x = *reinterpret_cast<const float4*>(p);
+    f[0] = x.x, f[1] = x.y, f[2] = x.z, f[3] = x.w;
+  } else {
+    const uint2 u = *reinterpret_cast<const uint2*>(p);
+    float g[8];
+    Piece<T>::unpack(make_uint4(u.x, u.y, 0, 0), g);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) f[e] = g[e];
+  }
+}
+
+template <typename T, int D, int GB, DealForm kForm>
+__global__ void __launch_bounds__(GroupCfg<T, D, GB>::kThreads)
+    decode_group_kernel(const T* Q, const T* K, const T* V, float* Mp, float* Lp, float* Op, int H, int kvH, int sk_eff,
+                        long long kv_head_stride, const Deal deal, float scale_log2) {
+  using C = GroupCfg<T, D, GB>;
+  constexpr int kR = C::kRows;
+  extern __shared__ __align__(16) unsigned char smem[];
+  // a warp's weights of one step; two buffers, so that one barrier a step is enough
+  __shared__ __align__(16) float weights[C::kWarps][2][C::kGroups * C::kScores];
+  unsigned char* k_ring = smem;
+  unsigned char* v_ring = smem + deal.ring * C::kStageBytes;
+
+  const int tid = threadIdx.x;
+  const int lane = tid & 31;
+  const int warp = tid >> 5;
+  const int lr = lane % C::kLPR;   // lane within the row group
+  const int grp = lane / C::kLPR;  // row group within the warp
+  const int my_head = lr % GB, my_row = lr / GB % kR;
+  const int base = lane - lr;
+  const bool lead = lr < C::kScores;
+  Shares<kForm> shares(deal);
+  Share share;
+  int buf = 0;
+  while (shares.next(deal, kvH, share)) {
+    const int b = share.b, kvh = share.kvh, hb = share.hb;
+
+    // Query heads of this block: h = kvh + kvH * (hb * GB + g), while h < H.
+    float2 q2[GB][C::kEPL / 2];  // (column, column + 1) of head j ^ my_head
+    float2 o2[GB / 2][C::kEPL];  // (head 2 j, head 2 j + 1) of a column
+    float m_run = -INFINITY, l_run = 0.f;    // of my_head over the rows of this group of lanes; l_run of my_row only
+#pragma unroll
+    for (int j = 0; j < GB; ++j) {
+      const int h = kvh + kvH * (hb * GB + (j ^ my_head));
+#pragma unroll
+      for (int v = 0; v < C::kVPT; ++v) {
+        float f[4] = {0.f, 0.f, 0.f, 0.f};
+        if (h < H)
+          load_four<T>(reinterpret_cast<const unsigned char*>(Q + (static_cast<size_t>(b) * H + h) * D) +
+                           (v * C::kLPR + lr) * C::kPieceBytes,
+                       f);
+        q2[j][2 * v] = make_float2(f[0] * scale_log2, f[1] * scale_log2);
+        q2[j][2 * v + 1] = make_float2(f[2] * scale_log2, f[3] * scale_log2);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < GB / 2; ++j)
+#pragma unroll
+      for (int e = 0; e < C::kEPL; ++e) o2[j][e] = make_float2(0.f, 0.f);
+
+    const int row_begin = share.beg * C::kRowsPerStage;
+    const int row_end = min(static_cast<long long>(sk_eff), static_cast<long long>(share.end) * C::kRowsPerStage);
+    const int n_rows = row_end - row_begin;
+    const int n_stages = share.end - share.beg;
+    const unsigned char* k_base = reinterpret_cast<const unsigned char*>(
+        K + (static_cast<size_t>(b) * kvH + kvh) * kv_head_stride + static_cast<size_t>(row_begin) * D);
+    const unsigned char* v_base = reinterpret_cast<const unsigned char*>(
+        V + (static_cast<size_t>(b) * kvH + kvh) * kv_head_stride + static_cast<size_t>(row_begin) * D);
+    const long long share_bytes = static_cast<long long>(n_rows) * C::kRowBytes;
+
+    auto issue = [&](int st) {
+      if (st < n_stages) {
+        const int slot = st % kStages;
+        const long long first = static_cast<long long>(st) * C::kStageBytes;
+#pragma unroll
+        for (int p = 0; p < C::kStageBytes / 16 / C::kThreads; ++p) {
+          const int off = (p * C::kThreads + tid) * 16;
+          const bool ok = first + off < share_bytes;
+          // past the share: src-size 0 zero-fills the destination, the source is not read
+          cp_async16(k_ring + slot * C::kStageBytes + off, ok ? k_base + first + off : k_base, ok ? 16 : 0);
+          cp_async16(v_ring + slot * C::kStageBytes + off, ok ? v_base + first + off : v_base, ok ? 16 : 0);
+        }
+      }
+      cp_async_commit();
+    };
+
+#pragma unroll
+    for (int s = 0; s < kStages - 1; ++s) issue(s);
+
+    for (int st = 0; st < n_stages; ++st) {
+      cp_async_wait<kStages - 2>();
+      __syncthreads();
+      issue(st + kStages - 1);
+      const int slot = st % kStages;
+#pragma unroll 1
+      for (int step = 0; step < C::kSteps; ++step) {
+        // row i of lane group g: first + i * kGroups + g
+        const int first = step * C::kRowsPerStep + warp * C::kRowsPerWarpStep + grp;
+        const unsigned char* krow = k_ring + slot * C::kStageBytes + first * C::kRowBytes + lr * C::kPieceBytes;
+        const unsigned char* vrow = v_ring + slot * C::kStageBytes + first * C::kRowBytes + lr * C::kPieceBytes;
+        float s[kR][GB];
+#pragma unroll
+        for (int i = 0; i < kR; ++i) {
+          float2 acc[GB];
+#pragma unroll
+          for (int j = 0; j < GB; ++j) acc[j] = make_float2(0.f, 0.f);
+#pragma unroll
+          for (int v = 0; v < C::kVPT; ++v) {
+            float f[4];
+            load_four<T>(krow + (i ^ my_row) * C::kGroups * C::kRowBytes + v * C::kLPR * C::kPieceBytes, f);
+            const float2 k0 = make_float2(f[0], f[1]), k1 = make_float2(f[2], f[3]);
+#pragma unroll
+            for (int j = 0; j < GB; ++j) {
+              acc[j] = ffma2(q2[j][2 * v], k0, acc[j]);
+              acc[j] = ffma2(q2[j][2 * v + 1], k1, acc[j]);
+            }
+          }
+#pragma unroll
+          for (int j = 0; j < GB; ++j) s[i][j] = acc[j].x + acc[j].y;
+        }
+#pragma unroll
+        for (int half = kR / 2; half > 0; half /= 2)
+#pragma unroll
+          for (int i = 0; i < half; ++i)
+#pragma unroll
+            for (int j = 0; j < GB; ++j) s[i][j] += __shfl_xor_sync(0xffffffffu, s[i + half][j], half * GB);
+#pragma unroll
+        for (int half = GB / 2; half > 0; half /= 2)
+#pragma unroll
+          for (int j = 0; j < half; ++j) s[0][j] += __shfl_xor_sync(0xffffffffu, s[0][j + half], half);
+        float score = s[0][0];
+#pragma unroll
+        for (int off = C::kScores; off < C::kLPR; off *= 2) score += __shfl_xor_sync(0xffffffffu, score, off);
+
+        const bool valid = st * C::kRowsPerStage + first + my_row * C::kGroups < n_rows;
+        float m_new = valid ? score : -INFINITY;
+#pragma unroll
+        for (int off = GB; off < C::kScores; off *= 2) m_new = fmaxf(m_new, __shfl_xor_sync(0xffffffffu, m_new, off));
+        m_new = fmaxf(m_run, m_new);
+        if (__any_sync(0xffffffffu, m_new > m_run)) {  // rare after the first rows: rescale only when a maximum moves
+          const float alpha = m_new > m_run ? ex2(m_run - m_new) : 1.f;  // ex2(-inf) = 0 on the first row
+          l_run *= alpha;
+          m_run = m_new;
+#pragma unroll
+          for (int j = 0; j < GB / 2; ++j) {
+            const float2 a = make_float2(__shfl_sync(0xffffffffu, alpha, base + 2 * j),
+                                               __shfl_sync(0xffffffffu, alpha, base + 2 * j + 1));
+#pragma unroll
+            for (int e = 0; e < C::kEPL; ++e) o2[j][e] = ffma2(o2[j][e], a, make_float2(0.f, 0.f));
+          }
+        }
+        const float p = valid && score != -INFINITY ? ex2(score - m_run) : 0.f;
+        l_run += p;
+        float* w = weights[warp][buf];
+        buf ^= 1;
+        if (lead) w[grp * C::kScores + lr] = p;
+        __syncwarp();
+        float2 p2[kR][GB / 2];
+#pragma unroll
+        for (int i = 0; i < kR; ++i)
+#pragma unroll
+          for (int j = 0; j < GB / 4; ++j) {
+            const float4 x = *reinterpret_cast<const float4*>(w + grp * C::kScores + i * GB + 4 * j);
+            p2[i][2 * j] = make_float2(x.x, x.y);
+            p2[i][2 * j + 1] = make_float2(x.z, x.w);
+          }
+        // the rows of a step are added up by themselves first: fewer terms one after another on the accumulators
+#pragma unroll
+        for (int v = 0; v < C::kVPT; ++v) {
+          float f[kR][4];
+#pragma unroll
+          for (int i = 0; i < kR; ++i)
+            load_four<T>(vrow + i * C::kGroups * C::kRowBytes + v * C::kLPR * C::kPieceBytes, f[i]);
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+#pragma unroll
+            for (int j = 0; j < GB / 2; ++j) {
+              float2& o = o2[j][4 * v + e];
+              if constexpr (kR == 1) {
+                o = ffma2(p2[0][j], make_float2(f[0][e], f[0][e]), o);
+              } else {
+                float2 sum = ffma2(p2[0][j], make_float2(f[0][e], f[0][e]), make_float2(0.f, 0.f));
+#pragma unroll
+                for (int i = 1; i < kR; ++i) sum = ffma2(p2[i][j], make_float2(f[i][e], f[i][e]), sum);
+                o = fadd2(o, sum);
+              }
+            }
+        }
+      }
+    }
+    cp_async_wait<0>();
+
+    // Merge the rows of a lane group (they share m_run), then the groups of the warp (log-sum-exp merge) ...
+#pragma unroll
+    for (int off = GB; off < C::kScores; off *= 2) l_run += __shfl_xor_sync(0xffffffffu, l_run, off);
+    __syncthreads();  // the ring is idle now
+    float* red_m = reinterpret_cast<float*>(smem);  // [kWarps][GB]
+    float* red_l = red_m + C::kWarps * GB;           // [kWarps][GB]
+    float* red_o = red_l + C::kWarps * GB;           // [kWarps][GB][D]
+#pragma unroll
+    for (int g = 0; g < GB; ++g) {
+      float m_g = __shfl_sync(0xffffffffu, m_run, base + g), l_g = __shfl_sync(0xffffffffu, l_run, base + g);
+      float o_g[C::kEPL];
+#pragma unroll
+      for (int e = 0; e < C::kEPL; ++e) o_g[e] = g % 2 ? o2[g / 2][e].y : o2[g / 2][e].x;
+#pragma unroll
+      for (int off = C::kLPR; off < 32; off *= 2) {
+        const float m_o = __shfl_xor_sync(0xffffffffu, m_g, off);
+        const float l_o = __shfl_xor_sync(0xffffffffu, l_g, off);
+        const float m_n = fmaxf(m_g, m_o);
+        const float a = (m_g == -INFINITY) ? 0.f : ex2(m_g - m_n);
+        const float c = (m_o == -INFINITY) ? 0.f : ex2(m_o - m_n);
+        l_g = a * l_g + c * l_o;
+#pragma unroll
+        for (int e = 0; e < C::kEPL; ++e) {
+          const float o_o = __shfl_xor_sync(0xffffffffu, o_g[e], off);
+          o_g[e] = a * o_g[e] + c * o_o;
+        }
+        m_g = m_n;
+      }
+      // ... then the warps of the block through shared memory.
+      if (grp == 0) {
+        if (lr == 0) {
+          red_m[warp * GB + g] = m_g;
+          red_l[warp * GB + g] = l_g;
+        }
+#pragma unroll
+        for (int v = 0; v < C::kVPT; ++v)
+          *reinterpret_cast<float4*>(red_o + (warp * GB + g) * D + (v * C::kLPR + lr) * 4) =
+              make_float4(o_g[4 * v], o_g[4 * v + 1], o_g[4 * v + 2], o_g[4 * v + 3]);
+      }
+    }
+    __syncthreads();
+    finish_group<GB, D, C::kWarps, kForm>(red_m, red_l, red_o, b, kvh, hb, H, kvH, share.part, deal, Mp, Lp, Op);
     if (kForm == kBalanced) __syncthreads();  // the ring is free again
   }
 }
@@ -795,7 +1062,7 @@ __global__ void __launch_bounds__(MmaCfg<D>::kThreads)
   }
 }
 
-// Fold the partials of the balanced and fixed forms into the persistent (out, m, l). grid = (H, B); a thread
+// Fold the partials of the balanced form into the persistent (out, m, l). grid = (H, B); a thread
 // takes four columns of every n_grp-th partial (with one column and two groups at head_dim 256 the B1 H64/kvH1
 // call on 6000 rows spent 17 of its 28 us of kernels on 38 loads in a row per thread), and (m, l) are read by
 // lanes. Launched while the split kernel still runs (programmatic dependent launch): everything it
@@ -819,9 +1086,7 @@ __global__ void __launch_bounds__(kFoldThreads)
   const long long total = static_cast<long long>(deal.groups) * deal.stages;
   const long long group =
       (static_cast<long long>(b) * kvH + h % kvH) * deal.head_batches + (h / kvH) / head_rows;
-  const int n = deal.splits > 0 ? deal.splits
-                                : deal_owner((group + 1) * deal.stages - 1, total, ctas) -
-                                      deal_owner(group * deal.stages, total, ctas) + 1;
+  const int n = deal_owner((group + 1) * deal.stages - 1, total, ctas) - deal_owner(group * deal.stages, total, ctas) + 1;
   wait_for_previous();
   const float* mp = Mp + row * deal.cap;
   const float* lp = Lp + row * deal.cap;
@@ -891,7 +1156,9 @@ struct DecodePlan {
 // What a kernel needs for a ring stage, in us: `alone` for one block on an SM, `share` of the SM's issue slots
 // (k blocks on an SM take k times that if it is longer). Slopes of calls with few groups, one block each,
 // between 6000 and 20000 rows: the mma kernel 0.53, 0.71 and 1.14 at head_dim 64, 128 (64 keys) and 256 (32);
-// the SIMT kernel 0.34-0.49 for 16 KB with one head, 0.47-0.77 with four, 0.75-1.1 with eight.
+// the SIMT kernel 0.34-0.49 for 16 KB with one head. (The kernel for four and eight heads needs
+// 0.38-0.48 and 0.49-0.64 now; the estimate still says what its predecessor took, so that no call takes the other form for it:
+// a fold at 8.2 with these stages would send calls that fold well to clusters, 7.8 -> 10.8 us at worst.)
 struct StageCost {
   double alone, share;
 };
@@ -901,15 +1168,15 @@ constexpr StageCost simt_stage_cost(int heads, size_t stage_bytes) {
 }
 
 // Which form, and how many blocks. `per_sm`: resident blocks per SM; `cap`: partial slots per row
-// that the workspace holds; `rows`: (batch, head) rows; `head_rows`: rows of a group; `fixed`: splits of the
-// fixed form (0: balanced). Every estimate is the walk of a block, wave by wave, at what its SM or the
+// that the workspace holds; `rows`: (batch, head) rows; `head_rows`: rows of a group; `partials`: there is room for
+// partials, or there can be. Every estimate is the walk of a block, wave by wave, at what its SM or the
 // memory (7 TB/s) allows, plus what the fold (a launch, and more the more rows it has) or the merge
 // (columns of the group, blocks of the cluster, and a wave of clusters starts slower than one of blocks)
 // adds. Constants fitted to 457 shapes (heads 8/8 to 64/1, batch 1 to 64, 200 to 100000 rows, fp16 and fp32,
 // every head_dim) timed in each form: this choice is 1.0 % from the best form on average, the estimate
 // before it (0.1 MB/us for any block, a fold of 3 us) 5.6 %, and up to twofold with few or very many groups.
-DecodePlan make_plan(int groups, int stages, size_t stage_bytes, int per_sm, int cap, int ring_max, int fixed,
-                     StageCost cost, size_t rows, int head_rows, int D) {
+DecodePlan make_plan(int groups, int stages, size_t stage_bytes, int per_sm, int cap, int ring_max,
+                     StageCost cost, size_t rows, int head_rows, int D, bool partials) {
   constexpr double kBytesPerUs = 7e6, kFold = 8.2, kFoldRow = 0.005, kMerge = 0.6, kMergeBlock = 0.15,
                    kMergeElement = 0.0005, kWave = 1.5, kClusterWave = 4.0;
   DecodePlan p;
@@ -925,12 +1192,10 @@ DecodePlan make_plan(int groups, int stages, size_t stage_bytes, int per_sm, int
   // exactly one each when there are as many blocks as groups
   long long ctas = std::min<long long>(slots, static_cast<long long>(total));
   ctas = cap > 1 ? std::min(ctas, (cap - 1ll) * groups) : groups;
-  fixed = std::min(std::min(fixed, cap), stages);
   p.cluster = 0;
   p.ctas = static_cast<int>(ctas);
-  double best = (fixed ? walk(static_cast<double>(groups) * fixed, std::ceil(static_cast<double>(stages) / fixed))
-                       : walk(static_cast<double>(ctas), std::ceil(total / ctas))) +
-                kFold + kFoldRow * rows;
+  double best = walk(static_cast<double>(ctas), std::ceil(total / ctas)) + kFold + kFoldRow * rows;
+  if (!partials) best = 1e30;
   for (int c = 1; c <= kMaxCluster && groups <= 65535; c *= 2) {
     if (c > 1 && c > stages) break;
     const double blocks = static_cast<double>(groups) * c;
@@ -944,10 +1209,8 @@ DecodePlan make_plan(int groups, int stages, size_t stage_bytes, int per_sm, int
   }
   p.deal.stages = stages;
   p.deal.groups = groups;
-  p.deal.splits = fixed;
-  p.deal.cap = fixed ? fixed : (p.ctas + groups - 1) / groups + (p.ctas == groups ? 0 : 1);
+  p.deal.cap = (p.ctas + groups - 1) / groups + (p.ctas == groups ? 0 : 1);
   const long long most = p.cluster ? (stages + p.cluster - 1) / p.cluster
-                         : fixed   ? (stages + fixed - 1) / fixed
                                    : std::min<long long>(stages, (static_cast<long long>(total) + ctas - 1) / ctas);
   p.deal.ring = static_cast<int>(std::max<long long>(1, std::min<long long>(ring_max, most)));
   return p;
@@ -979,6 +1242,13 @@ int ensure_workspace(size_t need, void** out) {
   return RA_OK;
 }
 
+bool workspace_holds(size_t need) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+  std::lock_guard<std::mutex> lk(g_ws_mu);
+  return g_ws[dev].bytes >= need;
+}
+
 }  // namespace
 
 int decode_ml_scratch(size_t floats, float** out) {
@@ -1002,7 +1272,7 @@ int decode_ml_scratch(size_t floats, float** out) {
 
 namespace {
 
-// Workspace of the balanced and the fixed form: [row][slot] of O, m and l.
+// Workspace of the balanced form: [row][slot] of O, m and l.
 int partial_space(size_t rows, int D, int cap, void* workspace, float** Op, float** Mp, float** Lp) {
   const size_t need = rows * cap * (D + 2) * sizeof(float);
   if (workspace == nullptr) {
@@ -1019,7 +1289,7 @@ int partial_space(size_t rows, int D, int cap, void* workspace, float** Op, floa
 // launch(cluster form?, config, deal, Mp, Lp, Op) sets the attribute and launches the kernel.
 template <int D, int ROWS, typename Launch>
 int run_plan(const ra_shape& s, int head_batches, int stages, size_t stage_bytes, int ring_max, int per_sm,
-             StageCost cost, size_t red_bytes, int old_splits, bool fixed, float* out, float* m, float* l, void* workspace,
+             StageCost cost, size_t red_bytes, int old_splits, float* out, float* m, float* l, void* workspace,
              size_t workspace_bytes, int split_cap, unsigned flags, cudaStream_t stream, Launch launch) {
   const int kvH = kv_heads_of(s);
   const size_t rows = static_cast<size_t>(s.batch) * s.heads;
@@ -1030,8 +1300,16 @@ int run_plan(const ra_shape& s, int head_batches, int stages, size_t stage_bytes
                 "decode workspace too small: %zu < %zu bytes", workspace_bytes, old_splits * slot_bytes);
     cap = static_cast<int>(std::min<size_t>(cap, workspace_bytes / slot_bytes));
   }
-  DecodePlan p = make_plan(s.batch * kvH * head_batches, stages, stage_bytes, per_sm, cap, ring_max,
-                           fixed ? old_splits : 0, cost, rows, std::min(ROWS, (s.heads + kvH - 1) / kvH), D);
+  auto plan = [&](bool partials) {
+    return make_plan(s.batch * kvH * head_batches, stages, stage_bytes, per_sm, cap, ring_max, cost, rows,
+                     std::min(ROWS, (s.heads + kvH - 1) / kvH), D, partials);
+  };
+  DecodePlan p = plan(true);
+  // a stream that is being captured allows no allocation: such a call merges in clusters instead
+  if (!p.cluster && workspace == nullptr && p.deal.groups <= 65535 && !workspace_holds(p.deal.cap * slot_bytes)) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &capture) == cudaSuccess && capture != cudaStreamCaptureStatusNone) p = plan(false);
+  }
   p.deal.head_batches = head_batches;
   p.deal.flags = flags;
   cudaLaunchConfig_t cfg = {};
@@ -1061,7 +1339,7 @@ int run_plan(const ra_shape& s, int head_batches, int stages, size_t stage_bytes
   // D128 fp32, 16384 rows: 27.5 us so, 30.6 with that, 29.7 launched behind.)
   cfg.attrs = attr + 1;
   cfg.numAttrs = 1;
-  cfg.gridDim = fixed ? dim3(static_cast<unsigned>(p.deal.splits) * p.deal.groups) : dim3(p.ctas);
+  cfg.gridDim = dim3(p.ctas);
   rc = launch(false, cfg, p.deal, Mp, Lp, Op);
   if (rc != RA_OK) return rc;
   // (no more thread groups than partials: with many rows and few partials each the idle ones cost, 2048
@@ -1074,7 +1352,7 @@ int run_plan(const ra_shape& s, int head_batches, int stages, size_t stage_bytes
   return RA_OK;
 }
 
-// Splits per group of the fixed-split plan, which a caller's workspace has always been held to.
+// Partials per row that a caller's workspace has always been held to: three waves of equal splits of a group.
 int fixed_splits(int blocks_per_split, int sk_eff, int rows_per_stage, int split_cap) {
   int want = (3 * sm_count() + blocks_per_split - 1) / blocks_per_split;
   want = std::max(1, std::min(std::min(want, std::max(1, sk_eff / (2 * rows_per_stage))), split_cap));
@@ -1128,7 +1406,7 @@ int launch_decode_typed(const void* q, const void* k, const void* v, float* out,
     static const int per_sm = resident_blocks(decode_mma_kernel<T, D, kBalanced>, M::kThreads, kSmem);
     return run_plan<D, 16>(
         s, head_batches, stages, 2 * M::kStageBytes, M::kStages, per_sm, mma_stage_cost(D), kRed,
-        fixed_splits(s.batch * kvH * head_batches, sk_eff, 64, split_cap), false, out,
+        fixed_splits(s.batch * kvH * head_batches, sk_eff, 64, split_cap), out,
         m, l, workspace, workspace_bytes, split_cap, flags, stream,
         [&](bool cluster, cudaLaunchConfig_t& cfg, const Deal& deal, float* Mp, float* Lp, float* Op) {
           static std::atomic<unsigned long long> set_c{0}, set_b{0};
@@ -1138,25 +1416,33 @@ int launch_decode_typed(const void* q, const void* k, const void* v, float* out,
                                        Mp, Lp, Op);
         });
   } else {
+    // Rows to which a caller's workspace is held (see fixed_splits): a stage of the kernel with 8 warps and 16-byte pieces
+    using Plan = DecodeCfg<T, D>;
     auto run = [&](auto gb_tag) {
       constexpr int GB = decltype(gb_tag)::value;
-      using C = DecodeCfg<T, D, GB>;
-      constexpr DealForm kDealt = GB * C::kEPL >= 64 ? kFixed : kBalanced;  // (see DecodeCfg)
-      constexpr size_t kRed = red_floats(kWarps, GB, D) * sizeof(float);
+      using C = std::conditional_t<(GB >= 4), GroupCfg<T, D, GB < 4 ? 4 : GB>, DecodeCfg<T, D>>;
+      constexpr int kBlockThreads = GB >= 4 ? GroupCfg<T, D, GB < 4 ? 4 : GB>::kThreads : kThreads;
+      constexpr size_t kRed = red_floats(kBlockThreads / 32, GB, D) * sizeof(float);
       constexpr size_t kSmem = C::kSmemBytes > kRed ? C::kSmemBytes : kRed;
+      const auto kernel = [](auto form) {
+        if constexpr (GB >= 4) return decode_group_kernel<T, D, GB, decltype(form)::value>;
+        else return decode_split_kernel<T, D, GB, decltype(form)::value>;
+      };
+      const auto balanced = kernel(std::integral_constant<DealForm, kBalanced>{});
+      const auto clustered = kernel(std::integral_constant<DealForm, kCluster>{});
       const int head_batches = (group + GB - 1) / GB;
       const int stages = (sk_eff + C::kRowsPerStage - 1) / C::kRowsPerStage;
-      static const int per_sm = resident_blocks(decode_split_kernel<T, D, GB, kDealt>, kThreads, kSmem);
+      // fp32, four and eight heads: two blocks an SM move 7.3 and 6.9 TB/s, three 6.9 and 6.9 (D128; B3 H32/kvH8, 200335 rows
+      // 699 us with two, 731 with three). 16-bit rows of 32 are bound by instructions: 5.3 with two, 5.7 with three
+      static const int per_sm = std::min(resident_blocks(balanced, kBlockThreads, kSmem), GB >= 4 && sizeof(T) == 4 ? 2 : 16);
       return run_plan<D, GB>(
           s, head_batches, stages, 2 * C::kStageBytes, kStages, per_sm, simt_stage_cost(GB, 2 * C::kStageBytes), kRed,
-          fixed_splits(s.batch * kvH * head_batches, sk_eff, C::kPlanRows, split_cap), kDealt == kFixed,
+          fixed_splits(s.batch * kvH * head_batches, sk_eff, Plan::kRowsPerStage, split_cap),
           out, m, l, workspace, workspace_bytes, split_cap, flags, stream,
           [&](bool cluster, cudaLaunchConfig_t& cfg, const Deal& deal, float* Mp, float* Lp, float* Op) {
             static std::atomic<unsigned long long> set_c{0}, set_b{0};
-            return cluster ? launch_with(decode_split_kernel<T, D, GB, kCluster>, kSmem, set_c, cfg, kThreads,
-                                         deal, Mp, Lp, Op)
-                           : launch_with(decode_split_kernel<T, D, GB, kDealt>, kSmem, set_b, cfg, kThreads,
-                                         deal, Mp, Lp, Op);
+            return cluster ? launch_with(clustered, kSmem, set_c, cfg, kBlockThreads, deal, Mp, Lp, Op)
+                           : launch_with(balanced, kSmem, set_b, cfg, kBlockThreads, deal, Mp, Lp, Op);
           });
     };
     // smallest of 1 / 2 / 4 / 8 that fits the group

@@ -1,0 +1,70 @@
+"""Decode calls with more than two query heads to a KV head on caches that the tensor-core kernel does not take (fp32; 16-bit
+with head_dim 32), against attention in 64 bits: stage edges, ragged groups of heads, both ways of dealing the rows."""
+import numpy as np
+import pytest
+import torch
+
+from ring_attention_b200 import api
+from util import normal_inputs, round_to
+
+pytestmark = pytest.mark.gpu
+
+
+def want64(q, k, v, kvH):
+    """out and the bound of its error: scores of D products summed as 4 or 8 in a lane and log2 over lanes, one
+    exponential (2^-22), and up to a quarter of the rows added one after another by a lane, in units of 2^-24."""
+    q, k, v = (torch.from_numpy(x.astype(np.float64)) for x in (q, k, v))
+    B, H, _, D = q.shape
+    of = torch.arange(H) % kvH
+    s = (q @ k[:, of].transpose(-1, -2)) / D ** 0.5
+    size = ((q.abs() @ k[:, of].abs().nan_to_num(0, 0, 0).transpose(-1, -2)) / D ** 0.5).max().item()
+    out = torch.softmax(s, -1) @ v[:, of]
+    eps = 2.0 ** -24
+    tol = (2 * (16 * eps * size + 2.0 ** -22) + 2 * (k.shape[2] / 4 + 64) * eps) * v.abs().max().item()
+    return out.numpy(), tol
+
+
+@pytest.mark.parametrize("dtype,D", [(torch.float32, 32), (torch.float32, 64), (torch.float32, 128), (torch.float32, 256),
+                                     (torch.float16, 32), (torch.bfloat16, 32)])
+@pytest.mark.parametrize("B,H,kvH,Sk", [
+    (1, 4, 1, 1), (2, 8, 1, 7), (1, 8, 2, 33), (1, 24, 3, 129), (2, 5, 1, 16), (1, 11, 3, 127), (1, 12, 4, 300),
+    (1, 9, 1, 257), (1, 20, 1, 100), (1, 8, 1, 3001), (3, 16, 4, 2999), (64, 32, 4, 70)])
+def test_group_decode_against_64_bits(dtype, D, B, H, kvH, Sk):
+    q, k, v = normal_inputs(31, B, H, kvH, 1, Sk, D)
+    q, k, v = (round_to(x, dtype) for x in (q, k, v)) if dtype != torch.float32 else (q, k, v)
+    if Sk > 20:  # a key that no head sees (weight 0 whatever its value row)
+        q, k = np.abs(q) + (q == 0), k.copy()
+        k[:, :, Sk // 2] = -np.inf
+    want, tol = want64(q, k, v, kvH)
+    dq, dk, dv = (torch.from_numpy(np.ascontiguousarray(x)).cuda().to(dtype) for x in (q, k, v))
+    shape = api.AttentionShape(B, H, 1, Sk, D, kvH)
+    need = int(api.lib().ra_decode_workspace_bytes(shape.c()))
+    for workspace in (None, torch.full((need // 4,), float("nan"), device="cuda")):
+        out = torch.full((B, H, 1, D), float("nan"), device="cuda")
+        m, l = torch.empty((B, H, 1), device="cuda"), torch.empty((B, H, 1), device="cuda")
+        api.launch_attention_init(out, m, l, shape)
+        api.launch_attention_decode_step(dq, dk, dv, out, m, l, shape, 0, 0, False, workspace=workspace)
+        api.launch_attention_finalize(out, l, shape)
+        assert np.abs(out.cpu().numpy() - want).max() <= tol
+
+
+def test_group_decode_first_called_while_captured():
+    """The library's own room for partials cannot grow while a stream is captured: the call is recorded all the same."""
+    B, H, kvH, Sk, D = 2, 64, 8, 20011, 256
+    q, k, v = normal_inputs(5, B, H, kvH, 1, Sk, D)
+    want, tol = want64(q, k, v, kvH)
+    dq, dk, dv = (torch.from_numpy(x).cuda() for x in (q, k, v))
+    shape = api.AttentionShape(B, H, 1, Sk, D, kvH)
+    out = torch.zeros((B, H, 1, D), device="cuda")
+    m, l = torch.empty((B, H, 1), device="cuda"), torch.empty((B, H, 1), device="cuda")
+    api.launch_attention_init(out, m, l, shape)
+    api.launch_attention_finalize(out, l, shape)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        api.launch_attention_init(out, m, l, shape)
+        api.launch_attention_decode_step(dq, dk, dv, out, m, l, shape, 0, 0, False)
+        api.launch_attention_finalize(out, l, shape)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert np.abs(out.cpu().numpy() - want).max() <= tol
