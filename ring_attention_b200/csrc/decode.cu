@@ -1072,6 +1072,7 @@ __global__ void __launch_bounds__(MmaCfg<D>::kThreads)
 // caller an init launch); RA_STEP_FINALIZE: divide by l after folding (saves the finalize
 // launch). vec: Op and O are 16-byte aligned (a caller's workspace and state need not be).
 constexpr int kFoldGroups = 16, kFoldThreads = kFoldGroups * 64;
+template <int kEach>  // partials a thread holds, a power of two: n_grp * kEach >= cap
 __global__ void __launch_bounds__(kFoldThreads)
     decode_reduce_kernel(const float* Mp, const float* Lp, const float* Op, float* M, float* L, float* O, int H,
                          int kvH, int D, int head_rows, int ctas, bool vec, const Deal deal) {
@@ -1092,10 +1093,28 @@ __global__ void __launch_bounds__(kFoldThreads)
   const float* lp = Lp + row * deal.cap;
   const float* op = Op + row * deal.cap * D + d;
   float* o_row = O + row * D + d;
+  // Everything the call reads is asked for at once: a thread's partials of O (no more than kEach), (m, l) of all partials in every warp, and the old state. One
+  // behind the other the loads were most of the fold's time: fp16 B1 H2/kvH1 D64, 8391 rows 8.8 -> 6.5 us a call, fp32 B1
+  // H24/kvH8 D128, 11229 rows 17.5 -> 16.3, B1 H8 16384 rows 27.0 -> 26.0; the same bits.
+  constexpr int kML = (kFoldGroups * kEach + 31) / 32;
+  float ms[kML], ls[kML];
+#pragma unroll
+  for (int i = 0; i < kML; ++i) {
+    const int s = lane + 32 * i;
+    ms[i] = s < n ? mp[s] : -INFINITY;
+    ls[i] = s < n ? lp[s] : 0.f;
+  }
+  float4 o[kEach];
+#pragma unroll
+  for (int i = 0; i < kEach; ++i) {
+    const int s = grp + i * n_grp;
+    o[i] = s < n ? ld4(op + static_cast<size_t>(s) * D, vec) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  const float m_old = fresh ? -INFINITY : M[row], l_old = fresh ? 0.f : L[row];
   // every warp works out the same maximum and sum; the scales go to shared memory once
-  const float m_old = fresh ? -INFINITY : M[row];
   float m_n = m_old;
-  for (int s = lane; s < n; s += 32) m_n = fmaxf(m_n, mp[s]);
+#pragma unroll
+  for (int i = 0; i < kML; ++i) m_n = fmaxf(m_n, ms[i]);
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) m_n = fmaxf(m_n, __shfl_xor_sync(0xffffffffu, m_n, off));
   if (m_n == -INFINITY) {
@@ -1110,20 +1129,21 @@ __global__ void __launch_bounds__(kFoldThreads)
     return;
   }
   float l_acc = 0.f;
-  for (int s = lane; s < n; s += 32) {
-    const float ms = mp[s];
-    const float f = (ms == -INFINITY) ? 0.f : expf(ms - m_n);
-    l_acc += f * lp[s];
-    if (threadIdx.x < 32) sc[s] = f;
+#pragma unroll
+  for (int i = 0; i < kML; ++i) {
+    const float f = (ms[i] == -INFINITY) ? 0.f : expf(ms[i] - m_n);
+    l_acc += f * ls[i];
+    if (threadIdx.x < 32) sc[lane + 32 * i] = f;
   }
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) l_acc += __shfl_xor_sync(0xffffffffu, l_acc, off);
   const float a = (m_old == -INFINITY) ? 0.f : expf(m_old - m_n);
-  if (m_old > -INFINITY) l_acc += a * L[row];
+  if (m_old > -INFINITY) l_acc += a * l_old;
   __syncthreads();
   float4 o_acc = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 4
-  for (int s = grp; s < n; s += n_grp) add_scaled(o_acc, sc[s], ld4(op + static_cast<size_t>(s) * D, vec));
+#pragma unroll
+  for (int i = 0; i < kEach; ++i)
+    if (grp + i * n_grp < n) add_scaled(o_acc, sc[grp + i * n_grp], o[i]);
   part_o[threadIdx.x] = o_acc;
   __syncthreads();
   if (grp > 0) return;
@@ -1344,8 +1364,11 @@ int run_plan(const ra_shape& s, int head_batches, int stages, size_t stage_bytes
   if (rc != RA_OK) return rc;
   // (no more thread groups than partials: with many rows and few partials each the idle ones cost, 2048
   // rows of D32 8 us)
-  RAB_CUDA(launch_overlapped(decode_reduce_kernel, dim3(s.heads, s.batch),
-                             dim3(std::max(32, std::min(kFoldGroups, p.deal.cap) * (D / 4))), 0, stream, Mp, Lp, Op, m, l,
+  const int groups = std::min(kFoldGroups, p.deal.cap);
+  const int each = (p.deal.cap + groups - 1) / groups;
+  const auto fold = each > 4 ? decode_reduce_kernel<8> : each > 2 ? decode_reduce_kernel<4>
+                    : each > 1 ? decode_reduce_kernel<2> : decode_reduce_kernel<1>;
+  RAB_CUDA(launch_overlapped(fold, dim3(s.heads, s.batch), dim3(std::max(32, groups * (D / 4))), 0, stream, Mp, Lp, Op, m, l,
                              out, s.heads, kvH, D, ROWS, p.ctas,
                              ((reinterpret_cast<uintptr_t>(Op) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0, p.deal));
   RAB_CUDA(cudaGetLastError());

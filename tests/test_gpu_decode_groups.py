@@ -10,9 +10,9 @@ from util import normal_inputs, round_to
 pytestmark = pytest.mark.gpu
 
 
-def want64(q, k, v, kvH):
+def want64(q, k, v, kvH, blocks=1):
     """out and the bound of its error: scores of D products summed as 4 or 8 in a lane and log2 over lanes, one
-    exponential (2^-22), and up to a quarter of the rows added one after another by a lane, in units of 2^-24."""
+    exponential (2^-22), and up to a quarter of a block's rows added one after another by a lane, in units of 2^-24."""
     q, k, v = (torch.from_numpy(x.astype(np.float64)) for x in (q, k, v))
     B, H, _, D = q.shape
     of = torch.arange(H) % kvH
@@ -20,7 +20,7 @@ def want64(q, k, v, kvH):
     size = ((q.abs() @ k[:, of].abs().nan_to_num(0, 0, 0).transpose(-1, -2)) / D ** 0.5).max().item()
     out = torch.softmax(s, -1) @ v[:, of]
     eps = 2.0 ** -24
-    tol = (2 * (16 * eps * size + 2.0 ** -22) + 2 * (k.shape[2] / 4 + 64) * eps) * v.abs().max().item()
+    tol = (2 * (16 * eps * size + 2.0 ** -22) + 2 * (k.shape[2] / blocks / 4 + 64 + blocks) * eps) * v.abs().max().item()
     return out.numpy(), tol
 
 
@@ -67,4 +67,24 @@ def test_group_decode_first_called_while_captured():
         api.launch_attention_finalize(out, l, shape)
     graph.replay()
     torch.cuda.synchronize()
+    assert np.abs(out.cpu().numpy() - want).max() <= tol
+
+
+@pytest.mark.parametrize("dtype,D", [(torch.float32, 64), (torch.float32, 256), (torch.float16, 32)])
+@pytest.mark.parametrize("B,kvH,Sk,blocks", [  # blocks: no more than a KV head has of them
+    (1, 1, 40000, 64), (1, 4, 20000, 64), (1, 8, 9001, 32), (1, 16, 6000, 16), (3, 16, 4100, 4), (8, 48, 700, 1)])
+def test_fold_of_few_and_many_partials(dtype, D, B, kvH, Sk, blocks):
+    """One to 128 partials to a row, by the number of groups, on a fresh and on an old state."""
+    q, k, v = normal_inputs(17, B, 2 * kvH, kvH, 1, Sk, D)
+    v = (v + np.sign(np.sin(np.arange(Sk) / 40.0))[:, None]).astype(np.float32)  # a lost share of the rows shows
+    q, k, v = (round_to(x, dtype) for x in (q, k, v)) if dtype != torch.float32 else (q, k, v)
+    want, tol = want64(q, k, v, kvH, blocks)
+    dq, dk, dv = (torch.from_numpy(np.ascontiguousarray(x)).cuda().to(dtype) for x in (q, k, v))
+    out = torch.full((B, 2 * kvH, 1, D), float("nan"), device="cuda")
+    m, l = (torch.empty((B, 2 * kvH, 1), device="cuda") for _ in range(2))
+    shape = api.AttentionShape(B, 2 * kvH, 1, Sk, D, kvH)
+    api.launch_attention_init(out, m, l, shape)
+    for _ in range(2):  # the same keys twice: every weight and the sum double, the quotient stays
+        api.launch_attention_decode_step(dq, dk, dv, out, m, l, shape, 0, 0, False)
+    api.launch_attention_finalize(out, l, shape)
     assert np.abs(out.cpu().numpy() - want).max() <= tol
