@@ -13,12 +13,14 @@
 //   blocks per KV head the grid is turned so that all query blocks of the heads sharing one KV
 //   head run before the next KV head (see launch_cfg).
 //
-// Five forms of the same kernel, tested against each other: P in tensor memory (default) or staged
+// Six forms of the same kernel, tested against each other: P in tensor memory (default) or staged
 // through shared memory (RA_STEP_P_IN_SMEM); cluster pairs (RA_STEP_CTA_PAIR, head_dim 128 / 256):
 // tcgen05.mma.cta_group::2 with M = 256 over the two blocks of a cluster, each block loading half of
 // every K and V tile; the key split (chosen by shape, pick_key_split): 2 to 8 blocks of a cluster
-// share the key tiles of one query block and merge their states (merge_key_split); and the fold (chosen by
-// shape, fold_rows): a block's two query tiles are a head's light and heavy ones instead of neighbours.
+// share the key tiles of one query block and merge their states (merge_key_split); the fold (chosen by
+// shape, fold_rows): a block's two query tiles are a head's light and heavy ones instead of neighbours; and
+// the spread form (chosen by shape where the caller gives a workspace, plan_spread): the key tiles of all query tiles in equal
+// shares over the SMs, whose partial states a second kernel folds, and heads with few rows in one query tile.
 //
 // Roles inside a block (384 threads)
 //   warp 0        TMA producer: Q tiles once, then K_j, V_j, K_j+1, ... into a shared-memory
