@@ -1198,6 +1198,9 @@ constexpr StageCost simt_stage_cost(int heads, size_t stage_bytes) {
 // adds. Constants fitted to 457 shapes (heads 8/8 to 64/1, batch 1 to 64, 200 to 100000 rows, fp16 and fp32,
 // every head_dim) timed in each form: this choice is 1.0 % from the best form on average, the estimate
 // before it (0.1 MB/us for any block, a fold of 3 us) 5.6 %, and up to twofold with few or very many groups.
+// Since launches overlap, a fold costs about 4: over 1700 calls the choice was 2.3 % from the best form, with kFold = 4 it would
+// be 0.7 %. It stays all the same: a fold goes through the library's partials, which calls on several streams must not
+// share, and calls that merge in clusters have none.
 DecodePlan make_plan(int groups, int stages, size_t stage_bytes, int per_sm, int cap, int ring_max,
                      StageCost cost, size_t rows, int head_rows, int D, bool partials) {
   constexpr double kBytesPerUs = 7e6, kFold = 8.2, kFoldRow = 0.005, kMerge = 0.6, kMergeBlock = 0.15,
@@ -1331,7 +1334,8 @@ int run_plan(const ra_shape& s, int head_batches, int stages, size_t stage_bytes
   // a stream that is being captured allows no allocation: such a call merges in clusters instead
   if (!p.cluster && workspace == nullptr && p.deal.groups <= 65535 && !workspace_holds(p.deal.cap * slot_bytes)) {
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(stream, &capture) == cudaSuccess && capture != cudaStreamCaptureStatusNone) p = plan(false);
+    if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess) cudaGetLastError();
+    else if (capture != cudaStreamCaptureStatusNone) p = plan(false);
   }
   p.deal.head_batches = head_batches;
   p.deal.flags = flags;
