@@ -50,7 +50,7 @@
 // time in which the tensor core is idle (P is always written when the warp comes to it). A satisfied wait costs it 100 to
 // 150 clocks, a sum of 64 bits in a descriptor half as much as an instruction. us, B1 H4 S16384 D128 causal: 824; descriptors
 // as 32-bit words 781; without a wait for V and with one for K 740; K and V split ahead 719; a warp for each query tile then
-// 672. At head_dim 64 it is the softmax (hi and lo of P beside the exponentials). Against one 128-row tile per block on
+// 686 (CUDA graphs). At head_dim 64 it is the softmax (hi and lo of P beside the exponentials). Against one 128-row tile per block on
 // TF32 pairs: B1 H8 S1024 D64 dense 20.6 (37), H4/kvH1 8231 x 9075 rows D64 causal 161 (272).
 //
 // Every wait on an mbarrier is bounded (see tc_common.cuh); a wait that runs out reports into
@@ -110,8 +110,9 @@ struct F32Cfg {
   static constexpr bool kQLoInTmem = D == 64;
   static constexpr bool kAlias = D == 128;
   // There one warp issues for both query tiles in turn, or, where no splitters take issue slots, a warp for each (B1 H4
-  // S16384 D128 causal: 672 against 719 with split operands, 770 against 740 us without).
+  // S16384 D128 causal: 686 against 719 with split operands, 770 against 740 us without).
   static constexpr bool kTurns = kAlias && kPre;
+  static constexpr bool kOneIssuer = kAlias && !kTurns;
   static constexpr int kBoxes = DR / 32;                // raw boxes: 32 fp32 = 128 bytes of a row
   static constexpr int kGroups = D / 64;                // 64-column groups of a split tile
   static constexpr int kBoxBytes = kBNf * 128;
@@ -348,7 +349,7 @@ __global__ void __launch_bounds__((F32Cfg<DR, kSplit, kPre>::kThreads), 1)
     for (int s = 0; s < C::kStages; ++s) {
       mbar_init(bar_kv_raw + 8 * s, 1);
       mbar_init(bar_kv_full + 8 * s, kPre ? 1 : kSplitThreads);
-      mbar_init(bar_kv_empty + 8 * s, C::kAlias ? 1 : live);
+      mbar_init(bar_kv_empty + 8 * s, C::kOneIssuer ? 1 : live);  // (a commit is about its own thread's MMAs)
     }
     *abort_flag = gone != 0;
     if (s_base & 1023u) {  // the swizzle of TMA and the descriptors below count on it
@@ -461,7 +462,7 @@ __global__ void __launch_bounds__((F32Cfg<DR, kSplit, kPre>::kThreads), 1)
           }
         }
       }
-    } else if (warp == 1 || ((!C::kAlias || C::kTurns) && warp == 2 && live == 2)) {
+    } else if (warp == 1 || (!C::kOneIssuer && warp == 2 && live == 2)) {
       // ----------------------------------------------------------- MMA issuers ----
       if (n_tiles > 0) {
         constexpr unsigned idesc_s = make_idesc(0u, 0, kBNf, kBM);
@@ -479,7 +480,7 @@ __global__ void __launch_bounds__((F32Cfg<DR, kSplit, kPre>::kThreads), 1)
         auto wait_kv = [&](int it, int which, int t) {
           return wait(bar_kv_full + 8 * (it % C::kStages), (it / C::kStages) & 1, which, t);
         };
-        // `last`: no other query tile reads the slot after this one
+        // `last`: no other of this thread's MMAs reads the slot, which is free when they are done (or the caller sees to it)
         auto issue_s = [&](int t, int w, bool last) {
           const int slot = (2 * t) % C::kStages;
           const unsigned kd = static_cast<unsigned>(desc_kmajor(s_kv + slot * C::kSlotBytes));
@@ -530,25 +531,35 @@ __global__ void __launch_bounds__((F32Cfg<DR, kSplit, kPre>::kThreads), 1)
         if constexpr (C::kTurns) {
           // As below, but with a warp for each query tile, whose turn comes with the end of the other's batch: it has done its
           // waits by then. The tensor core's queue holds a few instructions, so a batch that follows at once leaves no gap.
+          // A turn orders when batches are issued, not when they end, and a commit is about its own thread's MMAs: each warp
+          // commits to the slots it has read, and a slot is free when both have. These commits go behind the turn, out of the
+          // other warp's way: B1 H4 S16384 D128 causal 686 us in a CUDA graph, with each behind its MMAs 703, V's there and K's behind
+          // the turn 694.
           const int w = warp - 1;
           auto turn = [&](int n) { return live == 1 || wait(bar_turn + 8 * w, n & 1, 12, n); };
+          auto free_slot = [&](int it) {  // (nobody waits for the last ones, so nothing arrives late in a block that ends)
+            if (it + C::kStages < 2 * n_tiles && elect_one()) tc_commit(bar_kv_empty + 8 * (it % C::kStages));
+          };
           auto pass = [&]() {
             if (live == 2 && elect_one()) mbar_arrive(bar_turn + 8 * (1 - w));
           };
           ok = wait(bar_q_full + 8 * w, 0, 3, w) && wait_kv(0, 5, 0) && (w == 0 || turn(0));
           if (ok) {
             tc_fence_after();
-            issue_s(0, w, w == live - 1);
+            issue_s(0, w, false);
             pass();
+            free_slot(0);
           }
           for (int t = 0; t < n_tiles && ok; ++t) {
             const bool more = t + 1 < n_tiles;
             ok = (!more || wait_kv(2 * t + 2, 5, t)) && wait(bar_p_full + 8 * w, t & 1, 6, t) && turn(t + w);
             if (!ok) break;
             tc_fence_after();
-            issue_pv(t, w, w == live - 1);
-            if (more) issue_s(t + 1, w, w == live - 1);
+            issue_pv(t, w, false);
+            if (more) issue_s(t + 1, w, false);
             pass();
+            free_slot(2 * t + 1);
+            if (more) free_slot(2 * t + 2);
           }
         } else if constexpr (C::kAlias) {
           // One warp issues for both query tiles, in turn: P.V of tile t and the scores of tile t + 1, which
@@ -1219,7 +1230,7 @@ size_t split_bytes(const StepArgs& a) {
 }
 // Whether K and V are split ahead, given a workspace: a pair of query tiles saves 0.3 us a key tile (0.35 at head_dim 128), and the
 // launch ahead costs 5 us and the way of K, V and their terms through memory. us per call, split by every block / ahead:
-// B1 H4 S16384 D128 causal 753 / 674, H8 S8192 D64 causal 241 / 217, H16/kvH8 B2 1000 rows on 6000 keys D32 168 / 152,
+// B1 H4 S16384 D128 causal 753 / 686, H8 S8192 D64 causal 241 / 217, H16/kvH8 B2 1000 rows on 6000 keys D32 168 / 152,
 // H8/kvH1 3810 rows dense D64 117 / 101; not so H8 2048 rows causal D128 75 / 81, H8 1024 rows dense D64 21 / 27. Over 130
 // random calls (300 to 16384 rows) the 53 taken ones 0.87 in the mean, 0.96 at worst.
 template <int DR>

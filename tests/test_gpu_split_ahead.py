@@ -83,6 +83,26 @@ def test_split_ahead_gives_the_same_bits(D, split, case):
     assert (buf[need:] == 0xff).all() and api.device_status()[0] == 0
 
 
+@pytest.mark.parametrize("H,kvH,S,causal", [(4, 4, 8192, 1), (6, 2, 5000, 1), (128, 4, 129, 0), (3, 1, 7777, 0)])
+def test_head_dim_128_refills_slots_behind_both_issuing_warps(H, kvH, S, causal):
+    """Two warps issue, and a ring slot is free when the MMAs of both have read it: long walks, blocks with one and with two
+    query tiles, again and again, give the bits of the form with one issuing warp."""
+    Sk = max(S, 3000)
+    g = torch.Generator(device="cuda").manual_seed(S)
+    q, k, v = (torch.randn(1, h, n, 128, generator=g, device="cuda") for h, n in ((H, S), (kvH, Sk), (kvH, Sk)))
+    shape, qmap, kmap = api.AttentionShape(1, H, S, Sk, 128, kvH), SegMap.make([Sk - S], S), SegMap.make([0], Sk)
+    flags = causal * CAUSAL | FRESH | FINALIZE
+    ws = torch.empty(2 * kvH * (Sk + 64) * 128 * 4 + kvH * (Sk + 64) * 8, dtype=torch.uint8, device="cuda")
+    want, state = ([torch.empty(s, device="cuda") for s in (q.shape, q.shape[:3], q.shape[:3])] for _ in range(2))
+    assert not run(q, k, v, want, shape, qmap, kmap, 1, flags, 0, None) & AHEAD
+    for _ in range(10):
+        for t in state:
+            t.fill_(float("nan"))
+        assert run(q, k, v, state, shape, qmap, kmap, 1, flags, 0, ws) & AHEAD
+        assert all(torch.equal(x, y) for x, y in zip(want, state))
+    assert api.device_status()[0] == 0
+
+
 def test_flash_with_and_without_room_for_the_split():
     B, H, kvH, S, D = 1, 16, 2, 2500, 64
     g = torch.Generator(device="cuda").manual_seed(3)
