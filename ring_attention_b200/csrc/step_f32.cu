@@ -1233,8 +1233,10 @@ size_t split_bytes(const StepArgs& a) {
 // B1 H4 S16384 D128 causal 753 / 686, H8 S8192 D64 causal 241 / 217, H16/kvH8 B2 1000 rows on 6000 keys D32 168 / 152,
 // H8/kvH1 3810 rows dense D64 117 / 101; not so H8 2048 rows causal D128 75 / 81, H8 1024 rows dense D64 21 / 27. Over 130
 // random calls (300 to 16384 rows) the 53 taken ones 0.87 in the mean, 0.96 at worst.
+// Not for more (batch, KV head) pairs than the launch ahead has blocks in y; the step itself has its heads in x.
 template <int DR>
 bool split_ahead(const StepArgs& a) {
+  if (static_cast<long long>(a.B) * a.kvH > 65535) return false;
   long long steps = 0;  // of one head
   const int per_seg = (a.qmap.seg_len + 2 * kBM - 1) / (2 * kBM);
   for (int sq = 0; sq < a.qmap.n_seg; ++sq)

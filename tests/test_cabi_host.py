@@ -133,6 +133,17 @@ def test_workspace_size_queries():
     assert lib().ra_flash_workspace_bytes(C.byref(s2), 1) > lib().ra_flash_workspace_bytes(C.byref(s2), 0)
 
 
+@pytest.mark.parametrize("D", [32, 64, 128])
+def test_fp32_split_ahead_leaves_calls_that_its_launch_cannot_hold(D):
+    """The launch that splits K and V ahead has (batch, KV head) in y: 65535 at most."""
+    def wanted(B, H, kvH, Sq, Sk):
+        shape, qmap, kmap = Shape(B, H, Sq, Sk, D, kvH), SegMap.make([0], Sq), SegMap.make([0], Sk)
+        return lib().ra_attention_step_workspace_bytes(0, C.byref(shape), C.byref(qmap), C.byref(kmap), 1, 6, 0)
+
+    assert wanted(4095, 64, 16, 1024, 1024) > 0 and wanted(16383, 32, 4, 512, 512) > 0  # 65520 and 65532 pairs
+    assert wanted(4096, 64, 16, 1024, 1024) == wanted(16384, 32, 4, 512, 512) == wanted(65536, 8, 1, 2048, 512) == 0
+
+
 @pytest.mark.parametrize("N,G", [(1, 1), (1, 8), (8, 1), (2, 2), (2, 4), (3, 5), (4, 8)])
 def test_ring2d_schedule_bit_exact_and_covering(N, G):
     """ra_ring2d_source against the oracle, plus the properties the reference's own test checks
