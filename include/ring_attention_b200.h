@@ -249,7 +249,9 @@ RA_API int ra_prefill_host(int dtype, const void* q_host, const void* k_host, co
  * fp32 only). The causal cut-off is q_offset - k_offset + 1 rows
  * (src/attention_decode.cu:110-116). Partials go through `workspace`
  * (ra_decode_workspace_bytes bytes); NULL uses a per-device buffer the library grows on
- * demand, like the reference's process-static workspace (src/attention_decode.cu:55-65). */
+ * demand, like the reference's process-static workspace (src/attention_decode.cu:55-65), which calls
+ * on several streams must not use at once (nor ra_local_decode_step, whose partials, m and l go there too). A
+ * CUDA graph may hold such calls: a buffer that a capture has met is kept when a larger call needs a new one. */
 RA_API size_t ra_decode_workspace_bytes(const ra_shape* shape);
 RA_API int ra_attention_decode_step(int dtype, const void* q, const void* k, const void* v,
                                     float* out, float* m, float* l, const ra_shape* shape,

@@ -1247,25 +1247,42 @@ DecodePlan make_plan(int groups, int stages, size_t stage_bytes, int per_sm, int
 struct DevWorkspace {
   void* ptr = nullptr;
   size_t bytes = 0;
+  bool recorded = false;  // a capture has seen `ptr`
 };
 DevWorkspace g_ws[64];
 std::mutex g_ws_mu;
 
-int ensure_workspace(size_t need, void** out) {
+// At least `need` bytes. `record`: the address may become part of a CUDA graph, whose replays go on writing there when a
+// larger call has made the workspace grow: such a buffer is never given back. Its successor is twice as large (or, if there
+// is no room, as large as it must be), so that all buffers left behind take no more than the last one.
+int grow_workspace(DevWorkspace& w, size_t need, bool record, void** out) {
+  if (w.bytes < need) {
+    const size_t old = w.recorded ? w.bytes : 0;
+    if (w.ptr && !w.recorded) RAB_CUDA(cudaFree(w.ptr));
+    if (!w.recorded) w = DevWorkspace();
+    void* ptr = nullptr;
+    size_t bytes = std::max(need, 2 * old);
+    if (bytes > need && cudaMalloc(&ptr, bytes) != cudaSuccess) {
+      cudaGetLastError();
+      ptr = nullptr;
+      bytes = need;
+    }
+    if (ptr == nullptr) RAB_CUDA(cudaMalloc(&ptr, bytes));
+    w.ptr = ptr;
+    w.bytes = bytes;
+    w.recorded = false;
+  }
+  w.recorded = w.recorded || record;
+  *out = w.ptr;
+  return RA_OK;
+}
+
+int ensure_workspace(size_t need, bool record, void** out) {
   int dev = 0;
   RAB_CUDA(cudaGetDevice(&dev));
   RAB_REQUIRE(dev >= 0 && dev < 64, RA_ERR_INVALID, "device index %d out of range", dev);
   std::lock_guard<std::mutex> lk(g_ws_mu);
-  DevWorkspace& w = g_ws[dev];
-  if (w.bytes < need) {
-    if (w.ptr) RAB_CUDA(cudaFree(w.ptr));
-    w.ptr = nullptr;
-    w.bytes = 0;
-    RAB_CUDA(cudaMalloc(&w.ptr, need));
-    w.bytes = need;
-  }
-  *out = w.ptr;
-  return RA_OK;
+  return grow_workspace(g_ws[dev], need, record, out);
 }
 
 bool workspace_holds(size_t need) {
@@ -1277,32 +1294,26 @@ bool workspace_holds(size_t need) {
 
 }  // namespace
 
+// (a few KB: asking whether the stream is captured would cost every call more than keeping the old ones)
 int decode_ml_scratch(size_t floats, float** out) {
   static DevWorkspace ml[64];
   int dev = 0;
   RAB_CUDA(cudaGetDevice(&dev));
   RAB_REQUIRE(dev >= 0 && dev < 64, RA_ERR_INVALID, "device index %d out of range", dev);
   std::lock_guard<std::mutex> lk(g_ws_mu);
-  DevWorkspace& w = ml[dev];
-  const size_t need = floats * sizeof(float);
-  if (w.bytes < need) {
-    if (w.ptr) RAB_CUDA(cudaFree(w.ptr));
-    w.ptr = nullptr;
-    w.bytes = 0;
-    RAB_CUDA(cudaMalloc(&w.ptr, need));
-    w.bytes = need;
-  }
-  *out = static_cast<float*>(w.ptr);
-  return RA_OK;
+  void* ptr = nullptr;
+  const int rc = grow_workspace(ml[dev], floats * sizeof(float), true, &ptr);
+  *out = static_cast<float*>(ptr);
+  return rc;
 }
 
 namespace {
 
 // Workspace of the balanced form: [row][slot] of O, m and l.
-int partial_space(size_t rows, int D, int cap, void* workspace, float** Op, float** Mp, float** Lp) {
+int partial_space(size_t rows, int D, int cap, void* workspace, bool record, float** Op, float** Mp, float** Lp) {
   const size_t need = rows * cap * (D + 2) * sizeof(float);
   if (workspace == nullptr) {
-    const int rc = ensure_workspace(need, &workspace);
+    const int rc = ensure_workspace(need, record, &workspace);
     if (rc != RA_OK) return rc;
   }
   *Op = static_cast<float*>(workspace);
@@ -1332,10 +1343,12 @@ int run_plan(const ra_shape& s, int head_batches, int stages, size_t stage_bytes
   };
   DecodePlan p = plan(true);
   // a stream that is being captured allows no allocation: such a call merges in clusters instead
-  if (!p.cluster && workspace == nullptr && p.deal.groups <= 65535 && !workspace_holds(p.deal.cap * slot_bytes)) {
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess) cudaGetLastError();
-    else if (capture != cudaStreamCaptureStatusNone) p = plan(false);
+  bool captured = false;
+  if (!p.cluster && workspace == nullptr) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &status) != cudaSuccess) cudaGetLastError();
+    captured = status != cudaStreamCaptureStatusNone;
+    if (captured && p.deal.groups <= 65535 && !workspace_holds(p.deal.cap * slot_bytes)) p = plan(false);
   }
   p.deal.head_batches = head_batches;
   p.deal.flags = flags;
@@ -1359,7 +1372,7 @@ int run_plan(const ra_shape& s, int head_batches, int stages, size_t stage_bytes
     return launch(true, cfg, p.deal, m, l, out);
   }
   float *Op, *Mp, *Lp;
-  int rc = partial_space(rows, D, p.deal.cap, workspace, &Op, &Mp, &Lp);
+  int rc = partial_space(rows, D, p.deal.cap, workspace, captured, &Op, &Mp, &Lp);
   if (rc != RA_OK) return rc;
   // (these fill every slot, so it makes no difference where one begins. The fold does not let the next call's
   // blocks start: they would take the slots around its own, and the last of them would begin behind it. B1 H8

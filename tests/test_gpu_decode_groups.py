@@ -1,5 +1,9 @@
 """Decode calls with more than two query heads to a KV head on caches that the tensor-core kernel does not take (fp32; 16-bit
 with head_dim 32), against attention in 64 bits: stage edges, ragged groups of heads, both ways of dealing the rows."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 import torch
@@ -68,6 +72,72 @@ def test_group_decode_first_called_while_captured():
     graph.replay()
     torch.cuda.synchronize()
     assert np.abs(out.cpu().numpy() - want).max() <= tol
+
+
+CAPTURES = """
+import torch
+from ring_attention_b200 import api
+
+def call(B, H, kvH, Sk, D, seed, local):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    q, k, v = (torch.randn(B, h, n, D, generator=g, device="cuda") for h, n in ((H, 1), (kvH, Sk), (kvH, Sk)))
+    out, m, l = torch.empty_like(q), torch.empty(B, H, 1, device="cuda"), torch.empty(B, H, 1, device="cuda")
+    shape = api.AttentionShape(B, H, 1, Sk, D, kvH)
+    if local:
+        cache = api.DeviceKVCache(B, kvH, Sk, D, torch.float32)
+        cache.copy_prefill(k, v, Sk)
+        return out, lambda: api.run_local_decode_step(q, cache, H, Sk, 0, True, out), cache
+    def run():
+        api.launch_attention_init(out, m, l, shape)
+        api.launch_attention_decode_step(q, k, v, out, m, l, shape, 0, 0, False)
+        api.launch_attention_finalize(out, l, shape)
+    return out, run, None
+
+def captured(run):
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        run()
+    return graph
+
+if cold:  # the library has no room for partials yet and cannot allocate any now: the call is recorded all the same
+    out, run, _ = call(2, 64, 8, 20011, 256, 1, False)
+    api.launch_attention_init(out, *(torch.empty(2, 64, 1, device="cuda") for _ in "ml"), api.AttentionShape(2, 64, 1, 1, 256, 8))
+    graph = captured(run)
+    graph.replay()
+    torch.cuda.synchronize()
+    got = out.clone()
+    run()
+    torch.cuda.synchronize()
+    assert ((got - out).norm() / out.norm()).item() < 1e-6  # (a cluster and a fold add up in another order)
+else:  # the room for partials and the scratch for m and l grow while a graph holds the old ones
+    for local in (False, True):
+        graphs = []
+        for n, shape in enumerate([(1, 8, 8, 16384, 64), (2, 64, 8, 20011, 256), (6, 128, 16, 9000, 256)]):
+            out, run, keep = call(*shape, n, local)
+            run()
+            torch.cuda.synchronize()
+            want = out.clone()
+            graphs.append((captured(run), out, want, keep, run))  # (what a graph reads has to live as long as it does)
+            junk = [torch.full((1 << s,), float("nan"), device="cuda") for s in range(8, 24)]  # on what was given back, if anything was
+            torch.cuda.synchronize()
+            for graph, o, w, *_ in graphs:
+                o.fill_(0)
+                graph.replay()
+                torch.cuda.synchronize()
+                assert torch.equal(o, w)
+            assert all(j.isnan().all() for j in junk)
+            del junk
+assert api.device_status()[0] == 0
+"""
+
+
+@pytest.mark.parametrize("cold", [True, False])
+def test_graphs_keep_the_partials_they_were_captured_with(cold):
+    """In a process of its own: what the library has allocated before decides what a capture meets."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", f"cold = {cold}\n" + CAPTURES], cwd=root, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
 
 
 @pytest.mark.parametrize("dtype,D", [(torch.float32, 64), (torch.float32, 256), (torch.float16, 32)])
