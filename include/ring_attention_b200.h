@@ -216,9 +216,11 @@ RA_API int ra_int8_to_float(const signed char* src, float* dst, size_t n, ra_str
 /* Whole single-GPU attention, fp32 in and out, end-aligned causal mask
  * (j <= i + seq_k - seq_q). Replaces launch_flash_attention and launch_flash_attention_fp16
  * (src/attention.hpp:48-65). `workspace` must hold
- * ra_flash_workspace_bytes(shape, half_precision) bytes of device memory. (The size includes what
- * ra_attention_step_ws would use; a workspace without that part is accepted.) */
+ * ra_flash_workspace_bytes(shape, half_precision) bytes of device memory. The size includes what
+ * ra_attention_step_ws would use (for long fp32 calls as much as K and V, twice that at head_dim 32); a
+ * workspace without that part, of ra_flash_workspace_least_bytes bytes, is accepted where there is no room for it. */
 RA_API size_t ra_flash_workspace_bytes(const ra_shape* shape, int half_precision);
+RA_API size_t ra_flash_workspace_least_bytes(const ra_shape* shape, int half_precision);
 RA_API int ra_flash_attention(const float* q, const float* k, const float* v, float* out,
                               const ra_shape* shape, int causal, int half_precision,
                               void* workspace, size_t workspace_bytes, ra_stream stream);

@@ -97,6 +97,7 @@ _SIG = {
     "ra_float_to_int8": (C.c_int, [_P, _P, C.c_size_t, _P]),
     "ra_int8_to_float": (C.c_int, [_P, _P, C.c_size_t, _P]),
     "ra_flash_workspace_bytes": (C.c_size_t, [C.POINTER(Shape), C.c_int]),
+    "ra_flash_workspace_least_bytes": (C.c_size_t, [C.POINTER(Shape), C.c_int]),
     "ra_flash_attention": (C.c_int, [_P, _P, _P, _P, C.POINTER(Shape), C.c_int, C.c_int, _P,
                                      C.c_size_t, _P]),
     "ra_prefill_host": (C.c_int, [C.c_int, _P, _P, _P, _P, _P, C.POINTER(Shape),

@@ -58,24 +58,40 @@ ra_segmap to_c(const SegMap& m) {
   return c;
 }
 
-// One device scratch per process for the whole-attention entry points (grown on demand).
-void* flash_scratch(size_t bytes) {
+// One device scratch per process for the whole-attention entry points (grown on demand): `most` bytes, or, where
+// those are not free, no fewer than `least`. `bytes` gets its size.
+void* flash_scratch(size_t most, size_t least, size_t* bytes) {
   static void* ptr = nullptr;
   static size_t have = 0;
-  if (have < bytes) {
-    if (ptr) cudaFree(ptr);
-    cuda_must(cudaMalloc(&ptr, bytes), "flash scratch");
-    have = bytes;
+  if (have < most) {
+    void* larger = nullptr;
+    if (have < least && ptr) {  // no use any more
+      cudaFree(ptr);
+      ptr = nullptr;
+      have = 0;
+    }
+    if (cudaMalloc(&larger, most) == cudaSuccess) {
+      if (ptr) cudaFree(ptr);
+      ptr = larger;
+      have = most;
+    } else {
+      cudaGetLastError();
+      if (have < least) {
+        cuda_must(cudaMalloc(&ptr, least), "flash scratch");
+        have = least;
+      }
+    }
   }
+  *bytes = have;
   return ptr;
 }
 void flash(const float* q, const float* k, const float* v, float* out, const AttentionShape& s,
            bool causal, bool half_precision, cudaStream_t stream, const char* who) {
   const ra_shape c = to_c(s);
-  const size_t need = ra_flash_workspace_bytes(&c, half_precision);
-  must(ra_flash_attention(q, k, v, out, &c, causal, half_precision, flash_scratch(need), need,
-                          stream),
-       who);
+  size_t bytes = 0;
+  void* const scratch = flash_scratch(ra_flash_workspace_bytes(&c, half_precision),
+                                      ra_flash_workspace_least_bytes(&c, half_precision), &bytes);
+  must(ra_flash_attention(q, k, v, out, &c, causal, half_precision, scratch, bytes, stream), who);
 }
 
 }  // namespace

@@ -282,6 +282,8 @@ static int flash_step(int dtype, const void* q, const void* k, const void* v, fl
                  wanted);
 }
 
+size_t ra_flash_workspace_least_bytes(const ra_shape* s, int half_precision) { return s ? flash_bytes(*s, half_precision) : 0; }
+
 size_t ra_flash_workspace_bytes(const ra_shape* s, int half_precision) {
   if (!s) return 0;
   size_t most = 0;

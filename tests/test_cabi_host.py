@@ -131,6 +131,12 @@ def test_workspace_size_queries():
     assert lib().ra_decode_workspace_bytes(C.byref(s)) >= 4 * 32 * 130 * 4
     s2 = Shape(1, 8, 64, 64, 64, 0)
     assert lib().ra_flash_workspace_bytes(C.byref(s2), 1) > lib().ra_flash_workspace_bytes(C.byref(s2), 0)
+    s3 = Shape(1, 8, 8192, 8192, 128, 0)
+    for half in (0, 1):
+        assert lib().ra_flash_workspace_least_bytes(C.byref(s2), half) == lib().ra_flash_workspace_bytes(C.byref(s2), half)
+        least = 8 * 8192 * 8 + half * 3 * 8 * 8192 * 128 * 2
+        assert least <= lib().ra_flash_workspace_least_bytes(C.byref(s3), half) <= least + 1024
+    assert lib().ra_flash_workspace_bytes(C.byref(s3), 0) > 2 * 8 * 8192 * 128 * 4  # and K and V in split form
 
 
 @pytest.mark.parametrize("D", [32, 64, 128])

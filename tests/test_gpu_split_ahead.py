@@ -124,6 +124,38 @@ def test_flash_with_and_without_room_for_the_split():
     assert_close(outs[0][:, :, rows].cpu().numpy(), want[:, :, rows], 1e-5, 1e-5, "flash")
 
 
+def test_calls_run_without_the_split_where_there_is_no_room_for_it():
+    B, H, kvH, rows, keys, D = 1, 16, 8, 2048, 20000, 128
+    g = torch.Generator(device="cuda").manual_seed(3)
+    q, k, v = (torch.randn(B, h, n, D, generator=g, device="cuda") for h, n in ((H, rows), (kvH, keys), (kvH, keys)))
+    shape, qmap, kmap = api.AttentionShape(B, H, rows, keys, D, kvH), SegMap.make([0], rows), SegMap.make([0], keys)
+    state = [torch.empty(s, device="cuda") for s in (q.shape, q.shape[:3], q.shape[:3])]
+    flash = torch.empty_like(q)
+
+    def both():
+        api.attention_step_ex(q, k, v, *state, shape, qmap, kmap, fresh=True, finalize=True)
+        forms = [lib().ra_debug_step_form() & AHEAD]
+        api.launch_flash_attention(q, k, v, flash, shape, True)
+        return forms + [lib().ra_debug_step_form() & AHEAD]
+
+    assert both() == [AHEAD, AHEAD]
+    want = [t.clone() for t in (*state, flash)]
+    for t in (*state, flash):
+        t.fill_(0)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    room = torch.cuda.memory_reserved() + (64 << 20)  # K and V in split form take 164 MB
+    torch.cuda.set_per_process_memory_fraction(room / torch.cuda.get_device_properties(0).total_memory)
+    try:
+        assert both() == [0, 0]
+        with pytest.raises(torch.OutOfMemoryError):  # not even what the call cannot do without
+            api._workspace(1 << 30, 1 << 29)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert all(torch.equal(a, b) for a, b in zip((*state, flash), want))
+    assert both() == [AHEAD, AHEAD]
+
+
 @pytest.mark.parametrize("D", [64, 128])
 def test_split_ahead_steps_that_give_up_keep_their_state(D):
     B, H, kvH, rows, keys = 1, 16, 2, 2048, 3000
