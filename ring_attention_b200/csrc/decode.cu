@@ -123,8 +123,8 @@ struct DecodeCfg {
   static constexpr int kSmemBytes = 2 * kStages * kStageBytes;
 };
 
-// decode_group_kernel: a lane owns four columns of a row, or eight at head_dim 256, and a warp takes kRows rows of each of
-// its 32 / kLPR lane groups at a time.
+// decode_group_kernel: a lane owns four columns of a row, or eight at head_dim 256, and a warp takes kSets times kRows rows of
+// each of its 32 / kLPR lane groups at a time.
 template <typename T, int D, int GB>
 struct GroupCfg {
   static constexpr int kRowBytes = D * static_cast<int>(sizeof(T));
@@ -135,7 +135,8 @@ struct GroupCfg {
   static constexpr int kRows = D == 256 ? 2 : (kLPR / GB < 4 ? kLPR / GB : 4);
   static constexpr int kScores = kRows * GB;  // of a lane group; no more than it has lanes
   static constexpr int kGroups = 32 / kLPR;
-  static constexpr int kRowsPerWarpStep = kGroups * kRows;
+  static constexpr int kSets = sizeof(T) == 2 ? 2 : 1;  // such sets of scores a step
+  static constexpr int kRowsPerWarpStep = kGroups * kRows * kSets;
   static constexpr int kWarps =
       8192 / kRowBytes / kRowsPerWarpStep < 8 ? 8192 / kRowBytes / kRowsPerWarpStep : 8;
   static constexpr int kThreads = kWarps * 32;
@@ -144,7 +145,13 @@ struct GroupCfg {
   static constexpr int kRowsPerStage = kRowsPerStep * kSteps;
   static constexpr int kStageBytes = kRowsPerStage * kRowBytes;  // per tensor
   static constexpr int kSmemBytes = 2 * kStages * kStageBytes;
-  static_assert(kStageBytes == 8192 && kScores <= kLPR, "8 KB per tensor and stage, a score for each lane");
+  // Whether the rows of a step are added up by themselves before they reach the accumulators: fewer terms one after
+  // another there. So where a block has fewer lane groups, or (at head_dim 32) an SM fewer blocks or a row more lanes, than in
+  // the kernel above, whose error against 64 bits is not to be exceeded: 16 bits, head_dim 32, B5 H64/kvH16 150000 rows 4.8e-7
+  // so, 6.5e-7 without, H64/kvH8 3.5e-7 and 5.0e-7. (Elsewhere the errors are those of before either way, and the
+  // additions cost B5 H48/kvH6 D64, 55149 rows 175 us instead of 159.)
+  static constexpr bool kSumFirst = kRows * kSets > 1 && (kWarps < 8 || D == 32);
+  static_assert(kStageBytes == 8192 && kScores <= kLPR, "8 KB per tensor and stage, a score for each lane and set");
 };
 
 // ---- how the keys are dealt to blocks ----------------------------------------------------
@@ -559,9 +566,10 @@ __global__ void __launch_bounds__(kThreads)
 // lane holds head j ^ (lane % GB) and row i is row i ^ (lane / GB % kRows), so what a lane keeps and what it
 // gives away are the same registers in all of them. The softmax is one exponential a lane, the
 // weights go to all lanes through shared memory, both contractions are packed FMAs, and a step's rows are added up before they
-// reach the accumulators (without that the error against 64 bits grew from 2.4e-7 to 2.9e-7 on 40000 rows: an SM has fewer
+// reach the accumulators where kSumFirst says so (without that the error against 64 bits grew from 2.4e-7 to 2.9e-7 on 40000 rows: an SM has fewer
 // warps than before, so each adds more rows). With eight heads of 128 about 80 instead of 180 instructions a row and warp, 16
-// instead of 40 of them shuffles. fp32, eight heads, before / now (floor of the copy): B1 H64/kvH8 D256 135081 rows 939 / 332 us
+// instead of 40 of them shuffles. Two sets of rows a step, in 16 bits, share the maximum, the barrier and the reading of the
+// weights (64 random calls of head_dim 32: 0.97 of the time with one). fp32, eight heads, before / now (floor of the copy): B1 H64/kvH8 D256 135081 rows 939 / 332 us
 // (338), B3 H48/kvH6 D128 179592 rows 1073 / 508 (505), B1 H32/kvH4 D128 16049 rows 31 / 20 (10); bf16 rows of 32, B2 H32/kvH4
 // 225843 rows 179 / 96 (35). Four heads were near the copy in long calls (B3 H64/kvH16 D64 162905 rows 578 / 548);
 // short ones are 3 to 25 % faster (B2 H12/kvH4 D128 683 rows 8.2 / 6.9). 110 random calls: 0.85 in the mean, 0.99 at worst.
@@ -585,10 +593,10 @@ __global__ void __launch_bounds__(GroupCfg<T, D, GB>::kThreads)
     decode_group_kernel(const T* Q, const T* K, const T* V, float* Mp, float* Lp, float* Op, int H, int kvH, int sk_eff,
                         long long kv_head_stride, const Deal deal, float scale_log2) {
   using C = GroupCfg<T, D, GB>;
-  constexpr int kR = C::kRows;
+  constexpr int kR = C::kRows, kAll = kR * C::kSets;
   extern __shared__ __align__(16) unsigned char smem[];
   // a warp's weights of one step; two buffers, so that one barrier a step is enough
-  __shared__ __align__(16) float weights[C::kWarps][2][C::kGroups * C::kScores];
+  __shared__ __align__(16) float weights[C::kWarps][2][C::kGroups * C::kScores * C::kSets];
   unsigned char* k_ring = smem;
   unsigned char* v_ring = smem + deal.ring * C::kStageBytes;
 
@@ -665,46 +673,51 @@ __global__ void __launch_bounds__(GroupCfg<T, D, GB>::kThreads)
       const int slot = st % kStages;
 #pragma unroll 1
       for (int step = 0; step < C::kSteps; ++step) {
-        // row i of lane group g: first + i * kGroups + g
+        // row i of lane group g: first + i * kGroups + g; kR of them make a set
         const int first = step * C::kRowsPerStep + warp * C::kRowsPerWarpStep + grp;
         const unsigned char* krow = k_ring + slot * C::kStageBytes + first * C::kRowBytes + lr * C::kPieceBytes;
         const unsigned char* vrow = v_ring + slot * C::kStageBytes + first * C::kRowBytes + lr * C::kPieceBytes;
-        float s[kR][GB];
+        float score[C::kSets];
+        bool valid[C::kSets];
+        float m_new = -INFINITY;
 #pragma unroll
-        for (int i = 0; i < kR; ++i) {
-          float2 acc[GB];
+        for (int set = 0; set < C::kSets; ++set) {
+          float s[kR][GB];
 #pragma unroll
-          for (int j = 0; j < GB; ++j) acc[j] = make_float2(0.f, 0.f);
+          for (int i = 0; i < kR; ++i) {
+            float2 acc[GB];
 #pragma unroll
-          for (int v = 0; v < C::kVPT; ++v) {
-            float f[4];
-            load_four<T>(krow + (i ^ my_row) * C::kGroups * C::kRowBytes + v * C::kLPR * C::kPieceBytes, f);
-            const float2 k0 = make_float2(f[0], f[1]), k1 = make_float2(f[2], f[3]);
+            for (int j = 0; j < GB; ++j) acc[j] = make_float2(0.f, 0.f);
 #pragma unroll
-            for (int j = 0; j < GB; ++j) {
-              acc[j] = ffma2(q2[j][2 * v], k0, acc[j]);
-              acc[j] = ffma2(q2[j][2 * v + 1], k1, acc[j]);
+            for (int v = 0; v < C::kVPT; ++v) {
+              float f[4];
+              load_four<T>(krow + (set * kR + (i ^ my_row)) * C::kGroups * C::kRowBytes + v * C::kLPR * C::kPieceBytes, f);
+              const float2 k0 = make_float2(f[0], f[1]), k1 = make_float2(f[2], f[3]);
+#pragma unroll
+              for (int j = 0; j < GB; ++j) {
+                acc[j] = ffma2(q2[j][2 * v], k0, acc[j]);
+                acc[j] = ffma2(q2[j][2 * v + 1], k1, acc[j]);
+              }
             }
+#pragma unroll
+            for (int j = 0; j < GB; ++j) s[i][j] = acc[j].x + acc[j].y;
           }
 #pragma unroll
-          for (int j = 0; j < GB; ++j) s[i][j] = acc[j].x + acc[j].y;
+          for (int half = kR / 2; half > 0; half /= 2)
+#pragma unroll
+            for (int i = 0; i < half; ++i)
+#pragma unroll
+              for (int j = 0; j < GB; ++j) s[i][j] += __shfl_xor_sync(0xffffffffu, s[i + half][j], half * GB);
+#pragma unroll
+          for (int half = GB / 2; half > 0; half /= 2)
+#pragma unroll
+            for (int j = 0; j < half; ++j) s[0][j] += __shfl_xor_sync(0xffffffffu, s[0][j + half], half);
+          score[set] = s[0][0];
+#pragma unroll
+          for (int off = C::kScores; off < C::kLPR; off *= 2) score[set] += __shfl_xor_sync(0xffffffffu, score[set], off);
+          valid[set] = st * C::kRowsPerStage + first + (set * kR + my_row) * C::kGroups < n_rows;
+          m_new = fmaxf(m_new, valid[set] ? score[set] : -INFINITY);
         }
-#pragma unroll
-        for (int half = kR / 2; half > 0; half /= 2)
-#pragma unroll
-          for (int i = 0; i < half; ++i)
-#pragma unroll
-            for (int j = 0; j < GB; ++j) s[i][j] += __shfl_xor_sync(0xffffffffu, s[i + half][j], half * GB);
-#pragma unroll
-        for (int half = GB / 2; half > 0; half /= 2)
-#pragma unroll
-          for (int j = 0; j < half; ++j) s[0][j] += __shfl_xor_sync(0xffffffffu, s[0][j + half], half);
-        float score = s[0][0];
-#pragma unroll
-        for (int off = C::kScores; off < C::kLPR; off *= 2) score += __shfl_xor_sync(0xffffffffu, score, off);
-
-        const bool valid = st * C::kRowsPerStage + first + my_row * C::kGroups < n_rows;
-        float m_new = valid ? score : -INFINITY;
 #pragma unroll
         for (int off = GB; off < C::kScores; off *= 2) m_new = fmaxf(m_new, __shfl_xor_sync(0xffffffffu, m_new, off));
         m_new = fmaxf(m_run, m_new);
@@ -720,42 +733,44 @@ __global__ void __launch_bounds__(GroupCfg<T, D, GB>::kThreads)
             for (int e = 0; e < C::kEPL; ++e) o2[j][e] = ffma2(o2[j][e], a, make_float2(0.f, 0.f));
           }
         }
-        const float p = valid && score != -INFINITY ? ex2(score - m_run) : 0.f;
-        l_run += p;
         float* w = weights[warp][buf];
         buf ^= 1;
-        if (lead) w[grp * C::kScores + lr] = p;
-        __syncwarp();
-        float2 p2[kR][GB / 2];
+        float l_step = 0.f;
 #pragma unroll
-        for (int i = 0; i < kR; ++i)
+        for (int set = 0; set < C::kSets; ++set) {
+          const float p = valid[set] && score[set] != -INFINITY ? ex2(score[set] - m_run) : 0.f;
+          l_step += p;
+          if (lead) w[(grp * C::kSets + set) * C::kScores + lr] = p;
+        }
+        l_run += l_step;
+        __syncwarp();
+        float2 p2[kAll][GB / 2];
+#pragma unroll
+        for (int i = 0; i < kAll; ++i)
 #pragma unroll
           for (int j = 0; j < GB / 4; ++j) {
-            const float4 x = *reinterpret_cast<const float4*>(w + grp * C::kScores + i * GB + 4 * j);
+            const float4 x = *reinterpret_cast<const float4*>(w + grp * C::kSets * C::kScores + i * GB + 4 * j);
             p2[i][2 * j] = make_float2(x.x, x.y);
             p2[i][2 * j + 1] = make_float2(x.z, x.w);
           }
-        // Where a block has fewer than 8 warps, the rows of a step are added up by themselves first: fewer terms one
-        // after another on the accumulators. (With 8 the errors are those of before either way, and the additions cost
-        // B5 H48/kvH6 D64, 55149 rows 175 us instead of 159.)
 #pragma unroll
         for (int v = 0; v < C::kVPT; ++v) {
-          float f[kR][4];
+          float f[kAll][4];
 #pragma unroll
-          for (int i = 0; i < kR; ++i)
+          for (int i = 0; i < kAll; ++i)
             load_four<T>(vrow + i * C::kGroups * C::kRowBytes + v * C::kLPR * C::kPieceBytes, f[i]);
 #pragma unroll
           for (int e = 0; e < 4; ++e)
 #pragma unroll
             for (int j = 0; j < GB / 2; ++j) {
               float2& o = o2[j][4 * v + e];
-              if constexpr (C::kWarps == 8) {
+              if constexpr (!C::kSumFirst) {
 #pragma unroll
-                for (int i = 0; i < kR; ++i) o = ffma2(p2[i][j], make_float2(f[i][e], f[i][e]), o);
+                for (int i = 0; i < kAll; ++i) o = ffma2(p2[i][j], make_float2(f[i][e], f[i][e]), o);
               } else {
                 float2 sum = ffma2(p2[0][j], make_float2(f[0][e], f[0][e]), make_float2(0.f, 0.f));
 #pragma unroll
-                for (int i = 1; i < kR; ++i) sum = ffma2(p2[i][j], make_float2(f[i][e], f[i][e]), sum);
+                for (int i = 1; i < kAll; ++i) sum = ffma2(p2[i][j], make_float2(f[i][e], f[i][e]), sum);
                 o = fadd2(o, sum);
               }
             }
@@ -1192,7 +1207,7 @@ constexpr StageCost simt_stage_cost(int heads, size_t stage_bytes) {
 
 // Which form, and how many blocks. `per_sm`: resident blocks per SM; `cap`: partial slots per row
 // that the workspace holds; `rows`: (batch, head) rows; `head_rows`: rows of a group; `partials`: there is room for
-// partials, or there can be. Every estimate is the walk of a block, wave by wave, at what its SM or the
+// partials, or there can be; `long_share`: with more stages a block, twice as many blocks (0: never). Every estimate is the walk of a block, wave by wave, at what its SM or the
 // memory (7 TB/s) allows, plus what the fold (a launch, and more the more rows it has) or the merge
 // (columns of the group, blocks of the cluster, and a wave of clusters starts slower than one of blocks)
 // adds. Constants fitted to 457 shapes (heads 8/8 to 64/1, batch 1 to 64, 200 to 100000 rows, fp16 and fp32,
@@ -1202,7 +1217,7 @@ constexpr StageCost simt_stage_cost(int heads, size_t stage_bytes) {
 // be 0.7 %. It stays all the same: a fold goes through the library's partials, which calls on several streams must not
 // share, and calls that merge in clusters have none.
 DecodePlan make_plan(int groups, int stages, size_t stage_bytes, int per_sm, int cap, int ring_max,
-                     StageCost cost, size_t rows, int head_rows, int D, bool partials) {
+                     StageCost cost, size_t rows, int head_rows, int D, bool partials, int long_share) {
   constexpr double kBytesPerUs = 7e6, kFold = 8.2, kFoldRow = 0.005, kMerge = 0.6, kMergeBlock = 0.15,
                    kMergeElement = 0.0005, kWave = 1.5, kClusterWave = 4.0;
   DecodePlan p;
@@ -1217,6 +1232,7 @@ DecodePlan make_plan(int groups, int stages, size_t stage_bytes, int per_sm, int
   // no more partials than the workspace holds: a group meets at most ceil(ctas / groups) + 1 blocks,
   // exactly one each when there are as many blocks as groups
   long long ctas = std::min<long long>(slots, static_cast<long long>(total));
+  if (long_share > 0 && total > static_cast<double>(long_share) * slots) ctas *= 2;
   ctas = cap > 1 ? std::min(ctas, (cap - 1ll) * groups) : groups;
   p.cluster = 0;
   p.ctas = static_cast<int>(ctas);
@@ -1326,7 +1342,7 @@ int partial_space(size_t rows, int D, int cap, void* workspace, bool record, flo
 // launch(cluster form?, config, deal, Mp, Lp, Op) sets the attribute and launches the kernel.
 template <int D, int ROWS, typename Launch>
 int run_plan(const ra_shape& s, int head_batches, int stages, size_t stage_bytes, int ring_max, int per_sm,
-             StageCost cost, size_t red_bytes, int old_splits, float* out, float* m, float* l, void* workspace,
+             StageCost cost, int long_share, size_t red_bytes, int old_splits, float* out, float* m, float* l, void* workspace,
              size_t workspace_bytes, int split_cap, unsigned flags, cudaStream_t stream, Launch launch) {
   const int kvH = kv_heads_of(s);
   const size_t rows = static_cast<size_t>(s.batch) * s.heads;
@@ -1339,7 +1355,7 @@ int run_plan(const ra_shape& s, int head_batches, int stages, size_t stage_bytes
   }
   auto plan = [&](bool partials) {
     return make_plan(s.batch * kvH * head_batches, stages, stage_bytes, per_sm, cap, ring_max, cost, rows,
-                     std::min(ROWS, (s.heads + kvH - 1) / kvH), D, partials);
+                     std::min(ROWS, (s.heads + kvH - 1) / kvH), D, partials, long_share);
   };
   DecodePlan p = plan(true);
   // a stream that is being captured allows no allocation: such a call merges in clusters instead
@@ -1448,7 +1464,7 @@ int launch_decode_typed(const void* q, const void* k, const void* v, float* out,
     const int stages = (sk_eff + M::kStageRows - 1) / M::kStageRows;
     static const int per_sm = resident_blocks(decode_mma_kernel<T, D, kBalanced>, M::kThreads, kSmem);
     return run_plan<D, 16>(
-        s, head_batches, stages, 2 * M::kStageBytes, M::kStages, per_sm, mma_stage_cost(D), kRed,
+        s, head_batches, stages, 2 * M::kStageBytes, M::kStages, per_sm, mma_stage_cost(D), 0, kRed,
         fixed_splits(s.batch * kvH * head_batches, sk_eff, 64, split_cap), out,
         m, l, workspace, workspace_bytes, split_cap, flags, stream,
         [&](bool cluster, cudaLaunchConfig_t& cfg, const Deal& deal, float* Mp, float* Lp, float* Op) {
@@ -1476,10 +1492,16 @@ int launch_decode_typed(const void* q, const void* k, const void* v, float* out,
       const int head_batches = (group + GB - 1) / GB;
       const int stages = (sk_eff + C::kRowsPerStage - 1) / C::kRowsPerStage;
       // fp32, four and eight heads: two blocks an SM move 7.3 and 6.9 TB/s, three 6.9 and 6.9 (D128; B3 H32/kvH8, 200335 rows
-      // 699 us with two, 731 with three). 16-bit rows of 32 are bound by instructions: 5.3 with two, 5.7 with three
+      // 699 us with two, 731 with three). 16-bit rows of 32: as many as their registers allow (two; three with four heads in 80
+      // registers are 22 % faster to 6 % slower by shape, and their longer calls would have the larger errors)
       static const int per_sm = std::min(resident_blocks(balanced, kBlockThreads, kSmem), GB >= 4 && sizeof(T) == 4 ? 2 : 16);
+      // Eight heads, 16-bit rows of 32: a lane adds 1/64 of a block's rows one after another, so blocks with more than 24
+      // stages (3072 rows) are cut in two. Error against 64 bits of B5 H64/kvH8, 150000 rows: 3.9e-7 uncut, 3.2e-7 so, 3.5e-7 in the
+      // kernel with a butterfly for each head, which had two thirds of the rows a block; below that length there is no difference. It
+      // costs such calls 2 to 15 % (fp16 B1 H64/kvH8, 175724 rows 72 -> 77 us).
+      constexpr int kLongShare = GB == 8 && sizeof(T) == 2 ? 24 : 0;
       return run_plan<D, GB>(
-          s, head_batches, stages, 2 * C::kStageBytes, kStages, per_sm, simt_stage_cost(GB, 2 * C::kStageBytes), kRed,
+          s, head_batches, stages, 2 * C::kStageBytes, kStages, per_sm, simt_stage_cost(GB, 2 * C::kStageBytes), kLongShare, kRed,
           fixed_splits(s.batch * kvH * head_batches, sk_eff, Plan::kRowsPerStage, split_cap),
           out, m, l, workspace, workspace_bytes, split_cap, flags, stream,
           [&](bool cluster, cudaLaunchConfig_t& cfg, const Deal& deal, float* Mp, float* Lp, float* Op) {

@@ -74,6 +74,31 @@ def test_group_decode_first_called_while_captured():
     assert np.abs(out.cpu().numpy() - want).max() <= tol
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("B,H,kvH,Sk,blocks,added", [
+    (2, 64, 16, 262144, 296, 4),   # four heads a block: the rows of a step (4 a lane) are added up first
+    (4, 64, 8, 200000, 592, 2)])   # eight heads (2 a lane), and long shares are cut in two
+def test_long_group_decode_adds_no_longer_chains(dtype, B, H, kvH, Sk, blocks, added):
+    """The error of long calls is that of chains of additions: a lane group (32 a block) has k = rows / blocks / 32 / added of them
+    on each accumulator. Sums of terms of either sign walk like sqrt(i), and so do their roundings (0.3 to 0.5 units of 2^-24,
+    relative): about 0.2 sqrt(k) units, beside 3 to 4 of the scores and exponentials. Twice the chain is outside."""
+    D = 32
+    g = torch.Generator(device="cuda").manual_seed(11)
+    q, k, v = (torch.randn(B, h, n, D, generator=g, device="cuda").to(dtype) for h, n in ((H, 1), (kvH, Sk), (kvH, Sk)))
+    want = torch.empty(B, H, 1, D, dtype=torch.double, device="cuda")
+    for b in range(B):
+        for j in range(kvH):
+            s = q[b, j::kvH, 0].double() @ k[b, j].double().T / D ** 0.5
+            want[b, j::kvH, 0] = torch.softmax(s, -1) @ v[b, j].double()
+    out, m, l = torch.empty(B, H, 1, D, device="cuda"), torch.empty(B, H, 1, device="cuda"), torch.empty(B, H, 1, device="cuda")
+    shape = api.AttentionShape(B, H, 1, Sk, D, kvH)
+    api.launch_attention_init(out, m, l, shape)
+    api.launch_attention_decode_step(q, k, v, out, m, l, shape, 0, 0, False)
+    api.launch_attention_finalize(out, l, shape)
+    chain = B * kvH * Sk / blocks / 32 / added
+    assert ((out - want).norm() / want.norm()).item() <= 2.0 ** -24 * (4.5 + 0.2 * chain ** 0.5)
+
+
 CAPTURES = """
 import torch
 from ring_attention_b200 import api
