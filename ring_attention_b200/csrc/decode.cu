@@ -1492,8 +1492,8 @@ int launch_decode_typed(const void* q, const void* k, const void* v, float* out,
       const int head_batches = (group + GB - 1) / GB;
       const int stages = (sk_eff + C::kRowsPerStage - 1) / C::kRowsPerStage;
       // fp32, four and eight heads: two blocks an SM move 7.3 and 6.9 TB/s, three 6.9 and 6.9 (D128; B3 H32/kvH8, 200335 rows
-      // 699 us with two, 731 with three). 16-bit rows of 32: as many as their registers allow (two; three with four heads in 80
-      // registers are 22 % faster to 6 % slower by shape, and their longer calls would have the larger errors)
+      // 699 us with two, 731 with three). 16-bit rows of 32: as many as their registers allow (two; with four heads kept
+      // to 80 registers three fit, 22 % faster to 22 % slower by shape and even in the mean)
       static const int per_sm = std::min(resident_blocks(balanced, kBlockThreads, kSmem), GB >= 4 && sizeof(T) == 4 ? 2 : 16);
       // Eight heads, 16-bit rows of 32: a lane adds 1/64 of a block's rows one after another, so blocks with more than 24
       // stages (3072 rows) are cut in two. Error against 64 bits of B5 H64/kvH8, 150000 rows: 3.9e-7 uncut, 3.2e-7 so, 3.5e-7 in the
