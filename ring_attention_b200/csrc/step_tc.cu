@@ -1416,7 +1416,8 @@ size_t spread_bytes(const StepArgs& a, const Spread& spread) {
   return static_cast<size_t>(a.B) * a.kvH * spread.total * TcCfg<D, true>::kTiles * kBM * (a.D + 2) * sizeof(float);
 }
 
-// The form of a call that may choose: blocks that share a query block's keys, folded tiles, or (`spread` not null) the spread form.
+// The form of a call that may choose: blocks that share a query block's keys, folded tiles, or (`spread` not null, which a call
+// without a workspace need not ask for) the spread form.
 struct Form {
   int split = 1;
   bool fold = false, spread = false;
@@ -1433,7 +1434,7 @@ int pick_form(const StepArgs& a, Form* form, Spread* spread) {
     double tiles = 0;
     form->split = pick_key_split<kBN>(a, TcCfg<D, true>::kTiles * kBM, D == 64 ? 1.5 : D == 128 ? 2.5 : 4.5, slots, &tiles);
     if constexpr (D <= 128) form->fold = fold_rows<kBN>(a, D == 64 ? 0.75 : 0.87, tiles);
-    form->spread = !form->fold && plan_spread<kBN>(a, TcCfg<D, true>::kTiles, D <= 128 ? 4 : 6, slots[1], tiles, spread);
+    form->spread = spread && !form->fold && plan_spread<kBN>(a, TcCfg<D, true>::kTiles, D <= 128 ? 4 : 6, slots[1], tiles, spread);
   }
   return RA_OK;
 }
@@ -1445,11 +1446,11 @@ int launch_d(int dtype, const StepArgs& a, cudaStream_t stream) {
   const bool p_in_tmem = (a.flags & RA_STEP_P_IN_SMEM) == 0;
   Form form;
   Spread spread;
-  const int rc = pick_form<D>(a, &form, &spread);
+  const int rc = pick_form<D>(a, &form, a.workspace ? &spread : nullptr);
   if (rc != RA_OK) return rc;
   const int split = form.split;
   [[maybe_unused]] const bool fold = form.fold;
-  if (form.spread && a.workspace != nullptr && a.workspace_bytes >= spread_bytes<D>(a, spread) &&
+  if (form.spread && a.workspace_bytes >= spread_bytes<D>(a, spread) &&
       (reinterpret_cast<uintptr_t>(a.workspace) & 15u) == 0) {
     if constexpr (D == 64) {
       if (a.D == 32) return launch_spread<64, 32>(dtype, a, stream, spread);
