@@ -60,15 +60,18 @@ def _dtype(t):
         raise ValueError(f"unsupported dtype {t.dtype}") from None
 
 
-def _workspace(most, least, device="cuda"):
-    """Device memory of ``most`` bytes for a call on the current stream, or, where that much is not free, of the ``least``
+def _workspace(most, least=lambda: 0, device="cuda"):
+    """Device memory of ``most`` bytes for a call on the current stream, or, where that much is not free, of the ``least()``
     bytes that the call can do with (None for 0 bytes)."""
-    for n in (most, least):
-        try:
-            return torch.empty(n, dtype=torch.uint8, device=device) if n else None
-        except torch.OutOfMemoryError:
-            if n <= least:
-                raise
+    if not most:
+        return None
+    try:
+        return torch.empty(most, dtype=torch.uint8, device=device)
+    except torch.OutOfMemoryError:
+        n = least()
+        if n >= most:
+            raise
+    return torch.empty(n, dtype=torch.uint8, device=device) if n else None
 
 
 def tensor_numel(batch, heads, seq, head_dim):
@@ -120,7 +123,7 @@ def attention_step_ex(q, k, v, out, m, l, shape, qmap, kmap, pos_stride=1, causa
     # (below 2048 keys it has little or nothing to gain, and the question costs a short call a microsecond)
     need = 0 if s.seq_k < 2048 else lib().ra_attention_step_workspace_bytes(
         dt, C.byref(s), C.byref(qmap), C.byref(kmap), pos_stride, flags, doc_len)
-    ws = _workspace(need, 0)
+    ws = _workspace(need)
     check(lib().ra_attention_step_ws(dt, _ptr(q), _ptr(k), _ptr(v), _ptr(out), _ptr(m), _ptr(l), C.byref(s),
                                      C.byref(qmap), C.byref(kmap), pos_stride, flags, doc_len, kv_row_stride,
                                      _ptr(ws), need if ws is not None else 0, _stream()))
@@ -185,7 +188,7 @@ def launch_int8_to_float(src, dst):
 def _flash(q, k, v, out, shape, causal, half):
     s = shape.c()
     ws = _workspace(lib().ra_flash_workspace_bytes(C.byref(s), int(half)),
-                    lib().ra_flash_workspace_least_bytes(C.byref(s), int(half)), q.device)
+                    lambda: lib().ra_flash_workspace_least_bytes(C.byref(s), int(half)), q.device)
     check(lib().ra_flash_attention(_ptr(q), _ptr(k), _ptr(v), _ptr(out), C.byref(s), int(causal),
                                    int(half), _ptr(ws), ws.numel(), _stream()))
 

@@ -149,7 +149,7 @@ def test_calls_run_without_the_split_where_there_is_no_room_for_it():
     try:
         assert both() == [0, 0]
         with pytest.raises(torch.OutOfMemoryError):  # not even what the call cannot do without
-            api._workspace(1 << 30, 1 << 29)
+            api._workspace(1 << 30, lambda: 1 << 29)
     finally:
         torch.cuda.set_per_process_memory_fraction(1.0)
     assert all(torch.equal(a, b) for a, b in zip((*state, flash), want))
