@@ -163,6 +163,7 @@ RA_API int ra_attention_step_ex(int dtype, const void* q, const void* k, const v
  * terms once, by a launch ahead, instead of by every block (the results are the same bits). `workspace`: 128-byte aligned,
  * only read and written by this call's launches on `stream`, at least ra_attention_step_workspace_bytes(...) bytes (0: the
  * call does not use one). A smaller one, or NULL, is not an error: it is not used. */
+#define RA_STEP_SPREAD_KEYS 2048 /* 16-bit calls on fewer keys never have a use for one */
 RA_API size_t ra_attention_step_workspace_bytes(int dtype, const ra_shape* shape, const ra_segmap* qmap,
                                                 const ra_segmap* kmap, int pos_stride, unsigned flags,
                                                 long long doc_len);

@@ -16,6 +16,7 @@ RA_STEP_CAUSAL, RA_STEP_FRESH, RA_STEP_FINALIZE, RA_STEP_FORCE_SIMT = 1, 2, 4, 8
 RA_STEP_P_IN_SMEM = 16
 RA_STEP_CTA_PAIR = 32
 RA_STEP_KEY_SPLIT_SHIFT = 8
+RA_STEP_SPREAD_KEYS = 2048
 RA_MAX_SEG = 16
 
 STATUS_NAMES = {0: "RA_OK", 1: "RA_ERR_INVALID", 2: "RA_ERR_CUDA", 3: "RA_ERR_UNSUPPORTED",

@@ -120,8 +120,8 @@ def attention_step_ex(q, k, v, out, m, l, shape, qmap, kmap, pos_stride=1, causa
              (_lib.RA_STEP_P_IN_SMEM if p_in_smem else 0) |
              (_lib.RA_STEP_CTA_PAIR if cta_pair else 0) | key_split << _lib.RA_STEP_KEY_SPLIT_SHIFT)
     dt, s = _dtype(q), shape.c()
-    # (below 2048 keys it has little or nothing to gain, and the question costs a short call a microsecond)
-    need = 0 if s.seq_k < 2048 else lib().ra_attention_step_workspace_bytes(
+    # (on fewer keys a 16-bit call has no use for a workspace and an fp32 call little, and the question costs a microsecond)
+    need = 0 if s.seq_k < _lib.RA_STEP_SPREAD_KEYS else lib().ra_attention_step_workspace_bytes(
         dt, C.byref(s), C.byref(qmap), C.byref(kmap), pos_stride, flags, doc_len)
     ws = _workspace(need)
     check(lib().ra_attention_step_ws(dt, _ptr(q), _ptr(k), _ptr(v), _ptr(out), _ptr(m), _ptr(l), C.byref(s),

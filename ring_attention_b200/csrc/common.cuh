@@ -90,6 +90,8 @@ int read_device_status(int out[4], bool clear);
 // set, so every later step leaves its state as it is, until ra_device_status reads and clears it).
 int enqueue_status_read(cudaStream_t stream);
 int status_after_sync();
+// SMs of the current device (without one: a B200's 148).
+int sm_count();
 // Scratch for the (m, l) of the local decode op, per device, grown on demand.
 int decode_ml_scratch(size_t floats, float** out);
 

@@ -1178,13 +1178,6 @@ __global__ void __launch_bounds__(kFoldThreads)
   }
 }
 
-int sm_count() {
-  int dev = 0, v = 148;
-  if (cudaGetDevice(&dev) == cudaSuccess)
-    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
-  return v > 0 ? v : 148;
-}
-
 struct DecodePlan {
   int cluster;  // > 0: the cluster form with this many blocks per group
   int ctas;     // balanced form: blocks

@@ -68,6 +68,13 @@ int status_after_sync() {
   return RA_OK;
 }
 
+int sm_count() {
+  int dev = 0, v = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    cudaGetLastError();
+  return v > 0 ? v : 148;
+}
+
 int read_device_status(int out[4], bool clear) {
   int* p = device_status_ptr();
   RAB_REQUIRE(p != nullptr, RA_ERR_CUDA, "device status word unavailable");

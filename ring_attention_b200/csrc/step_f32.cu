@@ -1249,9 +1249,9 @@ bool split_ahead(const StepArgs& a) {
         steps += r.hi - r.lo;
       }
     }
-  constexpr double kSms = 148, kSaves = DR == 128 ? 0.35 : 0.3, kLaunch = 5, kBytesPerUs = 5e6;
+  constexpr double kSaves = DR == 128 ? 0.35 : 0.3, kLaunch = 5, kBytesPerUs = 5e6;
   const double bytes = 16.0 * a.B * a.kvH * split_tiles(a) * kBNf * DR;  // read and written
-  return kSaves * a.B * a.H * steps / kSms > kLaunch + bytes / kBytesPerUs;
+  return kSaves * a.B * a.H * steps / sm_count() > kLaunch + bytes / kBytesPerUs;
 }
 template <int DR, bool kSplit, bool kPre>
 int launch_f32(const StepArgs& a, cudaStream_t stream, int key_split) {

@@ -426,7 +426,7 @@ int launch_typed(const StepArgs& a, cudaStream_t stream) {
   // fewer blocks leave SMs empty, and under a causal mask the first to go have half the work: H4 1000 dense (64)
   // 273 / 313, H2 2700 causal (86) 740 / 808, H4 2500 causal (160) 852 / 751.
   const long long blocks4 = (a.Sq + SimtCfg<256, 4>::kRows - 1ll) / SimtCfg<256, 4>::kRows * a.H * a.B;
-  const bool four = sizeof(T) == 4 && blocks4 * ((a.flags & RA_STEP_CAUSAL) ? 1 : 2) >= 148;
+  const bool four = sizeof(T) == 4 && blocks4 * ((a.flags & RA_STEP_CAUSAL) ? 1 : 2) >= sm_count();
   switch (a.D) {
     RAB_SIMT_CASE(32, 2)
     RAB_SIMT_CASE(64, 2)

@@ -992,7 +992,7 @@ inline bool fold_rows(const StepArgs& a, double alone, double tiles) {
 // rows on 8336 keys H16/kvH8 D64 39 / 34. Over 104 random calls (16 to 2048 rows on 1000 to 40000 keys more) that gain by
 // more than 5 % in the estimate 0.69 in the mean, 1.05 at worst (19.7 / 20.7, a call that the four tiles now keep out);
 // over 41 of 16 to 128 rows, with heads that share tiles, 0.47 and 0.77.
-constexpr int kSpreadKeys = 2048;
+constexpr int kSpreadKeys = RA_STEP_SPREAD_KEYS;
 template <int kTileKeys>
 inline bool plan_spread(const StepArgs& a, int tiles_per_block, double fold_tiles, int sms, double best_other, Spread* out) {
   if (a.Sk < kSpreadKeys || best_other <= 0 || a.H % a.kvH != 0) return false;

@@ -34,6 +34,12 @@ def test_every_declared_symbol_is_bound_in_python():
     assert set(declared_symbols()) <= set(_lib._SIG)
 
 
+def test_step_constants_are_those_of_the_header():
+    text = open(os.path.join(ROOT, "include", "ring_attention_b200.h")).read()
+    found = {n: int(v) for n, v in re.findall(r"#define (RA_STEP_\w+) (\d+)u?\b", text)}
+    assert len(found) >= 8 and found == {n: getattr(_lib, n) for n in found}
+
+
 def test_version_and_error_text():
     assert lib().ra_version() == 100
     # invalid arguments are rejected before any CUDA call
