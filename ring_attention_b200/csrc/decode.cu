@@ -1187,9 +1187,10 @@ struct DecodePlan {
 // What a kernel needs for a ring stage, in us: `alone` for one block on an SM, `share` of the SM's issue slots
 // (k blocks on an SM take k times that if it is longer). Slopes of calls with few groups, one block each,
 // between 6000 and 20000 rows: the mma kernel 0.53, 0.71 and 1.14 at head_dim 64, 128 (64 keys) and 256 (32);
-// the SIMT kernel 0.34-0.49 for 16 KB with one head. (The kernel for four and eight heads needs
-// 0.38-0.48 and 0.49-0.64 now; the estimate still says what its predecessor took, so that no call takes the other form for it:
-// a fold at 8.2 with these stages would send calls that fold well to clusters, 7.8 -> 10.8 us at worst.)
+// the SIMT kernel 0.34-0.49 for 16 KB with one head, 0.47-0.77 with four and 0.75-1.1 with eight. (The kernel that four and eight
+// heads have now needs 0.38-0.48 and 0.49-0.64. Its stages count as its predecessor's because they stand against kFold,
+// which is as much too high: a fold at 8.2 with the lower stages sends calls that fold well to clusters, 7.8 -> 10.8 us at
+// worst. The two have to change together, see make_plan.)
 struct StageCost {
   double alone, share;
 };
@@ -1204,11 +1205,11 @@ constexpr StageCost simt_stage_cost(int heads, size_t stage_bytes) {
 // memory (7 TB/s) allows, plus what the fold (a launch, and more the more rows it has) or the merge
 // (columns of the group, blocks of the cluster, and a wave of clusters starts slower than one of blocks)
 // adds. Constants fitted to 457 shapes (heads 8/8 to 64/1, batch 1 to 64, 200 to 100000 rows, fp16 and fp32,
-// every head_dim) timed in each form: this choice is 1.0 % from the best form on average, the estimate
-// before it (0.1 MB/us for any block, a fold of 3 us) 5.6 %, and up to twofold with few or very many groups.
-// Since launches overlap, a fold costs about 4: over 1700 calls the choice was 2.3 % from the best form, with kFold = 4 it would
-// be 0.7 %. It stays all the same: a fold goes through the library's partials, which calls on several streams must not
-// share, and calls that merge in clusters have none.
+// every head_dim) timed in each form when a fold was a launch of its own. Launches overlap now and a fold costs about 4:
+// over 1700 calls the choice is 2.3 % from the best form on average (single calls of 3 to 100 MB by up to a third), with
+// kFold = 4 it would be 0.7 %. kFold stays at 8.2 because the form also decides what a call without a workspace touches:
+// a fold goes through the library's one buffer for partials, a merge in clusters through nothing that calls share, and a lower
+// kFold moves calls of the second kind to the first.
 DecodePlan make_plan(int groups, int stages, size_t stage_bytes, int per_sm, int cap, int ring_max,
                      StageCost cost, size_t rows, int head_rows, int D, bool partials, int long_share) {
   constexpr double kBytesPerUs = 7e6, kFold = 8.2, kFoldRow = 0.005, kMerge = 0.6, kMergeBlock = 0.15,

@@ -1130,7 +1130,8 @@ __global__ void __launch_bounds__((F32Cfg<DR, kSplit, kPre>::kThreads), 1)
 }
 
 // Splits K and V once for all query blocks of a call: a block per key tile and KV head writes, to the workspace, what the
-// splitter warps leave in a ring slot, byte for byte, and the tile's meta data. The step then copies whole slots, and has
+// splitter warps leave in a ring slot, byte for byte, and the tile's meta data. (At head_dim 32 a slot has room for 64 columns:
+// the other half is not written, and nothing reads what the step copies of it.) The step then copies whole slots, and has
 // neither splitter warps (two thirds of its issue slots at head_dim 64) nor their traffic in shared memory. Bound by
 // memory: H4 S16384 D128, 67 MB read and as many written, 27 us.
 template <int DR>
