@@ -99,6 +99,34 @@ def test_long_group_decode_adds_no_longer_chains(dtype, B, H, kvH, Sk, blocks, a
     assert ((out - want).norm() / want.norm()).item() <= 2.0 ** -24 * (4.5 + 0.2 * chain ** 0.5)
 
 
+@pytest.mark.parametrize("dtype,D", [(torch.float32, 32), (torch.float32, 64), (torch.float32, 128), (torch.float32, 256), (torch.float16, 32)])
+@pytest.mark.parametrize("H,kvH,Sk", [(4, 1, 37), (9, 2, 700), (16, 2, 20000)])
+def test_group_decode_is_finite_where_single_heads_are(dtype, D, H, kvH, Sk):
+    """Heads that share a butterfly and the weights of a step do not share what is not finite: as with a KV head for each head."""
+    g = torch.Generator(device="cuda").manual_seed(Sk)
+    q, k, v = (torch.randn(1, h, n, D, generator=g, device="cuda").to(dtype) for h, n in ((H, 1), (kvH, Sk), (kvH, Sk)))
+    q[:, 0] = float("nan")
+    q[:, H - 1, :, 1] = float("inf")
+    q[..., 0].abs_()
+    k[:, kvH - 1, Sk // 2, 0] = float("inf")
+    v[:, 0, Sk // 3, 3] = float("inf")
+    v[:, kvH - 1, Sk - 1, D - 1] = float("nan")
+    outs = []
+    for n in (kvH, H):
+        kk, vv = (t.repeat(1, (H + kvH - 1) // kvH, 1, 1)[:, :H].contiguous() if n == H else t for t in (k, v))
+        out, m, l = torch.empty(1, H, 1, D, device="cuda"), torch.empty(1, H, 1, device="cuda"), torch.empty(1, H, 1, device="cuda")
+        shape = api.AttentionShape(1, H, 1, Sk, D, n)
+        api.launch_attention_init(out, m, l, shape)
+        api.launch_attention_decode_step(q, kk, vv, out, m, l, shape, 0, 0, False)
+        api.launch_attention_finalize(out, l, shape)
+        outs.append(out)
+    finite = outs[1].isfinite()
+    assert torch.equal(outs[0].isfinite(), finite) and not finite.all() and (finite.any() or kvH == 1)
+    # (at most Sk additions of 2^-24 in either, and a few for scores and exponentials)
+    if finite.any():
+        assert (outs[0] - outs[1])[finite].abs().max().item() <= 2 * (Sk / 32 + 64) * 2.0 ** -24 * v[v.isfinite()].abs().max().item()
+
+
 CAPTURES = """
 import torch
 from ring_attention_b200 import api

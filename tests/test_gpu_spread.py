@@ -136,6 +136,56 @@ def test_random_spread_calls_match_the_key_split():
     assert taken >= 20 and api.device_status()[0] == 0
 
 
+def spoil(what, q, k, v):
+    last = k.shape[2] - 1 - q.shape[2]  # every row sees the keys up to here
+    if what == "scores":
+        k[:, :, 777, 1] = float("nan")       # NaN in every row
+    elif what == "scores, some heads":
+        k[:, 0, 5, 2] = float("inf")         # +inf or -inf by the sign of q
+        k[:, 0, last, 0] = float("nan")
+    elif what == "values":
+        v[:, :, 100, 3] = float("inf")
+        v[:, :, last - 70, 0] = float("nan")
+        v[:, :, 4000, 5], v[:, :, 4001, 5] = float("inf"), -float("inf")
+    elif what == "queries":
+        q[:, 1, 0] = float("nan")
+        q[:, -1, -1, 3] = float("inf")
+        q[:, 0, q.shape[2] // 2] = -float("inf")
+    elif what == "hidden key":
+        k[:, :, 300] = -float("inf")         # a score of -inf in every row, and nothing else
+        q.abs_()
+        q[q == 0] = 1
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("D", [32, 64, 128, 256])
+@pytest.mark.parametrize("H,kvH,rows", [(4, 2, 200), (6, 2, 24), (7, 1, 50), (5, 1, 1)])  # rows of a head, heads that share tiles
+@pytest.mark.parametrize("what", ["plain", "scores", "scores, some heads", "values", "queries", "hidden key"])
+def test_what_is_not_finite_stays_where_it_belongs(dtype, D, H, kvH, rows, what):
+    """Beside the key split, which rounds the same P: the same elements are finite, and they agree. Rows that only fill a tile hold
+    what shared memory held, here NaN."""
+    keys = 20000 + rows
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    q, k, v = (torch.randn(1, h, n, D, generator=g, device="cuda").to(dtype) for h, n in ((H, rows), (kvH, keys), (kvH, keys)))
+    nan = torch.full((1, 160, 256, D), float("nan"), device="cuda", dtype=dtype)
+    junk = [torch.empty(s, device="cuda") for s in (nan.shape, nan.shape[:3], nan.shape[:3])]
+    spoil(what, q, k, v)
+    shape, qmap, kmap = api.AttentionShape(1, H, rows, keys, D, kvH), SegMap.make([keys - rows], rows), SegMap.make([0], keys)
+    need = lib().ra_attention_step_workspace_bytes(RA_F16, C.byref(shape.c()), C.byref(qmap), C.byref(kmap), 1, CAUSAL | FRESH | FINALIZE, 0)
+    ws = torch.full((need,), 0xff, dtype=torch.uint8, device="cuda")
+    a, b = ([torch.full(s, 7.0, device="cuda") for s in (q.shape, q.shape[:3], q.shape[:3])] for _ in range(2))
+    assert not call("ex", q, k, v, a, shape, qmap, kmap, 1, CAUSAL | FRESH | FINALIZE, 0) & SPREAD
+    call("ex", nan, nan, nan, junk, api.AttentionShape(1, 160, 256, 256, D, 160), SegMap.make([0], 256), SegMap.make([0], 256), 1, FRESH, 0)
+    assert call("ws", q, k, v, b, shape, qmap, kmap, 1, CAUSAL | FRESH | FINALIZE, 0, ws.data_ptr(), need) & SPREAD
+    for x, y in zip(a, b):
+        assert torch.equal(x.isfinite(), y.isfinite())
+    finite = a[0].isfinite()
+    assert finite.all() == (what in ("plain", "hidden key"))
+    assert finite.any() == (what != "scores" and (what != "scores, some heads" or kvH > 1))
+    assert_close(b[0][finite].cpu().numpy(), a[0][finite].cpu().numpy(), TOL[dtype], TOL[dtype], what)
+    assert api.device_status()[0] == 0
+
+
 @pytest.mark.parametrize("D", [64, 256])
 def test_other_forms_run_without_a_usable_workspace(D):
     B, H, kvH, rows, keys = 1, 4, 2, 200, 20000
