@@ -1226,7 +1226,9 @@ DecodePlan make_plan(int groups, int stages, size_t stage_bytes, int per_sm, int
   // no more partials than the workspace holds: a group meets at most ceil(ctas / groups) + 1 blocks,
   // exactly one each when there are as many blocks as groups
   long long ctas = std::min<long long>(slots, static_cast<long long>(total));
-  if (long_share > 0 && total > static_cast<double>(long_share) * slots) ctas *= 2;
+  // (with few groups a row's partials are what limits the blocks, down to a second wave that is a quarter full: B3 H8/kvH1
+  // D256, 60000 rows 69 -> 83 us; below that there is nothing to cut)
+  if (long_share > 0 && total > static_cast<double>(long_share) * slots && (cap - 1.0) * groups > 1.2 * slots) ctas *= 2;
   ctas = cap > 1 ? std::min(ctas, (cap - 1ll) * groups) : groups;
   p.cluster = 0;
   p.ctas = static_cast<int>(ctas);
@@ -1489,11 +1491,12 @@ int launch_decode_typed(const void* q, const void* k, const void* v, float* out,
       // 699 us with two, 731 with three). 16-bit rows of 32: as many as their registers allow (two; with four heads kept
       // to 80 registers three fit, 22 % faster to 22 % slower by shape and even in the mean)
       static const int per_sm = std::min(resident_blocks(balanced, kBlockThreads, kSmem), GB >= 4 && sizeof(T) == 4 ? 2 : 16);
-      // Eight heads, 16-bit rows of 32: a lane adds 1/64 of a block's rows one after another, so blocks with more than 24
-      // stages (3072 rows) are cut in two. Error against 64 bits of B5 H64/kvH8, 150000 rows: 3.9e-7 uncut, 3.2e-7 so, 3.5e-7 in the
-      // kernel with a butterfly for each head, which had two thirds of the rows a block; below that length there is no difference. It
-      // costs such calls 2 to 15 % (fp16 B1 H64/kvH8, 175724 rows 72 -> 77 us).
-      constexpr int kLongShare = GB == 8 && sizeof(T) == 2 ? 24 : 0;
+      // Eight heads with rows of 32 in 16 bits or of 256: two blocks an SM are two thirds of the blocks that the kernel with a butterfly
+      // for each head had, so a lane adds up half as many rows again, one after another. Blocks with more than 24 stages are
+      // cut in two. Error against 64 bits in that kernel / uncut / so: fp16 D32 B5 H64/kvH8, 150000 rows 3.5e-7 / 3.9e-7 / 3.2e-7; fp32
+      // D256 B3 H64/kvH8, 20000 rows 2.9e-7 / 3.2e-7 / 2.7e-7; with shorter shares they differ by 2 % at most. It costs such calls 2 to
+      // 20 % (fp16 D32 B1 H64/kvH8, 175724 rows 72 -> 77 us, fp32 D256 B3 H64/kvH8, 20000 rows 160 -> 163, 5000 rows 50 -> 54).
+      constexpr int kLongShare = GB == 8 && (sizeof(T) == 2 || D == 256) ? 24 : 0;
       return run_plan<D, GB>(
           s, head_batches, stages, 2 * C::kStageBytes, kStages, per_sm, simt_stage_cost(GB, 2 * C::kStageBytes), kLongShare, kRed,
           fixed_splits(s.batch * kvH * head_batches, sk_eff, Plan::kRowsPerStage, split_cap),

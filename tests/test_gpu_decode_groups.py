@@ -74,15 +74,16 @@ def test_group_decode_first_called_while_captured():
     assert np.abs(out.cpu().numpy() - want).max() <= tol
 
 
-@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
-@pytest.mark.parametrize("B,H,kvH,Sk,blocks,added", [
-    (2, 64, 16, 262144, 296, 4),   # four heads a block: the rows of a step (4 a lane) are added up first
-    (4, 64, 8, 200000, 592, 2)])   # eight heads (2 a lane), and long shares are cut in two
-def test_long_group_decode_adds_no_longer_chains(dtype, B, H, kvH, Sk, blocks, added):
-    """The error of long calls is that of chains of additions: a lane group (32 a block) has k = rows / blocks / 32 / added of them
-    on each accumulator. Sums of terms of either sign walk like sqrt(i), and so do their roundings (0.3 to 0.5 units of 2^-24,
-    relative): about 0.2 sqrt(k) units, beside 3 to 4 of the scores and exponentials. Twice the chain is outside."""
-    D = 32
+@pytest.mark.parametrize("dtype,B,H,kvH,Sk,D,blocks,lanes", [
+    (torch.float16, 2, 64, 16, 262144, 32, 296, 128),   # four heads a block: 32 lane groups, each adds 4 rows of a step up first
+    (torch.bfloat16, 2, 64, 16, 262144, 32, 296, 128),
+    (torch.float16, 4, 64, 8, 200000, 32, 592, 64),     # eight heads: 2 rows, and long shares are cut in two
+    (torch.bfloat16, 4, 64, 8, 200000, 32, 592, 64),
+    (torch.float32, 3, 64, 8, 100000, 256, 592, 8)])    # 4 lane groups, 2 rows, cut in two
+def test_long_group_decode_adds_no_longer_chains(dtype, B, H, kvH, Sk, D, blocks, lanes):
+    """The error of long calls is that of chains of additions: an accumulator has k = rows / blocks / lanes of them. Sums of terms
+    of either sign walk like sqrt(i), and so do their roundings (0.3 to 0.5 units of 2^-24, relative): about 0.2 sqrt(k) units,
+    beside 3 to 4 of the scores and exponentials. Twice the chain is outside."""
     g = torch.Generator(device="cuda").manual_seed(11)
     q, k, v = (torch.randn(B, h, n, D, generator=g, device="cuda").to(dtype) for h, n in ((H, 1), (kvH, Sk), (kvH, Sk)))
     want = torch.empty(B, H, 1, D, dtype=torch.double, device="cuda")
@@ -95,7 +96,7 @@ def test_long_group_decode_adds_no_longer_chains(dtype, B, H, kvH, Sk, blocks, a
     api.launch_attention_init(out, m, l, shape)
     api.launch_attention_decode_step(q, k, v, out, m, l, shape, 0, 0, False)
     api.launch_attention_finalize(out, l, shape)
-    chain = B * kvH * Sk / blocks / 32 / added
+    chain = B * kvH * Sk / blocks / lanes
     assert ((out - want).norm() / want.norm()).item() <= 2.0 ** -24 * (4.5 + 0.2 * chain ** 0.5)
 
 
